@@ -80,7 +80,7 @@ int masks_update(mgx_ctx*, mgx_masks*, const double*, const double*, cudaStream_
 int masks_expand(const mgx_masks*, int, void*, int*, cudaStream_t);
 int gram_cuda_cores(mgx_ctx*, int, const void*, const void*, size_t, size_t,
     int, double, int, double*, cudaStream_t);
-int psi_theta_cuda_cores(int, const void*, size_t, size_t, int, const double*, int, int,
+int psi_theta_cuda_cores(mgx_ctx*, int, const void*, size_t, size_t, int, const double*, int, int,
     double, const void*, void*, cudaStream_t);
 int psi_theta_tcgen05(mgx_ctx*, int, const float*, size_t, size_t, int,
     const double*, int, int, float, const float*, float*, cudaStream_t, double* rho = nullptr);
@@ -872,7 +872,7 @@ static int mult_matrix(mgx_ctx* ctx, int mode, mgx_dtype dtype, const void* psi,
     {
         case MGX_GEMM_FP64:
             // FP64 accumulation for either orbital type, as MPgemmNN does
-            return psi_theta_cuda_cores(dtype == MGX_F64 ? 0 : 1, psi, ldv, npts, nfunc,
+            return psi_theta_cuda_cores(ctx, dtype == MGX_F64 ? 0 : 1, psi, ldv, npts, nfunc,
                 theta, nfunc, ncols, beta, cin, out, s);
         case MGX_GEMM_FP32:
         case MGX_GEMM_TF32:
@@ -881,7 +881,7 @@ static int mult_matrix(mgx_ctx* ctx, int mode, mgx_dtype dtype, const void* psi,
             if (dtype != MGX_F32)
                 return fail(MGX_BAD_ARG, "gemm mode %d needs FP32 orbitals", mode);
             if (mode == MGX_GEMM_FP32)
-                return psi_theta_cuda_cores(2, psi, ldv, npts, nfunc, theta, nfunc, ncols, beta,
+                return psi_theta_cuda_cores(ctx, 2, psi, ldv, npts, nfunc, theta, nfunc, ncols, beta,
                     cin, out, s);
             return psi_theta_tcgen05(ctx, mode, (const float*)psi, ldv, npts, nfunc, theta,
                 nfunc, ncols, (float)beta, (const float*)cin, (float*)out, s);

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "mgx_internal.cuh"
+#include "mgx_slice.cuh"
 #include "mgx_stencil.cuh"
 
 namespace mgx
@@ -49,15 +50,29 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e)
     e              = (a - (s - bb)) + (b - bb);
 }
 
+/* tiles of a launch: column tile by column tile; with lower only those that
+ * reach an entry i >= j + col0 */
+__host__ __device__ inline int gram_first_row(int j, int lower, int col0, int nti)
+{
+    const int f = lower ? col0 / GT + j : 0;
+    return f < nti ? f : nti;
+}
+
+/* only_if: nothing is done unless *only_if is set (the FP64 products that the
+ * tensor cores took over run here when an operand is not finite) */
 template <typename T>
 __global__ void __launch_bounds__(256) gram_splitk_kernel(const T* __restrict__ A,
     const T* __restrict__ B, size_t ld, int n, int ncols, size_t K, size_t kslice,
-    const int2* __restrict__ tiles, double* __restrict__ C)
+    int lower, int col0, const int* __restrict__ only_if, double* __restrict__ C)
 {
     __shared__ T As[GKC][GT + 1];
     __shared__ T Bs[GKC][GT + 1];
-    const int2 tile = tiles[blockIdx.x];
-    const int i0 = tile.x * GT, j0 = tile.y * GT;
+    if (only_if && *only_if == 0) return;
+    const int nti = (n + GT - 1) / GT;
+    int ti = blockIdx.x, tj = 0;
+    for (int f; (f = gram_first_row(tj, lower, col0, nti), ti >= nti - f); tj++)
+        ti -= nti - f;
+    const int i0 = (gram_first_row(tj, lower, col0, nti) + ti) * GT, j0 = tj * GT;
     const size_t k0 = (size_t)blockIdx.y * kslice;
     const size_t k1 = min(K, k0 + kslice);
     const int tid   = threadIdx.x;
@@ -177,37 +192,50 @@ __global__ void gram_finish_kernel(double* C, int n, double vel, int symmetric)
     }
 }
 
+/* C += A B^T of n x ncols functions of K points (with lower, at least the
+ * entries i >= j + col0).  FP64 products of some size are formed from slices
+ * on the tensor cores; the CUDA-core kernel behind them runs only when an
+ * operand is not finite. */
+static int gram_add(mgx_ctx* ctx, int dtype, const void* A, const void* B, size_t ld, size_t K,
+    int n, int ncols, int lower, int col0, double* C, cudaStream_t s)
+{
+    int* only_if = nullptr;
+    if (dtype == MGX_F64 && sl::pays(n, ncols, K))
+    {
+        const int st = sl::accumulate(ctx, (const double*)A, (const double*)B, ld, K, n, ncols,
+            lower, col0, C, &only_if, s);
+        if (st == MGX_NO_MEMORY)
+            only_if = nullptr; // no room for the planes: the CUDA cores do it
+        else if (st != MGX_OK)
+            return st;
+    }
+    const int nti = (n + GT - 1) / GT, ntj = (ncols + GT - 1) / GT;
+    int ntiles    = 0;
+    for (int j = 0; j < ntj; j++)
+        ntiles += nti - gram_first_row(j, lower, col0, nti);
+    int ksplit    = std::max(1, (8 * ctx->sm_count + ntiles - 1) / ntiles);
+    size_t kslice = (K + ksplit - 1) / ksplit;
+    kslice        = ((kslice + GKC - 1) / GKC) * GKC;
+    ksplit        = (int)((K + kslice - 1) / kslice);
+    if (ksplit > 65535) return fail(MGX_UNSUPPORTED, "K too large for split");
+    dim3 grid(ntiles, ksplit);
+    if (dtype == MGX_F64)
+        gram_splitk_kernel<double><<<grid, 256, 0, s>>>((const double*)A, (const double*)B, ld, n,
+            ncols, K, kslice, lower, col0, only_if, C);
+    else
+        gram_splitk_kernel<float><<<grid, 256, 0, s>>>((const float*)A, (const float*)B, ld, n,
+            ncols, K, kslice, lower, col0, only_if, C);
+    MGX_LAUNCH_CHECK("gram_splitk_kernel");
+    return MGX_OK;
+}
+
 int gram_cuda_cores(mgx_ctx* ctx, int dtype, const void* A, const void* B,
     size_t ld, size_t K, int n, double vel, int symmetric, double* C,
     cudaStream_t s)
 {
-    const int nt = (n + GT - 1) / GT;
-    std::vector<int2> tiles;
-    for (int j = 0; j < nt; j++)
-        for (int i = 0; i < nt; i++)
-            if (!symmetric || i >= j) tiles.push_back(make_int2(i, j));
-    const int ntiles = (int)tiles.size();
-    int ksplit       = std::max(1, (8 * ctx->sm_count + ntiles - 1) / ntiles);
-    size_t kslice    = (K + ksplit - 1) / ksplit;
-    kslice           = ((kslice + GKC - 1) / GKC) * GKC;
-    ksplit           = (int)((K + kslice - 1) / kslice);
-    if (ksplit > 65535) return fail(MGX_UNSUPPORTED, "K too large for split");
-    MGX_TRY(ctx->gemm_ws.ensure(tiles.size() * sizeof(int2)));
-    MGX_TRY(cuda_check(cudaMemcpyAsync(ctx->gemm_ws.ptr, tiles.data(),
-                           tiles.size() * sizeof(int2), cudaMemcpyHostToDevice, s),
-        "gram tiles upload"));
     MGX_TRY(cuda_check(cudaMemsetAsync(C, 0, (size_t)n * n * sizeof(double), s),
         "gram zero"));
-    dim3 grid(ntiles, ksplit);
-    if (dtype == MGX_F64)
-        gram_splitk_kernel<double><<<grid, 256, 0, s>>>((const double*)A,
-            (const double*)B, ld, n, n, K, kslice, (const int2*)ctx->gemm_ws.ptr, C);
-    else
-        gram_splitk_kernel<float><<<grid, 256, 0, s>>>((const float*)A,
-            (const float*)B, ld, n, n, K, kslice, (const int2*)ctx->gemm_ws.ptr, C);
-    MGX_LAUNCH_CHECK("gram_splitk_kernel");
-    // the tile list must stay alive until the kernel has read it
-    MGX_TRY(cuda_check(cudaStreamSynchronize(s), "gram sync"));
+    MGX_TRY(gram_add(ctx, dtype, A, B, ld, K, n, n, symmetric, 0, C, s));
     const int nb = (int)std::min<size_t>(((size_t)n * n + 255) / 256, 4096);
     gram_finish_kernel<<<nb, 256, 0, s>>>(C, n, vel, symmetric);
     MGX_LAUNCH_CHECK("gram_finish_kernel");
@@ -224,48 +252,14 @@ int matb_cuda_cores(mgx_ctx* ctx, int dtype, const void* psi, size_t ld, size_t 
 {
     if (wf <= 0) return fail(MGX_BAD_ARG, "matB: empty work block");
     const size_t es = dtype_size(dtype);
-    const int nt    = (n + GT - 1) / GT;
-    std::vector<int2> tiles;
-    std::vector<size_t> first;
+    MGX_TRY(cuda_check(cudaMemsetAsync(C, 0, (size_t)n * n * sizeof(double), s), "matB zero"));
     for (int c0 = 0; c0 < n; c0 += wf)
     {
         const int nc = std::min(wf, n - c0);
-        first.push_back(tiles.size());
-        for (int j = 0; j < (nc + GT - 1) / GT; j++)
-            for (int i = 0; i < nt; i++)
-                if (i * GT + GT - 1 >= c0 + j * GT) tiles.push_back(make_int2(i, j));
-    }
-    first.push_back(tiles.size());
-    const int nchunks = (int)first.size() - 1;
-    const int avg     = std::max(1, (int)(tiles.size() / nchunks));
-    int ksplit        = std::max(1, (8 * ctx->sm_count + avg - 1) / avg);
-    size_t kslice     = (K + ksplit - 1) / ksplit;
-    kslice            = ((kslice + GKC - 1) / GKC) * GKC;
-    ksplit            = (int)((K + kslice - 1) / kslice);
-    if (ksplit > 65535) return fail(MGX_UNSUPPORTED, "K too large for split");
-    MGX_TRY(ctx->gemm_ws.ensure(tiles.size() * sizeof(int2)));
-    const int2* dt = (const int2*)ctx->gemm_ws.ptr;
-    MGX_TRY(cuda_check(cudaMemcpyAsync(ctx->gemm_ws.ptr, tiles.data(),
-                           tiles.size() * sizeof(int2), cudaMemcpyHostToDevice, s),
-        "matB tiles upload"));
-    MGX_TRY(cuda_check(cudaMemsetAsync(C, 0, (size_t)n * n * sizeof(double), s), "matB zero"));
-    for (int c = 0; c < nchunks; c++)
-    {
-        const int c0 = c * wf, nc = std::min(wf, n - c0);
-        const int nct = (int)(first[c + 1] - first[c]);
         MGX_TRY(rhs_block(ctx->grid, dtype, (const char*)psi + (size_t)c0 * ld * es, ld, work,
             ld, nc, s));
-        dim3 grid(nct, ksplit);
-        if (dtype == MGX_F64)
-            gram_splitk_kernel<double><<<grid, 256, 0, s>>>((const double*)psi,
-                (const double*)work, ld, n, nc, K, kslice, dt + first[c], C + (size_t)c0 * n);
-        else
-            gram_splitk_kernel<float><<<grid, 256, 0, s>>>((const float*)psi,
-                (const float*)work, ld, n, nc, K, kslice, dt + first[c], C + (size_t)c0 * n);
-        MGX_LAUNCH_CHECK("gram_splitk_kernel");
+        MGX_TRY(gram_add(ctx, dtype, psi, work, ld, K, n, nc, 1, c0, C + (size_t)c0 * n, s));
     }
-    // the tile list must stay alive until the kernels have read it
-    MGX_TRY(cuda_check(cudaStreamSynchronize(s), "matB sync"));
     const int nb = (int)std::min<size_t>(((size_t)n * n + 255) / 256, 4096);
     gram_finish_kernel<<<nb, 256, 0, s>>>(C, n, vel, 1);
     MGX_LAUNCH_CHECK("gram_finish_kernel");
@@ -367,10 +361,11 @@ static int dgemm(bool ta, bool tb, int m, int n, int k, double alpha,
 template <typename T, typename ACC>
 __global__ void __launch_bounds__(256) psi_theta_kernel(size_t npts, int n,
     const T* __restrict__ psi, size_t ld, const double* __restrict__ theta, int ldt,
-    int ncols, double beta, const T* cin, T* out)
+    int ncols, double beta, const T* cin, T* out, const int* __restrict__ only_if)
 {
     __shared__ ACC As[16][128];
     __shared__ ACC Bs[16][65];
+    if (only_if && *only_if == 0) return;
     const size_t p0 = (size_t)blockIdx.x * 128;
     const int j0 = blockIdx.y * 64;
     const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
@@ -434,26 +429,43 @@ __global__ void __launch_bounds__(256) psi_theta_kernel(size_t npts, int n,
     }
 }
 
-/* kind 0: FP64 orbitals; 1: FP32 orbitals, FP64 accumulation; 2: FP32
- * orbitals, FP32 accumulation */
-int psi_theta_cuda_cores(int kind, const void* psi, size_t ld, size_t npts, int n,
+/* kind 0: FP64 orbitals (from slices on the tensor cores where they pay, the
+ * CUDA-core kernel then only for operands that are not finite); 1: FP32
+ * orbitals, FP64 accumulation; 2: FP32 orbitals, FP32 accumulation */
+int psi_theta_cuda_cores(mgx_ctx* ctx, int kind, const void* psi, size_t ld, size_t npts, int n,
     const double* theta, int ldt, int ncols, double beta, const void* cin, void* out,
     cudaStream_t s)
 {
     if (n <= 0 || ncols <= 0 || npts == 0) return MGX_OK;
-    dim3 grid((unsigned)((npts + 127) / 128), (unsigned)((ncols + 63) / 64));
-    if (grid.y > 65535) return fail(MGX_UNSUPPORTED, "too many functions");
-    if (kind == 0)
-        psi_theta_kernel<double, double><<<grid, 256, 0, s>>>(npts, n, (const double*)psi, ld,
-            theta, ldt, ncols, beta, (const double*)cin, (double*)out);
-    else if (kind == 1)
-        psi_theta_kernel<float, double><<<grid, 256, 0, s>>>(npts, n, (const float*)psi, ld,
-            theta, ldt, ncols, beta, (const float*)cin, (float*)out);
-    else
-        psi_theta_kernel<float, float><<<grid, 256, 0, s>>>(npts, n, (const float*)psi, ld,
-            theta, ldt, ncols, beta, (const float*)cin, (float*)out);
-    MGX_LAUNCH_CHECK("psi_theta_kernel");
-    return MGX_OK;
+    const unsigned gy = (unsigned)((ncols + 63) / 64);
+    if (gy > 65535) return fail(MGX_UNSUPPORTED, "too many functions");
+    auto cores = [&](size_t p0, size_t np, const int* only_if) -> int {
+        const dim3 grid((unsigned)((np + 127) / 128), gy);
+        if (kind == 0)
+            psi_theta_kernel<double, double><<<grid, 256, 0, s>>>(np, n, (const double*)psi + p0,
+                ld, theta, ldt, ncols, beta, cin ? (const double*)cin + p0 : nullptr,
+                (double*)out + p0, only_if);
+        else if (kind == 1)
+            psi_theta_kernel<float, double><<<grid, 256, 0, s>>>(np, n, (const float*)psi + p0, ld,
+                theta, ldt, ncols, beta, cin ? (const float*)cin + p0 : nullptr, (float*)out + p0,
+                only_if);
+        else
+            psi_theta_kernel<float, float><<<grid, 256, 0, s>>>(np, n, (const float*)psi + p0, ld,
+                theta, ldt, ncols, beta, cin ? (const float*)cin + p0 : nullptr, (float*)out + p0,
+                only_if);
+        MGX_LAUNCH_CHECK("psi_theta_kernel");
+        return MGX_OK;
+    };
+    if (kind == 0 && sl::pays(npts, ncols, n))
+    {
+        const sl::View a = { (const double*)psi, ld, npts, (size_t)n, false };
+        const sl::View b = { theta, (size_t)ldt, (size_t)ncols, (size_t)n, true };
+        const sl::Target t
+            = { (double*)out, ld, nullptr, 1., beta, (const double*)cin, ld, 0, 0 };
+        const int st = sl::store(ctx, a, b, t, s, cores);
+        if (st != MGX_NO_MEMORY) return st;
+    }
+    return cores(0, npts, nullptr);
 }
 
 /* ProjectedMatrices::updateTheta (src/ProjectedMatrices.h:218-225):

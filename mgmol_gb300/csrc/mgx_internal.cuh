@@ -114,6 +114,8 @@ struct mgx_ctx
         void* lo   = nullptr;
     } conv;
     int reuse_conversion = 0;
+    // FP64 products from bf16 slices: row exponents and digit planes
+    mgx::DeviceBuffer slices;
     // residual: Psi Theta when the caller passes no work block
     mgx::DeviceBuffer resid;
     // Poisson multigrid levels

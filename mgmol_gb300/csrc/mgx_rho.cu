@@ -19,7 +19,7 @@
 
 namespace mgx
 {
-int psi_theta_cuda_cores(int, const void*, size_t, size_t, int, const double*, int, int,
+int psi_theta_cuda_cores(mgx_ctx*, int, const void*, size_t, size_t, int, const double*, int, int,
     double, const void*, void*, cudaStream_t);
 int psi_theta_tcgen05(mgx_ctx*, int, const float*, size_t, size_t, int, const double*, int,
     int, float, const float*, float*, cudaStream_t, double* rho);
@@ -132,7 +132,7 @@ int mgx_rho(mgx_ctx* ctx, int mode, mgx_dtype dtype, const void* psi, size_t ld,
             for (int j0 = 0; j0 < nfunc; j0 += wf)
             {
                 const int nc = std::min(wf, nfunc - j0);
-                MGX_TRY(psi_theta_cuda_cores(kind, psi, ldv, np, nfunc, dm + (size_t)j0 * nfunc,
+                MGX_TRY(psi_theta_cuda_cores(ctx, kind, psi, ldv, np, nfunc, dm + (size_t)j0 * nfunc,
                     nfunc, nc, 0., nullptr, work, s));
                 if (dtype == MGX_F64)
                     rho_chunk_kernel<double><<<nb, 256, 0, s>>>((const double*)work, ldv,

@@ -1,0 +1,814 @@
+// FP64 products C = A B^T on the tcgen05 tensor cores of sm_103a, from exact
+// slices of the operands (the scheme of Ozaki, Ogita, Oishi and Rump,
+// "Error-free transformations of matrix multiplication", 2012).
+//
+// GB300 runs two FP64 multiply-adds per SM and clock, 1.18 TFLOP/s, and
+// 1.87 PFLOP/s of bf16 on the tensor cores.  So a product of FP64 operands is
+// formed from bf16 products whose sums are exact:
+//   - every row r of an operand is scaled by 2^-e_r, |x| < 2^e_r, and written
+//     as a 56-bit fixed-point number of seven balanced base-256 digits,
+//     x 2^(7 - e_r) = d_0 + d_1 2^-8 + ... + d_6 2^-48, |d| <= 128, each digit
+//     (with its power of 256) one bf16 value;
+//   - digit s of A times digit t of B are integers of at most 2^14 at weight
+//     2^(-8 (s + t)).  The products of one s + t add up in an FP32 accumulator
+//     of their own, which rounds nothing while |sum| <= 2^24: after 192 values
+//     of K it is read and added to a 64-bit integer.  (All of s + t <= 4 are
+//     exact for any input; of the 6 or 7 x 192 products of s + t = 5 and 6, at
+//     2^-40 and 2^-48, the last bit could round if all digits were extreme.)
+//     The sums have to be exact and not only FP32: the tensor cores truncate
+//     when they add, which biases a sum of squares by 2^-24 per addition;
+//   - products of s + t > 6, 2^-56 of |row maximum| |column maximum| and less,
+//     are left out.
+// 28 bf16 products stand for one FP64 product, at 2^-56 of the row maxima
+// where FP64 multiply-adds round every partial sum at 2^-53.
+//
+// A NaN or an infinity in an operand has no digits: it raises a flag, on
+// which the kernels here do nothing and the caller's CUDA-core kernel,
+// launched behind them, does the work instead of returning at once.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+
+#include "mgx_slice.cuh"
+#include "mgx_tcgen05.cuh"
+
+namespace mgx
+{
+namespace sl
+{
+constexpr int NS      = 7;   // slices
+constexpr int BM      = 128; // rows of a tile (A)
+constexpr int BN      = 128; // most columns of a tile (B)
+constexpr int BN1     = 64;  // most columns with all NS accumulators in TMEM at once
+constexpr int BK      = 32;  // K values of a stage (64 bytes, SWIZZLE_64B)
+constexpr int STAGES  = 2;
+constexpr int DRAIN   = 6;   // stages between reads of the accumulators
+constexpr int A_SLICE = BM * BK * 2;
+constexpr int B_SLICE = BN * BK * 2;
+constexpr int STAGE   = NS * (A_SLICE + B_SLICE);
+constexpr int EPI     = 8;   // epilogue warps
+constexpr int SUM_W   = 47;  // sums over items are kept in units of 2^-SUM_W
+constexpr int THREADS = 32 * (2 + EPI);
+constexpr size_t SMEM = (size_t)STAGES * STAGE + (2 * STAGES + 1 + NS) * 8 + 16 + 1024;
+static_assert(SMEM <= 227 * 1024, "two stages of seven slices fit one SM");
+static_assert(NS * BN1 <= 512 && 4 * BN <= 512, "the accumulators of a pass fit TMEM");
+
+/* The key of a row: the upper half of the bits of max |x|.  Exponent e with
+ * |x| < 2^e for every x of the row. */
+__device__ __forceinline__ int key_exponent(int key) { return max(key >> 20, 1) - 1022; }
+
+constexpr int KEY_NONFINITE = 0x7ff00000;
+
+__device__ __forceinline__ int abs_hi(double x) { return __double2hiint(x) & 0x7fffffff; }
+
+/* row maxima, K contiguous: blockIdx.y = row (grid-stride), blockIdx.x = a
+ * part of K */
+__global__ void __launch_bounds__(256) keys_kmajor_kernel(const double* __restrict__ x, size_t ld,
+    size_t rows, size_t K, int* __restrict__ keys, int* __restrict__ bad)
+{
+    const size_t part = ((K + gridDim.x - 1) / gridDim.x + 255) & ~size_t(255);
+    const size_t k0 = blockIdx.x * part, k1 = min(K, k0 + part);
+    for (size_t r = blockIdx.y; r < rows; r += gridDim.y)
+    {
+        int m             = 0;
+        const double* row = x + r * ld;
+        size_t k          = k0 + threadIdx.x;
+        for (; k + 3 * 256 < k1; k += 4 * 256)
+        {
+            const double a = row[k], b = row[k + 256], c = row[k + 512], d = row[k + 768];
+            m = max(m, max(max(abs_hi(a), abs_hi(b)), max(abs_hi(c), abs_hi(d))));
+        }
+        for (; k < k1; k += 256)
+            m = max(m, abs_hi(row[k]));
+        m = __reduce_max_sync(0xffffffffu, m);
+        if ((threadIdx.x & 31) == 0 && m > 0)
+        {
+            atomicMax(keys + r, m);
+            if (m >= KEY_NONFINITE) *bad = 1;
+        }
+    }
+}
+
+/* row maxima, rows contiguous: a thread owns a row, blockIdx.y a part of K */
+__global__ void __launch_bounds__(128) keys_rmajor_kernel(const double* __restrict__ x, size_t ld,
+    size_t rows, size_t K, int* __restrict__ keys, int* __restrict__ bad)
+{
+    const size_t part = (K + gridDim.y - 1) / gridDim.y;
+    const size_t k0 = blockIdx.y * part, k1 = min(K, k0 + part);
+    for (size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows;
+         r += (size_t)gridDim.x * blockDim.x)
+    {
+        int m = 0;
+#pragma unroll 8
+        for (size_t k = k0; k < k1; k++)
+            m = max(m, abs_hi(x[k * ld + r]));
+        if (m > 0)
+        {
+            atomicMax(keys + r, m);
+            if (m >= KEY_NONFINITE) *bad = 1;
+        }
+    }
+}
+
+/* x 2^(55 - e) rounded to an integer (half away from zero), |x| < 2^e, in
+ * integer arithmetic: the FP64 units are the scarce ones here */
+__device__ __forceinline__ long long to_fixed(double x, int e)
+{
+    const long long b = __double_as_longlong(x);
+    const int ex      = (int)(b >> 52) & 0x7ff;
+    long long m       = b & 0xfffffffffffffll;
+    if (ex) m |= 0x10000000000000ll;
+    // |x| = m 2^(max(ex, 1) - 1075)
+    const int sh = min(e + 1020 - max(ex, 1), 62);
+    m            = sh <= 0 ? m << (-sh) : (m + (1ll << (sh - 1))) >> sh;
+    return b < 0 ? -m : m;
+}
+
+/* the NS digits of q, most significant first, each times 2^(-8 s), as the
+ * upper halves of FP32 values (exact in bf16) */
+__device__ __forceinline__ void digits(long long q, uint32_t (&f)[NS])
+{
+    // with 128 added at the place of every digit but the first, the bytes of
+    // q are the balanced digits plus 128
+    const long long b = q + 0x0000808080808080ll;
+    const uint32_t lo = (uint32_t)b, hi = (uint32_t)((unsigned long long)b >> 32);
+    f[0] = __float_as_uint((float)((int)hi >> 16));
+#pragma unroll
+    for (int s = 1; s < NS; s++)
+    {
+        const int by         = 6 - s; // byte of b
+        const uint32_t byte  = ((by >= 4 ? hi : lo) >> (8 * (by & 3))) & 0xffu;
+        const uint32_t magic = (uint32_t)(150 - 8 * s) << 23; // 2^(23 - 8 s)
+        // (2^(23 - 8 s) + byte 2^(-8 s)) - (2^(23 - 8 s) + 128 2^(-8 s))
+        f[s] = __float_as_uint(
+            __uint_as_float(magic | byte) - __uint_as_float(magic | 128u));
+    }
+}
+
+/* stores the digits of 8 consecutive K values: 16 bytes in each plane.  The
+ * planes are K-blocked: element (row, k) of slice s at
+ * ((s * kblocks + k / 64) * rows + row) * 64 + k % 64. */
+__device__ __forceinline__ void store8(const long long (&q)[8], __nv_bfloat16* planes, size_t rows,
+    size_t kblocks, size_t kb, size_t r, int g)
+{
+    uint32_t w[NS][4];
+#pragma unroll
+    for (int p = 0; p < 4; p++)
+    {
+        uint32_t a[NS], b[NS];
+        digits(q[2 * p], a);
+        digits(q[2 * p + 1], b);
+#pragma unroll
+        for (int s = 0; s < NS; s++)
+            w[s][p] = __byte_perm(a[s], b[s], 0x7632);
+    }
+#pragma unroll
+    for (int s = 0; s < NS; s++)
+        *reinterpret_cast<uint4*>(planes + ((s * kblocks + kb) * rows + r) * 64 + g)
+            = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+}
+
+/* planes of a K-contiguous operand, 8 values of K per thread; HBM bound (8
+ * bytes read, 14 written per value) */
+__global__ void __launch_bounds__(256) planes_kmajor_kernel(const double* __restrict__ x, size_t ld,
+    size_t rows, size_t K, const int* __restrict__ keys, size_t kblocks,
+    __nv_bfloat16* __restrict__ planes)
+{
+    const size_t total = rows * kblocks * 8;
+    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+         t += (size_t)gridDim.x * blockDim.x)
+    {
+        const int g     = 8 * (int)(t % 8);
+        const size_t rk = t / 8;
+        const size_t kb = rk % kblocks, r = rk / kblocks;
+        const size_t k  = kb * 64 + g;
+        const int e     = key_exponent(keys[r]);
+        const double* p = x + r * ld + k;
+        long long q[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            q[i] = (k + i < K) ? to_fixed(p[i], e) : 0;
+        store8(q, planes, rows, kblocks, kb, r, g);
+    }
+}
+
+/* planes of a row-contiguous operand: a block takes 64 rows x 64 values of K
+ * through shared memory (73 values between rows: conflict-free stores along
+ * rows, two-way reads of the values k = 8 q + g in the order that puts g
+ * next to each other) */
+constexpr int TP = 73;
+
+__global__ void __launch_bounds__(256) planes_rmajor_kernel(const double* __restrict__ x, size_t ld,
+    size_t rows, size_t K, const int* __restrict__ keys, size_t kblocks,
+    __nv_bfloat16* __restrict__ planes)
+{
+    __shared__ long long t[64 * TP];
+    const size_t r0 = (size_t)blockIdx.x * 64, kb = blockIdx.y;
+    const int rr    = threadIdx.x % 64;
+    const size_t r  = r0 + rr;
+    const int e     = r < rows ? key_exponent(keys[r]) : 0;
+#pragma unroll 4
+    for (int kk = threadIdx.x / 64; kk < 64; kk += 4)
+    {
+        const size_t k = kb * 64 + kk;
+        // value k = 8 a + b of the block at place 8 b + a
+        t[rr * TP + (kk % 8) * 8 + kk / 8]
+            = (r < rows && k < K) ? to_fixed(x[k * ld + r], e) : 0;
+    }
+    __syncthreads();
+    for (int it = threadIdx.x; it < 64 * 8; it += 256)
+    {
+        const int a = it % 8, row = it / 8;
+        if (r0 + row >= rows) continue;
+        long long q[8];
+#pragma unroll
+        for (int b = 0; b < 8; b++)
+            q[b] = t[row * TP + 8 * b + a];
+        store8(q, planes, rows, kblocks, kb, r0 + row, 8 * a);
+    }
+}
+
+struct Params
+{
+    int nti, ntj;    // tiles
+    int bn;          // columns of a tile, a multiple of 16
+    int ntiles;      // tiles formed (with lower: those that reach i >= j + col0)
+    int nst;         // stages of K
+    int st_per_item; // stages of one item
+    int nitems;
+    int kblocks;     // 64-value blocks of K in each plane
+    int w;           // the sums are integers in units of 2^-w of a digit product
+    size_t m, n;
+    const int* ka;
+    const int* kb;
+    Target t;
+    const int* bad;
+    int* err;
+};
+
+/* item w: its tile and stages.  The tiles of one K range sit side by side in
+ * the list, so that CTAs that run together read the same planes. */
+__device__ __forceinline__ void decode(const Params& p, int w, int& ti, int& tj, int& st0, int& nst)
+{
+    int tile = w % p.ntiles;
+    st0      = (w / p.ntiles) * p.st_per_item;
+    nst      = min(p.nst - st0, p.st_per_item);
+    if (!p.t.lower)
+    {
+        ti = tile % p.nti;
+        tj = tile / p.nti;
+        return;
+    }
+    for (tj = 0; tj < p.ntj; tj++)
+    {
+        const int first = min((p.t.col0 + tj * p.bn) / BM, p.nti); // first row tile that counts
+        if (tile < p.nti - first)
+        {
+            ti = first + tile;
+            return;
+        }
+        tile -= p.nti - first;
+    }
+    ti = 0; // not reached
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
+{
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                 "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void tmem_wait_ld()
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+/* T 2^E, exactly where the result is a normal number */
+__device__ __forceinline__ double scaled(long long T, int E)
+{
+    const double v = (double)T;
+    const int ex   = (__double2hiint(v) >> 20) & 0x7ff;
+    if (T != 0 && (unsigned)(ex + E - 1) < 2045u)
+        return __hiloint2double(__double2hiint(v) + (E << 20), __double2loint(v));
+    return T == 0 ? 0. : scalbn(v, E);
+}
+
+/* One CTA per SM walks the items.  Warp 0 streams the slices of both operands
+ * (two stages of up to 114 KB), warp 1 issues the MMAs, one accumulator per
+ * s + t, and warps 2 .. 9 add the accumulators into 64-bit integers in
+ * registers (64 per thread) and finish the tile.  A tile has 128 columns,
+ * for which TMEM holds four accumulators: K is walked twice, for s + t = 4 .. 6
+ * (18 products of 7 slices) and 0 .. 3 (10 products of 4).  An MMA of 128 x 128
+ * x 16 reads 8 KB of shared memory in 64 clocks, just what the SM delivers; one
+ * of 128 x 64 would wait for it, so narrow tiles, which take all of s + t in
+ * one walk (NP = 1), serve only products of at most 64 columns.  The accumulators
+ * are handed over one by one: those of the next 192 values start while the
+ * epilogue warps still empty the later ones. */
+template <int NP>
+__global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
+    const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, const Params p)
+{
+    using namespace tc;
+    if (*p.bad) return;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* full  = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE);
+    uint64_t* empty = full + STAGES;
+    uint64_t* accf  = empty + STAGES; // the MMAs up to a drain are done
+    uint64_t* acce  = accf + 1;       // [NS] the epilogue warps have read accumulator a
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + NS);
+    __shared__ volatile int abort_all;
+
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    // diagonals s + t of walk ps: [pass_lo, pass_hi), which read slices < pass_hi
+    auto pass_lo = [](int ps) { return NP == 1 || ps == 1 ? 0 : 4; };
+    auto pass_hi = [](int ps) { return NP == 1 || ps == 0 ? NS : 4; };
+    if (threadIdx.x == 0)
+    {
+        for (int s = 0; s < STAGES; s++)
+        {
+            mbar_init(full + s, 1);
+            mbar_init(empty + s, 1);
+        }
+        mbar_init(accf, 1);
+        for (int a = 0; a < NS; a++)
+            mbar_init(acce + a, EPI);
+        abort_all = 0;
+        fence_mbar_init();
+    }
+    if (warp == 1)
+    {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(tslot)),
+            "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem = *tslot;
+
+    if (warp == 0 && lane == 0)
+    {
+        prefetch_map(&mA);
+        prefetch_map(&mB);
+        const uint32_t bytes = (uint32_t)(A_SLICE + p.bn * BK * 2); // of one slice
+        int g                = 0; // stages issued so far
+        for (int w = blockIdx.x; w < p.nitems && !abort_all; w += gridDim.x)
+        {
+            int ti, tj, st0, nst;
+            decode(p, w, ti, tj, st0, nst);
+            for (int ps = 0; ps < NP && !abort_all; ps++)
+            {
+                const int ns = pass_hi(ps);
+                for (int it = 0; it < nst; it++, g++)
+                {
+                    const int b = g % STAGES;
+                    if (!mbar_wait(empty + b, (uint32_t)(((g / STAGES) & 1) ^ 1)))
+                    {
+                        abort_all = 1;
+                        break;
+                    }
+                    unsigned char* st = smem + b * STAGE;
+                    mbar_arrive_expect_tx(full + b, ns * bytes);
+                    const int k = (st0 + it) * BK, e0 = k % 64, kb = k / 64;
+#pragma unroll 1
+                    for (int s = 0; s < ns; s++)
+                    {
+                        tma_load_3d(st + s * A_SLICE, &mA, e0, ti * BM, s * p.kblocks + kb,
+                            full + b);
+                        tma_load_3d(st + NS * A_SLICE + s * B_SLICE, &mB, e0, tj * p.bn,
+                            s * p.kblocks + kb, full + b);
+                    }
+                }
+            }
+        }
+    }
+    else if (warp == 1 && lane == 0)
+    {
+        const uint32_t id = instr_desc<1>(BM, 0) | ((uint32_t)(p.bn >> 3) << 17);
+        int g = 0, drains = 0; // drains committed so far
+        for (int w = blockIdx.x; w < p.nitems && !abort_all; w += gridDim.x)
+        {
+            int ti, tj, st0, nst;
+            decode(p, w, ti, tj, st0, nst);
+            bool ok = true;
+            for (int ps = 0; ps < NP && ok; ps++)
+            {
+                const int lo = pass_lo(ps), hi = pass_hi(ps);
+                for (int it = 0; it < nst && ok; it++, g++)
+                {
+                    const int b = g % STAGES;
+                    ok          = mbar_wait(full + b, (uint32_t)((g / STAGES) & 1));
+                    if (!ok) break;
+                    fence_after_sync();
+                    const uint32_t a0 = smem_u32(smem + b * STAGE);
+                    const uint32_t b0 = a0 + NS * A_SLICE;
+                    const bool fresh  = it % DRAIN == 0;
+                    for (int d = lo; d < hi && ok; d++)
+                    {
+                        if (fresh && drains > 0)
+                        {
+                            ok = mbar_wait(acce + (d - lo), (uint32_t)((drains - 1) & 1));
+                            if (!ok) break;
+                            fence_after_sync();
+                        }
+                        const uint32_t acc = tmem + (uint32_t)((d - lo) * p.bn);
+#pragma unroll
+                        for (int kk = 0; kk < BK / 16; kk++)
+#pragma unroll 1
+                            for (int s = 0; s <= d; s++)
+                                mma<1>(acc, desc_sw<64>(a0 + s * A_SLICE + kk * 32),
+                                    desc_sw<64>(b0 + (d - s) * B_SLICE + kk * 32), id,
+                                    (!fresh || kk > 0 || s > 0) ? 1u : 0u);
+                    }
+                    if (!ok) break;
+                    mma_commit(empty + b);
+                    if (it % DRAIN == DRAIN - 1 || it == nst - 1)
+                    {
+                        mma_commit(accf);
+                        drains++;
+                    }
+                }
+            }
+            if (!ok)
+            {
+                abort_all = 1;
+                mma_commit(accf);
+                break;
+            }
+        }
+    }
+    else if (warp >= 2)
+    {
+        const int q    = warp & 3;       // TMEM lane quarter of this warp
+        const int half = (warp - 2) / 4; // its half of the columns
+        const int nc   = p.bn / 2, c0 = half * nc;
+        const uint32_t tw = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
+        int drains        = 0;
+        for (int w = blockIdx.x; w < p.nitems; w += gridDim.x)
+        {
+            int ti, tj, st0, nst;
+            decode(p, w, ti, tj, st0, nst);
+            // s + t <= 3 in units of 2^-w (NP 2) or 2^-24 of a digit product,
+            // and s + t >= 4 in units of 2^-48: in T until the second walk
+            // begins (NP 2), or in L
+            constexpr int EL = NP == 1 ? BN1 / 2 : BN / 2;
+            long long T[EL], L[NP == 1 ? EL : 1];
+#pragma unroll
+            for (int c = 0; c < EL; c++)
+            {
+                T[c] = 0;
+                if (NP == 1) L[NP == 1 ? c : 0] = 0;
+            }
+            const int nd = (nst + DRAIN - 1) / DRAIN;
+            bool ok      = true;
+            for (int d = 0; d < nd * NP; d++, drains++)
+            {
+                ok = !abort_all && mbar_wait(accf, (uint32_t)(drains & 1)) && !abort_all;
+                if (!ok) break;
+                fence_after_sync();
+                const int ps = d / nd, lo = pass_lo(ps), hi = pass_hi(ps);
+                if (NP == 2 && d == nd)
+                {
+#pragma unroll
+                    for (int c = 0; c < EL; c++)
+                        T[c] = (T[c] + (1ll << (47 - p.w))) >> (48 - p.w);
+                }
+#pragma unroll 1
+                for (int a = 0; a < NS; a++)
+                {
+                    if (lo + a < hi)
+                    {
+                        const int dg = lo + a;
+                        // the accumulator holds integers times 2^(-8 dg): they
+                        // join the sum shifted left by sh bits
+                        const int sh   = (dg >= 4 ? 48 : NP == 1 ? 24 : p.w) - 8 * dg;
+                        const int e    = sh == 31 ? 1 : 0; // a factor of 2^31 is no int
+                        const float up = __uint_as_float((uint32_t)(127 + 8 * dg + e) << 23);
+                        const int mul  = 1 << ((sh - e) & 31);
+#pragma unroll
+                        for (int c = 0; c < EL; c += 8)
+                        {
+                            if (c >= nc) break;
+                            float v[8];
+                            tmem_ld8(tw + a * p.bn + c, v);
+                            tmem_wait_ld();
+                            if (NP == 2 && sh >= 32)
+                            {
+                                // only the upper half changes
+#pragma unroll
+                                for (int i = 0; i < 8; i++)
+                                    T[c + i] += (long long)((unsigned long long)(unsigned)(
+                                                                __float2int_rn(v[i] * up) * mul)
+                                                            << 32);
+                            }
+                            else
+                            {
+#pragma unroll
+                                for (int i = 0; i < 8; i++)
+                                {
+                                    const long long x = (long long)__float2int_rn(v[i] * up) * mul;
+                                    if (NP == 1 && dg >= 4)
+                                        L[NP == 1 ? c + i : 0] += x;
+                                    else
+                                        T[c + i] += x;
+                                }
+                            }
+                        }
+                    }
+                    fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acce + a);
+                }
+            }
+            if (!ok)
+            {
+                abort_all = 1;
+                break;
+            }
+            if (NP == 1)
+            {
+#pragma unroll
+                for (int c = 0; c < EL; c++)
+                    T[c] = (T[c] << (p.w - 24))
+                           + ((L[NP == 1 ? c : 0] + (1ll << (47 - p.w))) >> (48 - p.w));
+            }
+            const size_t i  = (size_t)ti * BM + q * 32 + lane;
+            const size_t j0 = (size_t)tj * p.bn + c0;
+            if (i < p.m)
+            {
+                const int ei = key_exponent(p.ka[i]) - 14 - p.w;
+#pragma unroll
+                for (int c = 0; c < EL; c++)
+                {
+                    const size_t j = j0 + c;
+                    if (c < nc && j < p.n && (!p.t.lower || i >= j + p.t.col0))
+                    {
+                        if (p.t.sum)
+                        {
+                            // T 2^(SUM_W - w) = upper 2^32 + lower
+                            const int l = SUM_W - p.w;
+                            atomicAdd(p.t.sum + j * p.m + i, (unsigned long long)(T[c] >> (32 - l)));
+                            atomicAdd(p.t.sum + (p.n + j) * p.m + i,
+                                (unsigned long long)((unsigned)T[c] << l));
+                            continue;
+                        }
+                        const double v = scaled(T[c], ei + key_exponent(p.kb[j]));
+                        double* o      = p.t.C + j * p.t.ldc + i;
+                        if (p.t.beta != 0.)
+                            *o = p.t.alpha * v + p.t.beta * p.t.cin[j * p.t.ldcin + i];
+                        else
+                            *o = p.t.alpha == 1. ? v : p.t.alpha * v;
+                    }
+                }
+            }
+        }
+    }
+    if (abort_all && threadIdx.x == 0 && p.err) atomicExch(p.err, MGX_TIMEOUT);
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512)
+                     : "memory");
+}
+
+/* C(i, j) += the integer sums of Target::sum */
+__global__ void __launch_bounds__(256) add_sums_kernel(const unsigned long long* __restrict__ sum,
+    int m, int n, const int* __restrict__ ka, const int* __restrict__ kb, int lower, int col0,
+    double* __restrict__ C, size_t ldc, const int* __restrict__ bad)
+{
+    if (*bad) return;
+    const size_t total = (size_t)m * n;
+    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+         t += (size_t)gridDim.x * blockDim.x)
+    {
+        const int i = (int)(t % m), j = (int)(t / m);
+        if (lower && i < j + col0) continue;
+        const unsigned long long lo = sum[total + t];
+        const long long hi          = (long long)(sum[t] + (lo >> 32));
+        const double v = (double)hi * 4294967296. + (double)(unsigned)lo;
+        C[j * ldc + i] += scalbn(v, key_exponent(ka[i]) + key_exponent(kb[j]) - 14 - SUM_W);
+    }
+}
+
+size_t plane_bytes(size_t rows, size_t K)
+{
+    return NS * rows * ((K + 63) / 64) * 128;
+}
+
+int row_keys(const View& v, int* keys, int* bad, cudaStream_t s)
+{
+    MGX_TRY(cuda_check(cudaMemsetAsync(keys, 0, v.rows * sizeof(int), s), "keys reset"));
+    if (v.kmajor)
+    {
+        const unsigned gy = (unsigned)std::min<size_t>(v.rows, 32768);
+        const unsigned gx = (unsigned)std::max<size_t>(1,
+            std::min<size_t>((v.K + 4095) / 4096, (4096 + gy - 1) / gy));
+        keys_kmajor_kernel<<<dim3(gx, gy), 256, 0, s>>>(v.x, v.ld, v.rows, v.K, keys, bad);
+    }
+    else
+    {
+        const unsigned gx = (unsigned)std::min<size_t>((v.rows + 127) / 128, 65536);
+        const unsigned gy = (unsigned)std::max<size_t>(1,
+            std::min<size_t>((v.K + 31) / 32, (1024 + gx - 1) / gx));
+        keys_rmajor_kernel<<<dim3(gx, gy), 128, 0, s>>>(v.x, v.ld, v.rows, v.K, keys, bad);
+    }
+    MGX_LAUNCH_CHECK("slice keys kernel");
+    return MGX_OK;
+}
+
+int make_planes(const View& v, size_t k0, size_t kc, const int* keys, void* planes,
+    cudaStream_t s)
+{
+    const size_t kblocks = (kc + 63) / 64;
+    if (v.kmajor)
+    {
+        const size_t total = v.rows * kblocks * 8;
+        planes_kmajor_kernel<<<(unsigned)std::min<size_t>((total + 255) / 256, 1u << 20), 256, 0,
+            s>>>(v.x + k0, v.ld, v.rows, kc, keys, kblocks, (__nv_bfloat16*)planes);
+    }
+    else
+    {
+        const dim3 grid((unsigned)((v.rows + 63) / 64), (unsigned)kblocks);
+        if (grid.y > 65535) return fail(MGX_UNSUPPORTED, "slices: K too large");
+        planes_rmajor_kernel<<<grid, 256, 0, s>>>(v.x + k0 * v.ld, v.ld, v.rows, kc, keys, kblocks,
+            (__nv_bfloat16*)planes);
+    }
+    MGX_LAUNCH_CHECK("slice planes kernel");
+    return MGX_OK;
+}
+
+int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const void* pb,
+    const int* kb, size_t kc, const Target& t, const int* bad, int* err, cudaStream_t s)
+{
+    if (m == 0 || n == 0 || kc == 0) return MGX_OK;
+    Params p;
+    p.m = m;
+    p.n = n;
+    // equal column tiles of at most BN
+    p.ntj = (int)((n + BN - 1) / BN);
+    p.bn  = (int)(((n + p.ntj - 1) / p.ntj + 15) / 16 * 16);
+    p.nti = (int)((m + BM - 1) / BM);
+    p.ntiles = p.nti * p.ntj;
+    if (t.lower)
+    {
+        p.ntiles = 0;
+        for (int j = 0; j < p.ntj; j++)
+            p.ntiles += p.nti - std::min((t.col0 + j * p.bn) / BM, p.nti);
+        if (p.ntiles == 0) return MGX_OK;
+    }
+    p.kblocks = (int)((kc + 63) / 64);
+    p.nst     = (int)((kc + BK - 1) / BK);
+    p.st_per_item = p.nst;
+    if (t.sum)
+    {
+        // K split into items of whole drains: the split whose busiest SM has
+        // the least to do (a drain's worth of work for the end of each item),
+        // of at most 2^17 values each, which bounds the integers below
+        const int nd = (p.nst + DRAIN - 1) / DRAIN;
+        long best    = -1;
+        for (int ks = 1; ks <= std::min(nd, std::max(1, 4 * sms / p.ntiles + 1)); ks++)
+        {
+            const int per    = (nd + ks - 1) / ks;
+            const long items = (long)p.ntiles * ((nd + per - 1) / per);
+            const long cost  = ((items + sms - 1) / sms) * (per + 1);
+            if (best < 0 || cost < best)
+            {
+                best          = cost;
+                p.st_per_item = per * DRAIN;
+            }
+        }
+        p.st_per_item = std::min(p.st_per_item, (1 << 17) / BK);
+    }
+    const int ks     = (p.nst + p.st_per_item - 1) / p.st_per_item;
+    const long items = (long)p.ntiles * ks;
+    if (items > (1L << 30)) return fail(MGX_UNSUPPORTED, "too many work items");
+    p.nitems = (int)items;
+    // |sum| <= 1.01 K 2^14 2^w < 2^63 (and, in units of 2^-48, s + t >= 4 adds
+    // up to 5.1 K 2^30)
+    int lg = 0;
+    while ((1L << lg) < (long)p.st_per_item * BK) lg++;
+    if (lg > 17) return fail(MGX_UNSUPPORTED, "slices: K too large for one sum");
+    p.w = std::min(SUM_W, 48 - lg);
+    p.ka  = ka;
+    p.kb  = kb;
+    p.t   = t;
+    p.bad = bad;
+    p.err = err;
+    CUtensorMap mA, mB;
+    MGX_TRY(tc::make_map_blocked(&mA, pa, m, (size_t)NS * p.kblocks, BM, 64));
+    MGX_TRY(tc::make_map_blocked(&mB, pb, n, (size_t)NS * p.kblocks, p.bn, 64));
+    auto kern = p.bn <= BN1 ? slice_product_kernel<1> : slice_product_kernel<2>;
+    MGX_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)SMEM),
+        "slice_product_kernel smem attribute"));
+    kern<<<(int)std::min<long>(items, sms), THREADS, SMEM, s>>>(mA, mB, p);
+    MGX_LAUNCH_CHECK("slice_product_kernel");
+    return MGX_OK;
+}
+
+bool pays(size_t m, size_t n, size_t K)
+{
+    return (double)m * (double)n * (double)K >= 16. * 1024. * 1024.;
+}
+
+namespace
+{
+size_t up256(size_t b) { return (b + 255) / 256 * 256; }
+
+/* keys of na + nb rows, the flag, the error word and the planes of `planes`
+ * bytes in ctx's workspace */
+int workspace(mgx_ctx* ctx, size_t na, size_t nb, size_t planes, int** ka, int** kb, int** bad,
+    int** err, char** pl)
+{
+    const size_t head = up256((na + nb + 2) * sizeof(int));
+    if (ctx->slices.ensure(head + planes) != MGX_OK) return MGX_NO_MEMORY;
+    *bad = (int*)ctx->slices.ptr;
+    *err = *bad + 1;
+    *ka  = *bad + 2;
+    *kb  = *ka + na;
+    *pl  = (char*)ctx->slices.ptr + head;
+    return MGX_OK;
+}
+} // namespace
+
+int accumulate(mgx_ctx* ctx, const double* A, const double* B, size_t ld, size_t K, int n,
+    int ncols, int lower, int col0, double* C, int** bad, cudaStream_t s)
+{
+    const bool same   = A == B && n == ncols;
+    const size_t rows = (size_t)n + (same ? 0 : ncols);
+    const size_t fit  = std::max<size_t>(1, PLANE_CAP / plane_bytes(rows, 64));
+    const size_t kc   = std::min((K + 63) / 64, fit) * 64;
+    int *ka, *kb, *err;
+    char* pl;
+    const size_t pa_bytes  = up256(plane_bytes(n, kc));
+    const size_t pb_bytes  = same ? 0 : up256(plane_bytes(ncols, kc));
+    const size_t sum_bytes = 2 * (size_t)n * ncols * sizeof(unsigned long long);
+    MGX_TRY(workspace(ctx, n, ncols, pa_bytes + pb_bytes + sum_bytes, &ka, &kb, bad, &err, &pl));
+    MGX_TRY(cuda_check(cudaMemsetAsync(*bad, 0, 2 * sizeof(int), s), "slice flags"));
+    auto* sum = (unsigned long long*)(pl + pa_bytes + pb_bytes);
+    MGX_TRY(cuda_check(cudaMemsetAsync(sum, 0, sum_bytes, s), "slice sums"));
+    const View va = { A, ld, (size_t)n, K, true }, vb = { B, ld, (size_t)ncols, K, true };
+    MGX_TRY(row_keys(va, ka, *bad, s));
+    if (!same) MGX_TRY(row_keys(vb, kb, *bad, s));
+    const Target t = { nullptr, 0, sum, 1., 0., nullptr, 0, lower, col0 };
+    for (size_t k0 = 0; k0 < K; k0 += kc)
+    {
+        const size_t k = std::min(kc, K - k0);
+        MGX_TRY(make_planes(va, k0, k, ka, pl, s));
+        if (!same) MGX_TRY(make_planes(vb, k0, k, kb, pl + pa_bytes, s));
+        MGX_TRY(product(ctx->sm_count, n, pl, ka, ncols, same ? pl : pl + pa_bytes, same ? ka : kb,
+            k, t, *bad, err, s));
+    }
+    const unsigned blocks
+        = (unsigned)std::min<size_t>(((size_t)n * ncols + 255) / 256, 2048);
+    add_sums_kernel<<<blocks, 256, 0, s>>>(sum, n, ncols, ka, same ? ka : kb, lower, col0, C, n,
+        *bad);
+    MGX_LAUNCH_CHECK("add_sums_kernel");
+    return MGX_OK;
+}
+
+int store_begin(mgx_ctx* ctx, const View& A, const View& B, StorePlan* p, cudaStream_t s)
+{
+    const size_t K  = A.K;
+    const size_t b1 = up256(plane_bytes(B.rows, K));
+    const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(BM, K));
+    p->chunk = std::min((A.rows + BM - 1) / BM, fit) * BM;
+    const size_t rows = std::min(p->chunk, A.rows);
+    char* pl;
+    MGX_TRY(workspace(ctx, rows, B.rows, b1 + plane_bytes(rows, K), &p->ka, &p->kb, &p->bad,
+        &p->err, &pl));
+    p->pb = pl;
+    p->pa = pl + b1;
+    MGX_TRY(cuda_check(cudaMemsetAsync(p->bad, 0, 2 * sizeof(int), s), "slice flags"));
+    MGX_TRY(row_keys(B, p->kb, p->bad, s));
+    return make_planes(B, 0, K, p->kb, p->pb, s);
+}
+
+int store_chunk(mgx_ctx* ctx, const View& A, const View& B, const Target& t, const StorePlan& p,
+    size_t r0, size_t rows, cudaStream_t s)
+{
+    View a = A;
+    a.x += A.kmajor ? r0 * A.ld : r0;
+    a.rows   = rows;
+    Target c = t;
+    c.C += r0;
+    if (c.cin) c.cin += r0;
+    MGX_TRY(row_keys(a, p.ka, p.bad, s));
+    MGX_TRY(make_planes(a, 0, A.K, p.ka, p.pa, s));
+    return product(ctx->sm_count, rows, p.pa, p.ka, B.rows, p.pb, p.kb, A.K, c, p.bad, p.err, s);
+}
+} // namespace sl
+} // namespace mgx

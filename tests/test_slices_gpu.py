@@ -1,0 +1,117 @@
+"""FP64 products formed from exact bf16 slices on the tensor cores, against
+64-bit torch: the Gram-type products, Psi Theta and the residual's column
+chunks, at the edges of tiles (128 x at most 96), of the 256-value sums and of
+the plane chunks, and with operands that are not finite."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _block(nf, npts, seed, spread=8.0):
+    """Values whose size varies over 2^-spread .. 1 within a row."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    x = torch.randn((nf, npts), generator=g, dtype=torch.float64, device="cuda")
+    return x * torch.exp2(-spread * torch.rand((nf, npts), generator=g, dtype=torch.float64,
+                                               device="cuda"))
+
+
+def _bound(A, B, K):
+    """What |error| of A B^T may be: a slice drops 2^-56 and the products left
+    out 6 x 2^-56 of (row maximum x row maximum) per value of K, with random
+    signs; FP64 sums (the comparison's too) round at 2^-53.  64 sqrt(K) 2^-53
+    covers both with room for the largest of all entries."""
+    return 64.0 * K ** 0.5 * 2.0 ** -53 * A.abs().amax(1)[:, None] * B.abs().amax(1)[None, :]
+
+
+def _product(A, B):
+    """A B^T with sums of 256 values of K added up by error-free two-sums, so
+    that the comparison's own rounding does not grow with K."""
+    hi = torch.zeros((A.shape[0], B.shape[0]), dtype=torch.float64, device="cuda")
+    lo = torch.zeros_like(hi)
+    for k in range(0, A.shape[1], 256):
+        p = A[:, k:k + 256] @ B[:, k:k + 256].T
+        t = hi + p
+        v = t - hi
+        lo += (hi - (t - v)) + (p - v)
+        hi = t
+    return hi + lo
+
+
+@pytest.mark.parametrize("nf,n", [(33, (24, 20, 36)), (64, (32, 32, 32)), (95, (16, 20, 18)),
+                                  (97, (20, 18, 14)), (129, (14, 16, 18)), (200, (33, 7, 9)),
+                                  (64, (112, 108, 104))])
+def test_gram_products(nf, n):
+    from mgmol_gb300 import capi
+    ctx = capi.Context(n, tuple(float(x) for x in n))  # unit volume element
+    K = ctx.npts
+    psi, hp = _block(nf, K, 1), _block(nf, K, 2)
+    S, H = ctx.gram(psi), ctx.hmat(psi, hp)
+    for got, a, b in ((S, psi, psi), (H, psi, hp)):
+        assert bool(((got - _product(a, b)).abs() <= _bound(a, b, K)).all())
+    assert torch.equal(S, S.T)
+    # B with work blocks that cut the functions unevenly
+    B = ctx.matb(psi, work=torch.empty((min(nf, 50), K), dtype=torch.float64, device="cuda"))
+    bp = ctx.rhs_mehr(psi)
+    low = (B - _product(psi, bp)).tril().abs() <= _bound(psi, bp, K)
+    assert bool(low.all()) and torch.equal(B, B.T)
+
+
+@pytest.mark.parametrize("nf,n", [(40, (24, 20, 36)), (64, (32, 32, 32)), (97, (20, 18, 14)),
+                                  (260, (17, 9, 11)), (520, (8, 10, 12))])
+def test_psi_theta(nf, n):
+    from mgmol_gb300 import capi
+    ctx = capi.Context(n, tuple(float(x) for x in n))
+    psi, hp = _block(nf, ctx.npts, 3), _block(nf, ctx.npts, 4)
+    theta = _block(nf, nf, 5)
+    got = ctx.mult_matrix(psi, theta)
+    a, b = psi.T.contiguous(), theta.T.contiguous()
+    assert bool(((got.T - a @ b.T).abs() <= _bound(a, b, nf)).all())
+    res = ctx.residual(psi, hp, theta, apply_B=False)
+    assert bool(((res.T + hp.T - a @ b.T).abs()
+                 <= _bound(a, b, nf) + 2.0 ** -51 * (hp.T.abs() + (a @ b.T).abs())).all())
+    # a few columns, over the block of H psi
+    j0, nc = 5, nf - 9
+    out = hp[j0:j0 + nc].clone()
+    cols = b[j0:j0 + nc].contiguous()
+    ctx.residual_cols(psi, out, cols, apply_B=False, out=out)
+    assert torch.equal(out, res[j0:j0 + nc])
+
+
+def test_scales_and_zeros():
+    """Rows of any exponent, subnormal and zero rows among them."""
+    from mgmol_gb300 import capi
+    n = (32, 32, 20)
+    ctx = capi.Context(n, tuple(float(x) for x in n))
+    psi = _block(64, ctx.npts, 6)
+    e = torch.linspace(-500, 500, 64, device="cuda", dtype=torch.float64).round()
+    psi *= torch.exp2(e)[:, None]
+    psi[7] = 0.0
+    psi[11] = 5e-310  # subnormal
+    H = ctx.hmat(psi, psi.flip(0).contiguous())
+    ref = psi @ psi.flip(0).T
+    ok = (H - ref).abs() <= _bound(psi, psi.flip(0), ctx.npts) + 1e-14
+    assert bool(ok.all()) and bool((H[7] == 0).all())
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+def test_not_finite(bad):
+    """An operand that is not finite gives what FP64 multiply-adds give."""
+    from mgmol_gb300 import capi
+    n = (32, 32, 20)
+    ctx = capi.Context(n, tuple(float(x) for x in n))
+    psi, hp = _block(64, ctx.npts, 7).abs() + 1.0, _block(64, ctx.npts, 8).abs() + 1.0
+    hp[5, 77] = bad
+    H = ctx.hmat(psi, hp)
+    ref = psi @ hp.T
+    ref = torch.where(ref.abs() > 1e-14, ref, torch.zeros_like(ref))  # the filter takes NaN to 0
+    assert torch.equal(torch.isinf(H), torch.isinf(ref)) and not bool(torch.isnan(H).any())
+    assert torch.equal(H[:, 5], ref[:, 5])
+    keep = [j for j in range(64) if j != 5]
+    assert bool(((H - ref)[:, keep].abs() <= _bound(psi, psi, ctx.npts)[:, keep] * 64).all())
+    theta = _block(64, 64, 9).abs() + 1.0
+    got = ctx.mult_matrix(hp, theta)
+    want = theta.T @ hp
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(torch.isinf(got), torch.isinf(want))
