@@ -80,6 +80,8 @@ int masks_update(mgx_ctx*, mgx_masks*, const double*, const double*, cudaStream_
 int masks_expand(const mgx_masks*, int, void*, int*, cudaStream_t);
 int gram_cuda_cores(mgx_ctx*, int, const void*, const void*, size_t, size_t,
     int, double, int, double*, cudaStream_t);
+int gram_hmat_matb_f64(mgx_ctx*, const double*, const double*, size_t, size_t, int, double, double*,
+    double*, double*, double*, cudaStream_t);
 int psi_theta_cuda_cores(mgx_ctx*, int, const void*, size_t, size_t, int, const double*, int, int,
     double, const void*, void*, cudaStream_t);
 int psi_theta_tcgen05(mgx_ctx*, int, const float*, size_t, size_t, int,
@@ -749,6 +751,13 @@ int mgx_gram_hmat_matb(mgx_ctx* ctx, int mode, const void* psi, const void* hpsi
         MGX_TRY(matb_work(ctx, mode, ldv, nfunc, &work, &wf));
         return gram_hmat_tcgen05(ctx, mode, psi, hpsi, ldv, L.npts(), nfunc, vel, S, H,
             (cudaStream_t)stream, Bm, work, wf);
+    }
+    if (mode == MGX_GEMM_FP64 && work && work_funcs >= nfunc)
+    {
+        const Level L = make_level(ctx->grid, 0);
+        return gram_hmat_matb_f64(ctx, (const double*)psi, (const double*)hpsi,
+            nfunc > 1 ? ld : L.npts(), L.npts(), nfunc, L.h[0] * L.h[1] * L.h[2], S, H, Bm,
+            (double*)work, (cudaStream_t)stream);
     }
     MGX_TRY(mgx_gram(ctx, mode, psi, ld, nfunc, S, stream));
     MGX_TRY(mgx_hmat(ctx, mode, psi, hpsi, ld, nfunc, H, stream));

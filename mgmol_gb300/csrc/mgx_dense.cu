@@ -193,39 +193,56 @@ __global__ void gram_finish_kernel(double* C, int n, double vel, int symmetric)
 }
 
 /* C += A B^T of n x ncols functions of K points (with lower, at least the
- * entries i >= j + col0).  FP64 products of some size are formed from slices
- * on the tensor cores; the CUDA-core kernel behind them runs only when an
- * operand is not finite. */
-static int gram_add(mgx_ctx* ctx, int dtype, const void* A, const void* B, size_t ld, size_t K,
-    int n, int ncols, int lower, int col0, double* C, cudaStream_t s)
+ * entries i >= j + col0) for each of nf products with the same A.  FP64
+ * products of some size are formed from slices on the tensor cores; the
+ * CUDA-core kernels behind them run only when an operand is not finite. */
+static int gram_add(mgx_ctx* ctx, int dtype, const void* A, size_t ld, size_t K, int n,
+    const sl::Factor* f, int nf, cudaStream_t s)
 {
     int* only_if = nullptr;
-    if (dtype == MGX_F64 && sl::pays(n, ncols, K))
+    if (dtype == MGX_F64 && sl::pays(n, f[0].ncols, K))
     {
-        const int st = sl::accumulate(ctx, (const double*)A, (const double*)B, ld, K, n, ncols,
-            lower, col0, C, &only_if, s);
+        const int st = sl::accumulate(ctx, (const double*)A, ld, K, n, f, nf, &only_if, s);
         if (st == MGX_NO_MEMORY)
             only_if = nullptr; // no room for the planes: the CUDA cores do it
         else if (st != MGX_OK)
             return st;
     }
-    const int nti = (n + GT - 1) / GT, ntj = (ncols + GT - 1) / GT;
-    int ntiles    = 0;
-    for (int j = 0; j < ntj; j++)
-        ntiles += nti - gram_first_row(j, lower, col0, nti);
-    int ksplit    = std::max(1, (8 * ctx->sm_count + ntiles - 1) / ntiles);
-    size_t kslice = (K + ksplit - 1) / ksplit;
-    kslice        = ((kslice + GKC - 1) / GKC) * GKC;
-    ksplit        = (int)((K + kslice - 1) / kslice);
-    if (ksplit > 65535) return fail(MGX_UNSUPPORTED, "K too large for split");
-    dim3 grid(ntiles, ksplit);
-    if (dtype == MGX_F64)
-        gram_splitk_kernel<double><<<grid, 256, 0, s>>>((const double*)A, (const double*)B, ld, n,
-            ncols, K, kslice, lower, col0, only_if, C);
-    else
-        gram_splitk_kernel<float><<<grid, 256, 0, s>>>((const float*)A, (const float*)B, ld, n,
-            ncols, K, kslice, lower, col0, only_if, C);
-    MGX_LAUNCH_CHECK("gram_splitk_kernel");
+    const int nti = (n + GT - 1) / GT;
+    for (int q = 0; q < nf; q++)
+    {
+        const int ncols = f[q].ncols, lower = f[q].lower, col0 = f[q].col0;
+        const int ntj = (ncols + GT - 1) / GT;
+        int ntiles    = 0;
+        for (int j = 0; j < ntj; j++)
+            ntiles += nti - gram_first_row(j, lower, col0, nti);
+        int ksplit    = std::max(1, (8 * ctx->sm_count + ntiles - 1) / ntiles);
+        size_t kslice = (K + ksplit - 1) / ksplit;
+        kslice        = ((kslice + GKC - 1) / GKC) * GKC;
+        ksplit        = (int)((K + kslice - 1) / kslice);
+        if (ksplit > 65535) return fail(MGX_UNSUPPORTED, "K too large for split");
+        dim3 grid(ntiles, ksplit);
+        if (dtype == MGX_F64)
+            gram_splitk_kernel<double><<<grid, 256, 0, s>>>((const double*)A, f[q].B, ld, n, ncols,
+                K, kslice, lower, col0, only_if, f[q].C);
+        else
+            gram_splitk_kernel<float><<<grid, 256, 0, s>>>((const float*)A, (const float*)f[q].B,
+                ld, n, ncols, K, kslice, lower, col0, only_if, f[q].C);
+        MGX_LAUNCH_CHECK("gram_splitk_kernel");
+    }
+    return MGX_OK;
+}
+
+static int gram_begin(double* C, int n, cudaStream_t s)
+{
+    return cuda_check(cudaMemsetAsync(C, 0, (size_t)n * n * sizeof(double), s), "gram zero");
+}
+
+static int gram_finish(double* C, int n, double vel, int symmetric, cudaStream_t s)
+{
+    const int nb = (int)std::min<size_t>(((size_t)n * n + 255) / 256, 4096);
+    gram_finish_kernel<<<nb, 256, 0, s>>>(C, n, vel, symmetric);
+    MGX_LAUNCH_CHECK("gram_finish_kernel");
     return MGX_OK;
 }
 
@@ -233,12 +250,25 @@ int gram_cuda_cores(mgx_ctx* ctx, int dtype, const void* A, const void* B,
     size_t ld, size_t K, int n, double vel, int symmetric, double* C,
     cudaStream_t s)
 {
-    MGX_TRY(cuda_check(cudaMemsetAsync(C, 0, (size_t)n * n * sizeof(double), s),
-        "gram zero"));
-    MGX_TRY(gram_add(ctx, dtype, A, B, ld, K, n, n, symmetric, 0, C, s));
-    const int nb = (int)std::min<size_t>(((size_t)n * n + 255) / 256, 4096);
-    gram_finish_kernel<<<nb, 256, 0, s>>>(C, n, vel, symmetric);
-    MGX_LAUNCH_CHECK("gram_finish_kernel");
+    MGX_TRY(gram_begin(C, n, s));
+    const sl::Factor f = { (const double*)B, n, symmetric, 0, C };
+    MGX_TRY(gram_add(ctx, dtype, A, ld, K, n, &f, 1, s));
+    return gram_finish(C, n, vel, symmetric, s);
+}
+
+/* S, H and B of FP64 blocks in one go, B Psi whole in `work`: Psi is sliced
+ * once for the three products */
+int gram_hmat_matb_f64(mgx_ctx* ctx, const double* psi, const double* hpsi, size_t ld, size_t K,
+    int n, double vel, double* S, double* H, double* Bm, double* work, cudaStream_t s)
+{
+    MGX_TRY(rhs_block(ctx->grid, MGX_F64, psi, ld, work, ld, n, s));
+    double* C[3]         = { S, H, Bm };
+    const sl::Factor f[] = { { psi, n, 1, 0, S }, { hpsi, n, 0, 0, H }, { work, n, 1, 0, Bm } };
+    for (double* c : C)
+        MGX_TRY(gram_begin(c, n, s));
+    MGX_TRY(gram_add(ctx, MGX_F64, psi, ld, K, n, f, 3, s));
+    for (int i = 0; i < 3; i++)
+        MGX_TRY(gram_finish(C[i], n, vel, f[i].lower, s));
     return MGX_OK;
 }
 
@@ -252,18 +282,16 @@ int matb_cuda_cores(mgx_ctx* ctx, int dtype, const void* psi, size_t ld, size_t 
 {
     if (wf <= 0) return fail(MGX_BAD_ARG, "matB: empty work block");
     const size_t es = dtype_size(dtype);
-    MGX_TRY(cuda_check(cudaMemsetAsync(C, 0, (size_t)n * n * sizeof(double), s), "matB zero"));
+    MGX_TRY(gram_begin(C, n, s));
     for (int c0 = 0; c0 < n; c0 += wf)
     {
         const int nc = std::min(wf, n - c0);
         MGX_TRY(rhs_block(ctx->grid, dtype, (const char*)psi + (size_t)c0 * ld * es, ld, work,
             ld, nc, s));
-        MGX_TRY(gram_add(ctx, dtype, psi, work, ld, K, n, nc, 1, c0, C + (size_t)c0 * n, s));
+        const sl::Factor f = { (const double*)work, nc, 1, c0, C + (size_t)c0 * n };
+        MGX_TRY(gram_add(ctx, dtype, psi, ld, K, n, &f, 1, s));
     }
-    const int nb = (int)std::min<size_t>(((size_t)n * n + 255) / 256, 4096);
-    gram_finish_kernel<<<nb, 256, 0, s>>>(C, n, vel, 1);
-    MGX_LAUNCH_CHECK("gram_finish_kernel");
-    return MGX_OK;
+    return gram_finish(C, n, vel, 1, s);
 }
 
 /* ------------------------------------------------------------------ */

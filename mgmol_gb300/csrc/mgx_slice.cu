@@ -12,7 +12,7 @@
 //   - digit s of A times digit t of B are integers of at most 2^14 at weight
 //     2^(-8 (s + t)).  The products of one s + t add up in an FP32 accumulator
 //     of their own, which rounds nothing while |sum| <= 2^24: after 192 values
-//     of K it is read and added to a 64-bit integer.  (All of s + t <= 4 are
+//     of K (256 where only s + t <= 3 are summed) it is read and added to a 64-bit integer.  (All of s + t <= 4 are
 //     exact for any input; of the 6 or 7 x 192 products of s + t = 5 and 6, at
 //     2^-40 and 2^-48, the last bit could round if all digits were extreme.)
 //     The sums have to be exact and not only FP32: the tensor cores truncate
@@ -30,6 +30,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
+#include <vector>
 
 #include "mgx_slice.cuh"
 #include "mgx_tcgen05.cuh"
@@ -45,10 +47,11 @@ constexpr int BN1     = 64;  // most columns with all NS accumulators in TMEM at
 constexpr int BK      = 32;  // K values of a stage (64 bytes, SWIZZLE_64B)
 constexpr int STAGES  = 2;
 constexpr int DRAIN   = 6;   // stages between reads of the accumulators
+constexpr int DRAIN2  = 8;   // the same for the walk of s + t = 0 .. 3 alone
 constexpr int A_SLICE = BM * BK * 2;
 constexpr int B_SLICE = BN * BK * 2;
 constexpr int STAGE   = NS * (A_SLICE + B_SLICE);
-constexpr int EPI     = 8;   // epilogue warps
+constexpr int EPI     = 16;  // epilogue warps: four per scheduler hide the TMEM reads
 constexpr int SUM_W   = 47;  // sums over items are kept in units of 2^-SUM_W
 constexpr int THREADS = 32 * (2 + EPI);
 constexpr size_t SMEM = (size_t)STAGES * STAGE + (2 * STAGES + 1 + NS) * 8 + 16 + 1024;
@@ -233,7 +236,7 @@ __global__ void __launch_bounds__(256) planes_rmajor_kernel(const double* __rest
 struct Params
 {
     int nti, ntj;    // tiles
-    int bn;          // columns of a tile, a multiple of 16
+    int bn;          // columns of a tile, a multiple of 32
     int ntiles;      // tiles formed (with lower: those that reach i >= j + col0)
     int nst;         // stages of K
     int st_per_item; // stages of one item
@@ -276,19 +279,20 @@ __device__ __forceinline__ void decode(const Params& p, int w, int& ti, int& tj,
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
 {
-    uint32_t r[8];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-                 "=r"(r[6]), "=r"(r[7])
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]),
+                 "=f"(v[6]), "=f"(v[7])
                  : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-        v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void tmem_wait_ld()
+/* waits for the loads in flight; the values of v are used only behind it */
+__device__ __forceinline__ void tmem_wait_ld(float (&v)[8])
 {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]),
+                 "+f"(v[6]), "+f"(v[7])
+                 :
+                 : "memory");
 }
 
 /* T 2^E, exactly where the result is a normal number */
@@ -303,8 +307,8 @@ __device__ __forceinline__ double scaled(long long T, int E)
 
 /* One CTA per SM walks the items.  Warp 0 streams the slices of both operands
  * (two stages of up to 114 KB), warp 1 issues the MMAs, one accumulator per
- * s + t, and warps 2 .. 9 add the accumulators into 64-bit integers in
- * registers (64 per thread) and finish the tile.  A tile has 128 columns,
+ * s + t, and warps 2 .. 17 add the accumulators into 64-bit integers in
+ * registers (32 per thread) and finish the tile.  A tile has 128 columns,
  * for which TMEM holds four accumulators: K is walked twice, for s + t = 4 .. 6
  * (18 products of 7 slices) and 0 .. 3 (10 products of 4).  An MMA of 128 x 128
  * x 16 reads 8 KB of shared memory in 64 clocks, just what the SM delivers; one
@@ -332,6 +336,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
     // diagonals s + t of walk ps: [pass_lo, pass_hi), which read slices < pass_hi
     auto pass_lo = [](int ps) { return NP == 1 || ps == 1 ? 0 : 4; };
     auto pass_hi = [](int ps) { return NP == 1 || ps == 0 ? NS : 4; };
+    auto drain   = [](int ps) { return ps == 0 ? DRAIN : DRAIN2; };
     if (threadIdx.x == 0)
     {
         for (int s = 0; s < STAGES; s++)
@@ -412,29 +417,39 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                     ok          = mbar_wait(full + b, (uint32_t)((g / STAGES) & 1));
                     if (!ok) break;
                     fence_after_sync();
-                    const uint32_t a0 = smem_u32(smem + b * STAGE);
-                    const uint32_t b0 = a0 + NS * A_SLICE;
-                    const bool fresh  = it % DRAIN == 0;
-                    for (int d = lo; d < hi && ok; d++)
-                    {
+                    const uint64_t ad = desc_sw<64>(smem_u32(smem + b * STAGE));
+                    const uint64_t bd = desc_sw<64>(smem_u32(smem + b * STAGE) + NS * A_SLICE);
+                    const bool fresh  = it % drain(ps) == 0;
+                    // one descriptor addition per operand and MMA: the issuing
+                    // thread has 64 clocks for each
+                    auto diagonal = [&](auto dc) {
+                        constexpr int d = decltype(dc)::value;
+                        if (d < lo || d >= hi || !ok) return;
                         if (fresh && drains > 0)
                         {
                             ok = mbar_wait(acce + (d - lo), (uint32_t)((drains - 1) & 1));
-                            if (!ok) break;
+                            if (!ok) return;
                             fence_after_sync();
                         }
                         const uint32_t acc = tmem + (uint32_t)((d - lo) * p.bn);
 #pragma unroll
                         for (int kk = 0; kk < BK / 16; kk++)
-#pragma unroll 1
+#pragma unroll
                             for (int s = 0; s <= d; s++)
-                                mma<1>(acc, desc_sw<64>(a0 + s * A_SLICE + kk * 32),
-                                    desc_sw<64>(b0 + (d - s) * B_SLICE + kk * 32), id,
+                                mma<1>(acc, ad + ((s * A_SLICE + kk * 32) >> 4),
+                                    bd + (((d - s) * B_SLICE + kk * 32) >> 4), id,
                                     (!fresh || kk > 0 || s > 0) ? 1u : 0u);
-                    }
+                    };
+                    diagonal(std::integral_constant<int, 0>());
+                    diagonal(std::integral_constant<int, 1>());
+                    diagonal(std::integral_constant<int, 2>());
+                    diagonal(std::integral_constant<int, 3>());
+                    diagonal(std::integral_constant<int, 4>());
+                    diagonal(std::integral_constant<int, 5>());
+                    diagonal(std::integral_constant<int, 6>());
                     if (!ok) break;
                     mma_commit(empty + b);
-                    if (it % DRAIN == DRAIN - 1 || it == nst - 1)
+                    if (it % drain(ps) == drain(ps) - 1 || it == nst - 1)
                     {
                         mma_commit(accf);
                         drains++;
@@ -451,9 +466,8 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
     }
     else if (warp >= 2)
     {
-        const int q    = warp & 3;       // TMEM lane quarter of this warp
-        const int half = (warp - 2) / 4; // its half of the columns
-        const int nc   = p.bn / 2, c0 = half * nc;
+        const int q    = warp & 3; // TMEM lane quarter of this warp
+        const int nc   = p.bn / 4, c0 = (warp - 2) / 4 * nc; // its columns
         const uint32_t tw = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
         int drains        = 0;
         for (int w = blockIdx.x; w < p.nitems; w += gridDim.x)
@@ -463,7 +477,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
             // s + t <= 3 in units of 2^-w (NP 2) or 2^-24 of a digit product,
             // and s + t >= 4 in units of 2^-48: in T until the second walk
             // begins (NP 2), or in L
-            constexpr int EL = NP == 1 ? BN1 / 2 : BN / 2;
+            constexpr int EL = NP == 1 ? BN1 / 4 : BN / 4;
             long long T[EL], L[NP == 1 ? EL : 1];
 #pragma unroll
             for (int c = 0; c < EL; c++)
@@ -471,14 +485,15 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                 T[c] = 0;
                 if (NP == 1) L[NP == 1 ? c : 0] = 0;
             }
-            const int nd = (nst + DRAIN - 1) / DRAIN;
+            const int nd = (nst + DRAIN - 1) / DRAIN; // of the first walk
+            const int na = NP == 1 ? nd : nd + (nst + DRAIN2 - 1) / DRAIN2;
             bool ok      = true;
-            for (int d = 0; d < nd * NP; d++, drains++)
+            for (int d = 0; d < na; d++, drains++)
             {
                 ok = !abort_all && mbar_wait(accf, (uint32_t)(drains & 1)) && !abort_all;
                 if (!ok) break;
                 fence_after_sync();
-                const int ps = d / nd, lo = pass_lo(ps), hi = pass_hi(ps);
+                const int ps = d < nd ? 0 : 1, lo = pass_lo(ps), hi = pass_hi(ps);
                 if (NP == 2 && d == nd)
                 {
 #pragma unroll
@@ -501,16 +516,16 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                         for (int c = 0; c < EL; c += 8)
                         {
                             if (c >= nc) break;
-                            float v[8];
-                            tmem_ld8(tw + a * p.bn + c, v);
-                            tmem_wait_ld();
+                            float x[8];
+                            tmem_ld8(tw + a * p.bn + c, x);
+                            tmem_wait_ld(x);
                             if (NP == 2 && sh >= 32)
                             {
                                 // only the upper half changes
 #pragma unroll
                                 for (int i = 0; i < 8; i++)
                                     T[c + i] += (long long)((unsigned long long)(unsigned)(
-                                                                __float2int_rn(v[i] * up) * mul)
+                                                                __float2int_rn(x[i] * up) * mul)
                                                             << 32);
                             }
                             else
@@ -518,11 +533,11 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
 #pragma unroll
                                 for (int i = 0; i < 8; i++)
                                 {
-                                    const long long x = (long long)__float2int_rn(v[i] * up) * mul;
+                                    const long long y = (long long)__float2int_rn(x[i] * up) * mul;
                                     if (NP == 1 && dg >= 4)
-                                        L[NP == 1 ? c + i : 0] += x;
+                                        L[NP == 1 ? c + i : 0] += y;
                                     else
-                                        T[c + i] += x;
+                                        T[c + i] += y;
                                 }
                             }
                         }
@@ -659,7 +674,7 @@ int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const vo
     p.n = n;
     // equal column tiles of at most BN
     p.ntj = (int)((n + BN - 1) / BN);
-    p.bn  = (int)(((n + p.ntj - 1) / p.ntj + 15) / 16 * 16);
+    p.bn  = (int)(((n + p.ntj - 1) / p.ntj + 31) / 32 * 32);
     p.nti = (int)((m + BM - 1) / BM);
     p.ntiles = p.nti * p.ntj;
     if (t.lower)
@@ -744,39 +759,76 @@ int workspace(mgx_ctx* ctx, size_t na, size_t nb, size_t planes, int** ka, int**
 }
 } // namespace
 
-int accumulate(mgx_ctx* ctx, const double* A, const double* B, size_t ld, size_t K, int n,
-    int ncols, int lower, int col0, double* C, int** bad, cudaStream_t s)
+int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const Factor* f, int nf,
+    int** bad, cudaStream_t s)
 {
-    const bool same   = A == B && n == ncols;
-    const size_t rows = (size_t)n + (same ? 0 : ncols);
-    const size_t fit  = std::max<size_t>(1, PLANE_CAP / plane_bytes(rows, 64));
-    const size_t kc   = std::min((K + 63) / 64, fit) * 64;
+    // the planes of A and, in turn, those of each B that is not A; a sum and
+    // the keys of each
+    size_t brows = 0, bkeys = 0, sums = 0;
+    for (int i = 0; i < nf; i++)
+    {
+        if (f[i].B != A || f[i].ncols != n)
+        {
+            brows = std::max<size_t>(brows, f[i].ncols);
+            bkeys += f[i].ncols;
+        }
+        sums += 2 * (size_t)n * f[i].ncols;
+    }
+    const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(n + brows, 64));
+    const size_t kc  = std::min((K + 63) / 64, fit) * 64;
+    const size_t pa_bytes = up256(plane_bytes(n, kc)), pb_bytes = up256(plane_bytes(brows, kc));
     int *ka, *kb, *err;
     char* pl;
-    const size_t pa_bytes  = up256(plane_bytes(n, kc));
-    const size_t pb_bytes  = same ? 0 : up256(plane_bytes(ncols, kc));
-    const size_t sum_bytes = 2 * (size_t)n * ncols * sizeof(unsigned long long);
-    MGX_TRY(workspace(ctx, n, ncols, pa_bytes + pb_bytes + sum_bytes, &ka, &kb, bad, &err, &pl));
+    MGX_TRY(workspace(ctx, n, bkeys, pa_bytes + pb_bytes + sums * sizeof(unsigned long long), &ka,
+        &kb, bad, &err, &pl));
+    char* pb  = pl + pa_bytes;
+    auto* sum = (unsigned long long*)(pb + pb_bytes);
     MGX_TRY(cuda_check(cudaMemsetAsync(*bad, 0, 2 * sizeof(int), s), "slice flags"));
-    auto* sum = (unsigned long long*)(pl + pa_bytes + pb_bytes);
-    MGX_TRY(cuda_check(cudaMemsetAsync(sum, 0, sum_bytes, s), "slice sums"));
-    const View va = { A, ld, (size_t)n, K, true }, vb = { B, ld, (size_t)ncols, K, true };
+    MGX_TRY(cuda_check(cudaMemsetAsync(sum, 0, sums * sizeof(unsigned long long), s), "slice sums"));
+    const View va = { A, ld, (size_t)n, K, true };
     MGX_TRY(row_keys(va, ka, *bad, s));
-    if (!same) MGX_TRY(row_keys(vb, kb, *bad, s));
-    const Target t = { nullptr, 0, sum, 1., 0., nullptr, 0, lower, col0 };
+    struct Part
+    {
+        bool same;
+        View v;
+        int* keys;
+        Target t;
+    };
+    std::vector<Part> parts;
+    for (int i = 0; i < nf; i++)
+    {
+        Part q;
+        q.same = f[i].B == A && f[i].ncols == n;
+        q.v    = { f[i].B, ld, (size_t)f[i].ncols, K, true };
+        q.keys = q.same ? ka : kb;
+        q.t    = { nullptr, 0, sum, 1., 0., nullptr, 0, f[i].lower, f[i].col0 };
+        sum += 2 * (size_t)n * f[i].ncols;
+        if (!q.same)
+        {
+            MGX_TRY(row_keys(q.v, kb, *bad, s));
+            kb += f[i].ncols;
+        }
+        parts.push_back(q);
+    }
     for (size_t k0 = 0; k0 < K; k0 += kc)
     {
         const size_t k = std::min(kc, K - k0);
         MGX_TRY(make_planes(va, k0, k, ka, pl, s));
-        if (!same) MGX_TRY(make_planes(vb, k0, k, kb, pl + pa_bytes, s));
-        MGX_TRY(product(ctx->sm_count, n, pl, ka, ncols, same ? pl : pl + pa_bytes, same ? ka : kb,
-            k, t, *bad, err, s));
+        for (const Part& q : parts)
+        {
+            if (!q.same) MGX_TRY(make_planes(q.v, k0, k, q.keys, pb, s));
+            MGX_TRY(product(ctx->sm_count, n, pl, ka, q.v.rows, q.same ? pl : pb, q.keys, k, q.t,
+                *bad, err, s));
+        }
     }
-    const unsigned blocks
-        = (unsigned)std::min<size_t>(((size_t)n * ncols + 255) / 256, 2048);
-    add_sums_kernel<<<blocks, 256, 0, s>>>(sum, n, ncols, ka, same ? ka : kb, lower, col0, C, n,
-        *bad);
-    MGX_LAUNCH_CHECK("add_sums_kernel");
+    for (int i = 0; i < nf; i++)
+    {
+        const unsigned blocks
+            = (unsigned)std::min<size_t>(((size_t)n * f[i].ncols + 255) / 256, 2048);
+        add_sums_kernel<<<blocks, 256, 0, s>>>(parts[i].t.sum, n, f[i].ncols, ka, parts[i].keys,
+            f[i].lower, f[i].col0, f[i].C, n, *bad);
+        MGX_LAUNCH_CHECK("add_sums_kernel");
+    }
     return MGX_OK;
 }
 

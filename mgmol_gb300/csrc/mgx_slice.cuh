@@ -55,14 +55,24 @@ int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const vo
 /* whether a product of this size is formed from slices */
 bool pays(size_t m, size_t n, size_t K);
 
-/* C(i, j) += sum_k A(i, k) B(j, k) over K-contiguous blocks of ld (n rows of
- * A, ncols of B) in chunks of K that bound the planes to PLANE_CAP bytes;
- * with lower, entries i >= j + col0 only.  *bad (device) tells whether the
- * operands were not finite and nothing was added.  MGX_NO_MEMORY: no
- * workspace, nothing was added. */
+/* One product with a shared left operand: C(i, j) += sum_k A(i, k) B(j, k),
+ * j < ncols, C of leading dimension n; with lower, entries i >= j + col0. */
+struct Factor
+{
+    const double* B;
+    int ncols;
+    int lower;
+    int col0;
+    double* C;
+};
+
+/* The products of K-contiguous blocks of leading dimension ld (n rows of A),
+ * in chunks of K that bound the planes to PLANE_CAP bytes; the planes of A
+ * serve all of them.  *bad (device) tells whether an operand was not finite
+ * and nothing was added.  MGX_NO_MEMORY: no workspace, nothing was added. */
 constexpr size_t PLANE_CAP = size_t(1) << 30;
-int accumulate(mgx_ctx* ctx, const double* A, const double* B, size_t ld, size_t K, int n,
-    int ncols, int lower, int col0, double* C, int** bad, cudaStream_t s);
+int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const Factor* f, int nf,
+    int** bad, cudaStream_t s);
 
 /* C = alpha A B^T + beta cin of FP64 operands of any layout, the rows of A in
  * chunks that bound the planes to PLANE_CAP bytes.  After each chunk
