@@ -86,7 +86,7 @@ int psi_theta_cuda_cores(mgx_ctx*, int, const void*, size_t, size_t, int, const 
     double, const void*, void*, cudaStream_t);
 int psi_theta_tcgen05(mgx_ctx*, int, const float*, size_t, size_t, int,
     const double*, int, int, float, const float*, float*, cudaStream_t, double* rho = nullptr);
-int theta_product(int, const double*, const double*, double*, cudaStream_t);
+int theta_product(mgx_ctx*, int, const double*, const double*, double*, cudaStream_t);
 int theta_from_cholesky(mgx_ctx*, int, const double*, const double*, double*, double*,
     cudaStream_t);
 int mgm_solve(mgx_ctx*, const mgx_mgm_params*, int, void*, const void*, mgx_mgm_result*,
@@ -100,7 +100,7 @@ int matb_cuda_cores(mgx_ctx*, int, const void*, size_t, size_t, int, double, dou
     void*, int, cudaStream_t);
 int matb_tcgen05(mgx_ctx*, int, const void*, size_t, size_t, int, double, double*, void*, int,
     cudaStream_t);
-int update_hb(int, const double*, const double*, double*, cudaStream_t);
+int update_hb(mgx_ctx*, int, const double*, const double*, double*, cudaStream_t);
 int normalize(mgx_ctx*, int, void*, size_t, size_t, int, double, double*, cudaStream_t);
 int diag_rsqrt(mgx_ctx*, int, const double*, double*, cudaStream_t);
 int cholesky(mgx_ctx*, int, double*, int*, cudaStream_t, int* info_dev = nullptr);
@@ -795,7 +795,7 @@ int mgx_update_hb(mgx_ctx* ctx, int n, const double* S, const double* theta, dou
     void* stream)
 {
     if (!ctx) return fail(MGX_BAD_ARG, "ctx is NULL");
-    return update_hb(n, S, theta, HB, (cudaStream_t)stream);
+    return update_hb(ctx, n, S, theta, HB, (cudaStream_t)stream);
 }
 
 int mgx_normalize(mgx_ctx* ctx, mgx_dtype dtype, void* psi, size_t ld, int nfunc,
@@ -863,7 +863,7 @@ int mgx_theta(mgx_ctx* ctx, int n, const double* Sinv, const double* H,
 {
     if (!ctx) return fail(MGX_BAD_ARG, "ctx is NULL");
     if (theta == Sinv || theta == H) return fail(MGX_BAD_ARG, "theta aliases an input");
-    return theta_product(n, Sinv, H, theta, (cudaStream_t)stream);
+    return theta_product(ctx, n, Sinv, H, theta, (cudaStream_t)stream);
 }
 }
 

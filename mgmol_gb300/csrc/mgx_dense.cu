@@ -297,61 +297,75 @@ int matb_cuda_cores(mgx_ctx* ctx, int dtype, const void* psi, size_t ld, size_t 
 /* ------------------------------------------------------------------ */
 /* generic FP64 GEMM, column-major: C = alpha op(A) op(B) + beta C        */
 /* ------------------------------------------------------------------ */
-// sym_a: A is symmetric and only its lower triangle is read (BLAS symm
-// with side 'l', uplo 'l'); used without TA.
-template <bool TA, bool TB>
+// On the FP64 units, 2 multiply-adds per SM and clock: a tile of TS x TS x k
+// takes TS^2 k / 2 clocks of its SM, so the tile is the largest one that
+// still spreads over all SMs (64^3: 69 us on one SM, 5 us in 16 x 16 tiles).
+// lower_only: entries i + roff >= j; blockIdx.z: a batch of equal products at
+// strides sA, sB, sC; only_if as in gram_splitk_kernel.
+template <bool TA, bool TB, int TS>
 __global__ void __launch_bounds__(256) dgemm_kernel(int m, int n, int k,
     double alpha, const double* __restrict__ A, int lda,
     const double* __restrict__ B, int ldb, double beta, double* C, int ldc,
-    int lower_only, int sym_a)
+    int lower_only, int roff, size_t sA, size_t sB, size_t sC, const int* __restrict__ only_if)
 {
-    __shared__ double As[16][65];
-    __shared__ double Bs[16][65];
-    const int i0 = blockIdx.x * 64, j0 = blockIdx.y * 64;
-    if (lower_only && i0 + 63 < j0) return;
+    constexpr int R = TS / 16;
+    __shared__ double As[16][TS + 1];
+    __shared__ double Bs[16][TS + 1];
+    if (only_if && *only_if == 0) return;
+    A += blockIdx.z * sA;
+    B += blockIdx.z * sB;
+    C += blockIdx.z * sC;
+    const int i0 = blockIdx.x * TS, j0 = blockIdx.y * TS;
+    if (lower_only && i0 + TS - 1 + roff < j0) return;
     const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-    double acc[4][4] = {};
+    double acc[R][R] = {};
     for (int kc = 0; kc < k; kc += 16)
     {
 #pragma unroll
-        for (int r = 0; r < 4; r++)
+        for (int r = 0; r < R; r++)
         {
-            const int e  = tid + r * 256;
-            const int mm = e % 64, kk = e / 64;
-            const int i = i0 + mm, j = j0 + mm, kq = kc + kk;
-            double av = 0., bv = 0.;
-            if (i < m && kq < k)
-                av = (TA || (sym_a && kq > i)) ? A[(size_t)i * lda + kq] : A[(size_t)kq * lda + i];
-            if (j < n && kq < k) bv = TB ? B[(size_t)kq * ldb + j] : B[(size_t)j * ldb + kq];
-            As[kk][mm] = av;
-            Bs[kk][mm] = bv;
+            // the 16 x TS elements of each operand along the direction in
+            // which it is contiguous
+            const int e = tid + r * 256;
+            {
+                const int mm = TA ? e / 16 : e % TS, kk = TA ? e % 16 : e / TS;
+                const int i = i0 + mm, kq = kc + kk;
+                As[kk][mm] = (i < m && kq < k) ? (TA ? A[(size_t)i * lda + kq] : A[(size_t)kq * lda + i])
+                                               : 0.;
+            }
+            {
+                const int mm = TB ? e % TS : e / 16, kk = TB ? e / TS : e % 16;
+                const int j = j0 + mm, kq = kc + kk;
+                Bs[kk][mm] = (j < n && kq < k) ? (TB ? B[(size_t)kq * ldb + j] : B[(size_t)j * ldb + kq])
+                                               : 0.;
+            }
         }
         __syncthreads();
 #pragma unroll
         for (int kk = 0; kk < 16; kk++)
         {
-            double a[4], b[4];
+            double a[R], b[R];
 #pragma unroll
-            for (int q = 0; q < 4; q++)
+            for (int q = 0; q < R; q++)
             {
-                a[q] = As[kk][ty + 16 * q];
-                b[q] = Bs[kk][tx + 16 * q];
+                a[q] = As[kk][tx + 16 * q];
+                b[q] = Bs[kk][ty + 16 * q];
             }
 #pragma unroll
-            for (int p = 0; p < 4; p++)
+            for (int p = 0; p < R; p++)
 #pragma unroll
-                for (int q = 0; q < 4; q++)
+                for (int q = 0; q < R; q++)
                     acc[p][q] = fma(a[p], b[q], acc[p][q]);
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int p = 0; p < 4; p++)
+    for (int p = 0; p < R; p++)
 #pragma unroll
-        for (int q = 0; q < 4; q++)
+        for (int q = 0; q < R; q++)
         {
-            const int i = i0 + ty + 16 * p, j = j0 + tx + 16 * q;
-            if (i < m && j < n && (!lower_only || i >= j))
+            const int i = i0 + tx + 16 * p, j = j0 + ty + 16 * q;
+            if (i < m && j < n && (!lower_only || i + roff >= j))
             {
                 double* c = C + (size_t)j * ldc + i;
                 *c        = alpha * acc[p][q] + (beta == 0. ? 0. : beta * *c);
@@ -359,22 +373,71 @@ __global__ void __launch_bounds__(256) dgemm_kernel(int m, int n, int k,
         }
 }
 
-static int dgemm(bool ta, bool tb, int m, int n, int k, double alpha,
-    const double* A, int lda, const double* B, int ldb, double beta, double* C,
-    int ldc, int lower_only, cudaStream_t s, int sym_a = 0)
+/* C = alpha op(A) op(B) + beta C on the FP64 units */
+struct Gemm
 {
-    if (m <= 0 || n <= 0) return MGX_OK;
-    dim3 grid((m + 63) / 64, (n + 63) / 64);
-    if (!ta && !tb)
-        dgemm_kernel<false, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower_only, sym_a);
-    else if (!ta && tb)
-        dgemm_kernel<false, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower_only, sym_a);
-    else if (ta && !tb)
-        dgemm_kernel<true, false><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower_only, sym_a);
-    else
-        dgemm_kernel<true, true><<<grid, 256, 0, s>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, lower_only, sym_a);
+    bool ta, tb;
+    int m, n, k;
+    double alpha;
+    const double* A;
+    int lda;
+    const double* B;
+    int ldb;
+    double beta;
+    double* C;
+    int ldc;
+    int lower = 0;
+    int batch = 1;
+    size_t sA = 0, sB = 0, sC = 0;
+};
+
+template <bool TA, bool TB>
+static int dgemm_t(const Gemm& g, int roff, const int* only_if, int sms, cudaStream_t s)
+{
+    auto tiles = [&](int ts) {
+        return (long)((g.m + ts - 1) / ts) * ((g.n + ts - 1) / ts) * g.batch;
+    };
+    const int ts = tiles(64) >= sms ? 64 : tiles(32) >= sms ? 32 : 16;
+    const dim3 grid((g.m + ts - 1) / ts, (g.n + ts - 1) / ts, g.batch);
+    auto kern = ts == 64 ? dgemm_kernel<TA, TB, 64>
+                         : ts == 32 ? dgemm_kernel<TA, TB, 32> : dgemm_kernel<TA, TB, 16>;
+    kern<<<grid, 256, 0, s>>>(g.m, g.n, g.k, g.alpha, g.A, g.lda, g.B, g.ldb, g.beta, g.C, g.ldc,
+        g.lower, roff, g.sA, g.sB, g.sC, only_if);
     MGX_LAUNCH_CHECK("dgemm_kernel");
     return MGX_OK;
+}
+
+static int dgemm(const Gemm& g, int sms, cudaStream_t s, int roff = 0, const int* only_if = nullptr)
+{
+    if (g.m <= 0 || g.n <= 0) return MGX_OK;
+    if (!g.ta && !g.tb) return dgemm_t<false, false>(g, roff, only_if, sms, s);
+    if (!g.ta && g.tb) return dgemm_t<false, true>(g, roff, only_if, sms, s);
+    if (g.ta && !g.tb) return dgemm_t<true, false>(g, roff, only_if, sms, s);
+    return dgemm_t<true, true>(g, roff, only_if, sms, s);
+}
+
+/* C = alpha op(A) op(B) + beta C, from slices on the tensor cores where they
+ * pay (C may then alias A or B only as far as it may for the kernel above,
+ * which takes over when an operand is not finite) */
+static int gemm(mgx_ctx* ctx, const Gemm& g, cudaStream_t s)
+{
+    if (g.m <= 0 || g.n <= 0) return MGX_OK;
+    if (g.batch == 1 && sl::pays(g.m, g.n, g.k))
+    {
+        const sl::View a = { g.A, (size_t)g.lda, (size_t)g.m, (size_t)g.k, g.ta };
+        const sl::View b = { g.B, (size_t)g.ldb, (size_t)g.n, (size_t)g.k, !g.tb };
+        const sl::Target t
+            = { g.C, (size_t)g.ldc, nullptr, g.alpha, g.beta, g.C, (size_t)g.ldc, g.lower, 0 };
+        const int st = sl::store(ctx, a, b, t, s, [&](size_t r0, size_t rows, const int* bad) {
+            Gemm c = g;
+            c.m    = (int)rows;
+            c.A += g.ta ? r0 * g.lda : r0;
+            c.C += r0;
+            return dgemm(c, ctx->sm_count, s, (int)r0, bad);
+        });
+        if (st != MGX_NO_MEMORY) return st;
+    }
+    return dgemm(g, ctx->sm_count, s);
 }
 
 /* ------------------------------------------------------------------ */
@@ -496,115 +559,157 @@ int psi_theta_cuda_cores(mgx_ctx* ctx, int kind, const void* psi, size_t ld, siz
     return cores(0, npts, nullptr);
 }
 
-/* ProjectedMatrices::updateTheta (src/ProjectedMatrices.h:218-225):
- * theta = Sinv H with Sinv symmetric, read from its lower triangle. */
-int theta_product(int n, const double* Sinv, const double* H, double* theta,
-    cudaStream_t s)
-{
-    if (n <= 0 || !Sinv || !H || !theta) return fail(MGX_BAD_ARG, "theta: bad arguments");
-    return dgemm(false, false, n, n, n, 1., Sinv, n, H, n, 0., theta, n, 0, s, 1);
-}
-
 /* ------------------------------------------------------------------ */
 /* Cholesky                                                             */
 /* ------------------------------------------------------------------ */
-constexpr int NB        = 64;
+constexpr int NB        = 64;  // diagonal blocks, factored and inverted by one CTA
+constexpr int OB        = 256; // blocks of the products between them
 constexpr int DIAG_SMEM = 2 * NB * (NB + 1) * sizeof(double);
+
+/* 1 / d to the last bit or two for d of exponent -1020 .. 1020: an FP32
+ * reciprocal of the leading mantissa bits and one cubic Newton step.  Three
+ * FP64 operations: each occupies its SM's FP64 unit for 16 clocks per warp, and
+ * the division this replaces stood on the critical path of every column. */
+__device__ __forceinline__ bool reciprocal_ok(double d)
+{
+    const int hi = __double2hiint(d); // positive, no extreme exponent
+    return hi >= 0x00300000 && hi < 0x7fb00000;
+}
+__device__ __forceinline__ double reciprocal(double d)
+{
+    const int hi   = __double2hiint(d), lo = __double2loint(d);
+    const double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, lo); // [1, 2)
+    const unsigned t
+        = __float_as_uint(__frcp_rn(__uint_as_float(0x3f800000u | ((hi & 0xfffff) << 3) | ((unsigned)lo >> 29))));
+    const double r = __hiloint2double((int)(t >> 3) + ((1023 - 127) << 20), (int)(t << 29));
+    const double e = fma(-m, r, 1.);
+    const double q = fma(r, fma(e, e, e), r); // in (1/2, 1]
+    return __hiloint2double(__double2hiint(q) - (((hi >> 20) - 1023) << 20), __double2loint(q));
+}
 
 /* Factor the diagonal block A[k0:k0+nb, k0:k0+nb] (lower), write L_kk in
  * place (upper part zeroed) and its inverse W (nb x nb, column-major, ld
  * NB) to `winv`.  Sets *info to the 1-based global pivot index on failure.
- * Right-looking by columns, the column scaled by the reciprocal of its
- * pivot (as LAPACK's dpotf2 scales); the trailing update has a thread per
- * column of the block and four row groups.  The inverse is formed row by
- * row, W(i, c) = -W(i, i) sum_{c <= q < i} L(i, q) W(q, c), four threads per
- * column summing a quarter of each dot product. */
+ *
+ * One sweep over the columns factors and inverts: with A = G D G^T, G unit
+ * lower, column j takes G(i, j) = u_i / d_j times row j of [G^-1 | A] from
+ * each row i > j, in one array whose columns before j already hold G^-1 and
+ * the others what is left of A (in-place Gauss-Jordan).  L = G D^1/2 and W =
+ * D^-1/2 G^-1 are scaled at the end, all columns at once.  Eight warps: two
+ * column halves x four row groups, a lane per column, so that all four FP64
+ * units work; the warp that updates the next pivot forms its reciprocal
+ * before its other rows, so that the others need not wait for it.  Bound by
+ * the FP64 units of its SM (175 k multiply-adds at 2 per clock would be 23 us
+ * at 64). */
 __global__ void __launch_bounds__(256) potrf_diag_kernel(double* A, int n, int k0,
     int nb, double* winv, int* info)
 {
     extern __shared__ double dsm[];
-    double(*L)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(dsm);
-    double(*W)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(dsm + NB * (NB + 1));
-    __shared__ double rdiag[NB];
+    double(*X)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(dsm);
+    double(*U)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(dsm + NB * (NB + 1)); // u columns
+    __shared__ double inv[NB], sq[NB];
     __shared__ int bad;
     if (*info != 0) return;
     const int tid = threadIdx.x;
     for (int e = tid; e < NB * NB; e += blockDim.x)
     {
         const int i = e % NB, j = e / NB;
-        L[i][j]     = (i >= j && i < nb && j < nb) ? A[(size_t)(k0 + j) * n + k0 + i] : 0.;
-        W[i][j]     = 0.;
+        const double v = (i >= j && i < nb && j < nb) ? A[(size_t)(k0 + j) * n + k0 + i] : 0.;
+        X[i][j]        = v;
+        if (j == 0) U[i][0] = v;
     }
     if (tid == 0) bad = 0;
     __syncthreads();
-    const int cl = tid & 63, rg = tid >> 6;
+    // the pivot d of column j: its reciprocal, or -1 for a failure
+    auto pivot = [&](int j, double d) {
+        if (reciprocal_ok(d))
+            inv[j] = reciprocal(d);
+        else if (d > 0. && isfinite(d))
+            inv[j] = 1. / d;
+        else
+        {
+            inv[j] = -1.;
+            bad    = k0 + j + 1;
+        }
+    };
+    if (tid == 0) pivot(0, X[0][0]);
+    __syncthreads();
+    const int warp = tid / 32, lane = tid & 31;
+    const int half = warp >> 2, wr = warp & 3;
+    const int c = 32 * half + lane;
     for (int j = 0; j < nb; j++)
     {
-        if (tid == 0)
+        if (__double2hiint(inv[j]) < 0) break;
+        // row j of [G^-1 | A] over d_j at this lane's column
+        const double v = (c < j ? X[j][c] : c == j ? 1. : U[c][j]) * inv[j];
+        // its rows from the diagonal down, the first of all with the pivot, the
+        // others four at a time (the loads of four before the first store)
+        int i = j + 1 + wr;
+        if (wr == 0 && i < nb)
         {
-            const double d = L[j][j];
-            if (!(d > 0.) || !isfinite(d))
-                bad = k0 + j + 1;
-            else
+            if (i >= 32 * half)
             {
-                const double sq = sqrt(d);
-                L[j][j]         = sq;
-                rdiag[j]        = 1. / sq;
+                const double x = (c == j ? 0. : X[i][c]) - U[i][j] * v;
+                if (c <= i) X[i][c] = x;
+                if (c == j + 1) U[i][j + 1] = x;
+                if (half == (i >> 5))
+                {
+                    const double d = __shfl_sync(0xffffffffu, x, i & 31);
+                    if (lane == 0) pivot(i, d);
+                }
+            }
+            i += 4;
+        }
+        if (i < 32 * half) i += (32 * half - i + 3) / 4 * 4; // columns past the diagonal
+        for (; i < nb; i += 16)
+        {
+            double x[4], u[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+            {
+                const int r = min(i + 4 * q, nb - 1);
+                x[q]        = X[r][c];
+                u[q]        = U[r][j];
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+            {
+                const int r = i + 4 * q;
+                if (r >= nb) break;
+                const double y = (c == j ? 0. : x[q]) - u[q] * v;
+                if (c <= r) X[r][c] = y;
+                if (c == j + 1) U[r][j + 1] = y;
             }
         }
         __syncthreads();
-        if (bad) break;
-        const double r = rdiag[j];
-        for (int i = j + 1 + tid; i < nb; i += blockDim.x)
-            L[i][j] *= r;
-        __syncthreads();
-        // trailing update of the block: column c, rows i >= c
-        const int c = j + 1 + cl;
-        if (c < nb)
-        {
-            const double lcj = L[c][j];
-            for (int i = j + 1 + rg; i < nb; i += 4)
-                if (i >= c) L[i][c] -= L[i][j] * lcj;
-        }
-        __syncthreads();
     }
-    if (bad)
+    if (bad) // set before the last barrier that every thread has passed
     {
         if (tid == 0) atomicCAS(info, 0, bad);
         return;
     }
     for (int i = tid; i < nb; i += blockDim.x)
-        W[i][i] = rdiag[i];
-    __syncthreads();
     {
-        const int c = tid >> 2, part = tid & 3;
-        for (int i = 1; i < nb; i++)
-        {
-            double sum = 0.;
-            if (c < i)
-                for (int q = c + part; q < i; q += 4)
-                    sum += L[i][q] * W[q][c];
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            if (c < i && part == 0) W[i][c] = -rdiag[i] * sum;
-            __syncthreads();
-        }
+        const double r = sqrt(U[i][i]);
+        sq[i]          = r;
+        inv[i]         = 1. / r;
     }
+    __syncthreads();
     for (int e = tid; e < nb * nb; e += blockDim.x)
     {
         const int i = e % nb, j = e / nb;
-        A[(size_t)(k0 + j) * n + k0 + i] = (i >= j) ? L[i][j] : 0.;
-        winv[(size_t)j * NB + i]         = W[i][j];
+        A[(size_t)(k0 + j) * n + k0 + i] = i > j ? U[i][j] * inv[j] : i == j ? sq[i] : 0.;
+        winv[(size_t)j * NB + i]         = i > j ? X[i][j] * inv[i] : i == j ? inv[i] : 0.;
     }
 }
 
-/* The panel of a Cholesky step in place: rows [k0 + nb, n) of columns
+/* The panel of a Cholesky step in place: rows [k0 + nb, rend) of columns
  * k0 .. k0+nb of A (column-major, leading dimension n) become
  * A_panel W^T, W = L_kk^-1 (lower, column-major, leading dimension NB):
  * the L_ik = A_ik L_kk^-T of the blocked algorithm.  16 rows per CTA. */
 constexpr int PANEL_ROWS = 16;
 
-__global__ void __launch_bounds__(256) panel_trsm_kernel(double* A, int n, int k0, int nb,
+__global__ void __launch_bounds__(256) panel_trsm_kernel(double* A, int n, int k0, int nb, int rend,
     const double* __restrict__ winv)
 {
     __shared__ double Ws[NB][NB + 1];
@@ -619,7 +724,7 @@ __global__ void __launch_bounds__(256) panel_trsm_kernel(double* A, int n, int k
     for (int e = tid; e < PANEL_ROWS * NB; e += blockDim.x)
     {
         const int rr = e % PANEL_ROWS, q = e / PANEL_ROWS;
-        As[rr][q]    = (q < nb && r0 + rr < n) ? A[(size_t)(k0 + q) * n + r0 + rr] : 0.;
+        As[rr][q]    = (q < nb && r0 + rr < rend) ? A[(size_t)(k0 + q) * n + r0 + rr] : 0.;
     }
     __syncthreads();
     const int rr = tid % PANEL_ROWS;
@@ -628,7 +733,7 @@ __global__ void __launch_bounds__(256) panel_trsm_kernel(double* A, int n, int k
         double acc = 0.;
         for (int q = 0; q <= c; q++)
             acc += As[rr][q] * Ws[c][q];
-        if (r0 + rr < n) A[(size_t)(k0 + c) * n + r0 + rr] = acc;
+        if (r0 + rr < rend) A[(size_t)(k0 + c) * n + r0 + rr] = acc;
     }
 }
 
@@ -643,6 +748,13 @@ __global__ void copy_panel_kernel(const double* src, int lds, double* dst,
     }
 }
 
+static int copy_panel(const double* src, int lds, double* dst, int ldd, int m, int n, cudaStream_t s)
+{
+    copy_panel_kernel<<<std::min(1024, (m * n + 255) / 256), 256, 0, s>>>(src, lds, dst, ldd, m, n);
+    MGX_LAUNCH_CHECK("copy_panel_kernel");
+    return MGX_OK;
+}
+
 __global__ void zero_upper_kernel(double* A, int n)
 {
     const size_t nn = (size_t)n * n;
@@ -654,53 +766,127 @@ __global__ void zero_upper_kernel(double* A, int n)
     }
 }
 
-/* workspace: diagonal inverses (nblocks x NB x NB) + panel (n x NB) + X */
-static int dense_ws(mgx_ctx* ctx, int n, double** winv, double** panel,
-    double** X, int** info)
+/* copies the NB x NB inverses of a block's diagonal (packed, leading
+ * dimension NB) to the diagonal of W (leading dimension OB) */
+__global__ void place_diag_kernel(const double* __restrict__ winv, double* __restrict__ W, int kb)
 {
-    const int nbk = (n + NB - 1) / NB;
-    const size_t b_w = (size_t)nbk * NB * NB * 8, b_p = (size_t)n * NB * 8,
+    const int k0 = blockIdx.x * NB, nb = min(NB, kb - k0);
+    for (int e = threadIdx.x; e < nb * nb; e += blockDim.x)
+    {
+        const int i = e % nb, j = e / nb;
+        W[(size_t)(k0 + j) * OB + k0 + i] = winv[(size_t)k0 * NB + (size_t)j * NB + i];
+    }
+}
+
+/* workspace: diagonal inverses (nblocks x NB x NB), OB x OB inverses, a panel
+ * (n x OB) and an n x n matrix */
+struct DenseWs
+{
+    double *winv, *wob, *panel, *X;
+    int* info;
+};
+
+static int dense_ws(mgx_ctx* ctx, int n, DenseWs* w)
+{
+    const size_t nbk = (n + NB - 1) / NB, nob = (n + OB - 1) / OB;
+    const size_t b_w = nbk * NB * NB * 8, b_o = nob * OB * OB * 8, b_p = (size_t)n * OB * 8,
                  b_x = (size_t)n * n * 8;
-    MGX_TRY(ctx->dense_ws.ensure(b_w + b_p + b_x + 256));
+    MGX_TRY(ctx->dense_ws.ensure(b_w + b_o + b_p + b_x + 256));
     char* base = (char*)ctx->dense_ws.ptr;
-    *winv      = (double*)base;
-    *panel     = (double*)(base + b_w);
-    *X         = (double*)(base + b_w + b_p);
-    *info      = (int*)(base + b_w + b_p + b_x);
+    w->winv    = (double*)base;
+    w->wob     = (double*)(base + b_w);
+    w->panel   = (double*)(base + b_w + b_o);
+    w->X       = (double*)(base + b_w + b_o + b_p);
+    w->info    = (int*)(base + b_w + b_o + b_p + b_x);
+    return MGX_OK;
+}
+
+/* W (leading dimension ldw, lower) holds the inverses of L's diagonal blocks
+ * of `step` rows; on return those of 2 step, for `batch` matrices of kb rows
+ * at strides sL and sW: the block below the first inverse W1 of a pair is
+ * -W2 (L21 W1), T a scratch of (step x step) per product at stride sT */
+static int merge_inverses(mgx_ctx* ctx, int kb, int step, const double* L, int ldl, double* W,
+    int ldw, double* T, int batch, size_t sL, size_t sW, size_t sT, cudaStream_t s)
+{
+    for (int o = 0; o + step < kb; o += 2 * step)
+    {
+        const int m = std::min(step, kb - o - step);
+        Gemm g{ false, false, m, step, step, 1., L + (size_t)o * ldl + o + step, ldl,
+            W + (size_t)o * ldw + o, ldw, 0., T, m };
+        g.batch = batch;
+        g.sA    = sL;
+        g.sB    = sW;
+        g.sC    = sT;
+        MGX_TRY(gemm(ctx, g, s));
+        Gemm h{ false, false, m, step, m, -1., W + (size_t)(o + step) * ldw + o + step, ldw, T, m,
+            0., W + (size_t)o * ldw + o + step, ldw };
+        h.batch = batch;
+        h.sA    = sW;
+        h.sB    = sT;
+        h.sC    = sW;
+        MGX_TRY(gemm(ctx, h, s));
+    }
+    return MGX_OK;
+}
+
+/* the OB x OB inverse of one diagonal block of kb rows from its NB x NB ones */
+static int block_inverse(mgx_ctx* ctx, int kb, const double* L, int n, const double* winv,
+    double* W, double* T, cudaStream_t s)
+{
+    MGX_TRY(cuda_check(cudaMemsetAsync(W, 0, sizeof(double) * OB * OB, s), "block inverse reset"));
+    place_diag_kernel<<<(kb + NB - 1) / NB, 256, 0, s>>>(winv, W, kb);
+    MGX_LAUNCH_CHECK("place_diag_kernel");
+    for (int step = NB; step < kb; step *= 2)
+        MGX_TRY(merge_inverses(ctx, kb, step, L, n, W, OB, T, 1, 0, 0, 0, s));
     return MGX_OK;
 }
 
 /* info_host set: synchronous, *info_host receives the pivot index; else
- * info_dev (device) receives it and nothing waits for the factorization */
+ * info_dev (device) receives it and nothing waits for the factorization.
+ * Blocks of OB columns: their diagonal block by NB columns on the FP64 units,
+ * then the panel below it, A W^T with the block's inverse W, and the trailing
+ * update, both products of OB values that the tensor cores form from slices */
 int cholesky(mgx_ctx* ctx, int n, double* A, int* info_host, cudaStream_t s,
     int* info_dev = nullptr)
 {
     if (n <= 0 || !A || (!info_host && !info_dev))
         return fail(MGX_BAD_ARG, "cholesky: bad arguments");
-    double *winv, *panel, *X;
-    int* dinfo;
-    MGX_TRY(dense_ws(ctx, n, &winv, &panel, &X, &dinfo));
-    if (info_dev) dinfo = info_dev;
+    DenseWs w;
+    MGX_TRY(dense_ws(ctx, n, &w));
+    int* dinfo = info_dev ? info_dev : w.info;
     MGX_TRY(cuda_check(cudaMemsetAsync(dinfo, 0, sizeof(int), s), "info reset"));
     MGX_TRY(cuda_check(cudaFuncSetAttribute(potrf_diag_kernel,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, DIAG_SMEM),
         "potrf smem attribute"));
-    const int nbk = (n + NB - 1) / NB;
-    for (int kb = 0; kb < nbk; kb++)
+    for (int o = 0; o < n; o += OB)
     {
-        const int k0 = kb * NB, nb = std::min(NB, n - k0);
-        potrf_diag_kernel<<<1, 256, DIAG_SMEM, s>>>(A, n, k0, nb, winv + (size_t)kb * NB * NB, dinfo);
-        MGX_LAUNCH_CHECK("potrf_diag_kernel");
-        const int m = n - k0 - nb; // rows below the block
+        const int kb = std::min(OB, n - o), end = o + kb;
+        for (int k0 = o; k0 < end; k0 += NB)
+        {
+            const int nb = std::min(NB, end - k0);
+            double* wk   = w.winv + (size_t)k0 * NB;
+            potrf_diag_kernel<<<1, 256, DIAG_SMEM, s>>>(A, n, k0, nb, wk, dinfo);
+            MGX_LAUNCH_CHECK("potrf_diag_kernel");
+            const int m = end - k0 - nb; // rows below, in this block
+            if (m <= 0) continue;
+            panel_trsm_kernel<<<(m + PANEL_ROWS - 1) / PANEL_ROWS, 256, 0, s>>>(A, n, k0, nb, end, wk);
+            MGX_LAUNCH_CHECK("panel_trsm_kernel");
+            const double* P = A + (size_t)k0 * n + k0 + nb;
+            Gemm g{ false, true, m, m, nb, -1., P, n, P, n, 1.,
+                A + (size_t)(k0 + nb) * n + k0 + nb, n };
+            g.lower = 1;
+            MGX_TRY(gemm(ctx, g, s));
+        }
+        const int m = n - end;
         if (m <= 0) continue;
-        double* Ap = A + (size_t)k0 * n + k0 + nb; // panel A[k0+nb:, k0:k0+nb]
-        // panel <- A_panel * W^T   (L_ik = A_ik L_kk^-T), in place
-        panel_trsm_kernel<<<(m + PANEL_ROWS - 1) / PANEL_ROWS, 256, 0, s>>>(A, n, k0, nb,
-            winv + (size_t)kb * NB * NB);
-        MGX_LAUNCH_CHECK("panel_trsm_kernel");
-        // trailing update A22 -= P P^T (lower)
-        double* A22 = A + (size_t)(k0 + nb) * n + k0 + nb;
-        MGX_TRY(dgemm(false, true, m, m, nb, -1., Ap, n, Ap, n, 1., A22, n, 1, s));
+        double* P = A + (size_t)o * n + end;
+        double* W = w.wob;
+        MGX_TRY(block_inverse(ctx, kb, A + (size_t)o * n + o, n, w.winv + (size_t)o * NB, W, w.X, s));
+        MGX_TRY(gemm(ctx, Gemm{ false, true, m, kb, kb, 1., P, n, W, OB, 0., w.panel, m }, s));
+        MGX_TRY(copy_panel(w.panel, m, P, n, m, kb, s));
+        Gemm g{ false, true, m, m, kb, -1., P, n, P, n, 1., A + (size_t)end * n + end, n };
+        g.lower = 1;
+        MGX_TRY(gemm(ctx, g, s));
     }
     zero_upper_kernel<<<std::min<size_t>(((size_t)n * n + 255) / 256, 4096), 256, 0, s>>>(A, n);
     MGX_LAUNCH_CHECK("zero_upper_kernel");
@@ -714,133 +900,171 @@ int cholesky(mgx_ctx* ctx, int n, double* A, int* info_host, cudaStream_t s,
     return MGX_OK;
 }
 
-/* inverse of a lower-triangular factor, blocked by rows:
- * X_ii = L_ii^-1 ; X_i,0:i = -X_ii (L_i,0:i X_0:i,0:i) */
+/* inverses of the NB x NB diagonal blocks of a lower-triangular factor, one
+ * CTA each, into the diagonal of X (leading dimension ldx; with stride > 0 the
+ * blocks of each OB rows go to X + stride * (row / OB)).  Column by column on
+ * all rows below, a lane per column (as potrf_diag_kernel does). */
 __global__ void __launch_bounds__(256) trinv_diag_kernel(const double* L, int n,
-    double* X)
+    double* X, int ldx, size_t stride)
 {
     extern __shared__ double dsm[];
     double(*T)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(dsm);
     double(*W)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(dsm + NB * (NB + 1));
-    const int kb = blockIdx.x, k0 = kb * NB, nb = min(NB, n - k0);
+    __shared__ double inv[NB];
+    const int k0 = blockIdx.x * NB, nb = min(NB, n - k0);
     const int tid = threadIdx.x;
     for (int e = tid; e < nb * nb; e += blockDim.x)
     {
         const int i = e % nb, j = e / nb;
         T[i][j]     = (i >= j) ? L[(size_t)(k0 + j) * n + k0 + i] : 0.;
-        W[i][j]     = 0.;
+        W[i][j]     = i == j ? 1. : 0.;
     }
     __syncthreads();
-    // row by row as in potrf_diag_kernel: W(i, c) = -W(i, i) sum_{c <= q < i}
-    // T(i, q) W(q, c), four threads per column
     for (int i = tid; i < nb; i += blockDim.x)
-        W[i][i] = 1. / T[i][i];
+        inv[i] = 1. / T[i][i];
     __syncthreads();
+    const int warp = tid / 32, lane = tid & 31;
+    const int half = warp >> 2, wr = warp & 3;
+    const int c = 32 * half + lane;
+    for (int j = 0; j < nb; j++)
     {
-        const int c = tid >> 2, part = tid & 3;
-        for (int i = 1; i < nb; i++)
+        // row j is final but for its factor; the rows below lose T(i, j) of it
+        if (32 * half <= j && c < nb)
         {
-            double sum = 0.;
-            if (c < i)
-                for (int q = c + part; q < i; q += 4)
-                    sum += T[i][q] * W[q][c];
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            if (c < i && part == 0) W[i][c] = -W[i][i] * sum;
-            __syncthreads();
+            const double v = W[j][c] * inv[j];
+            for (int i = j + 1 + wr; i < nb; i += 16)
+            {
+                double x[4], t[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                {
+                    const int r = min(i + 4 * q, nb - 1);
+                    x[q]        = W[r][c];
+                    t[q]        = T[r][j];
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (i + 4 * q < nb && c <= j) W[i + 4 * q][c] = x[q] - t[q] * v;
+            }
         }
+        __syncthreads();
     }
+    double* out = X + (stride ? stride * (k0 / OB) : 0);
+    const int q = stride ? k0 % OB : k0;
     for (int e = tid; e < nb * nb; e += blockDim.x)
     {
         const int i = e % nb, j = e / nb;
-        X[(size_t)(k0 + j) * n + k0 + i] = W[i][j];
+        out[(size_t)(q + j) * ldx + q + i] = i >= j ? W[i][j] * inv[i] : 0.;
     }
 }
 
-/* forward substitution L Y = B in place on Y (n x ncols, leading dimension
- * n), with the inverses of L's diagonal blocks in the diagonal blocks of
- * X: per 64-row block, Y_k <- W_k Y_k through the panel, then the rows
- * below lose L[below, k] Y_k (one (n - k) x ncols x 64 product, parallel
- * over all of Y's columns) */
-static int forward_subst(int n, const double* L, const double* X, double* Y, int ncols,
-    double* panel, cudaStream_t s, bool lower_rhs = false)
+static int diag_inverses(int n, const double* L, double* X, int ldx, size_t stride, cudaStream_t s)
 {
-    const int nbk = (n + NB - 1) / NB;
-    for (int kb = 0; kb < nbk; kb++)
+    MGX_TRY(cuda_check(cudaFuncSetAttribute(trinv_diag_kernel,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, DIAG_SMEM),
+        "trinv smem attribute"));
+    trinv_diag_kernel<<<(n + NB - 1) / NB, 256, DIAG_SMEM, s>>>(L, n, X, ldx, stride);
+    MGX_LAUNCH_CHECK("trinv_diag_kernel");
+    return MGX_OK;
+}
+
+/* the inverses of L's OB x OB diagonal blocks into w.wob (leading dimension
+ * OB), all full blocks in batches */
+static int ob_inverses(mgx_ctx* ctx, int n, const double* L, const DenseWs& w, cudaStream_t s)
+{
+    const size_t so = (size_t)OB * OB;
+    const int full = n / OB, rest = n - full * OB, nob = full + (rest ? 1 : 0);
+    MGX_TRY(cuda_check(cudaMemsetAsync(w.wob, 0, nob * so * sizeof(double), s), "inverses reset"));
+    MGX_TRY(diag_inverses(n, L, w.wob, OB, so, s));
+    for (int step = NB; step < OB; step *= 2)
     {
-        const int k0 = kb * NB, nb = std::min(NB, n - k0);
-        // a lower-triangular right-hand side (the identity) keeps Y lower
-        // triangular: columns past this block row are still zero
-        const int nc = lower_rhs ? std::min(ncols, k0 + nb) : ncols;
-        MGX_TRY(dgemm(false, false, nb, nc, nb, 1., X + (size_t)k0 * n + k0, n, Y + k0, n,
-            0., panel, NB, 0, s));
-        copy_panel_kernel<<<std::min(1024, (nb * nc + 255) / 256), 256, 0, s>>>(panel, NB,
-            Y + k0, n, nb, nc);
-        MGX_LAUNCH_CHECK("copy_panel_kernel");
-        const int m = n - k0 - nb;
-        if (m > 0)
-            MGX_TRY(dgemm(false, false, m, nc, nb, -1., L + (size_t)k0 * n + k0 + nb, n,
-                Y + k0, n, 1., Y + k0 + nb, n, 0, s));
+        if (full)
+            MGX_TRY(merge_inverses(ctx, OB, step, L, n, w.wob, OB, w.panel, full,
+                (size_t)OB * n + OB, so, (size_t)step * step, s));
+        if (step < rest)
+            MGX_TRY(merge_inverses(ctx, rest, step, L + (size_t)full * OB * (n + 1), n,
+                w.wob + full * so, OB, w.panel, 1, 0, 0, 0, s));
     }
     return MGX_OK;
 }
 
-// upper triangle <- lower triangle
-__global__ void mirror_lower_kernel(double* A, int n)
+// upper triangle <- lower triangle (of src, into dst; they may be the same)
+__global__ void mirror_lower_kernel(const double* src, double* dst, int n)
 {
     const size_t nn = (size_t)n * n;
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < nn;
          t += (size_t)gridDim.x * blockDim.x)
     {
         const size_t i = t % n, j = t / n;
-        if (i < j) A[t] = A[i * n + j];
+        if (i < j)
+            dst[t] = src[i * n + j];
+        else if (src != dst)
+            dst[t] = src[t];
     }
 }
 
-__global__ void identity_kernel(double* X, int n)
+static int mirror_lower(const double* src, double* dst, int n, cudaStream_t s)
 {
-    const size_t nn = (size_t)n * n;
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < nn;
-         t += (size_t)gridDim.x * blockDim.x)
-        X[t] = ((t % n) == (t / n)) ? 1. : 0.;
+    const int nb = (int)std::min<size_t>(((size_t)n * n + 255) / 256, 4096);
+    mirror_lower_kernel<<<nb, 256, 0, s>>>(src, dst, n);
+    MGX_LAUNCH_CHECK("mirror_lower_kernel");
+    return MGX_OK;
 }
 
-/* Sinv = (L L^T)^-1 = X^T X with X = L^-1 formed by forward substitution
- * on the identity (parallel over its n columns), then one product. */
+/* S M for a symmetric S of which the lower triangle is read (BLAS symm 'l',
+ * 'l') */
+static int symm(mgx_ctx* ctx, int n, const double* S, const double* M, double* out, cudaStream_t s)
+{
+    DenseWs w;
+    MGX_TRY(dense_ws(ctx, n, &w));
+    MGX_TRY(mirror_lower(S, w.X, n, s));
+    // S = S^T: read along the columns, the values of k
+    return gemm(ctx, Gemm{ true, false, n, n, n, 1., w.X, n, M, n, 0., out, n }, s);
+}
+
+/* ProjectedMatrices::updateTheta (src/ProjectedMatrices.h:218-225):
+ * theta = Sinv H with Sinv symmetric, read from its lower triangle. */
+int theta_product(mgx_ctx* ctx, int n, const double* Sinv, const double* H, double* theta,
+    cudaStream_t s)
+{
+    if (n <= 0 || !Sinv || !H || !theta) return fail(MGX_BAD_ARG, "theta: bad arguments");
+    return symm(ctx, n, Sinv, H, theta, s);
+}
+
+/* Sinv = (L L^T)^-1 = X^T X with X = L^-1, whose diagonal blocks are inverted
+ * and merged in pairs until one is left. */
 int inverse_from_cholesky(mgx_ctx* ctx, int n, const double* L, double* Sinv,
     cudaStream_t s)
 {
     if (n <= 0 || !L || !Sinv) return fail(MGX_BAD_ARG, "inverse: bad arguments");
     if (Sinv == L) return fail(MGX_BAD_ARG, "inverse: Sinv aliases L");
-    double *winv, *panel, *X;
-    int* dinfo;
-    MGX_TRY(dense_ws(ctx, n, &winv, &panel, &X, &dinfo));
-    const int nbk = (n + NB - 1) / NB;
-    MGX_TRY(cuda_check(cudaFuncSetAttribute(trinv_diag_kernel,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, DIAG_SMEM),
-        "trinv smem attribute"));
-    // inverses of the diagonal blocks into X, then Y = I in Sinv, solved
-    trinv_diag_kernel<<<nbk, 256, DIAG_SMEM, s>>>(L, n, X);
-    MGX_LAUNCH_CHECK("trinv_diag_kernel");
-    const int nb = (int)std::min<size_t>(((size_t)n * n + 255) / 256, 4096);
-    identity_kernel<<<nb, 256, 0, s>>>(Sinv, n);
-    MGX_LAUNCH_CHECK("identity_kernel");
-    MGX_TRY(forward_subst(n, L, X, Sinv, n, panel, s, true));
-    // X <- L^-1, then the lower triangle of S^-1 = X^T X, mirrored
-    MGX_TRY(cuda_check(cudaMemcpyAsync(X, Sinv, (size_t)n * n * 8, cudaMemcpyDeviceToDevice, s),
-        "L^-1 copy"));
-    MGX_TRY(dgemm(true, false, n, n, n, 1., X, n, X, n, 0., Sinv, n, 1, s));
-    mirror_lower_kernel<<<nb, 256, 0, s>>>(Sinv, n);
-    MGX_LAUNCH_CHECK("mirror_lower_kernel");
-    return MGX_OK;
+    DenseWs w;
+    MGX_TRY(dense_ws(ctx, n, &w));
+    MGX_TRY(cuda_check(cudaMemsetAsync(w.X, 0, (size_t)n * n * 8, s), "inverse reset"));
+    MGX_TRY(diag_inverses(n, L, w.X, n, 0, s));
+    for (int step = NB; step < n; step *= 2)
+    {
+        // the full pairs of small blocks in one batch each
+        const int pairs = step < OB ? n / (2 * step) : 0, done = pairs * 2 * step;
+        if (pairs)
+            MGX_TRY(merge_inverses(ctx, 2 * step, step, L, n, w.X, n, Sinv, pairs,
+                (size_t)2 * step * (n + 1), (size_t)2 * step * (n + 1), (size_t)step * step, s));
+        MGX_TRY(merge_inverses(ctx, n - done, step, L + (size_t)done * (n + 1), n,
+            w.X + (size_t)done * (n + 1), n, Sinv, 1, 0, 0, 0, s));
+    }
+    // the lower triangle of S^-1 = X^T X, mirrored
+    Gemm g{ true, false, n, n, n, 1., w.X, n, w.X, n, 0., Sinv, n };
+    g.lower = 1;
+    MGX_TRY(gemm(ctx, g, s));
+    return mirror_lower(Sinv, Sinv, n, s);
 }
 
 /* theta = S^-1 H = L^-T (L^-1 H) from the Cholesky factor L, without
  * forming S^-1: blocked forward substitution L Y = H and back substitution
- * L^T theta = Y with the n columns of H as right-hand sides.  The diagonal
- * blocks are applied through their inverses (trinv_diag_kernel); the
- * off-diagonal updates are (n - k) x n x 64 products with full-width
- * parallelism.  2 n^3 flop instead of the n^3 / 3 + 2 n^3 + 2 n^3 of
+ * L^T theta = Y with the n columns of H as right-hand sides.  The OB x OB
+ * diagonal blocks are applied through their inverses; the off-diagonal
+ * updates are (n - k) x n x OB products, from slices on the tensor cores.
+ * 2 n^3 flop instead of the n^3 / 3 + 2 n^3 + 2 n^3 of
  * computeInverse followed by updateTheta (src/GramMatrix.cc:75-91,
  * src/ProjectedMatrices.h:218-225).  trace (device, may be NULL) receives
  * tr(theta) = tr(S^-1 H). */
@@ -865,36 +1089,35 @@ int theta_from_cholesky(mgx_ctx* ctx, int n, const double* L, const double* H,
 {
     if (n <= 0 || !L || !H || !theta) return fail(MGX_BAD_ARG, "theta: bad arguments");
     if (theta == H || theta == L) return fail(MGX_BAD_ARG, "theta aliases an input");
-    double *winv, *panel, *X;
-    int* dinfo;
-    MGX_TRY(dense_ws(ctx, n, &winv, &panel, &X, &dinfo));
-    const int nbk = (n + NB - 1) / NB;
-    MGX_TRY(cuda_check(cudaFuncSetAttribute(trinv_diag_kernel,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, DIAG_SMEM),
-        "trinv smem attribute"));
-    trinv_diag_kernel<<<nbk, 256, DIAG_SMEM, s>>>(L, n, X);
-    MGX_LAUNCH_CHECK("trinv_diag_kernel");
+    DenseWs w;
+    MGX_TRY(dense_ws(ctx, n, &w));
+    MGX_TRY(ob_inverses(ctx, n, L, w, s));
     MGX_TRY(cuda_check(cudaMemcpyAsync(theta, H, (size_t)n * n * 8, cudaMemcpyDeviceToDevice, s),
         "theta init"));
-    auto apply_diag = [&](int k0, int nb, bool transpose) -> int {
-        // rows k0..k0+nb of theta <- W^(T) * rows k0..k0+nb, through the panel
-        MGX_TRY(dgemm(transpose, false, nb, n, nb, 1., X + (size_t)k0 * n + k0, n, theta + k0,
-            n, 0., panel, NB, 0, s));
-        copy_panel_kernel<<<std::min(1024, (nb * n + 255) / 256), 256, 0, s>>>(panel, NB,
-            theta + k0, n, nb, n);
-        MGX_LAUNCH_CHECK("copy_panel_kernel");
-        return MGX_OK;
+    // rows o .. o + kb of theta <- W^(T) times them, through the panel
+    auto apply_diag = [&](int o, int kb, bool transpose) -> int {
+        MGX_TRY(gemm(ctx, Gemm{ transpose, false, kb, n, kb, 1., w.wob + (size_t)(o / OB) * OB * OB,
+                              OB, theta + o, n, 0., w.panel, kb }, s));
+        return copy_panel(w.panel, kb, theta + o, n, kb, n, s);
     };
+    const int nob = (n + OB - 1) / OB;
     // forward: L Y = H
-    MGX_TRY(forward_subst(n, L, X, theta, n, panel, s));
-    // backward: L^T theta = Y
-    for (int kb = nbk - 1; kb >= 0; kb--)
+    for (int b = 0; b < nob; b++)
     {
-        const int k0 = kb * NB, nb = std::min(NB, n - k0);
-        MGX_TRY(apply_diag(k0, nb, true));
-        if (k0 > 0)
-            MGX_TRY(dgemm(true, false, k0, n, nb, -1., L + k0, n, theta + k0, n, 1., theta, n,
-                0, s));
+        const int o = b * OB, kb = std::min(OB, n - o), m = n - o - kb;
+        MGX_TRY(apply_diag(o, kb, false));
+        if (m > 0)
+            MGX_TRY(gemm(ctx, Gemm{ false, false, m, n, kb, -1., L + (size_t)o * n + o + kb, n,
+                                  theta + o, n, 1., theta + o + kb, n }, s));
+    }
+    // backward: L^T theta = Y
+    for (int b = nob - 1; b >= 0; b--)
+    {
+        const int o = b * OB, kb = std::min(OB, n - o);
+        MGX_TRY(apply_diag(o, kb, true));
+        if (o > 0)
+            MGX_TRY(gemm(ctx, Gemm{ true, false, o, n, kb, -1., L + o, n, theta + o, n, 1., theta, n },
+                s));
     }
     if (trace)
     {
@@ -981,11 +1204,11 @@ __global__ void sym_average_kernel(double* A, int n)
     }
 }
 
-int update_hb(int n, const double* S, const double* theta, double* HB, cudaStream_t s)
+int update_hb(mgx_ctx* ctx, int n, const double* S, const double* theta, double* HB, cudaStream_t s)
 {
     if (n <= 0 || !S || !theta || !HB) return fail(MGX_BAD_ARG, "updateHB: bad arguments");
     if (HB == S || HB == theta) return fail(MGX_BAD_ARG, "HB aliases an input");
-    MGX_TRY(dgemm(false, false, n, n, n, 1., S, n, theta, n, 0., HB, n, 0, s, 1));
+    MGX_TRY(symm(ctx, n, S, theta, HB, s));
     const int nb = (int)std::min<size_t>(((size_t)n * n + 255) / 256, 4096);
     sym_average_kernel<<<nb, 256, 0, s>>>(HB, n);
     MGX_LAUNCH_CHECK("sym_average_kernel");

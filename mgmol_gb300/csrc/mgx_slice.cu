@@ -251,6 +251,13 @@ struct Params
     int* err;
 };
 
+/* the first row tile that reaches an entry i >= c */
+__host__ __device__ inline int first_tile(int c, int nti)
+{
+    const int f = c > 0 ? c / BM : 0;
+    return f < nti ? f : nti;
+}
+
 /* item w: its tile and stages.  The tiles of one K range sit side by side in
  * the list, so that CTAs that run together read the same planes. */
 __device__ __forceinline__ void decode(const Params& p, int w, int& ti, int& tj, int& st0, int& nst)
@@ -266,7 +273,7 @@ __device__ __forceinline__ void decode(const Params& p, int w, int& ti, int& tj,
     }
     for (tj = 0; tj < p.ntj; tj++)
     {
-        const int first = min((p.t.col0 + tj * p.bn) / BM, p.nti); // first row tile that counts
+        const int first = first_tile(p.t.col0 + tj * p.bn, p.nti);
         if (tile < p.nti - first)
         {
             ti = first + tile;
@@ -295,14 +302,21 @@ __device__ __forceinline__ void tmem_wait_ld(float (&v)[8])
                  : "memory");
 }
 
-/* T 2^E, exactly where the result is a normal number */
+/* T 2^E rounded to FP64, in integer arithmetic (a conversion would take the
+ * FP64 unit, which the conversions of a tile of few values of K kept busy four
+ * times as long as its MMAs ran); scalbn where the result is not normal */
 __device__ __forceinline__ double scaled(long long T, int E)
 {
-    const double v = (double)T;
-    const int ex   = (__double2hiint(v) >> 20) & 0x7ff;
-    if (T != 0 && (unsigned)(ex + E - 1) < 2045u)
-        return __hiloint2double(__double2hiint(v) + (E << 20), __double2loint(v));
-    return T == 0 ? 0. : scalbn(v, E);
+    if (T == 0) return 0.;
+    const unsigned long long a = T < 0 ? 0ull - (unsigned long long)T : (unsigned long long)T;
+    const int lz               = __clzll(a);
+    const unsigned long long u = a << lz; // leading bit at 63
+    // 53 bits, the leading one of which adds 1 to the exponent field
+    const unsigned long long m = (u >> 11) + ((u >> 10) & 1);
+    const int field            = 1023 + 62 - lz + E;
+    if ((unsigned)(field - 1) >= 2044u) return scalbn((double)T, E);
+    return __longlong_as_double(
+        (long long)(m + ((unsigned long long)field << 52) + (T < 0 ? 1ull << 63 : 0ull)));
 }
 
 /* One CTA per SM walks the items.  Warp 0 streams the slices of both operands
@@ -474,6 +488,12 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
         {
             int ti, tj, st0, nst;
             decode(p, w, ti, tj, st0, nst);
+            // the exponents of this thread's row and of column j0 + lane, fetched
+            // while the MMAs run
+            const size_t i     = (size_t)ti * BM + q * 32 + lane;
+            const long long j0 = (long long)tj * p.bn + c0;
+            const int ei = i < p.m ? key_exponent(p.ka[i]) - 14 - p.w : 0;
+            const int ej = lane < nc && j0 + lane < (long long)p.n ? key_exponent(p.kb[j0 + lane]) : 0;
             // s + t <= 3 in units of 2^-w (NP 2) or 2^-24 of a digit product,
             // and s + t >= 4 in units of 2^-48: in T until the second walk
             // begins (NP 2), or in L
@@ -559,34 +579,52 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                     T[c] = (T[c] << (p.w - 24))
                            + ((L[NP == 1 ? c : 0] + (1ll << (47 - p.w))) >> (48 - p.w));
             }
-            const size_t i  = (size_t)ti * BM + q * 32 + lane;
-            const size_t j0 = (size_t)tj * p.bn + c0;
-            if (i < p.m)
-            {
-                const int ei = key_exponent(p.ka[i]) - 14 - p.w;
+            // entries of this thread: row i, columns j0 .. j0 + nc - 1 that exist
+            // (lower: from the diagonal down)
+            const int cols = i < p.m ? (int)min((long long)nc, (long long)p.n - j0) : 0;
+            const int last = p.t.lower ? (int)min((long long)cols, (long long)i + 1 - j0 - p.t.col0)
+                                       : cols;
 #pragma unroll
-                for (int c = 0; c < EL; c++)
+            for (int c = 0; c < EL; c += 8)
+            {
+                if (c >= nc) break;
+                if (p.t.sum)
                 {
-                    const size_t j = j0 + c;
-                    if (c < nc && j < p.n && (!p.t.lower || i >= j + p.t.col0))
-                    {
-                        if (p.t.sum)
+                    // T 2^(SUM_W - w) = upper 2^32 + lower
+                    const int l = SUM_W - p.w;
+#pragma unroll
+                    for (int x = 0; x < 8; x++)
+                        if (c + x < last)
                         {
-                            // T 2^(SUM_W - w) = upper 2^32 + lower
-                            const int l = SUM_W - p.w;
-                            atomicAdd(p.t.sum + j * p.m + i, (unsigned long long)(T[c] >> (32 - l)));
-                            atomicAdd(p.t.sum + (p.n + j) * p.m + i,
-                                (unsigned long long)((unsigned)T[c] << l));
-                            continue;
+                            unsigned long long* o = p.t.sum + (j0 + c + x) * p.m + i;
+                            atomicAdd(o, (unsigned long long)(T[c + x] >> (32 - l)));
+                            atomicAdd(o + p.n * p.m, (unsigned long long)((unsigned)T[c + x] << l));
                         }
-                        const double v = scaled(T[c], ei + key_exponent(p.kb[j]));
-                        double* o      = p.t.C + j * p.t.ldc + i;
-                        if (p.t.beta != 0.)
-                            *o = p.t.alpha * v + p.t.beta * p.t.cin[j * p.t.ldcin + i];
-                        else
-                            *o = p.t.alpha == 1. ? v : p.t.alpha * v;
-                    }
+                    continue;
                 }
+                double v[8];
+#pragma unroll
+                for (int x = 0; x < 8; x++)
+                    v[x] = scaled(T[c + x], ei + __shfl_sync(0xffffffffu, ej, c + x));
+                if (p.t.beta != 0.)
+                {
+                    double y[8];
+#pragma unroll
+                    for (int x = 0; x < 8; x++)
+                        y[x] = c + x < last ? p.t.cin[(j0 + c + x) * p.t.ldcin + i] : 0.;
+#pragma unroll
+                    for (int x = 0; x < 8; x++)
+                        v[x] = p.t.alpha * v[x] + p.t.beta * y[x];
+                }
+                else if (p.t.alpha != 1.)
+                {
+#pragma unroll
+                    for (int x = 0; x < 8; x++)
+                        v[x] *= p.t.alpha;
+                }
+#pragma unroll
+                for (int x = 0; x < 8; x++)
+                    if (c + x < last) p.t.C[(j0 + c + x) * p.t.ldc + i] = v[x];
             }
         }
     }
@@ -672,16 +710,34 @@ int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const vo
     Params p;
     p.m = m;
     p.n = n;
-    // equal column tiles of at most BN
-    p.ntj = (int)((n + BN - 1) / BN);
-    p.bn  = (int)(((n + p.ntj - 1) / p.ntj + 31) / 32 * 32);
     p.nti = (int)((m + BM - 1) / BM);
+    // equal column tiles of at most `width`: BN where K is split over the SMs;
+    // else the width whose tiles are done first (an MMA of bn columns takes
+    // about 64 + bn / 4 clocks, a tile some 12000 besides)
+    int width = BN;
+    if (!t.sum)
+    {
+        double best = 0.;
+        for (int c = BN; c >= 32; c -= 32)
+        {
+            const long tiles = (long)p.nti * ((n + c - 1) / c);
+            const double cost = (double)((tiles + sms - 1) / sms)
+                                * (28. * (kc + 15) / 16 * (64 + c / 4) + 12000.);
+            if (c == BN || cost < best)
+            {
+                best  = cost;
+                width = c;
+            }
+        }
+    }
+    p.ntj = (int)((n + width - 1) / width);
+    p.bn  = (int)(((n + p.ntj - 1) / p.ntj + 31) / 32 * 32);
     p.ntiles = p.nti * p.ntj;
     if (t.lower)
     {
         p.ntiles = 0;
         for (int j = 0; j < p.ntj; j++)
-            p.ntiles += p.nti - std::min((t.col0 + j * p.bn) / BM, p.nti);
+            p.ntiles += p.nti - first_tile(t.col0 + j * p.bn, p.nti);
         if (p.ntiles == 0) return MGX_OK;
     }
     p.kblocks = (int)((kc + 63) / 64);
@@ -858,6 +914,7 @@ int store_chunk(mgx_ctx* ctx, const View& A, const View& B, const Target& t, con
     Target c = t;
     c.C += r0;
     if (c.cin) c.cin += r0;
+    c.col0 -= (int)r0;
     MGX_TRY(row_keys(a, p.ka, p.bad, s));
     MGX_TRY(make_planes(a, 0, A.K, p.ka, p.pa, s));
     return product(ctx->sm_count, rows, p.pa, p.ka, B.rows, p.pb, p.kb, A.K, c, p.bad, p.err, s);
