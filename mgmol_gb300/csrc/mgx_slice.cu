@@ -8,7 +8,10 @@
 //   - every row r of an operand is scaled by 2^-e_r, |x| < 2^e_r, and written
 //     as a 56-bit fixed-point number of seven balanced base-256 digits,
 //     x 2^(7 - e_r) = d_0 + d_1 2^-8 + ... + d_6 2^-48, |d| <= 128, each digit
-//     (with its power of 256) one bf16 value;
+//     (with its power of 256) one bf16 value.  Products of the orbitals'
+//     matrices, whose rows hold entries of very different size, take an eighth
+//     digit: with seven the errors of S theta were 7 to 10 times those of
+//     FP64 multiply-adds at 256 .. 2048 functions;
 //   - digit s of A times digit t of B are integers of at most 2^14 at weight
 //     2^(-8 (s + t)).  The products of one s + t add up in an FP32 accumulator
 //     of their own, which rounds nothing while |sum| <= 2^24: after 192 values
@@ -17,10 +20,10 @@
 //     2^-40 and 2^-48, the last bit could round if all digits were extreme.)
 //     The sums have to be exact and not only FP32: the tensor cores truncate
 //     when they add, which biases a sum of squares by 2^-24 per addition;
-//   - products of s + t > 6, 2^-56 of |row maximum| |column maximum| and less,
-//     are left out.
-// 28 bf16 products stand for one FP64 product, at 2^-56 of the row maxima
-// where FP64 multiply-adds round every partial sum at 2^-53.
+//   - products of s + t > 6 (7), 2^-56 (2^-64) of |row maximum| |column maximum|
+//     and less, are left out.
+// 28 (36) bf16 products stand for one FP64 product, at 2^-56 (2^-64) of the row
+// maxima where FP64 multiply-adds round every partial sum at 2^-53.
 //
 // A NaN or an infinity in an operand has no digits: it raises a flag, on
 // which the kernels here do nothing and the caller's CUDA-core kernel,
@@ -40,7 +43,6 @@ namespace mgx
 {
 namespace sl
 {
-constexpr int NS      = 7;   // slices
 constexpr int BM      = 128; // rows of a tile (A)
 constexpr int BN      = 128; // most columns of a tile (B)
 constexpr int BN1     = 64;  // most columns with all NS accumulators in TMEM at once
@@ -49,18 +51,32 @@ constexpr int STAGES  = 2;
 constexpr int DRAIN   = 6;   // stages between reads of the accumulators
 constexpr int DRAIN2  = 8;   // the same for the walk of s + t = 0 .. 3 alone
 constexpr int A_SLICE = BM * BK * 2;
-constexpr int B_SLICE = BN * BK * 2;
-constexpr int STAGE   = NS * (A_SLICE + B_SLICE);
 constexpr int EPI     = 16;  // epilogue warps: four per scheduler hide the TMEM reads
-constexpr int SUM_W   = 47;  // sums over items are kept in units of 2^-SUM_W
+constexpr int SUM_W   = 48;  // sums over items are kept in units of 2^-SUM_W
 constexpr int THREADS = 32 * (2 + EPI);
-constexpr size_t SMEM = (size_t)STAGES * STAGE + (2 * STAGES + 1 + NS) * 8 + 16 + 1024;
-static_assert(SMEM <= 227 * 1024, "two stages of seven slices fit one SM");
-static_assert(NS * BN1 <= 512 && 4 * BN <= 512, "the accumulators of a pass fit TMEM");
+
+/* the kernel's two forms: NP 1, all s + t in one walk over K, at most 64
+ * columns; NP 2, two walks, at most 128 */
+template <int NP, int NS>
+struct Form
+{
+    static constexpr int W       = NP == 1 ? BN1 : BN;
+    static constexpr int B_SLICE = W * BK * 2;
+    static constexpr int STAGE   = NS * (A_SLICE + B_SLICE);
+    static constexpr size_t SMEM
+        = (size_t)STAGES * STAGE + (2 * STAGES + 1 + NS) * 8 + 16 + 1024;
+    static_assert(SMEM <= 227 * 1024, "two stages fit one SM");
+    static_assert((NP == 1 ? NS : 4) * W <= 512, "the accumulators of a walk fit TMEM");
+};
 
 /* The key of a row: the upper half of the bits of max |x|.  Exponent e with
- * |x| < 2^e for every x of the row. */
-__device__ __forceinline__ int key_exponent(int key) { return max(key >> 20, 1) - 1022; }
+ * |x| < 2^e for every x of the row (one more with eight digits, whose first
+ * then fits the upper byte of 64 bits). */
+template <int NS>
+__device__ __forceinline__ int key_exponent(int key)
+{
+    return max(key >> 20, 1) - 1022 + (NS == 8);
+}
 
 constexpr int KEY_NONFINITE = 0x7ff00000;
 
@@ -115,8 +131,9 @@ __global__ void __launch_bounds__(128) keys_rmajor_kernel(const double* __restri
     }
 }
 
-/* x 2^(55 - e) rounded to an integer (half away from zero), |x| < 2^e, in
+/* x 2^(8 NS - 1 - e) rounded to an integer (half away from zero), |x| < 2^e, in
  * integer arithmetic: the FP64 units are the scarce ones here */
+template <int NS>
 __device__ __forceinline__ long long to_fixed(double x, int e)
 {
     const long long b = __double_as_longlong(x);
@@ -124,24 +141,25 @@ __device__ __forceinline__ long long to_fixed(double x, int e)
     long long m       = b & 0xfffffffffffffll;
     if (ex) m |= 0x10000000000000ll;
     // |x| = m 2^(max(ex, 1) - 1075)
-    const int sh = min(e + 1020 - max(ex, 1), 62);
+    const int sh = min(e + 1076 - 8 * NS - max(ex, 1), 62);
     m            = sh <= 0 ? m << (-sh) : (m + (1ll << (sh - 1))) >> sh;
     return b < 0 ? -m : m;
 }
 
 /* the NS digits of q, most significant first, each times 2^(-8 s), as the
  * upper halves of FP32 values (exact in bf16) */
+template <int NS>
 __device__ __forceinline__ void digits(long long q, uint32_t (&f)[NS])
 {
     // with 128 added at the place of every digit but the first, the bytes of
     // q are the balanced digits plus 128
-    const long long b = q + 0x0000808080808080ll;
+    const long long b = q + (NS == 8 ? 0x0080808080808080ll : 0x0000808080808080ll);
     const uint32_t lo = (uint32_t)b, hi = (uint32_t)((unsigned long long)b >> 32);
-    f[0] = __float_as_uint((float)((int)hi >> 16));
+    f[0] = __float_as_uint((float)((int)hi >> (NS == 8 ? 24 : 16)));
 #pragma unroll
     for (int s = 1; s < NS; s++)
     {
-        const int by         = 6 - s; // byte of b
+        const int by         = NS - 1 - s; // byte of b
         const uint32_t byte  = ((by >= 4 ? hi : lo) >> (8 * (by & 3))) & 0xffu;
         const uint32_t magic = (uint32_t)(150 - 8 * s) << 23; // 2^(23 - 8 s)
         // (2^(23 - 8 s) + byte 2^(-8 s)) - (2^(23 - 8 s) + 128 2^(-8 s))
@@ -153,6 +171,7 @@ __device__ __forceinline__ void digits(long long q, uint32_t (&f)[NS])
 /* stores the digits of 8 consecutive K values: 16 bytes in each plane.  The
  * planes are K-blocked: element (row, k) of slice s at
  * ((s * kblocks + k / 64) * rows + row) * 64 + k % 64. */
+template <int NS>
 __device__ __forceinline__ void store8(const long long (&q)[8], __nv_bfloat16* planes, size_t rows,
     size_t kblocks, size_t kb, size_t r, int g)
 {
@@ -161,8 +180,8 @@ __device__ __forceinline__ void store8(const long long (&q)[8], __nv_bfloat16* p
     for (int p = 0; p < 4; p++)
     {
         uint32_t a[NS], b[NS];
-        digits(q[2 * p], a);
-        digits(q[2 * p + 1], b);
+        digits<NS>(q[2 * p], a);
+        digits<NS>(q[2 * p + 1], b);
 #pragma unroll
         for (int s = 0; s < NS; s++)
             w[s][p] = __byte_perm(a[s], b[s], 0x7632);
@@ -175,6 +194,7 @@ __device__ __forceinline__ void store8(const long long (&q)[8], __nv_bfloat16* p
 
 /* planes of a K-contiguous operand, 8 values of K per thread; HBM bound (8
  * bytes read, 14 written per value) */
+template <int NS>
 __global__ void __launch_bounds__(256) planes_kmajor_kernel(const double* __restrict__ x, size_t ld,
     size_t rows, size_t K, const int* __restrict__ keys, size_t kblocks,
     __nv_bfloat16* __restrict__ planes)
@@ -187,13 +207,13 @@ __global__ void __launch_bounds__(256) planes_kmajor_kernel(const double* __rest
         const size_t rk = t / 8;
         const size_t kb = rk % kblocks, r = rk / kblocks;
         const size_t k  = kb * 64 + g;
-        const int e     = key_exponent(keys[r]);
+        const int e     = key_exponent<NS>(keys[r]);
         const double* p = x + r * ld + k;
         long long q[8];
 #pragma unroll
         for (int i = 0; i < 8; i++)
-            q[i] = (k + i < K) ? to_fixed(p[i], e) : 0;
-        store8(q, planes, rows, kblocks, kb, r, g);
+            q[i] = (k + i < K) ? to_fixed<NS>(p[i], e) : 0;
+        store8<NS>(q, planes, rows, kblocks, kb, r, g);
     }
 }
 
@@ -203,6 +223,7 @@ __global__ void __launch_bounds__(256) planes_kmajor_kernel(const double* __rest
  * next to each other) */
 constexpr int TP = 73;
 
+template <int NS>
 __global__ void __launch_bounds__(256) planes_rmajor_kernel(const double* __restrict__ x, size_t ld,
     size_t rows, size_t K, const int* __restrict__ keys, size_t kblocks,
     __nv_bfloat16* __restrict__ planes)
@@ -211,14 +232,14 @@ __global__ void __launch_bounds__(256) planes_rmajor_kernel(const double* __rest
     const size_t r0 = (size_t)blockIdx.x * 64, kb = blockIdx.y;
     const int rr    = threadIdx.x % 64;
     const size_t r  = r0 + rr;
-    const int e     = r < rows ? key_exponent(keys[r]) : 0;
+    const int e     = r < rows ? key_exponent<NS>(keys[r]) : 0;
 #pragma unroll 4
     for (int kk = threadIdx.x / 64; kk < 64; kk += 4)
     {
         const size_t k = kb * 64 + kk;
         // value k = 8 a + b of the block at place 8 b + a
         t[rr * TP + (kk % 8) * 8 + kk / 8]
-            = (r < rows && k < K) ? to_fixed(x[k * ld + r], e) : 0;
+            = (r < rows && k < K) ? to_fixed<NS>(x[k * ld + r], e) : 0;
     }
     __syncthreads();
     for (int it = threadIdx.x; it < 64 * 8; it += 256)
@@ -229,7 +250,7 @@ __global__ void __launch_bounds__(256) planes_rmajor_kernel(const double* __rest
 #pragma unroll
         for (int b = 0; b < 8; b++)
             q[b] = t[row * TP + 8 * b + a];
-        store8(q, planes, rows, kblocks, kb, r0 + row, 8 * a);
+        store8<NS>(q, planes, rows, kblocks, kb, r0 + row, 8 * a);
     }
 }
 
@@ -302,21 +323,28 @@ __device__ __forceinline__ void tmem_wait_ld(float (&v)[8])
                  : "memory");
 }
 
-/* T 2^E rounded to FP64, in integer arithmetic (a conversion would take the
+/* V 2^E rounded to FP64, in integer arithmetic (a conversion would take the
  * FP64 unit, which the conversions of a tile of few values of K kept busy four
  * times as long as its MMAs ran); scalbn where the result is not normal */
-__device__ __forceinline__ double scaled(long long T, int E)
+__device__ __forceinline__ double scaled(__int128 V, int E)
 {
-    if (T == 0) return 0.;
-    const unsigned long long a = T < 0 ? 0ull - (unsigned long long)T : (unsigned long long)T;
-    const int lz               = __clzll(a);
-    const unsigned long long u = a << lz; // leading bit at 63
+    if (V == 0) return 0.;
+    const bool neg               = V < 0;
+    const unsigned __int128 a    = neg ? (unsigned __int128)0 - (unsigned __int128)V
+                                       : (unsigned __int128)V;
+    const unsigned long long hi  = (unsigned long long)(a >> 64), lo = (unsigned long long)a;
+    const int lz                 = hi ? __clzll(hi) : 64 + __clzll(lo);
+    const unsigned long long u   = (unsigned long long)((a << lz) >> 64); // leading bit at 63
     // 53 bits, the leading one of which adds 1 to the exponent field
     const unsigned long long m = (u >> 11) + ((u >> 10) & 1);
-    const int field            = 1023 + 62 - lz + E;
-    if ((unsigned)(field - 1) >= 2044u) return scalbn((double)T, E);
+    const int field            = 1023 + 126 - lz + E;
+    if ((unsigned)(field - 1) >= 2044u)
+    {
+        const double v = scalbn((double)u, E + 64 - lz);
+        return neg ? -v : v;
+    }
     return __longlong_as_double(
-        (long long)(m + ((unsigned long long)field << 52) + (T < 0 ? 1ull << 63 : 0ull)));
+        (long long)(m + ((unsigned long long)field << 52) + (neg ? 1ull << 63 : 0ull)));
 }
 
 /* One CTA per SM walks the items.  Warp 0 streams the slices of both operands
@@ -330,11 +358,12 @@ __device__ __forceinline__ double scaled(long long T, int E)
  * one walk (NP = 1), serve only products of at most 64 columns.  The accumulators
  * are handed over one by one: those of the next 192 values start while the
  * epilogue warps still empty the later ones. */
-template <int NP>
+template <int NP, int NS>
 __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
     const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, const Params p)
 {
     using namespace tc;
+    constexpr int B_SLICE = Form<NP, NS>::B_SLICE, STAGE = Form<NP, NS>::STAGE;
     if (*p.bad) return;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -461,6 +490,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                     diagonal(std::integral_constant<int, 4>());
                     diagonal(std::integral_constant<int, 5>());
                     diagonal(std::integral_constant<int, 6>());
+                    if (NS == 8) diagonal(std::integral_constant<int, NS - 1>());
                     if (!ok) break;
                     mma_commit(empty + b);
                     if (it % drain(ps) == drain(ps) - 1 || it == nst - 1)
@@ -492,12 +522,13 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
             // while the MMAs run
             const size_t i     = (size_t)ti * BM + q * 32 + lane;
             const long long j0 = (long long)tj * p.bn + c0;
-            const int ei = i < p.m ? key_exponent(p.ka[i]) - 14 - p.w : 0;
-            const int ej = lane < nc && j0 + lane < (long long)p.n ? key_exponent(p.kb[j0 + lane]) : 0;
-            // s + t <= 3 in units of 2^-w (NP 2) or 2^-24 of a digit product,
-            // and s + t >= 4 in units of 2^-48: in T until the second walk
-            // begins (NP 2), or in L
-            constexpr int EL = NP == 1 ? BN1 / 4 : BN / 4;
+            const int ei = i < p.m ? key_exponent<NS>(p.ka[i]) - 14 : 0;
+            const int ej
+                = lane < nc && j0 + lane < (long long)p.n ? key_exponent<NS>(p.kb[j0 + lane]) : 0;
+            // s + t >= 4 in units of 2^-LOW of a digit product, in L (NP 1) or, until
+            // the second walk begins, in T; s + t <= 3 in units of 2^-24 (NP 1) or
+            // 2^-w, for which the sum is then rounded once
+            constexpr int EL = Form<NP, NS>::W / 4, LOW = 8 * (NS - 1);
             long long T[EL], L[NP == 1 ? EL : 1];
 #pragma unroll
             for (int c = 0; c < EL; c++)
@@ -518,7 +549,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                 {
 #pragma unroll
                     for (int c = 0; c < EL; c++)
-                        T[c] = (T[c] + (1ll << (47 - p.w))) >> (48 - p.w);
+                        T[c] = (T[c] + (1ll << (LOW - 1 - p.w))) >> (LOW - p.w);
                 }
 #pragma unroll 1
                 for (int a = 0; a < NS; a++)
@@ -528,7 +559,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                         const int dg = lo + a;
                         // the accumulator holds integers times 2^(-8 dg): they
                         // join the sum shifted left by sh bits
-                        const int sh   = (dg >= 4 ? 48 : NP == 1 ? 24 : p.w) - 8 * dg;
+                        const int sh   = (dg >= 4 ? LOW : NP == 1 ? 24 : p.w) - 8 * dg;
                         const int e    = sh == 31 ? 1 : 0; // a factor of 2^31 is no int
                         const float up = __uint_as_float((uint32_t)(127 + 8 * dg + e) << 23);
                         const int mul  = 1 << ((sh - e) & 31);
@@ -572,13 +603,11 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                 abort_all = 1;
                 break;
             }
-            if (NP == 1)
-            {
-#pragma unroll
-                for (int c = 0; c < EL; c++)
-                    T[c] = (T[c] << (p.w - 24))
-                           + ((L[NP == 1 ? c : 0] + (1ll << (47 - p.w))) >> (48 - p.w));
-            }
+            // the whole sum, in units of 2^-unit
+            const int unit = NP == 1 ? LOW : p.w;
+            auto whole     = [&](int c) -> __int128 {
+                return NP == 1 ? ((__int128)T[c] << (LOW - 24)) + L[NP == 1 ? c : 0] : (__int128)T[c];
+            };
             // entries of this thread: row i, columns j0 .. j0 + nc - 1 that exist
             // (lower: from the diagonal down)
             const int cols = i < p.m ? (int)min((long long)nc, (long long)p.n - j0) : 0;
@@ -590,22 +619,22 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                 if (c >= nc) break;
                 if (p.t.sum)
                 {
-                    // T 2^(SUM_W - w) = upper 2^32 + lower
-                    const int l = SUM_W - p.w;
+                    // in units of 2^-SUM_W: upper 2^32 + lower
 #pragma unroll
                     for (int x = 0; x < 8; x++)
                         if (c + x < last)
                         {
+                            const __int128 y      = whole(c + x) << (SUM_W - unit);
                             unsigned long long* o = p.t.sum + (j0 + c + x) * p.m + i;
-                            atomicAdd(o, (unsigned long long)(T[c + x] >> (32 - l)));
-                            atomicAdd(o + p.n * p.m, (unsigned long long)((unsigned)T[c + x] << l));
+                            atomicAdd(o, (unsigned long long)(long long)(y >> 32));
+                            atomicAdd(o + p.n * p.m, (unsigned long long)(unsigned)y);
                         }
                     continue;
                 }
                 double v[8];
 #pragma unroll
                 for (int x = 0; x < 8; x++)
-                    v[x] = scaled(T[c + x], ei + __shfl_sync(0xffffffffu, ej, c + x));
+                    v[x] = scaled(whole(c + x), ei - unit + __shfl_sync(0xffffffffu, ej, c + x));
                 if (p.t.beta != 0.)
                 {
                     double y[8];
@@ -652,13 +681,13 @@ __global__ void __launch_bounds__(256) add_sums_kernel(const unsigned long long*
         const unsigned long long lo = sum[total + t];
         const long long hi          = (long long)(sum[t] + (lo >> 32));
         const double v = (double)hi * 4294967296. + (double)(unsigned)lo;
-        C[j * ldc + i] += scalbn(v, key_exponent(ka[i]) + key_exponent(kb[j]) - 14 - SUM_W);
+        C[j * ldc + i] += scalbn(v, key_exponent<7>(ka[i]) + key_exponent<7>(kb[j]) - 14 - SUM_W);
     }
 }
 
-size_t plane_bytes(size_t rows, size_t K)
+size_t plane_bytes(size_t rows, size_t K, int ns)
 {
-    return NS * rows * ((K + 63) / 64) * 128;
+    return ns * rows * ((K + 63) / 64) * 128;
 }
 
 int row_keys(const View& v, int* keys, int* bad, cudaStream_t s)
@@ -682,21 +711,22 @@ int row_keys(const View& v, int* keys, int* bad, cudaStream_t s)
     return MGX_OK;
 }
 
-int make_planes(const View& v, size_t k0, size_t kc, const int* keys, void* planes,
+int make_planes(const View& v, size_t k0, size_t kc, const int* keys, void* planes, int ns,
     cudaStream_t s)
 {
     const size_t kblocks = (kc + 63) / 64;
     if (v.kmajor)
     {
         const size_t total = v.rows * kblocks * 8;
-        planes_kmajor_kernel<<<(unsigned)std::min<size_t>((total + 255) / 256, 1u << 20), 256, 0,
-            s>>>(v.x + k0, v.ld, v.rows, kc, keys, kblocks, (__nv_bfloat16*)planes);
+        auto kern = ns == 8 ? planes_kmajor_kernel<8> : planes_kmajor_kernel<7>;
+        kern<<<(unsigned)std::min<size_t>((total + 255) / 256, 1u << 20), 256, 0, s>>>(v.x + k0, v.ld, v.rows, kc, keys, kblocks, (__nv_bfloat16*)planes);
     }
     else
     {
         const dim3 grid((unsigned)((v.rows + 63) / 64), (unsigned)kblocks);
         if (grid.y > 65535) return fail(MGX_UNSUPPORTED, "slices: K too large");
-        planes_rmajor_kernel<<<grid, 256, 0, s>>>(v.x + k0 * v.ld, v.ld, v.rows, kc, keys, kblocks,
+        auto kern = ns == 8 ? planes_rmajor_kernel<8> : planes_rmajor_kernel<7>;
+        kern<<<grid, 256, 0, s>>>(v.x + k0 * v.ld, v.ld, v.rows, kc, keys, kblocks,
             (__nv_bfloat16*)planes);
     }
     MGX_LAUNCH_CHECK("slice planes kernel");
@@ -704,7 +734,7 @@ int make_planes(const View& v, size_t k0, size_t kc, const int* keys, void* plan
 }
 
 int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const void* pb,
-    const int* kb, size_t kc, const Target& t, const int* bad, int* err, cudaStream_t s)
+    const int* kb, size_t kc, const Target& t, int ns, const int* bad, int* err, cudaStream_t s)
 {
     if (m == 0 || n == 0 || kc == 0) return MGX_OK;
     Params p;
@@ -714,16 +744,18 @@ int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const vo
     // equal column tiles of at most `width`: BN where K is split over the SMs;
     // else the width whose tiles are done first (an MMA of bn columns takes
     // about 64 + bn / 4 clocks, a tile some 12000 besides)
-    int width = BN;
+    // (an eighth digit leaves room for one walk over 64 columns only)
+    const int most = ns == 8 ? BN1 : BN;
+    int width      = most;
     if (!t.sum)
     {
         double best = 0.;
-        for (int c = BN; c >= 32; c -= 32)
+        for (int c = most; c >= 32; c -= 32)
         {
             const long tiles = (long)p.nti * ((n + c - 1) / c);
             const double cost = (double)((tiles + sms - 1) / sms)
-                                * (28. * (kc + 15) / 16 * (64 + c / 4) + 12000.);
-            if (c == BN || cost < best)
+                                * (ns * (ns + 1) / 2. * (kc + 15) / 16 * (64 + c / 4) + 12000.);
+            if (c == most || cost < best)
             {
                 best  = cost;
                 width = c;
@@ -767,25 +799,28 @@ int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const vo
     const long items = (long)p.ntiles * ks;
     if (items > (1L << 30)) return fail(MGX_UNSUPPORTED, "too many work items");
     p.nitems = (int)items;
-    // |sum| <= 1.01 K 2^14 2^w < 2^63 (and, in units of 2^-48, s + t >= 4 adds
-    // up to 5.1 K 2^30)
+    // |sum| <= 1.01 K 2^14 2^w < 2^63 (NP 2; in units of 2^-48, s + t >= 4 adds up
+    // to 5.1 K 2^30 before)
     int lg = 0;
     while ((1L << lg) < (long)p.st_per_item * BK) lg++;
     if (lg > 17) return fail(MGX_UNSUPPORTED, "slices: K too large for one sum");
-    p.w = std::min(SUM_W, 48 - lg);
+    p.w = std::min(47, 48 - lg);
     p.ka  = ka;
     p.kb  = kb;
     p.t   = t;
     p.bad = bad;
     p.err = err;
     CUtensorMap mA, mB;
-    MGX_TRY(tc::make_map_blocked(&mA, pa, m, (size_t)NS * p.kblocks, BM, 64));
-    MGX_TRY(tc::make_map_blocked(&mB, pb, n, (size_t)NS * p.kblocks, p.bn, 64));
-    auto kern = p.bn <= BN1 ? slice_product_kernel<1> : slice_product_kernel<2>;
+    MGX_TRY(tc::make_map_blocked(&mA, pa, m, (size_t)ns * p.kblocks, BM, 64));
+    MGX_TRY(tc::make_map_blocked(&mB, pb, n, (size_t)ns * p.kblocks, p.bn, 64));
+    const bool two    = p.bn > BN1;
+    auto kern         = ns == 8 ? slice_product_kernel<1, 8>
+                        : two   ? slice_product_kernel<2, 7> : slice_product_kernel<1, 7>;
+    const size_t smem = ns == 8 ? Form<1, 8>::SMEM : two ? Form<2, 7>::SMEM : Form<1, 7>::SMEM;
     MGX_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)SMEM),
+                           (int)smem),
         "slice_product_kernel smem attribute"));
-    kern<<<(int)std::min<long>(items, sms), THREADS, SMEM, s>>>(mA, mB, p);
+    kern<<<(int)std::min<long>(items, sms), THREADS, smem, s>>>(mA, mB, p);
     MGX_LAUNCH_CHECK("slice_product_kernel");
     return MGX_OK;
 }
@@ -830,9 +865,9 @@ int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const 
         }
         sums += 2 * (size_t)n * f[i].ncols;
     }
-    const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(n + brows, 64));
+    const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(n + brows, 64, 7));
     const size_t kc  = std::min((K + 63) / 64, fit) * 64;
-    const size_t pa_bytes = up256(plane_bytes(n, kc)), pb_bytes = up256(plane_bytes(brows, kc));
+    const size_t pa_bytes = up256(plane_bytes(n, kc, 7)), pb_bytes = up256(plane_bytes(brows, kc, 7));
     int *ka, *kb, *err;
     char* pl;
     MGX_TRY(workspace(ctx, n, bkeys, pa_bytes + pb_bytes + sums * sizeof(unsigned long long), &ka,
@@ -869,12 +904,12 @@ int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const 
     for (size_t k0 = 0; k0 < K; k0 += kc)
     {
         const size_t k = std::min(kc, K - k0);
-        MGX_TRY(make_planes(va, k0, k, ka, pl, s));
+        MGX_TRY(make_planes(va, k0, k, ka, pl, 7, s));
         for (const Part& q : parts)
         {
-            if (!q.same) MGX_TRY(make_planes(q.v, k0, k, q.keys, pb, s));
+            if (!q.same) MGX_TRY(make_planes(q.v, k0, k, q.keys, pb, 7, s));
             MGX_TRY(product(ctx->sm_count, n, pl, ka, q.v.rows, q.same ? pl : pb, q.keys, k, q.t,
-                *bad, err, s));
+                7, *bad, err, s));
         }
     }
     for (int i = 0; i < nf; i++)
@@ -888,21 +923,22 @@ int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const 
     return MGX_OK;
 }
 
-int store_begin(mgx_ctx* ctx, const View& A, const View& B, StorePlan* p, cudaStream_t s)
+int store_begin(mgx_ctx* ctx, const View& A, const View& B, int ns, StorePlan* p, cudaStream_t s)
 {
+    p->ns = ns;
     const size_t K  = A.K;
-    const size_t b1 = up256(plane_bytes(B.rows, K));
-    const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(BM, K));
+    const size_t b1 = up256(plane_bytes(B.rows, K, ns));
+    const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(BM, K, ns));
     p->chunk = std::min((A.rows + BM - 1) / BM, fit) * BM;
     const size_t rows = std::min(p->chunk, A.rows);
     char* pl;
-    MGX_TRY(workspace(ctx, rows, B.rows, b1 + plane_bytes(rows, K), &p->ka, &p->kb, &p->bad,
+    MGX_TRY(workspace(ctx, rows, B.rows, b1 + plane_bytes(rows, K, ns), &p->ka, &p->kb, &p->bad,
         &p->err, &pl));
     p->pb = pl;
     p->pa = pl + b1;
     MGX_TRY(cuda_check(cudaMemsetAsync(p->bad, 0, 2 * sizeof(int), s), "slice flags"));
     MGX_TRY(row_keys(B, p->kb, p->bad, s));
-    return make_planes(B, 0, K, p->kb, p->pb, s);
+    return make_planes(B, 0, K, p->kb, p->pb, ns, s);
 }
 
 int store_chunk(mgx_ctx* ctx, const View& A, const View& B, const Target& t, const StorePlan& p,
@@ -916,8 +952,9 @@ int store_chunk(mgx_ctx* ctx, const View& A, const View& B, const Target& t, con
     if (c.cin) c.cin += r0;
     c.col0 -= (int)r0;
     MGX_TRY(row_keys(a, p.ka, p.bad, s));
-    MGX_TRY(make_planes(a, 0, A.K, p.ka, p.pa, s));
-    return product(ctx->sm_count, rows, p.pa, p.ka, B.rows, p.pb, p.kb, A.K, c, p.bad, p.err, s);
+    MGX_TRY(make_planes(a, 0, A.K, p.ka, p.pa, p.ns, s));
+    return product(ctx->sm_count, rows, p.pa, p.ka, B.rows, p.pb, p.kb, A.K, c, p.ns, p.bad, p.err,
+        s);
 }
 } // namespace sl
 } // namespace mgx
