@@ -428,7 +428,7 @@ static int gemm(mgx_ctx* ctx, const Gemm& g, cudaStream_t s)
         const sl::View b = { g.B, (size_t)g.ldb, (size_t)g.n, (size_t)g.k, !g.tb };
         const sl::Target t
             = { g.C, (size_t)g.ldc, nullptr, g.alpha, g.beta, g.C, (size_t)g.ldc, g.lower, 0 };
-        const int st = sl::store(ctx, a, b, t, 8, s, [&](size_t r0, size_t rows, const int* bad) {
+        const int st = sl::store(ctx, a, b, t, s, [&](size_t r0, size_t rows, const int* bad) {
             Gemm c = g;
             c.m    = (int)rows;
             c.A += g.ta ? r0 * g.lda : r0;
@@ -553,7 +553,7 @@ int psi_theta_cuda_cores(mgx_ctx* ctx, int kind, const void* psi, size_t ld, siz
         const sl::View b = { theta, (size_t)ldt, (size_t)ncols, (size_t)n, true };
         const sl::Target t
             = { (double*)out, ld, nullptr, 1., beta, (const double*)cin, ld, 0, 0 };
-        const int st = sl::store(ctx, a, b, t, 7, s, cores);
+        const int st = sl::store(ctx, a, b, t, s, cores);
         if (st != MGX_NO_MEMORY) return st;
     }
     return cores(0, npts, nullptr);

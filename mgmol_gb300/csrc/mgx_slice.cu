@@ -8,10 +8,11 @@
 //   - every row r of an operand is scaled by 2^-e_r, |x| < 2^e_r, and written
 //     as a 56-bit fixed-point number of seven balanced base-256 digits,
 //     x 2^(7 - e_r) = d_0 + d_1 2^-8 + ... + d_6 2^-48, |d| <= 128, each digit
-//     (with its power of 256) one bf16 value.  Products of the orbitals'
-//     matrices, whose rows hold entries of very different size, take an eighth
-//     digit: with seven the errors of S theta were 7 to 10 times those of
-//     FP64 multiply-adds at 256 .. 2048 functions;
+//     (with its power of 256) one bf16 value.  Seven digits serve the sums
+//     over grid points; the products of N x N matrices and Psi Theta, where one
+//     entry of a row may be far larger than the rest, take an eighth (with
+//     seven S theta and the residual were off 5 to 10 times as far as with FP64
+//     multiply-adds, with eight no further);
 //   - digit s of A times digit t of B are integers of at most 2^14 at weight
 //     2^(-8 (s + t)).  The products of one s + t add up in an FP32 accumulator
 //     of their own, which rounds nothing while |sum| <= 2^24: after 192 values
@@ -734,8 +735,9 @@ int make_planes(const View& v, size_t k0, size_t kc, const int* keys, void* plan
 }
 
 int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const void* pb,
-    const int* kb, size_t kc, const Target& t, int ns, const int* bad, int* err, cudaStream_t s)
+    const int* kb, size_t kc, const Target& t, const int* bad, int* err, cudaStream_t s)
 {
+    const int ns = t.sum ? NS_SUM : NS_STORE;
     if (m == 0 || n == 0 || kc == 0) return MGX_OK;
     Params p;
     p.m = m;
@@ -865,9 +867,10 @@ int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const 
         }
         sums += 2 * (size_t)n * f[i].ncols;
     }
-    const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(n + brows, 64, 7));
+    const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(n + brows, 64, NS_SUM));
     const size_t kc  = std::min((K + 63) / 64, fit) * 64;
-    const size_t pa_bytes = up256(plane_bytes(n, kc, 7)), pb_bytes = up256(plane_bytes(brows, kc, 7));
+    const size_t pa_bytes = up256(plane_bytes(n, kc, NS_SUM)),
+                 pb_bytes = up256(plane_bytes(brows, kc, NS_SUM));
     int *ka, *kb, *err;
     char* pl;
     MGX_TRY(workspace(ctx, n, bkeys, pa_bytes + pb_bytes + sums * sizeof(unsigned long long), &ka,
@@ -904,12 +907,12 @@ int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const 
     for (size_t k0 = 0; k0 < K; k0 += kc)
     {
         const size_t k = std::min(kc, K - k0);
-        MGX_TRY(make_planes(va, k0, k, ka, pl, 7, s));
+        MGX_TRY(make_planes(va, k0, k, ka, pl, NS_SUM, s));
         for (const Part& q : parts)
         {
-            if (!q.same) MGX_TRY(make_planes(q.v, k0, k, q.keys, pb, 7, s));
+            if (!q.same) MGX_TRY(make_planes(q.v, k0, k, q.keys, pb, NS_SUM, s));
             MGX_TRY(product(ctx->sm_count, n, pl, ka, q.v.rows, q.same ? pl : pb, q.keys, k, q.t,
-                7, *bad, err, s));
+                *bad, err, s));
         }
     }
     for (int i = 0; i < nf; i++)
@@ -923,9 +926,9 @@ int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const 
     return MGX_OK;
 }
 
-int store_begin(mgx_ctx* ctx, const View& A, const View& B, int ns, StorePlan* p, cudaStream_t s)
+int store_begin(mgx_ctx* ctx, const View& A, const View& B, StorePlan* p, cudaStream_t s)
 {
-    p->ns = ns;
+    constexpr int ns = NS_STORE;
     const size_t K  = A.K;
     const size_t b1 = up256(plane_bytes(B.rows, K, ns));
     const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(BM, K, ns));
@@ -952,9 +955,8 @@ int store_chunk(mgx_ctx* ctx, const View& A, const View& B, const Target& t, con
     if (c.cin) c.cin += r0;
     c.col0 -= (int)r0;
     MGX_TRY(row_keys(a, p.ka, p.bad, s));
-    MGX_TRY(make_planes(a, 0, A.K, p.ka, p.pa, p.ns, s));
-    return product(ctx->sm_count, rows, p.pa, p.ka, B.rows, p.pb, p.kb, A.K, c, p.ns, p.bad, p.err,
-        s);
+    MGX_TRY(make_planes(a, 0, A.K, p.ka, p.pa, NS_STORE, s));
+    return product(ctx->sm_count, rows, p.pa, p.ka, B.rows, p.pb, p.kb, A.K, c, p.bad, p.err, s);
 }
 } // namespace sl
 } // namespace mgx

@@ -38,7 +38,10 @@ struct Target
     int col0;
 };
 
-/* bytes of the ns planes (digits per value: 7 or 8) of `rows` rows of K values */
+/* digits per value: of the sums over grid points, and of the other products */
+constexpr int NS_SUM = 7, NS_STORE = 8;
+
+/* bytes of the ns planes of `rows` rows of K values */
 size_t plane_bytes(size_t rows, size_t K, int ns);
 
 /* resets the keys of `rows` rows (and *bad when given) and takes the row
@@ -47,10 +50,10 @@ int row_keys(const View& v, int* keys, int* bad, cudaStream_t s);
 /* planes of columns [k0, k0 + kc) of the view */
 int make_planes(const View& v, size_t k0, size_t kc, const int* keys, void* planes, int ns,
     cudaStream_t s);
-/* the product of two sets of planes of kc values of K; does nothing when
- * *bad is set */
+/* the product of two sets of planes (NS_SUM with Target::sum, else NS_STORE) of
+ * kc values of K; does nothing when *bad is set */
 int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const void* pb,
-    const int* kb, size_t kc, const Target& t, int ns, const int* bad, int* err, cudaStream_t s);
+    const int* kb, size_t kc, const Target& t, const int* bad, int* err, cudaStream_t s);
 
 /* whether a product of this size is formed from slices */
 bool pays(size_t m, size_t n, size_t K);
@@ -74,34 +77,30 @@ constexpr size_t PLANE_CAP = size_t(1) << 30;
 int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const Factor* f, int nf,
     int** bad, cudaStream_t s);
 
-/* C = alpha A B^T + beta cin of FP64 operands of any layout from ns digits per
- * value, the rows of A in chunks that bound the planes to PLANE_CAP bytes.  After each chunk
+/* C = alpha A B^T + beta cin of FP64 operands of any layout, the rows of A
+ * in chunks that bound the planes to PLANE_CAP bytes.  After each chunk
  * fallback(r0, rows, bad) enqueues the CUDA-core kernel of these rows, which
  * does nothing unless *bad is set.  MGX_NO_MEMORY: no workspace, nothing was
  * written. */
 template <typename F>
-int store(mgx_ctx* ctx, const View& A, const View& B, const Target& t, int ns, cudaStream_t s,
-    F fallback);
+int store(mgx_ctx* ctx, const View& A, const View& B, const Target& t, cudaStream_t s, F fallback);
 
 /* the parts of store() */
 struct StorePlan
 {
     size_t chunk;
-    int ns;
     int *ka, *kb, *bad, *err;
     char *pa, *pb;
 };
-int store_begin(mgx_ctx* ctx, const View& A, const View& B, int ns, StorePlan* plan,
-    cudaStream_t s);
+int store_begin(mgx_ctx* ctx, const View& A, const View& B, StorePlan* plan, cudaStream_t s);
 int store_chunk(mgx_ctx* ctx, const View& A, const View& B, const Target& t, const StorePlan& plan,
     size_t r0, size_t rows, cudaStream_t s);
 
 template <typename F>
-int store(mgx_ctx* ctx, const View& A, const View& B, const Target& t, int ns, cudaStream_t s,
-    F fallback)
+int store(mgx_ctx* ctx, const View& A, const View& B, const Target& t, cudaStream_t s, F fallback)
 {
     StorePlan p;
-    MGX_TRY(store_begin(ctx, A, B, ns, &p, s));
+    MGX_TRY(store_begin(ctx, A, B, &p, s));
     for (size_t r0 = 0; r0 < A.rows; r0 += p.chunk)
     {
         const size_t rows = p.chunk < A.rows - r0 ? p.chunk : A.rows - r0;
