@@ -1508,6 +1508,237 @@ __global__ void __launch_bounds__(NT, 512 / NT) plane_jj_kernel(PlaneParams p, D
 }
 
 /* ------------------------------------------------------------------ */
+/* axis stencils of radius 2 .. 4 on FP32 blocks                        */
+/* ------------------------------------------------------------------ */
+// One CTA owns one function, TY rows and a chunk of x planes, which arrive
+// whole (TY + 2R rows) in a ring of R + 4 stages, as in plane_kernel.  A thread
+// owns 4 z points of two neighbouring rows: the 2R + 2 rows around them are
+// read once for both (1.75 16-byte reads per point at R = 4, where a point at a
+// time took 17 scalar ones), the x neighbours stay in registers, and every
+// neighbour is one FMA.  What bounded the scalar form was its instruction
+// count: H psi of 512 orbitals on 128^3 with the 8th-order operator took 7.27 ms
+// (1.2 TB/s).
+template <int OP, int R>
+__global__ void __launch_bounds__(256, 2) plane_axis_kernel(PlaneParams p, DevCoef<float> c)
+{
+    constexpr int S = R + 4, QL = 2 * R + 1;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int nx = p.n[0], ny = p.n[1], nz = p.n[2];
+    const int TY      = p.ty;
+    const int rows    = TY + 2 * R;
+    const int tile_y  = blockIdx.x % p.ntile_y;
+    const int tile_x  = blockIdx.x / p.ntile_y;
+    const int f       = blockIdx.y;
+    const int y0      = tile_y * TY;
+    const int x0      = tile_x * p.xc;
+    const int nplanes = min(p.xc, nx - x0) + 2 * R;
+    const bool scaled = is_jacobi(OP) && (p.gamma_in != 0.); // first sweep from gamma f
+    const float gam   = (float)p.gamma_in;
+
+    const size_t stage_elems = (size_t)rows * nz;
+    float* stages            = reinterpret_cast<float*>(smem_raw);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + S * stage_elems * sizeof(float));
+    const float* ubase = reinterpret_cast<const float*>(scaled ? p.f : p.u)
+                         + (size_t)f * (scaled ? p.ldf : p.ldu);
+
+    // staged rows y0 - R .. (mod ny) as at most two runs
+    int ya = y0 - R, na = rows;
+    if (ya < 0)
+    {
+        na = -ya;
+        ya += ny;
+    }
+    else if (ya + rows > ny)
+        na = ny - ya;
+    const int nb = rows - na;
+    auto issue = [&](int i) {
+        const int x      = wrap(x0 - R + i, nx);
+        uint64_t* bar    = bars + i % S;
+        float* dst       = stages + (i % S) * stage_elems;
+        const float* src = ubase + (size_t)x * ny * nz;
+        mbar_arrive_expect_tx(bar, (uint32_t)(stage_elems * sizeof(float)));
+        bulk_g2s(dst, src + (size_t)ya * nz, (uint32_t)(na * nz * sizeof(float)), bar);
+        if (nb > 0)
+            bulk_g2s(dst + (size_t)na * nz, src, (uint32_t)(nb * nz * sizeof(float)), bar);
+    };
+    if (threadIdx.x == 0)
+    {
+        for (int s = 0; s < S; s++)
+            mbar_init(bars + s, 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    int issued = min(S, nplanes) - 1;
+    if (threadIdx.x == 0)
+        for (int i = 0; i <= issued; i++)
+            issue(i);
+
+    const int hz   = nz / 4;
+    const int pair = threadIdx.x / hz, g = threadIdx.x - pair * hz;
+    const int ry   = 2 * pair; // first of the thread's rows, in the tile
+    const bool on  = ry < TY && y0 + ry < ny;
+    const bool on1 = on && ry + 1 < TY && y0 + ry + 1 < ny;
+    const int o    = on ? (ry + R) * nz + 4 * g : R * nz; // centre in a stage
+    const int ol = o + (g > 0 ? -4 : nz - 4), orr = o + (g < hz - 1 ? 4 : 4 - nz);
+    const int row1 = nz; // the stage holds the second row also where it is not the thread's
+    const size_t gidx = (size_t)(y0 + ry) * nz + 4 * g; // in a plane of the grid
+
+    float* __restrict__ outp = reinterpret_cast<float*>(p.out) + (size_t)f * p.ldo;
+    float* __restrict__ updp
+        = (OP == OP_JACOBI_UPD) ? reinterpret_cast<float*>(p.upd) + (size_t)f * p.ldupd : nullptr;
+    const float ualpha = (float)p.upd_alpha;
+    const float uscale = (OP == OP_JACOBI_UPD && p.upd_scale) ? (float)p.upd_scale[f] : 1.f;
+    float* __restrict__ wp = p.w ? reinterpret_cast<float*>(p.w) + (size_t)f * p.ldw : nullptr;
+    // pointwise operand: f of a Jacobi sweep, V of V psi
+    constexpr bool POINTWISE = is_jacobi(OP) || OP == OP_HPSI_V;
+    const float* __restrict__ pw
+        = OP == OP_HPSI_V ? reinterpret_cast<const float*>(p.V)
+                          : (p.f ? reinterpret_cast<const float*>(p.f) + (size_t)f * p.ldf : nullptr);
+
+    float q[2][4][QL]; // the centre columns x - R .. x + R
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+        for (int v = 0; v < 4; v++)
+#pragma unroll
+            for (int j = 0; j < QL; j++)
+                q[r][v][j] = 0.f;
+    auto load4 = [](const float* a, float (&v)[4]) {
+        const float4 t = *reinterpret_cast<const float4*>(a);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    };
+
+    bool ok    = true;
+    int waited = -1;
+    for (int i = 0; i < nplanes; i++)
+    {
+        const bool emit = i >= 2 * R;
+        const int x     = x0 + i - 2 * R;
+        const size_t gx = (size_t)x * ny * nz + gidx;
+        float pv[2][4], up[2][4];
+        if (emit && on)
+        {
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+            {
+                if (r == 1 && !on1) break;
+                if (POINTWISE && !scaled) load4(pw + gx + r * nz, pv[r]);
+                if (OP == OP_JACOBI_UPD) load4(updp + gx + r * nz, up[r]);
+            }
+        }
+        ok = ok && mbar_wait(bars + (i % S), (uint32_t)((i / S) & 1));
+        if (ok) waited = i;
+        const float* st = stages + (i % S) * stage_elems;
+        const float* sc = stages + ((i - R + S) % S) * stage_elems; // plane x
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+        {
+            float nw[4];
+            load4(st + o + r * row1, nw);
+#pragma unroll
+            for (int v = 0; v < 4; v++)
+            {
+#pragma unroll
+                for (int j = 0; j < QL - 1; j++)
+                    q[r][v][j] = q[r][v][j + 1];
+                q[r][v][QL - 1] = nw[v];
+            }
+        }
+        if (emit && on)
+        {
+            // the neighbours at distance 2 .. R first, on their own: their sum is
+            // small next to the terms below, and so are its roundings
+            float a[2][4];
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+#pragma unroll
+                for (int v = 0; v < 4; v++)
+                {
+                    a[r][v] = 0.f;
+#pragma unroll
+                    for (int d = R; d >= 2; d--)
+                        a[r][v] += c.cx[d - 1] * (q[r][v][R - d] + q[r][v][R + d]);
+                }
+            // rows k = -R .. R + 1 around the first one
+#pragma unroll
+            for (int k = -R; k <= R + 1; k++)
+            {
+                if (k == 0 || k == 1) continue;
+                float w[4];
+                load4(sc + o + k * nz, w);
+#pragma unroll
+                for (int v = 0; v < 4; v++)
+                {
+                    if (k != -1 && k <= R) a[0][v] += c.cy[(k < 0 ? -k : k) - 1] * w[v];
+                    if (k != 2 && k > -R) a[1][v] += c.cy[(k < 1 ? 1 - k : k - 1) - 1] * w[v];
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+            {
+                if (r == 1 && !on1) break;
+                float z[12], yn[4]; // yn: the neighbour row that is not the thread's
+                {
+                    float l[4], h[4];
+                    load4(sc + ol + r * row1, l);
+                    load4(sc + orr + r * row1, h);
+                    load4(sc + o + (r ? 2 : -1) * nz, yn);
+#pragma unroll
+                    for (int v = 0; v < 4; v++)
+                    {
+                        z[v]     = l[v];
+                        z[4 + v] = q[r][v][R];
+                        z[8 + v] = h[v];
+                    }
+                }
+                float res[4], wv[4];
+#pragma unroll
+                for (int v = 0; v < 4; v++)
+                {
+#pragma unroll
+                    for (int d = R; d >= 2; d--)
+                        a[r][v] += c.cz[d - 1] * (z[4 + v - d] + z[4 + v + d]);
+                    float lap = c.c0 * z[4 + v];
+                    lap += c.cx[0] * (q[r][v][R - 1] + q[r][v][R + 1]);
+                    lap += c.cy[0] * (yn[v] + q[1 - r][v][R]);
+                    lap += c.cz[0] * (z[3 + v] + z[5 + v]);
+                    lap += a[r][v];
+                    const float u = z[4 + v];
+                    res[v]        = lap;
+                    if (OP == OP_HPSI_V) res[v] = lap + u * pv[r][v];
+                    if (is_jacobi(OP))
+                        res[v] = jacobi_point<float>(lap, u, scaled ? 0.f : pv[r][v], c.jf, scaled,
+                            gam, wv[v]);
+                    if (OP == OP_JACOBI_UPD) res[v] = update_point<float>(up[r][v], res[v], ualpha, uscale);
+                }
+                float* dst = (OP == OP_JACOBI_UPD ? updp : outp) + gx + r * nz;
+                *reinterpret_cast<float4*>(dst) = make_float4(res[0], res[1], res[2], res[3]);
+                if (is_jacobi(OP) && wp != nullptr)
+                    *reinterpret_cast<float4*>(wp + gx + r * nz)
+                        = make_float4(wv[0], wv[1], wv[2], wv[3]);
+            }
+        }
+        __syncthreads();
+        const int nxt = i - R + S;
+        if (nxt < nplanes && nxt > issued)
+        {
+            if (threadIdx.x == 0)
+            {
+                fence_proxy_async_smem();
+                issue(nxt);
+            }
+            issued = nxt;
+        }
+    }
+    if (!ok && threadIdx.x == 0)
+    {
+        if (p.err != nullptr) atomicExch(p.err, MGX_TIMEOUT);
+        for (int i = waited + 1; i <= issued; i++)
+            mbar_wait(bars + (i % S), (uint32_t)((i / S) & 1));
+    }
+}
+
+/* ------------------------------------------------------------------ */
 /* direct kernel (global loads with wrap), for small / unaligned cases  */
 /* ------------------------------------------------------------------ */
 template <typename T, typename TV, int LAP, int OP, int R>
@@ -1635,12 +1866,71 @@ static int launch_vec(const PlaneParams& p0, const DevCoef<T>& c, int nfunc,
     return MGX_OK;
 }
 
+/* Can plane_axis_kernel run this launch?  FP32 blocks of whole 16-byte
+ * vectors, an axis stencil of radius 2 .. 4 without localization masks, and a
+ * tile of at least two rows that wraps at most once and leaves two CTAs on an
+ * SM.  *ty: the rows of a tile, equal cuts of ny. */
+template <typename T, typename TV, int LAP, int OP, int R>
+static bool axis_ok(const PlaneParams& p, int force_direct, int* ty)
+{
+    if (force_direct || R < 2 || sizeof(T) != 4 || sizeof(TV) != 4 || LAP == 0 || p.mask.state)
+        return false;
+    if (OP != OP_LAP && OP != OP_HPSI_V && OP != OP_JACOBI && OP != OP_JACOBI_UPD) return false;
+    const int nx = p.n[0], ny = p.n[1], nz = p.n[2];
+    auto al = [](const void* q, size_t ld) {
+        return q == nullptr || (((uintptr_t)q % 16) == 0 && ld % 4 == 0);
+    };
+    if (nz % 4 || nz < 2 * R + 1 || nz > 1024 || nx < R) return false;
+    if (!al(p.u, p.ldu) || !al(p.out, p.ldo) || !al(p.w, p.ldw) || !al(p.f, p.ldf)
+        || !al(p.upd, p.ldupd) || !al(p.V, 0))
+        return false;
+    int t = std::min(2 * (256 / (nz / 4)), (ny - 2 * R) & ~1);
+    while (t >= 2 && (size_t)(R + 4) * ((t + 2 * R) * nz * sizeof(float) + 8) > 110 * 1024)
+        t -= 2;
+    if (t < 2) return false;
+    const int n = (ny + t - 1) / t;
+    *ty         = ((ny + n - 1) / n + 1) & ~1;
+    return true;
+}
+
+template <int OP, int R>
+static int launch_axis(const PlaneParams& p0, const DevCoef<float>& c, int nfunc, int ty,
+    cudaStream_t stream)
+{
+    PlaneParams p = p0;
+    const int nx = p.n[0], ny = p.n[1], nz = p.n[2];
+    p.ty      = ty;
+    p.ntile_y = (ny + ty - 1) / ty;
+    // x chunks: the march's 2R extra planes are read again by each, so no more
+    // of them than give every SM several CTAs
+    int cuts = 1;
+    while ((size_t)p.ntile_y * cuts * nfunc < 6 * 152 && (nx + cuts - 1) / cuts > 2 * R)
+        cuts *= 2;
+    p.xc      = (nx + cuts - 1) / cuts;
+    p.ntile_x = (nx + p.xc - 1) / p.xc;
+    const size_t smem = (size_t)(R + 4) * ((size_t)(ty + 2 * R) * nz * sizeof(float) + 8);
+    auto kern         = plane_axis_kernel<OP, R>;
+    MGX_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)smem),
+        "plane_axis_kernel smem attribute"));
+    kern<<<dim3(p.ntile_y * p.ntile_x, nfunc), 256, smem, stream>>>(p, c);
+    MGX_LAUNCH_CHECK("plane_axis_kernel");
+    return MGX_OK;
+}
+
 template <typename T, typename TV, int LAP, int OP, int R>
 static int launch_t(const PlaneParams& p0, const DevCoef<T>& c, int nfunc,
     cudaStream_t stream, int force_direct)
 {
     if (vec_ok<T, TV, LAP, OP, R>(p0, force_direct) && (OP != OP_JACOBI_RST || !p0.mask.state))
         return launch_vec<T, TV, LAP, OP, R>(p0, c, nfunc, stream);
+    if constexpr (R >= 2 && sizeof(T) == 4 && sizeof(TV) == 4
+                  && (OP == OP_LAP || OP == OP_HPSI_V || OP == OP_JACOBI || OP == OP_JACOBI_UPD))
+    {
+        int ty = 0;
+        if (axis_ok<T, TV, LAP, OP, R>(p0, force_direct, &ty))
+            return launch_axis<OP, R>(p0, c, nfunc, ty, stream);
+    }
     if (OP == OP_JACOBI_RST)
         return fail(MGX_UNSUPPORTED, "the fused restriction needs the vector kernel, no masks");
     if (p0.gamma_in != 0.)

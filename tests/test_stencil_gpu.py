@@ -158,3 +158,29 @@ def test_dropin_rhs_and_transfers():
     capi.mgkernel_extend3d(n, ll, g, C, F, nf)
     e_ref = O.extend(n, ll, c_ref)
     assert rel_err(F[:, 1:-1, 1:-1, 1:-1].reshape(nf, -1).cpu().numpy(), e_ref) < TOL_F64
+
+
+@pytest.mark.parametrize("n", [(9, 10, 12), (10, 11, 16), (17, 33, 128), (70, 37, 64), (12, 20, 1024),
+                               (40, 128, 36)])
+@pytest.mark.parametrize("lap", [2, 3, 4])
+def test_axis_kernel_tiles(n, lap):
+    """The FP32 kernel of the radius 2 .. 4 operators at odd row counts, cut
+    tiles and x chunks, against the FP64 kernels (H psi, the smoothing sweeps and
+    the fused update): FP32 roundings of up to 27 terms, TOL_F32 as above."""
+    ll = tuple(0.3 * x for x in n)
+    ctx = capi.Context(n, ll)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    u = torch.randn((3, ctx.npts), generator=g, device="cuda")
+    V = torch.randn(ctx.npts, generator=g, device="cuda")
+    psi = torch.randn((3, ctx.npts), generator=g, device="cuda")
+
+    def close(a, b):
+        return float((a.double() - b).abs().max() / b.abs().max()) < TOL_F32
+
+    assert close(ctx.hpsi(u, V, lap), ctx.hpsi(u.double(), V.double(), lap))
+    assert close(ctx.fd_apply(u, lap), ctx.fd_apply(u.double(), lap))
+    out = ctx.precond_mg(u, lap, 0, 0.2)
+    assert close(out, ctx.precond_mg(u.double(), lap, 0, 0.2))
+    a = ctx.precond_update(u, psi.clone(), 0.4, lap, 0, 0.2)
+    assert close(a, ctx.precond_update(u.double(), psi.double(), 0.4, lap, 0, 0.2))
