@@ -1797,6 +1797,43 @@ constexpr int stages_for()
     return ((LAP == 0) || is_rhs_op(OP)) ? 4 : R + 4;
 }
 
+/* Tile rows and x chunk of a plane kernel that cannot fill the GPU with large
+ * tiles (one field, few functions): the pair whose busiest SM has the least to
+ * do.  A CTA works on (xc + halo) planes of ty rows; a point and plane costs its
+ * SM about 10 clocks in FP64 (2 operations per clock) and 0.5 in FP32, a plane
+ * some 500 more of latency, which two resident CTAs hide from each other.  *ty
+ * comes in as the most rows that fit.  With tiles of the most rows and chunks
+ * of 4 planes, one FP64 sweep on 96^3 took 240 CTAs on 152 SMs. */
+static void few_tiles(int nx, int ny, int nz, int nfunc, int halo, int esz, bool even, int* ty,
+    int* xc)
+{
+    static const int cuts[] = { 1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 32, 48, 64 };
+    const double point = esz == 8 ? 10. : 0.5;
+    const int most     = *ty;
+    double best        = -1.;
+    auto up2 = [&](int v) { return even ? (v + 1) & ~1 : v; };
+    for (int ky : cuts)
+    {
+        const int t = up2((ny + ky - 1) / ky);
+        if (t > most) continue;
+        for (int kx : cuts)
+        {
+            const int x       = up2((nx + kx - 1) / kx);
+            const long ctas   = (long)((ny + t - 1) / t) * ((nx + x - 1) / x) * nfunc;
+            const long per_sm = (ctas + 151) / 152;
+            const double cost = (x + halo) * (per_sm * (double)t * nz * point + 500. * ((per_sm + 1) / 2));
+            if (best < 0. || cost < best)
+            {
+                best = cost;
+                *ty  = t;
+                *xc  = x;
+            }
+            if (x <= 2) break;
+        }
+        if (t <= 2) break;
+    }
+}
+
 /* Can the vectorised radius-1 kernel run this launch?  It needs the
  * operator to be radius 1 with a uniform element type, and every block it
  * touches 16-byte aligned with rows of whole vectors. */
@@ -1847,14 +1884,13 @@ static int launch_vec(const PlaneParams& p0, const DevCoef<T>& c, int nfunc,
     for (; ty >= 1; ty -= RST ? 2 : 1)
         if (smem_for(ty) <= smem_cap) break;
     if (ty < 1) return fail(MGX_UNSUPPORTED, "plane too large for the vector kernel");
+    int xc = std::min(32, nx);
+    if ((size_t)((ny + ty - 1) / ty) * ((nx + xc - 1) / xc) * nfunc < 4 * 152)
+        few_tiles(nx, ny, nz, nfunc, 2 + YO, (int)sizeof(T), RST, &ty, &xc);
     p.ty      = ty;
     p.ntile_y = (ny + ty - 1) / ty;
-    int xc = 32;
-    while (xc > 4 && (size_t)p.ntile_y * ((nx + xc - 1) / xc) * nfunc < 4 * 152)
-        xc /= 2;
-    if (xc > nx) xc = nx;
-    p.xc       = xc;
-    p.ntile_x  = (nx + xc - 1) / xc;
+    p.xc      = xc;
+    p.ntile_x = (nx + xc - 1) / xc;
     const size_t smem = smem_for(ty);
     auto kern         = plane_vec_kernel<T, LAP == 1 ? 1 : 0, OP, S, NG>;
     cudaError_t e     = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
