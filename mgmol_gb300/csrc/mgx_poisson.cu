@@ -30,8 +30,11 @@ int restrict_launch(int, const Level&, const void*, size_t, void*, size_t, int,
     const MaskDev&, cudaStream_t);
 int prolong_launch(int, int, const Level&, const void*, size_t, void*, size_t,
     int, const MaskDev&, cudaStream_t);
+int scale_launch(int, const void*, size_t, void*, size_t, size_t, int, double, cudaStream_t);
 
 constexpr int NORM_BLOCKS = 512;
+// levels of at most so many points are swept without the plane pipeline
+constexpr size_t DIRECT_PTS = 16384;
 
 template <typename T>
 __global__ void __launch_bounds__(256) sumsq_partial_kernel(const T* __restrict__ u,
@@ -72,6 +75,153 @@ __global__ void __launch_bounds__(256) sum_partials_kernel(const double* __restr
     if (threadIdx.x == 0) *out = red[0];
 }
 
+/* The part of the cycle below a level of at most BOTTOM_PTS points, in one
+ * launch of one CTA: there a sweep's work is under a microsecond, and the ten to
+ * twenty launches of its own that each level took (4 to 8 us each) were a tenth
+ * of the solve on 96^3.  Every level's fields live in shared memory; the steps
+ * are those of PoissonMG::cycle.  LAP: 0 (Laph4M) or 1 (Laph2), on all of these
+ * levels. */
+constexpr int BOTTOM_PTS    = 512;
+constexpr int BOTTOM_LEVELS = 4;
+
+template <typename T>
+struct BottomParams
+{
+    int nlev, nu1, nu2;
+    int n[BOTTOM_LEVELS][3];
+    T c0[BOTTOM_LEVELS], cf[BOTTOM_LEVELS][3], ce[BOTTOM_LEVELS][3], jf[BOTTOM_LEVELS];
+    const T* f; // right-hand side of the first level
+    T* x;       // its result
+};
+
+template <typename T, int LAP>
+__global__ void __launch_bounds__(256) bottom_kernel(const BottomParams<T> p)
+{
+    // x, x', w and f of every level: 4 (1 + 1/8 + ...) BOTTOM_PTS values
+    __shared__ T mem[4 * (BOTTOM_PTS + BOTTOM_PTS / 8 + BOTTOM_PTS / 64 + BOTTOM_PTS / 512)];
+    T* base[BOTTOM_LEVELS];
+    int np[BOTTOM_LEVELS], cur[BOTTOM_LEVELS];
+    {
+        T* b = mem;
+        for (int l = 0; l < p.nlev; l++)
+        {
+            np[l]   = p.n[l][0] * p.n[l][1] * p.n[l][2];
+            cur[l]  = 0;
+            base[l] = b;
+            b += 4 * np[l];
+        }
+    }
+    auto X = [&](int l) { return base[l] + cur[l] * np[l]; };
+    auto Y = [&](int l) { return base[l] + (1 - cur[l]) * np[l]; };
+    auto W = [&](int l) { return base[l] + 2 * np[l]; };
+    auto F = [&](int l) { return base[l] + 3 * np[l]; };
+    const int tid = threadIdx.x;
+    for (int i = tid; i < np[0]; i += 256)
+        F(0)[i] = p.f[i];
+    __syncthreads();
+
+    // w = A x - f, and x' = x - jf w unless only the residual is wanted
+    auto sweep = [&](int l, bool residual) {
+        const int ny = p.n[l][1], nz = p.n[l][2], nx = p.n[l][0];
+        const T *x = X(l), *f = F(l);
+        T *y = Y(l), *w = W(l);
+        for (int i = tid; i < np[l]; i += 256)
+        {
+            const int iz = i % nz, iy = (i / nz) % ny, ix = i / (nz * ny);
+            const int zm = iz ? -1 : nz - 1, zp = iz + 1 < nz ? 1 : 1 - nz;
+            const int ym = (iy ? -1 : ny - 1) * nz, yp = (iy + 1 < ny ? 1 : 1 - ny) * nz;
+            const int xm = (ix ? -1 : nx - 1) * ny * nz, xp = (ix + 1 < nx ? 1 : 1 - nx) * ny * nz;
+            const T* q = x + i;
+            const T sz = q[zm] + q[zp], sy = q[ym] + q[yp], sx = q[xm] + q[xp];
+            T r        = p.c0[l] * q[0] + p.cf[l][2] * sz + p.cf[l][1] * sy + p.cf[l][0] * sx;
+            if (LAP == 0)
+            {
+                r += p.ce[l][0] * (q[xm + zm] + q[xm + zp] + q[xp + zm] + q[xp + zp]); // x z
+                r += p.ce[l][1] * (q[ym + zm] + q[ym + zp] + q[yp + zm] + q[yp + zp]); // y z
+                r += p.ce[l][2] * (q[xm + ym] + q[xp + ym] + q[xm + yp] + q[xp + yp]); // x y
+            }
+            r -= f[i];
+            if (residual)
+                w[i] = r;
+            else
+                y[i] = q[0] - p.jf[l] * r;
+        }
+        __syncthreads();
+        if (!residual) cur[l] ^= 1;
+    };
+
+    for (int l = 0; l < p.nlev; l++)
+    {
+        // the first sweep from x = 0 is jf f
+        for (int i = tid; i < np[l]; i += 256)
+            X(l)[i] = p.nu1 > 0 ? p.jf[l] * F(l)[i] : (T)0;
+        __syncthreads();
+        for (int s = 1; s < p.nu1; s++)
+            sweep(l, false);
+        if (l + 1 == p.nlev) break;
+        sweep(l, true);
+        // full weighting (restrict_kernel)
+        const int nx = p.n[l][0], ny = p.n[l][1], nz = p.n[l][2];
+        const int cy = ny >> 1, cz = nz >> 1;
+        const T* w = W(l);
+        for (int i = tid; i < np[l + 1]; i += 256)
+        {
+            const int iz = 2 * (i % cz), iy = 2 * ((i / cz) % cy), ix = 2 * (i / (cz * cy));
+            const int zm = iz ? -1 : nz - 1, zp = 1;
+            const int ym = (iy ? -1 : ny - 1) * nz, yp = nz;
+            const int xm = (ix ? -1 : nx - 1) * ny * nz, xp = ny * nz;
+            const T* q = w + (ix * ny + iy) * nz + iz;
+            const T face   = q[xp] + q[xm] + q[yp] + q[ym] + q[zm] + q[zp];
+            const T corner = q[xp + yp + zm] + q[xp + yp + zp] + q[xp + ym + zm] + q[xp + ym + zp]
+                             + q[xm + yp + zm] + q[xm + yp + zp] + q[xm + ym + zm] + q[xm + ym + zp];
+            const T edge   = q[yp + zm] + q[yp + zp] + q[ym + zm] + q[ym + zp] + q[xp + zm]
+                           + q[xp + zp] + q[xm + zm] + q[xm + zp] + q[xm + ym] + q[xp + ym]
+                           + q[xm + yp] + q[xp + yp];
+            F(l + 1)[i] = (T)(1. / 64.) * ((T)8. * q[0] + (T)4. * face + (T)2. * edge + corner);
+        }
+        __syncthreads();
+    }
+    for (int l = p.nlev - 1; l >= 0; l--)
+    {
+        if (l + 1 < p.nlev)
+        {
+            // x -= trilinear interpolation of the level below (prolong_kernel)
+            const int ny = p.n[l][1], nz = p.n[l][2];
+            const int cx = p.n[l][0] >> 1, cy = ny >> 1, cz = nz >> 1;
+            const T* e = X(l + 1);
+            T* x       = X(l);
+            for (int i = tid; i < np[l]; i += 256)
+            {
+                const int iz = i % nz, iy = (i / nz) % ny, ix = i / (nz * ny);
+                const int az = iz & 1, ay = iy & 1, ax = ix & 1;
+                const int jz = iz >> 1, jy = iy >> 1, jx = ix >> 1;
+                const int dz = az ? (jz + 1 < cz ? 1 : 1 - cz) : 0;
+                const int dy = ay ? (jy + 1 < cy ? 1 : 1 - cy) * cz : 0;
+                const int dx = ax ? (jx + 1 < cx ? 1 : 1 - cx) * cy * cz : 0;
+                const T* q   = e + (jx * cy + jy) * cz + jz;
+                // every odd direction halves a sum of two
+                T v = q[0];
+                if (az) v = v + q[dz];
+                if (ay) v = v + (az ? q[dy] + q[dy + dz] : q[dy]);
+                if (ax)
+                {
+                    T u = q[dx];
+                    if (az) u = u + q[dx + dz];
+                    if (ay) u = u + (az ? q[dx + dy] + q[dx + dy + dz] : q[dx + dy]);
+                    v = v + u;
+                }
+                x[i] -= v * (T)(1. / (1 << (ax + ay + az)));
+            }
+            __syncthreads();
+        }
+        for (int s = 0; s < p.nu2; s++)
+            sweep(l, false);
+    }
+    const T* x = X(0);
+    for (int i = tid; i < np[0]; i += 256)
+        p.x[i] = x[i];
+}
+
 namespace
 {
 struct PoissonMG
@@ -87,7 +237,8 @@ struct PoissonMG
     int* err      = nullptr;
     size_t es     = 8;
 
-    int sweep(int l, const void* u, void* out, void* wout, double factor)
+    // one Jacobi sweep; gamma: from gamma f[l] instead of u
+    int sweep(int l, const void* u, void* out, void* wout, double factor, double gamma = 0.)
     {
         PlaneParams p;
         p.u   = u;
@@ -100,20 +251,87 @@ struct PoissonMG
         p.ldw = lev[l].npts();
         for (int i = 0; i < 3; i++)
             p.n[i] = lev[l].n[i];
-        p.err = err;
-        return stencil_launch(OP_JACOBI, op[l], dtype, dtype, p, lev[l], factor, 1, s);
+        p.err      = err;
+        p.gamma_in = gamma;
+        // small levels: the kernel without a plane pipeline starts sooner (4
+        // against 8 us a sweep at 12^3 and 24^3)
+        return stencil_launch(OP_JACOBI, op[l], dtype, dtype, p, lev[l], factor, 1, s,
+            lev[l].npts() <= DIRECT_PTS ? 1 : 0);
+    }
+
+    // the cycle from level l down in bottom_kernel; MGX_UNSUPPORTED where it
+    // cannot run.  The result goes to x0[l].
+    int bottom(int l)
+    {
+        const int nl = (int)lev.size() - l;
+        if (nl > BOTTOM_LEVELS || lev[l].npts() > BOTTOM_PTS || op[l] > 1) return MGX_UNSUPPORTED;
+        for (int k = l; k < (int)lev.size(); k++)
+            if (op[k] != op[l]) return MGX_UNSUPPORTED;
+        return dtype == MGX_F64 ? bottom_t<double>(l, nl) : bottom_t<float>(l, nl);
+    }
+
+    template <typename T>
+    int bottom_t(int l, int nl)
+    {
+        BottomParams<T> p;
+        p.nlev = nl;
+        p.nu1  = nu1;
+        p.nu2  = nu2;
+        for (int k = 0; k < nl; k++)
+        {
+            const Level& L        = lev[l + k];
+            const StencilCoeffs c = stencil_coeffs(op[l], L.h);
+            for (int i = 0; i < 3; i++)
+                p.n[k][i] = L.n[i];
+            p.c0[k]    = (T)c.c0;
+            p.cf[k][0] = (T)c.cx[0];
+            p.cf[k][1] = (T)c.cy[0];
+            p.cf[k][2] = (T)c.cz[0];
+            p.ce[k][0] = (T)c.cxz;
+            p.ce[k][1] = (T)c.cyz;
+            p.ce[k][2] = (T)c.cxy;
+            p.jf[k]    = (T)jf[l + k];
+        }
+        p.f = (const T*)f[l];
+        p.x = (T*)x0[l];
+        if (op[l] == 0)
+            bottom_kernel<T, 0><<<1, 256, 0, s>>>(p);
+        else
+            bottom_kernel<T, 1><<<1, 256, 0, s>>>(p);
+        MGX_LAUNCH_CHECK("bottom_kernel");
+        return MGX_OK;
     }
 
     // Vcycle at level l from x = 0; returns the buffer (0: x0, 1: x1) that
     // holds the result, or a negative status
     int cycle(int l)
     {
-        const size_t bytes = lev[l].npts() * es;
-        int st = cuda_check(cudaMemsetAsync(x0[l], 0, bytes, s), "mgm zero");
+        int st = bottom(l);
+        if (st == MGX_OK) return 0;
+        if (st != MGX_UNSUPPORTED) return -st - 1;
+        int cur      = 0;
+        auto X       = [&](int b) { return b ? x1[l] : x0[l]; };
+        const size_t np = lev[l].npts();
+        // the first sweep from x = 0 is x = jf f, and the second one reads f
+        // times jf where its kernel can
+        int done = std::min(nu1, 1);
+        if (nu1 >= 2)
+        {
+            st = sweep(l, f[l], x1[l], nullptr, jf[l], jf[l]);
+            if (st == MGX_OK)
+            {
+                done = 2;
+                cur  = 1;
+            }
+            else if (st != MGX_UNSUPPORTED)
+                return -st - 1;
+        }
+        if (done == 0)
+            st = cuda_check(cudaMemsetAsync(x0[l], 0, np * es, s), "mgm zero");
+        else if (done == 1)
+            st = scale_launch(dtype, f[l], np, x0[l], np, np, 1, jf[l], s);
         if (st != MGX_OK) return -st - 1;
-        int cur = 0;
-        auto X  = [&](int b) { return b ? x1[l] : x0[l]; };
-        for (int i = 0; i < nu1; i++)
+        for (int i = done; i < nu1; i++)
         {
             st = sweep(l, X(cur), X(cur ^ 1), nullptr, jf[l]);
             if (st != MGX_OK) return -st - 1;

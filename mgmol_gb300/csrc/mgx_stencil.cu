@@ -1747,7 +1747,10 @@ __global__ void __launch_bounds__(256) direct_kernel(PlaneParams p, DevCoef<T> c
     const int nx = p.n[0], ny = p.n[1], nz = p.n[2];
     const size_t npts = (size_t)nx * ny * nz;
     const int f       = blockIdx.y;
-    const T* ub       = reinterpret_cast<const T*>(p.u) + (size_t)f * p.ldu;
+    const bool scaled = is_jacobi(OP) && p.gamma_in != 0.; // first sweep from gamma f
+    const T gam       = scaled ? (T)p.gamma_in : (T)1;
+    const T* ub       = reinterpret_cast<const T*>(scaled ? p.f : p.u)
+                  + (size_t)f * (scaled ? p.ldf : p.ldu);
     const TV* vb      = reinterpret_cast<const TV*>(p.V);
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < npts;
          idx += (size_t)gridDim.x * blockDim.x)
@@ -1756,8 +1759,9 @@ __global__ void __launch_bounds__(256) direct_kernel(PlaneParams p, DevCoef<T> c
         const int y = (int)((idx / nz) % ny);
         const int x = (int)(idx / ((size_t)nz * ny));
         auto at     = [&](int dx, int dy, int dz) -> T {
-            return ub[((size_t)wrap(x + dx, nx) * ny + wrap(y + dy, ny)) * nz
-                      + wrap(z + dz, nz)];
+            const T v = ub[((size_t)wrap(x + dx, nx) * ny + wrap(y + dy, ny)) * nz
+                           + wrap(z + dz, nz)];
+            return scaled ? gam * v : v;
         };
         auto vat = [&](int dx, int dy, int dz) -> TV {
             return vb[((size_t)wrap(x + dx, nx) * ny + wrap(y + dy, ny)) * nz
@@ -1969,7 +1973,7 @@ static int launch_t(const PlaneParams& p0, const DevCoef<T>& c, int nfunc,
     }
     if (OP == OP_JACOBI_RST)
         return fail(MGX_UNSUPPORTED, "the fused restriction needs the vector kernel, no masks");
-    if (p0.gamma_in != 0.)
+    if (p0.gamma_in != 0. && !force_direct)
         return fail(MGX_UNSUPPORTED, "scaled first sweep needs the vector kernel");
     PlaneParams p = p0;
     constexpr int S  = stages_for<LAP, OP, R>();
@@ -2024,9 +2028,11 @@ static int launch_t(const PlaneParams& p0, const DevCoef<T>& c, int nfunc,
         return MGX_OK;
     }
     const size_t npts = (size_t)nx * ny * nz;
-    int bx            = (int)std::min<size_t>((npts + 255) / 256, 4096);
+    // small blocks spread a small grid over the SMs
+    const int nt = npts * nfunc <= 65536 ? 64 : 256;
+    int bx       = (int)std::min<size_t>((npts + nt - 1) / nt, 4096);
     dim3 grid(bx, nfunc);
-    direct_kernel<T, TV, LAP, OP, R><<<grid, 256, 0, stream>>>(p, c);
+    direct_kernel<T, TV, LAP, OP, R><<<grid, nt, 0, stream>>>(p, c);
     MGX_LAUNCH_CHECK("direct_kernel");
     return MGX_OK;
 }

@@ -87,3 +87,24 @@ def test_mgm_rejects_bad_arguments():
         ctx.mgm(a, a)                       # vh and rho alias
     with pytest.raises(capi.MgxError):
         ctx.mgm(a, torch.zeros_like(a), lap_type=4, ghosts=2)   # ghosts below radius
+
+
+@pytest.mark.parametrize("n", [(8, 8, 8), (16, 8, 4), (32, 16, 16), (6, 10, 4), (40, 24, 24), (48, 8, 2)])
+@pytest.mark.parametrize("lap,nu1,nu2", [(0, 2, 2), (1, 2, 2), (0, 1, 3), (1, 0, 1), (2, 3, 0)])
+def test_mgm_small_levels(n, lap, nu1, nu2):
+    """Grids whose cycle ends in, or is nothing but, the levels that one block
+    works on in shared memory, with every kind of smoothing count."""
+    if min(n) < lap:
+        pytest.skip("below the operator's radius")
+    ll = tuple(x * 0.3 for x in n)
+    rho = synth.gaussian_wells(n, ll, 5, 78)
+    rho = rho - rho.mean()
+    vh0 = np.zeros_like(rho)
+    ref, ri = O.mgm(n, ll, lap, vh0, rho, max_sweeps=4, tol=1e-12, nu1=nu1, nu2=nu2)
+    ctx = capi.Context(n, ll)
+    for dt, tol in ((np.float64, TOL_F64), (np.float32, 1e-4)):
+        vh = _dev(vh0, dt)
+        info = ctx.mgm(vh, _dev(rho, dt), lap_type=lap, max_sweeps=4, tol=1e-12, nu1=nu1,
+                       nu2=nu2)
+        assert info["levels"] == ri["levels"]
+        assert rel_err(vh.double().cpu().numpy(), ref) < tol
