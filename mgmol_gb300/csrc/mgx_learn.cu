@@ -50,8 +50,11 @@ constexpr size_t NPARAM = 139104;
 static_assert(NPARAM == MGX_UNET_PARAMS, "parameter count");
 
 // output tile of a convolution block: TXP x TY x TZ points, one thread per
-// (y, z) column computing TXP points along x
-constexpr int TY = 8, TZ = 32, THREADS = TY * TZ;
+// (y, z) column computing TXP points along x; TY x TZ is 8 x 32, or 16 x 16 for
+// levels with fewer than 32 points along z
+constexpr int THREADS = 256;
+constexpr int WGROUP  = 16; // output channels of a group of weights
+template <int TZ> struct TileY { static constexpr int N = THREADS / TZ; };
 
 __device__ __forceinline__ int wrapi(int i, int n)
 {
@@ -59,23 +62,57 @@ __device__ __forceinline__ int wrapi(int i, int n)
     return i < 0 ? i + n : i;
 }
 
-/* stages the periodic halo tile (TXP + 2) x (TY + 2) x (TZ + 2) of CI
- * channels starting at channel c0 of function block x (channel stride
- * npts) into xs */
-template <int CI, int TXP>
-__device__ __forceinline__ void stage_halo(float* xs, const float* __restrict__ x, int c0,
-    size_t npts, int nx, int ny, int nz, int x0, int y0, int z0)
+/* asynchronous copies global -> shared: 4 bytes (zero where !on) and 16 */
+__device__ __forceinline__ void copy4(float* dst, const float* src, bool on = true)
 {
-    constexpr int HY = TY + 2, HZ = TZ + 2, HP = (TXP + 2) * HY * HZ;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src),
+        "r"(on ? 4 : 0)
+        : "memory");
+}
+__device__ __forceinline__ void copy16(float* dst, const float* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copy_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+/* The periodic halo tile (NX + 2) x (TY + 2) x (TZ + 2) around (x0, y0, z0): the
+ * offsets of its z rows in a field, wrapped once per tile, for all channels
+ * (wrapping them again for each cost more than the convolution). */
+template <int NX, int TZ, int NT>
+__device__ __forceinline__ void halo_rows(int* rows, int nx, int ny, int nz, int x0, int y0)
+{
+    constexpr int HX = NX + 2, HY = TileY<TZ>::N + 2;
+    for (int q = threadIdx.x; q < HX * HY; q += NT)
+        rows[q] = (wrapi(x0 - 1 + q / HY, nx) * ny + wrapi(y0 - 1 + q % HY, ny)) * nz;
+}
+
+/* starts the copies of CI channels of the tile, from channel c0 of function
+ * block x (channel stride npts), into xs (channel stride CS); a warp takes a z
+ * row at a time */
+template <int CI, int NX, int TZ, int CS, int NT>
+__device__ __forceinline__ void stage_halo(float* xs, const float* __restrict__ x, int c0,
+    size_t npts, int nz, int z0, const int* rows)
+{
+    constexpr int HX = NX + 2, HY = TileY<TZ>::N + 2, HZ = TZ + 2;
+    const int lane = threadIdx.x % 32;
+    const int za   = wrapi(z0 - 1 + lane, nz);
+    const int zb   = wrapi(z0 + 31 + lane, nz); // the two last of a row of 34
+#pragma unroll 1
     for (int c = 0; c < CI; c++)
     {
         const float* src = x + (size_t)(c0 + c) * npts;
-        for (int h = threadIdx.x; h < HP; h += THREADS)
+        float* dst       = xs + c * CS;
+#pragma unroll 4
+        for (int q = threadIdx.x / 32; q < HX * HY; q += NT / 32)
         {
-            const int hz = h % HZ, r = h / HZ, hy = r % HY, hx = r / HY;
-            const int gx = wrapi(x0 - 1 + hx, nx), gy = wrapi(y0 - 1 + hy, ny),
-                      gz = wrapi(z0 - 1 + hz, nz);
-            xs[c * HP + h] = src[((size_t)gx * ny + gy) * nz + gz];
+            const int o = rows[q];
+            if (lane < HZ) copy4(dst + q * HZ + lane, src + o + za);
+            if (HZ > 32 && lane < HZ - 32) copy4(dst + q * HZ + 32 + lane, src + o + zb);
         }
     }
 }
@@ -83,16 +120,23 @@ __device__ __forceinline__ void stage_halo(float* xs, const float* __restrict__ 
 /* y[f][co] = act(oscale[f] * sum_{ci, t} W[co][ci][t] x[f][ci][p + off(t)]),
  * a periodic 3x3x3 cross-correlation; CO output channels per block
  * (blockIdx.y = f * (cout / CO) + output block), CI input channels staged
- * at a time.  xf / yf: function strides of x and y. */
-template <int CI, int CO, int TXP>
-__global__ void __launch_bounds__(THREADS) conv_fwd_kernel(const float* __restrict__ x,
-    size_t xf, int cin, const __nv_bfloat16* __restrict__ W, float* __restrict__ y, size_t yf,
+ * at a time, the next ones on their way while these are used.  W: FP32 values
+ * in the order of weight_index.  xf / yf: function strides of x and y.  Bound by
+ * the FP32 multiply-adds, which are issued for two output channels at once (a
+ * pair of weights times one value twice), so that half the issue slots are left
+ * for the shared-memory reads. */
+template <int CI, int CO, int TXP, int TZ>
+__global__ void __launch_bounds__(THREADS, 2) conv_fwd_kernel(const float* __restrict__ x,
+    size_t xf, int cin, const float* __restrict__ W, float* __restrict__ y, size_t yf,
     int cout, int nx, int ny, int nz, int relu, const float* __restrict__ oscale)
 {
+    constexpr int TY = TileY<TZ>::N;
     constexpr int HY = TY + 2, HZ = TZ + 2, HP = (TXP + 2) * HY * HZ;
-    extern __shared__ __align__(16) float smem[];
-    float* xs = smem;           // CI * HP
-    float* ws = smem + CI * HP; // [c][tap][co]
+    constexpr int C2 = CO > 1 ? CO / 2 : 1;
+    constexpr int CG = CO > 1 ? WGROUP : 1; // output channels of a weight group
+    constexpr int BUF = CI * 27 * CO + CI * HP;
+    extern __shared__ __align__(16) float smem[]; // two of: weights [c][tap][co], x CI * HP
+    __shared__ int rows[(TXP + 2) * HY];
     const int ntz = (nz + TZ - 1) / TZ, nty = (ny + TY - 1) / TY;
     int t          = blockIdx.x;
     const int z0   = (t % ntz) * TZ;
@@ -105,23 +149,41 @@ __global__ void __launch_bounds__(THREADS) conv_fwd_kernel(const float* __restri
     const int ty = threadIdx.x / TZ, tz = threadIdx.x % TZ;
     const float* xb = x + (size_t)f * xf;
 
-    float acc[TXP][CO];
+    float2 acc[TXP][C2]; // channels 2 q and 2 q + 1 (CO 1: the first alone)
 #pragma unroll
     for (int p = 0; p < TXP; p++)
 #pragma unroll
-        for (int o = 0; o < CO; o++)
-            acc[p][o] = 0.f;
+        for (int o = 0; o < C2; o++)
+            acc[p][o] = make_float2(0.f, 0.f);
 
-    for (int ci0 = 0; ci0 < cin; ci0 += CI)
+    auto stage = [&](int k) {
+        float* ws       = smem + (k & 1) * (BUF + 3) / 4 * 4;
+        const float* wg = W + ((size_t)(cob * CO / CG) * cin + k * CI) * 27 * CG + cob * CO % CG;
+        if constexpr (CO % 4 == 0)
+            for (int i = threadIdx.x; i < CI * 27 * CO / 4; i += THREADS)
+                copy16(ws + 4 * i, wg + (i / (CO / 4)) * CG + 4 * (i % (CO / 4)));
+        else
+            for (int i = threadIdx.x; i < CI * 27 * CO; i += THREADS)
+                copy4(ws + i, wg + i);
+        stage_halo<CI, TXP, TZ, HP, THREADS>(ws + CI * 27 * CO, xb, k * CI, npts, nz, z0, rows);
+        copy_commit();
+    };
+    const int nk = cin / CI;
+    halo_rows<TXP, TZ, THREADS>(rows, nx, ny, nz, x0, y0);
+    __syncthreads();
+    stage(0);
+    for (int k = 0; k < nk; k++)
     {
-        __syncthreads();
-        stage_halo<CI, TXP>(xs, xb, ci0, npts, nx, ny, nz, x0, y0, z0);
-        for (int i = threadIdx.x; i < CI * 27 * CO; i += THREADS)
+        if (k + 1 < nk)
         {
-            const int o = i % CO, r = i / CO, tap = r % 27, c = r / 27;
-            ws[i] = __bfloat162float(W[((size_t)(cob * CO + o) * cin + ci0 + c) * 27 + tap]);
+            stage(k + 1);
+            copy_wait<1>();
         }
+        else
+            copy_wait<0>();
         __syncthreads();
+        const float* ws = smem + (k & 1) * (BUF + 3) / 4 * 4;
+        const float* xs = ws + CI * 27 * CO;
 #pragma unroll 1
         for (int c = 0; c < CI; c++)
         {
@@ -149,28 +211,26 @@ __global__ void __launch_bounds__(THREADS) conv_fwd_kernel(const float* __restri
 #pragma unroll
                                 for (int p = 0; p < TXP; p++)
                                 {
-                                    const float v = col[p + dx];
-                                    acc[p][4 * q + 0] = fmaf(w4.x, v, acc[p][4 * q + 0]);
-                                    acc[p][4 * q + 1] = fmaf(w4.y, v, acc[p][4 * q + 1]);
-                                    acc[p][4 * q + 2] = fmaf(w4.z, v, acc[p][4 * q + 2]);
-                                    acc[p][4 * q + 3] = fmaf(w4.w, v, acc[p][4 * q + 3]);
+                                    const float2 v = make_float2(col[p + dx], col[p + dx]);
+                                    acc[p][2 * q]
+                                        = __ffma2_rn(make_float2(w4.x, w4.y), v, acc[p][2 * q]);
+                                    acc[p][2 * q + 1]
+                                        = __ffma2_rn(make_float2(w4.z, w4.w), v, acc[p][2 * q + 1]);
                                 }
                             }
                         }
                         else
                         {
+                            static_assert(CO == 1 || CO % 4 == 0, "output channels of a block");
+                            const float w = wv[0];
 #pragma unroll
-                            for (int o = 0; o < CO; o++)
-                            {
-                                const float w = wv[o];
-#pragma unroll
-                                for (int p = 0; p < TXP; p++)
-                                    acc[p][o] = fmaf(w, col[p + dx], acc[p][o]);
-                            }
+                            for (int p = 0; p < TXP; p++)
+                                acc[p][0].x = fmaf(w, col[p + dx], acc[p][0].x);
                         }
                     }
                 }
         }
+        __syncthreads(); // the buffer is filled again two steps on
     }
     const float sc = oscale ? oscale[f] : 1.f;
     const int gy = y0 + ty, gz = z0 + tz;
@@ -185,7 +245,7 @@ __global__ void __launch_bounds__(THREADS) conv_fwd_kernel(const float* __restri
 #pragma unroll
         for (int o = 0; o < CO; o++)
         {
-            float v = acc[p][o] * sc;
+            float v = (o & 1 ? acc[p][o / 2].y : acc[p][o / 2].x) * sc;
             if (relu) v = fmaxf(v, 0.f);
             yb[(size_t)o * npts + idx] = v;
         }
@@ -193,34 +253,52 @@ __global__ void __launch_bounds__(THREADS) conv_fwd_kernel(const float* __restri
 }
 
 /* dW[co][ci][t] += sum_{f, p} dy[f][co][p] x[f][ci][p + off(t)] over the
- * points of the blocks' tiles (TXW = 2 planes of x).  A thread owns one
- * (input channel, tap) pair and CO output channels; PS threads split the
- * points of a tile between them.  blockIdx.y = output block * (cin / CI)
- * + input block; blocks stride over (function, tile) items. */
-constexpr int TXW = 2;
-template <int CI, int CO, int PS>
-__global__ void __launch_bounds__(THREADS) conv_wgrad_kernel(const float* __restrict__ x,
+ * points of the blocks' tiles (TXW = 2 planes of x).  A thread owns an input
+ * channel, the x offset of the taps and NCO output channels: their 9 NCO sums
+ * stay in registers while it walks segments of 8 points along z, whose 3 x 10
+ * values of x and 8 NCO of dy it reads once (72 multiply-adds per 5 reads of
+ * shared memory; a thread per tap made 16 per 5).  PS groups of threads
+ * split the segments.  blockIdx.y = output block * (cin / CI) + input block;
+ * blocks stride over (function, tile) items. */
+constexpr int TXW = 2, WT = 192;
+template <int CI, int CO, int TZ>
+struct Wgrad
+{
+    static constexpr int NCO = CO >= 8 ? 8 : 1, G = CO / NCO;
+    static constexpr int PS = WT / (CI * 3 * G);
+    static constexpr int TY = TileY<TZ>::N, HY = TY + 2, HZ = TZ + 2, HP = (TXW + 2) * HY * HZ;
+    // channel stride of x: the 8 channels and 3 x offsets of a warp in 24
+    // different banks
+    static constexpr int CS = HP + ((TZ == 32 ? 1 : 11) - HP % 32 + 32) % 32;
+    static constexpr int NP = TXW * TY * TZ, SEG = NP / 8;
+    static constexpr size_t smem = (size_t)(CI * CS + 3) / 4 * 16 + (size_t)NP * CO * 4;
+    static_assert(PS * CI * 3 * G == WT && SEG % PS == 0, "threads");
+    static_assert(CI * 27 * CO * 4 <= smem, "the block's sums fit its buffers");
+};
+template <int CI, int CO, int TZ>
+__global__ void __launch_bounds__(WT) conv_wgrad_kernel(const float* __restrict__ x,
     int cin, const float* __restrict__ dy, int cout, float* __restrict__ dW, int nf, int nx,
     int ny, int nz)
 {
-    static_assert(CI * 27 * PS <= THREADS, "threads");
-    constexpr int HY = TY + 2, HZ = TZ + 2, HP = (TXW + 2) * HY * HZ, NP = TXW * TY * TZ;
+    using K = Wgrad<CI, CO, TZ>;
+    constexpr int NCO = K::NCO, N2 = NCO > 1 ? NCO / 2 : 1, TY = K::TY, HY = K::HY, HZ = K::HZ;
     extern __shared__ __align__(16) float smem[];
-    float* xs  = smem;           // CI * HP
-    float* dys = smem + CI * HP; // [p][co]
+    float* xs  = smem;                            // CI * CS
+    float* dys = smem + (CI * K::CS + 3) / 4 * 4; // [p][co]
+    __shared__ int rows[(TXW + 2) * HY];
     const int ncib = cin / CI;
     const int cob = blockIdx.y / ncib, cib = blockIdx.y % ncib;
-    const int q = threadIdx.x % (CI * 27), sp = threadIdx.x / (CI * 27);
-    const bool active = sp < PS;
-    const int c = q / 27, tap = q % 27;
-    const int dx = tap / 9, dyy = (tap / 3) % 3, dz = tap % 3;
+    const int dx = threadIdx.x % 3, c = threadIdx.x / 3 % CI, cg = threadIdx.x / (3 * CI) % K::G,
+              sp = threadIdx.x / (3 * CI * K::G);
     const int ntz = (nz + TZ - 1) / TZ, nty = (ny + TY - 1) / TY, ntx = (nx + TXW - 1) / TXW;
     const int ntiles  = ntx * nty * ntz;
     const size_t npts = (size_t)nx * ny * nz;
-    float acc[CO];
+    float2 acc[9][N2];
 #pragma unroll
-    for (int o = 0; o < CO; o++)
-        acc[o] = 0.f;
+    for (int t = 0; t < 9; t++)
+#pragma unroll
+        for (int o = 0; o < N2; o++)
+            acc[t][o] = make_float2(0.f, 0.f);
     for (int item = blockIdx.x; item < nf * ntiles; item += gridDim.x)
     {
         const int f = item / ntiles;
@@ -230,51 +308,81 @@ __global__ void __launch_bounds__(THREADS) conv_wgrad_kernel(const float* __rest
         const int y0 = (t % nty) * TY;
         const int x0 = (t / nty) * TXW;
         __syncthreads();
-        stage_halo<CI, TXW>(xs, x + (size_t)f * cin * npts, cib * CI, npts, nx, ny, nz, x0, y0,
-            z0);
-        for (int i = threadIdx.x; i < NP * CO; i += THREADS)
-        {
-            const int p = i % NP, o = i / NP;
-            const int px = x0 + p / (TY * TZ), py = y0 + (p / TZ) % TY, pz = z0 + p % TZ;
-            float v = 0.f;
-            if (px < nx && py < ny && pz < nz)
-                v = dy[((size_t)f * cout + cob * CO + o) * npts + ((size_t)px * ny + py) * nz + pz];
-            dys[p * CO + o] = v;
-        }
+        halo_rows<TXW, TZ, WT>(rows, nx, ny, nz, x0, y0);
         __syncthreads();
-        if (active)
+        stage_halo<CI, TXW, TZ, K::CS, WT>(xs, x + (size_t)f * cin * npts, cib * CI, npts, nz, z0,
+            rows);
+        for (int i = threadIdx.x; i < K::NP * CO; i += WT)
         {
-            const float* xt = xs + c * HP + (dx * HY + dyy) * HZ + dz;
-            for (int p = sp; p < NP; p += PS)
-            {
-                const int px = p / (TY * TZ), py = (p / TZ) % TY, pz = p % TZ;
-                const float xv = xt[(px * HY + py) * HZ + pz];
-                const float* dv = dys + p * CO;
-                if constexpr (CO % 4 == 0)
-                {
+            const int p = i % K::NP, o = i / K::NP;
+            const int px = x0 + p / (TY * TZ), py = y0 + (p / TZ) % TY, pz = z0 + p % TZ;
+            const bool in = px < nx && py < ny && pz < nz;
+            copy4(dys + p * CO + o,
+                dy + (in ? ((size_t)f * cout + cob * CO + o) * npts + ((size_t)px * ny + py) * nz + pz
+                         : 0),
+                in);
+        }
+        copy_commit();
+        copy_wait<0>();
+        __syncthreads();
+#pragma unroll 1
+        for (int g = sp; g < K::SEG; g += K::PS)
+        {
+            const int row = g / (TZ / 8), pz = 8 * (g % (TZ / 8)); // row: (x, y) of the tile
+            const float* xt = xs + c * K::CS + ((row / TY + dx) * HY + row % TY) * HZ + pz;
+            const float* dv = dys + (row * TZ + pz) * CO + cg * NCO;
+            float w[3][10];
 #pragma unroll
-                    for (int o4 = 0; o4 < CO / 4; o4++)
-                    {
-                        const float4 d4 = reinterpret_cast<const float4*>(dv)[o4];
-                        acc[4 * o4 + 0] = fmaf(d4.x, xv, acc[4 * o4 + 0]);
-                        acc[4 * o4 + 1] = fmaf(d4.y, xv, acc[4 * o4 + 1]);
-                        acc[4 * o4 + 2] = fmaf(d4.z, xv, acc[4 * o4 + 2]);
-                        acc[4 * o4 + 3] = fmaf(d4.w, xv, acc[4 * o4 + 3]);
-                    }
+            for (int d = 0; d < 3; d++)
+#pragma unroll
+                for (int i = 0; i < 10; i++)
+                    w[d][i] = xt[d * HZ + i];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+            {
+                float2 d2[N2];
+                if constexpr (NCO == 8)
+                {
+                    const float4 a = reinterpret_cast<const float4*>(dv + i * CO)[0];
+                    const float4 b = reinterpret_cast<const float4*>(dv + i * CO)[1];
+                    d2[0] = make_float2(a.x, a.y);
+                    d2[1] = make_float2(a.z, a.w);
+                    d2[2] = make_float2(b.x, b.y);
+                    d2[3] = make_float2(b.z, b.w);
                 }
                 else
-                {
+                    d2[0] = make_float2(dv[i * CO], 0.f);
 #pragma unroll
-                    for (int o = 0; o < CO; o++)
-                        acc[o] = fmaf(dv[o], xv, acc[o]);
+                for (int t = 0; t < 9; t++)
+                {
+                    const float v = w[t / 3][i + t % 3];
+#pragma unroll
+                    for (int o = 0; o < N2; o++)
+                        if constexpr (NCO == 8)
+                            acc[t][o] = __ffma2_rn(d2[o], make_float2(v, v), acc[t][o]);
+                        else
+                            acc[t][o].x = fmaf(d2[o].x, v, acc[t][o].x);
                 }
             }
         }
     }
-    if (!active) return;
+    // the PS groups meet in shared memory, the blocks in dW
+    __syncthreads();
+    for (int i = threadIdx.x; i < CI * 27 * CO; i += WT)
+        xs[i] = 0.f;
+    __syncthreads();
 #pragma unroll
-    for (int o = 0; o < CO; o++)
-        atomicAdd(&dW[((size_t)(cob * CO + o) * cin + cib * CI + c) * 27 + tap], acc[o]);
+    for (int t = 0; t < 9; t++)
+#pragma unroll
+        for (int o = 0; o < NCO; o++)
+            atomicAdd(xs + (c * 27 + dx * 9 + t) * CO + cg * NCO + o,
+                o & 1 ? acc[t][o / 2].y : acc[t][o / 2].x);
+    __syncthreads();
+    for (int i = threadIdx.x; i < CI * 27 * CO; i += WT)
+    {
+        const int o = i % CO, r = i / CO; // r = channel * 27 + tap
+        atomicAdd(&dW[((size_t)(cob * CO + o) * cin + cib * CI) * 27 + r], xs[i]);
+    }
 }
 
 /* ---------------- pointwise kernels ---------------- */
@@ -381,18 +489,27 @@ __global__ void __launch_bounds__(256) loss_kernel(const float* __restrict__ y,
     if (threadIdx.x == 0) atomicAdd(loss, s * lscale);
 }
 
-// w = bf16(m); wt[ci][co][26 - t] = bf16(m[co][ci][t]) (the flipped,
-// transposed kernel of the data gradient)
+/* Place of weight (co, ci, tap) of a convolution cin -> cout: groups of WGROUP
+ * output channels (one, for a single output), their channels next to each
+ * other, which is how conv_fwd_kernel stages and reads them. */
+__host__ __device__ inline size_t weight_index(int cin, int cout, int co, int ci, int tap)
+{
+    const int g = cout % WGROUP == 0 ? WGROUP : 1;
+    return ((size_t)(co / g * cin + ci) * 27 + tap) * g + co % g;
+}
+
+// w: the master weights rounded to bf16, as FP32 values; wt: those of the data
+// gradient's convolution cout -> cin, wt(ci, co, 26 - t) = w(co, ci, t)
 __global__ void __launch_bounds__(256) to_bf16_kernel(const float* __restrict__ m,
-    __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt, int cin, int cout)
+    float* __restrict__ w, float* __restrict__ wt, int cin, int cout)
 {
     const int n = cin * cout * 27;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     {
         const int t = i % 27, r = i / 27, ci = r % cin, co = r / cin;
-        const __nv_bfloat16 b = __float2bfloat16_rn(m[i]);
-        w[i]                                     = b;
-        wt[((size_t)ci * cout + co) * 27 + 26 - t] = b;
+        const float b = __bfloat162float(__float2bfloat16_rn(m[i]));
+        w[weight_index(cin, cout, co, ci, t)]       = b;
+        wt[weight_index(cout, cin, ci, co, 26 - t)] = b;
     }
 }
 
@@ -440,83 +557,100 @@ inline dim3 pw_grid(size_t n, int rows = 1)
 }
 
 /* ---------------- launchers ---------------- */
-template <int CI, int CO, int TXP> constexpr size_t conv_smem()
-{
-    return (size_t)(CI * (TXP + 2) * (TY + 2) * (TZ + 2) + CI * 27 * CO) * sizeof(float);
-}
-template <int CI, int CO> constexpr size_t wgrad_smem()
-{
-    return (size_t)(CI * (TXW + 2) * (TY + 2) * (TZ + 2) + TXW * TY * TZ * CO) * sizeof(float);
-}
-
-template <int CI, int CO>
-int conv_launch_t(const float* x, size_t xf, int cin, const __nv_bfloat16* W, float* y,
+template <int CI, int CO, int TXP, int TZ>
+int conv_launch_t(const float* x, size_t xf, int cin, const float* W, float* y,
     size_t yf, int cout, const Level& L, int nf, bool relu, const float* oscale, cudaStream_t s)
 {
-    constexpr int TXP = 4;
-    constexpr size_t sm = conv_smem<CI, CO, TXP>();
-    static bool attr    = false;
-    if (!attr)
-    {
-        MGX_TRY(cuda_check(cudaFuncSetAttribute(conv_fwd_kernel<CI, CO, TXP>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
-            "conv smem"));
-        attr = true;
-    }
+    constexpr int TY    = TileY<TZ>::N;
+    constexpr size_t sm
+        = 2 * (size_t)((CI * (TXP + 2) * (TY + 2) * (TZ + 2) + CI * 27 * CO + 3) / 4 * 4) * sizeof(float);
+    MGX_TRY(cuda_check(cudaFuncSetAttribute(conv_fwd_kernel<CI, CO, TXP, TZ>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
+        "conv smem"));
     const long tiles = (long)((L.n[0] + TXP - 1) / TXP) * ((L.n[1] + TY - 1) / TY)
         * ((L.n[2] + TZ - 1) / TZ);
     const long rows = (long)nf * (cout / CO);
     if (rows > 65535) return fail(MGX_BAD_ARG, "conv: %ld function-channel blocks", rows);
-    conv_fwd_kernel<CI, CO, TXP><<<dim3((unsigned)tiles, (unsigned)rows), THREADS, sm, s>>>(x, xf,
-        cin, W, y, yf, cout, L.n[0], L.n[1], L.n[2], relu ? 1 : 0, oscale);
+    conv_fwd_kernel<CI, CO, TXP, TZ><<<dim3((unsigned)tiles, (unsigned)rows), THREADS, sm, s>>>(x,
+        xf, cin, W, y, yf, cout, L.n[0], L.n[1], L.n[2], relu ? 1 : 0, oscale);
     MGX_LAUNCH_CHECK("conv_fwd_kernel");
     return MGX_OK;
 }
 
-int conv_launch(const float* x, size_t xf, int cin, const __nv_bfloat16* W, float* y, size_t yf,
-    int cout, const Level& L, int nf, bool relu, const float* oscale, cudaStream_t s)
+/* Columns of TXP points along x and CO output channels; half of the one, and
+ * then of the other, where the blocks would leave SMs with one or none (the
+ * halo and the reads of shared memory weigh more per multiply-add then). */
+template <int CI, int CO, int TXP>
+int conv_launch_z(const float* x, size_t xf, int cin, const float* W, float* y, size_t yf,
+    int cout, const Level& L, int nf, bool relu, const float* oscale, int sms, cudaStream_t s)
+{
+    const bool narrow = L.n[2] <= 16;
+    auto blocks = [&](int txp, int co) {
+        return (long)((L.n[0] + txp - 1) / txp)
+               * (narrow ? (L.n[1] + 15) / 16 : (long)((L.n[1] + 7) / 8) * ((L.n[2] + 31) / 32)) * nf
+               * (cout / co);
+    };
+#define MGX_CONV(CO_, TXP_)                                                                        \
+    (narrow ? conv_launch_t<CI, CO_, TXP_, 16>(x, xf, cin, W, y, yf, cout, L, nf, relu, oscale, s) \
+            : conv_launch_t<CI, CO_, TXP_, 32>(x, xf, cin, W, y, yf, cout, L, nf, relu, oscale, s))
+    if (blocks(TXP, CO) >= 2 * sms) return MGX_CONV(CO, TXP);
+    if constexpr (CO > 8)
+    {
+        if (blocks(TXP / 2, CO) < 2 * sms) return MGX_CONV(8, TXP / 2);
+    }
+    return MGX_CONV(CO, TXP / 2);
+#undef MGX_CONV
+}
+
+int conv_launch(const float* x, size_t xf, int cin, const float* W, float* y, size_t yf,
+    int cout, const Level& L, int nf, bool relu, const float* oscale, int sms, cudaStream_t s)
 {
     if (cin == 1 && cout % 16 == 0)
-        return conv_launch_t<1, 16>(x, xf, cin, W, y, yf, cout, L, nf, relu, oscale, s);
-    if (cin % 8 == 0 && cout % 16 == 0)
-        return conv_launch_t<8, 16>(x, xf, cin, W, y, yf, cout, L, nf, relu, oscale, s);
-    if (cin % 8 == 0 && cout == 1)
-        return conv_launch_t<8, 1>(x, xf, cin, W, y, yf, cout, L, nf, relu, oscale, s);
+        return conv_launch_z<1, 16, 4>(x, xf, cin, W, y, yf, cout, L, nf, relu, oscale, sms, s);
+    if (cin % 4 == 0 && cout % 16 == 0)
+        return conv_launch_z<4, 16, 4>(x, xf, cin, W, y, yf, cout, L, nf, relu, oscale, sms, s);
+    if (cin % 4 == 0 && cout == 1)
+        return conv_launch_z<4, 1, 8>(x, xf, cin, W, y, yf, cout, L, nf, relu, oscale, sms, s);
     return fail(MGX_UNSUPPORTED, "conv %d -> %d channels", cin, cout);
 }
 
-template <int CI, int CO, int PS>
+template <int CI, int CO, int TZ>
 int wgrad_launch_t(const float* x, int cin, const float* dy, int cout, float* dW,
     const Level& L, int nf, int sms, cudaStream_t s)
 {
-    constexpr size_t sm = wgrad_smem<CI, CO>();
-    static bool attr    = false;
-    if (!attr)
-    {
-        MGX_TRY(cuda_check(cudaFuncSetAttribute(conv_wgrad_kernel<CI, CO, PS>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
-            "wgrad smem"));
-        attr = true;
-    }
-    const long tiles = (long)((L.n[0] + TXW - 1) / TXW) * ((L.n[1] + TY - 1) / TY)
+    using K = Wgrad<CI, CO, TZ>;
+    MGX_TRY(cuda_check(cudaFuncSetAttribute(conv_wgrad_kernel<CI, CO, TZ>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::smem),
+        "wgrad smem"));
+    const long tiles = (long)((L.n[0] + TXW - 1) / TXW) * ((L.n[1] + K::TY - 1) / K::TY)
         * ((L.n[2] + TZ - 1) / TZ);
     const int rows   = (cout / CO) * (cin / CI);
     const long items = tiles * nf;
+    // at most four blocks per SM, each with the same number of items
     const long want  = std::max<long>(1, (long)4 * sms / rows);
-    const unsigned gx = (unsigned)std::min(items, want);
-    conv_wgrad_kernel<CI, CO, PS><<<dim3(gx, rows), THREADS, sm, s>>>(x, cin, dy, cout, dW, nf,
+    const long each  = (items + want - 1) / want;
+    const unsigned gx = (unsigned)((items + each - 1) / each);
+    conv_wgrad_kernel<CI, CO, TZ><<<dim3(gx, rows), WT, K::smem, s>>>(x, cin, dy, cout, dW, nf,
         L.n[0], L.n[1], L.n[2]);
     MGX_LAUNCH_CHECK("conv_wgrad_kernel");
     return MGX_OK;
 }
 
+template <int CI, int CO>
+int wgrad_launch_z(const float* x, int cin, const float* dy, int cout, float* dW, const Level& L,
+    int nf, int sms, cudaStream_t s)
+{
+    return L.n[2] <= 16 ? wgrad_launch_t<CI, CO, 16>(x, cin, dy, cout, dW, L, nf, sms, s)
+                        : wgrad_launch_t<CI, CO, 32>(x, cin, dy, cout, dW, L, nf, sms, s);
+}
+
 int wgrad_launch(const float* x, int cin, const float* dy, int cout, float* dW, const Level& L,
     int nf, int sms, cudaStream_t s)
 {
-    if (cin == 1 && cout % 16 == 0) return wgrad_launch_t<1, 16, 8>(x, cin, dy, cout, dW, L, nf, sms, s);
+    if (cin == 1 && cout % 16 == 0) return wgrad_launch_z<1, 16>(x, cin, dy, cout, dW, L, nf, sms, s);
     if (cin % 8 == 0 && cout % 16 == 0)
-        return wgrad_launch_t<8, 16, 1>(x, cin, dy, cout, dW, L, nf, sms, s);
-    if (cin % 8 == 0 && cout == 1) return wgrad_launch_t<8, 1, 1>(x, cin, dy, cout, dW, L, nf, sms, s);
+        return wgrad_launch_z<8, 16>(x, cin, dy, cout, dW, L, nf, sms, s);
+    if (cin % 8 == 0 && cout == 1) return wgrad_launch_z<8, 1>(x, cin, dy, cout, dW, L, nf, sms, s);
     return fail(MGX_UNSUPPORTED, "wgrad %d -> %d channels", cin, cout);
 }
 
@@ -631,13 +765,13 @@ Acts carve(mgx_unet* net, int nf, bool train)
     return A;
 }
 
-const __nv_bfloat16* W(const mgx_unet* net, int l)
+const float* W(const mgx_unet* net, int l)
 {
-    return (const __nv_bfloat16*)net->wbf.ptr + layer_offset(l);
+    return (const float*)net->wbf.ptr + layer_offset(l);
 }
-const __nv_bfloat16* Wt(const mgx_unet* net, int l)
+const float* Wt(const mgx_unet* net, int l)
 {
-    return (const __nv_bfloat16*)net->wbft.ptr + layer_offset(l);
+    return (const float*)net->wbft.ptr + layer_offset(l);
 }
 
 int refresh_bf16(mgx_unet* net, cudaStream_t s)
@@ -646,7 +780,7 @@ int refresh_bf16(mgx_unet* net, cudaStream_t s)
     {
         const size_t o = layer_offset(l);
         to_bf16_kernel<<<pw_grid(layer_size(l)), 256, 0, s>>>((const float*)net->master.ptr + o,
-            (__nv_bfloat16*)net->wbf.ptr + o, (__nv_bfloat16*)net->wbft.ptr + o, LAYERS[l].cin,
+            (float*)net->wbf.ptr + o, (float*)net->wbft.ptr + o, LAYERS[l].cin,
             LAYERS[l].cout);
         MGX_LAUNCH_CHECK("to_bf16_kernel");
     }
@@ -659,6 +793,7 @@ int forward(mgx_unet* net, const Acts& A, const float* x, size_t ld, int nf, flo
     size_t ldy, cudaStream_t s)
 {
     const Level *L = net->lev;
+    const int sms  = net->ctx->sm_count;
     const size_t n0 = L[0].npts(), n1 = L[1].npts(), n2 = L[2].npts();
     double* acc = (double*)net->red.ptr;
     float* sc   = (float*)net->scal.ptr; // s[nf], inv[nf]
@@ -671,20 +806,20 @@ int forward(mgx_unet* net, const Acts& A, const float* x, size_t ld, int nf, flo
     scale_in_kernel<<<pw_grid(n0, nf), 256, 0, s>>>(x, ld, A.xh, n0, inv);
     MGX_LAUNCH_CHECK("scale_in_kernel");
     const MaskDev none;
-    MGX_TRY(conv_launch(A.xh, n0, 1, W(net, 0), A.a0, 16 * n0, 16, L[0], nf, true, nullptr, s));
+    MGX_TRY(conv_launch(A.xh, n0, 1, W(net, 0), A.a0, 16 * n0, 16, L[0], nf, true, nullptr, sms, s));
     MGX_TRY(restrict_launch(MGX_F32, L[0], A.a0, n0, A.p1, n1, nf * 16, none, s));
-    MGX_TRY(conv_launch(A.p1, 16 * n1, 16, W(net, 1), A.a1, 32 * n1, 32, L[1], nf, true, nullptr, s));
+    MGX_TRY(conv_launch(A.p1, 16 * n1, 16, W(net, 1), A.a1, 32 * n1, 32, L[1], nf, true, nullptr, sms, s));
     MGX_TRY(restrict_launch(MGX_F32, L[1], A.a1, n1, A.p2, n2, nf * 32, none, s));
-    MGX_TRY(conv_launch(A.p2, 32 * n2, 32, W(net, 2), A.a2, 64 * n2, 64, L[2], nf, true, nullptr, s));
-    MGX_TRY(conv_launch(A.a2, 64 * n2, 64, W(net, 3), A.z2, 32 * n2, 32, L[2], nf, false, nullptr, s));
+    MGX_TRY(conv_launch(A.p2, 32 * n2, 32, W(net, 2), A.a2, 64 * n2, 64, L[2], nf, true, nullptr, sms, s));
+    MGX_TRY(conv_launch(A.a2, 64 * n2, 64, W(net, 3), A.z2, 32 * n2, 32, L[2], nf, false, nullptr, sms, s));
     MGX_TRY(prolong_launch(MGX_F32, 0, L[1], A.z2, n2, A.s1, n1, nf * 32, none, s));
     MGX_TRY(add_relu(A.s1, A.a1, (size_t)nf * 32 * n1, s));
-    MGX_TRY(conv_launch(A.s1, 32 * n1, 32, W(net, 4), A.z1, 16 * n1, 16, L[1], nf, false, nullptr, s));
+    MGX_TRY(conv_launch(A.s1, 32 * n1, 32, W(net, 4), A.z1, 16 * n1, 16, L[1], nf, false, nullptr, sms, s));
     MGX_TRY(prolong_launch(MGX_F32, 0, L[0], A.z1, n1, A.s0, n0, nf * 16, none, s));
     MGX_TRY(add_relu(A.s0, A.a0, (size_t)nf * 16 * n0, s));
     if (y)
-        return conv_launch(A.s0, 16 * n0, 16, W(net, 5), y, ldy, 1, L[0], nf, false, sc, s);
-    return conv_launch(A.s0, 16 * n0, 16, W(net, 5), A.y, n0, 1, L[0], nf, false, nullptr, s);
+        return conv_launch(A.s0, 16 * n0, 16, W(net, 5), y, ldy, 1, L[0], nf, false, sc, sms, s);
+    return conv_launch(A.s0, 16 * n0, 16, W(net, 5), A.y, n0, 1, L[0], nf, false, nullptr, sms, s);
 }
 
 /* backward pass after forward(..., y = NULL): A.gy holds d loss / d y;
@@ -698,29 +833,29 @@ int backward(mgx_unet* net, const Acts& A, int nf, float* grad, cudaStream_t s)
     auto G = [&](int l) { return grad + layer_offset(l); };
     // D0
     MGX_TRY(wgrad_launch(A.s0, 16, A.gy, 1, G(5), L[0], nf, sms, s));
-    MGX_TRY(conv_launch(A.gy, n0, 1, Wt(net, 5), A.gs0, 16 * n0, 16, L[0], nf, false, nullptr, s));
+    MGX_TRY(conv_launch(A.gy, n0, 1, Wt(net, 5), A.gs0, 16 * n0, 16, L[0], nf, false, nullptr, sms, s));
     MGX_TRY(relu_grad(A.gs0, nullptr, 0.f, A.s0, (size_t)nf * 16 * n0, s));
     // D1 (through the prolongation: P^T = 8 R)
     MGX_TRY(restrict_launch(MGX_F32, L[0], A.gs0, n0, A.gz1, n1, nf * 16, none, s));
     MGX_TRY(scale_inplace(A.gz1, 8.f, (size_t)nf * 16 * n1, s));
     MGX_TRY(wgrad_launch(A.s1, 32, A.gz1, 16, G(4), L[1], nf, sms, s));
-    MGX_TRY(conv_launch(A.gz1, 16 * n1, 16, Wt(net, 4), A.gs1, 32 * n1, 32, L[1], nf, false, nullptr, s));
+    MGX_TRY(conv_launch(A.gz1, 16 * n1, 16, Wt(net, 4), A.gs1, 32 * n1, 32, L[1], nf, false, nullptr, sms, s));
     MGX_TRY(relu_grad(A.gs1, nullptr, 0.f, A.s1, (size_t)nf * 32 * n1, s));
     // D2
     MGX_TRY(restrict_launch(MGX_F32, L[1], A.gs1, n1, A.gz2, n2, nf * 32, none, s));
     MGX_TRY(scale_inplace(A.gz2, 8.f, (size_t)nf * 32 * n2, s));
     MGX_TRY(wgrad_launch(A.a2, 64, A.gz2, 32, G(3), L[2], nf, sms, s));
-    MGX_TRY(conv_launch(A.gz2, 32 * n2, 32, Wt(net, 3), A.ga2, 64 * n2, 64, L[2], nf, false, nullptr, s));
+    MGX_TRY(conv_launch(A.gz2, 32 * n2, 32, Wt(net, 3), A.ga2, 64 * n2, 64, L[2], nf, false, nullptr, sms, s));
     MGX_TRY(relu_grad(A.ga2, nullptr, 0.f, A.a2, (size_t)nf * 64 * n2, s));
     // E2
     MGX_TRY(wgrad_launch(A.p2, 32, A.ga2, 64, G(2), L[2], nf, sms, s));
-    MGX_TRY(conv_launch(A.ga2, 64 * n2, 64, Wt(net, 2), A.gp2, 32 * n2, 32, L[2], nf, false, nullptr, s));
+    MGX_TRY(conv_launch(A.ga2, 64 * n2, 64, Wt(net, 2), A.gp2, 32 * n2, 32, L[2], nf, false, nullptr, sms, s));
     // through the restriction (R^T = P / 8) into the skip of level 1
     MGX_TRY(prolong_launch(MGX_F32, 0, L[1], A.gp2, n2, A.gt1, n1, nf * 32, none, s));
     MGX_TRY(relu_grad(A.gs1, A.gt1, 0.125f, A.a1, (size_t)nf * 32 * n1, s));
     // E1
     MGX_TRY(wgrad_launch(A.p1, 16, A.gs1, 32, G(1), L[1], nf, sms, s));
-    MGX_TRY(conv_launch(A.gs1, 32 * n1, 32, Wt(net, 1), A.gp1, 16 * n1, 16, L[1], nf, false, nullptr, s));
+    MGX_TRY(conv_launch(A.gs1, 32 * n1, 32, Wt(net, 1), A.gp1, 16 * n1, 16, L[1], nf, false, nullptr, sms, s));
     MGX_TRY(prolong_launch(MGX_F32, 0, L[0], A.gp1, n1, A.gt0, n0, nf * 16, none, s));
     MGX_TRY(relu_grad(A.gs0, A.gt0, 0.125f, A.a0, (size_t)nf * 16 * n0, s));
     // E0
@@ -838,8 +973,8 @@ int mgx_unet_create(mgx_ctx* ctx, mgx_unet** out)
     MGX_TRY(net->adam_m.ensure(pb));
     MGX_TRY(net->adam_v.ensure(pb));
     MGX_TRY(net->grad.ensure(pb));
-    MGX_TRY(net->wbf.ensure(nn::NPARAM * sizeof(__nv_bfloat16)));
-    MGX_TRY(net->wbft.ensure(nn::NPARAM * sizeof(__nv_bfloat16)));
+    MGX_TRY(net->wbf.ensure(pb));
+    MGX_TRY(net->wbft.ensure(pb));
     MGX_TRY(cuda_check(cudaMemset(net->master.ptr, 0, pb), "net zero"));
     MGX_TRY(cuda_check(cudaMemset(net->adam_m.ptr, 0, pb), "net zero"));
     MGX_TRY(cuda_check(cudaMemset(net->adam_v.ptr, 0, pb), "net zero"));
