@@ -77,6 +77,9 @@ struct Params
     float beta       = 0.f;
     int nrows        = 0;
     int ntj          = 1;
+    // columns of a tile of the persistent kernel: a multiple of 32, at most BN (0:
+    // BN)
+    int bn = 0;
     // the operand maps are K-blocked 3-D maps (rows of 64 K elements, one
     // contiguous block of all rows per 64 K) instead of row-major 2-D maps
     int blocked = 0;
@@ -326,6 +329,15 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel(
                      : "memory");
 }
 
+/* Columns of the tiles of a store product: equal tiles of at most `most`, so
+ * that 257 functions make two tiles of 160 columns and not of 256 (an MMA of n
+ * columns takes about 64 + n / 4 clocks). */
+inline int tile_cols(int ncols, int most)
+{
+    const int nt = (ncols + most - 1) / most;
+    return ((ncols + nt - 1) / nt + 31) / 32 * 32;
+}
+
 /* The persistent form of gram_kernel: one CTA per SM walks the work items
  * w = blockIdx.x, blockIdx.x + gridDim.x, ... (split-K: tile w % ntiles of
  * the list, K slice w / ntiles; store: output tile w), with two TMEM
@@ -366,13 +378,14 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
     __shared__ volatile int abort_all;
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int bn   = p.bn ? p.bn : BN;
 
     // the item's output tile and K-block range
     auto decode = [&](int w, int& i0, int& j0, int& kb0, int& nkb) {
         if (STORE)
         {
             i0  = (w / p.ntj) * BM;
-            j0  = (w % p.ntj) * BN;
+            j0  = (w % p.ntj) * bn;
             kb0 = 0;
             nkb = p.kblocks;
         }
@@ -438,7 +451,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
                     break;
                 }
                 unsigned char* st = smem + s * STAGE;
-                mbar_arrive_expect_tx(full + s, STAGE);
+                mbar_arrive_expect_tx(full + s, (uint32_t)(NOP * (A_BYTES + bn * SW)));
                 const int kc = (kb0 + it) * BK;
                 if (AMN)
                 {
@@ -475,7 +488,8 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
     }
     else if (warp == 1 && lane == 0)
     {
-        constexpr uint32_t idesc = instr_desc<KIND>(BM, BN) | (AMN ? (1u << 15) : 0u);
+        const uint32_t idesc
+            = instr_desc<KIND>(BM, 0) | ((uint32_t)(bn >> 3) << 17) | (AMN ? (1u << 15) : 0u);
         int g = 0, t = 0;
         for (int w = blockIdx.x; w < nitems && !abort_all; w += gridDim.x, t++)
         {
@@ -551,7 +565,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
             if (nkb > 0)
             {
 #pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += 32)
+                for (int c0 = 0; c0 < bn; c0 += 32)
                 {
                     float v[32];
                     tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + c0), v);
@@ -1737,14 +1751,15 @@ int psi_theta_tcgen05(mgx_ctx* ctx, int mode, const float* psi, size_t ld, size_
                 nkbf, (__nv_bfloat16*)bhi, (__nv_bfloat16*)blo, nullptr);
             MGX_LAUNCH_CHECK("matrix_split_kernel");
             const int BN = (ncols > 128) ? 256 : 128;
+            const int bn = sms ? tile_cols(ncols, BN) : BN;
             const int BK = sw / 2;
             CUtensorMap mb0, mb1, ma0, ma1;
-            MGX_TRY(make_map_blocked(&mb0, bhi, ncols, nkbf, BN, sw));
-            MGX_TRY(make_map_blocked(&mb1, blo, ncols, nkbf, BN, sw));
+            MGX_TRY(make_map_blocked(&mb0, bhi, ncols, nkbf, bn, sw));
+            MGX_TRY(make_map_blocked(&mb1, blo, ncols, nkbf, bn, sw));
             const size_t kbp = (npts + 63) / 64;
             MGX_TRY(make_map_mn(&ma0, cv.hi, (size_t)n, kbp, BK));
             MGX_TRY(make_map_mn(&ma1, cv.lo, (size_t)n, kbp, BK));
-            const int ntj = (ncols + BN - 1) / BN;
+            const int ntj = (ncols + bn - 1) / bn;
             Params p;
             p.tiles      = nullptr;
             p.kblocks    = (n + BK - 1) / BK;
@@ -1760,6 +1775,7 @@ int psi_theta_tcgen05(mgx_ctx* ctx, int mode, const float* psi, size_t ld, size_
             p.beta       = cin ? beta : 0.f;
             p.nrows      = (int)npts;
             p.ntj        = ntj;
+            p.bn         = bn;
             p.blocked    = 1;
             if (rho)
             {
@@ -1811,6 +1827,7 @@ int psi_theta_tcgen05(mgx_ctx* ctx, int mode, const float* psi, size_t ld, size_
     void* ahi = ws + b_bytes;
     void* alo = ws + b_bytes + a_plane;
     const bool blk = half || (bf && blocked_planes());
+    const bool mn  = blk && !half; // bf16 planes, rows = functions, read MN-major
     const int nkb  = (int)(ldk / 64);
     ScaleSlot* sa  = nullptr;
     ScaleSlot* sb  = nullptr;
@@ -1839,34 +1856,45 @@ int psi_theta_tcgen05(mgx_ctx* ctx, int mode, const float* psi, size_t ld, size_
         MGX_LAUNCH_CHECK("matrix_split_kernel");
     }
     const int BN = (ncols > 128) ? 256 : 128;
+    const int bn = sms ? tile_cols(ncols, BN) : BN;
     const int sw = half ? 64 : bf ? bf16_swizzle() : 128;
     CUtensorMap mb0, mb1, ma0, ma1;
     if (blk)
     {
-        MGX_TRY(make_map_blocked(&mb0, bhi, ncols, nkb, BN, sw, half));
-        MGX_TRY(make_map_blocked(&mb1, blo, ncols, nkb, BN, sw, half));
+        MGX_TRY(make_map_blocked(&mb0, bhi, ncols, nkb, bn, sw, half));
+        MGX_TRY(make_map_blocked(&mb1, blo, ncols, nkb, bn, sw, half));
     }
     else
     {
-        MGX_TRY(make_map(&mb0, bhi, bf, n, ncols, ldk, BN, sw));
+        MGX_TRY(make_map(&mb0, bhi, bf, n, ncols, ldk, bn, sw));
         mb1 = mb0;
-        if (bf) MGX_TRY(make_map(&mb1, blo, true, n, ncols, ldk, BN, sw));
+        if (bf) MGX_TRY(make_map(&mb1, blo, true, n, ncols, ldk, bn, sw));
     }
     const int bkk     = bf ? sw / 2 : 32;
     const int kblocks = (int)((n + bkk - 1) / bkk);
-    const int ntj     = (ncols + BN - 1) / BN;
+    const int ntj     = (ncols + bn - 1) / bn;
     for (size_t p0 = 0; p0 < npts; p0 += P)
     {
         const int Pc = (int)std::min(P, npts - p0);
-        if (blk)
+        if (mn)
+        {
+            // the planes of the Gram products, read MN-major: their conversion
+            // runs along the points (6.4 TB/s) where the transposing one made
+            // 2.8 TB/s
+            const size_t kbp = (size_t)(Pc + 63) / 64;
+            const int vec4   = ((ld % 4) == 0 && ((uintptr_t)(psi + p0) % 16) == 0) ? 1 : 0;
+            const int nb8    = (int)std::min<size_t>((kbp * 8 * n + 255) / 256, 1 << 20);
+            split8_kernel<__nv_bfloat16><<<nb8, 256, 0, s>>>(psi + p0, ld, n, Pc, kbp,
+                (__nv_bfloat16*)ahi, (__nv_bfloat16*)alo, nullptr, vec4);
+            MGX_LAUNCH_CHECK("split8_kernel");
+            MGX_TRY(make_map_mn(&ma0, ahi, (size_t)n, kbp, sw / 2));
+            MGX_TRY(make_map_mn(&ma1, alo, (size_t)n, kbp, sw / 2));
+        }
+        else if (blk)
         {
             dim3 tg((Pc + TB_P - 1) / TB_P, nkb);
-            if (half)
-                transpose_split_blocked_kernel<__half><<<tg, 256, 0, s>>>(psi, ld, n, p0, Pc,
-                    (__half*)ahi, (__half*)alo, sa);
-            else
-                transpose_split_blocked_kernel<__nv_bfloat16><<<tg, 256, 0, s>>>(psi, ld, n, p0,
-                    Pc, (__nv_bfloat16*)ahi, (__nv_bfloat16*)alo, nullptr);
+            transpose_split_blocked_kernel<__half><<<tg, 256, 0, s>>>(psi, ld, n, p0, Pc,
+                (__half*)ahi, (__half*)alo, sa);
             MGX_LAUNCH_CHECK("transpose_split_blocked_kernel");
             MGX_TRY(make_map_blocked(&ma0, ahi, Pc, nkb, BM, sw, half));
             MGX_TRY(make_map_blocked(&ma1, alo, Pc, nkb, BM, sw, half));
@@ -1906,6 +1934,7 @@ int psi_theta_tcgen05(mgx_ctx* ctx, int mode, const float* psi, size_t ld, size_
         p.beta       = cin ? beta : 0.f;
         p.nrows      = Pc;
         p.ntj        = ntj;
+        p.bn         = bn;
         p.blocked    = blk ? 1 : 0;
         p.sa         = sa;
         p.sb         = sb;
@@ -1916,6 +1945,17 @@ int psi_theta_tcgen05(mgx_ctx* ctx, int mode, const float* psi, size_t ld, size_
                 MGX_TRY((launch<2, 3, 256, 4, true, 64>(ma0, ma1, mb0, mb1, p, ntiles, 1, s, sms)));
             else
                 MGX_TRY((launch<2, 3, 128, 6, true, 64>(ma0, ma1, mb0, mb1, p, ntiles, 1, s, sms)));
+        }
+        else if (mn)
+        {
+            if (sw == 64 && BN == 256)
+                MGX_TRY((launch<1, 3, 256, 4, true, 64, true>(ma0, ma1, mb0, mb1, p, ntiles, 1, s, sms)));
+            else if (sw == 64)
+                MGX_TRY((launch<1, 3, 128, 6, true, 64, true>(ma0, ma1, mb0, mb1, p, ntiles, 1, s, sms)));
+            else if (BN == 256)
+                MGX_TRY((launch<1, 3, 256, 2, true, 128, true>(ma0, ma1, mb0, mb1, p, ntiles, 1, s, sms)));
+            else
+                MGX_TRY((launch<1, 3, 128, 3, true, 128, true>(ma0, ma1, mb0, mb1, p, ntiles, 1, s, sms)));
         }
         else if (BN == 256)
         {

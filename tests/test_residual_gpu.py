@@ -331,3 +331,19 @@ def test_abpg_step_lean_schedule_matches_full(mode, gemm):
     na = O.normalize(grid, ll, a.cpu().numpy().astype(np.float64))[0]
     nc = O.normalize(grid, ll, c.cpu().numpy().astype(np.float64))[0]
     assert rel_err(nc, na) < (1e-12 if mode == "plain" else 1e-6)
+
+
+@pytest.mark.parametrize("mode", [capi.GEMM_TF32, capi.GEMM_BF16X3, capi.GEMM_FP16X3])
+@pytest.mark.parametrize("nf,grid", [(33, (16, 9, 12)), (130, (16, 9, 12)), (257, (17, 8, 12)),
+                                     (290, (20, 16, 8))])
+def test_mult_matrix_tile_columns(mode, nf, grid):
+    """Psi Theta on column tiles of 64, 96, 160 and 160 columns (equal tiles, the
+    last one partly empty), point counts that end inside a 128-point tile."""
+    ll = tuple(x * 0.35 for x in grid)
+    psi, _, _ = synth.gaussian_orbitals(grid, ll, nf, 37)
+    th = _theta(nf, 37)
+    ctx = capi.Context(grid, ll)
+    dp = _dev(psi, np.float32)
+    out = ctx.mult_matrix(dp, _dev(th), mode).double()
+    ref = _dev(th).T @ dp.double()
+    assert float((out - ref).abs().max() / ref.abs().max()) < TOL[mode]
