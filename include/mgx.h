@@ -643,7 +643,9 @@ int mgx_precond_learned(mgx_ctx* ctx, mgx_unet* net, const mgx_precond_params* p
  * centres and radii, so the same boxes.  Each box extent must leave room for
  * a halo of 3 points inside the grid.  Both mask sets must outlive the
  * handle, and the boxes are read once: after mgx_masks_update moves the
- * centres, create the handle again. */
+ * centres, create the handle again.  (An update that leaves the boxes as they
+ * are keeps the handle usable; the step then visits whole boxes instead of the
+ * points that the masks reached at creation.) */
 typedef struct mgx_local mgx_local;
 
 int mgx_local_create(mgx_ctx* ctx, const mgx_masks* masks, const mgx_masks* corr,
@@ -669,9 +671,8 @@ int mgx_local_scatter(mgx_local* loc, const float* packed, float* full, size_t l
  * argument or the configuration changes. */
 int mgx_local_step(mgx_local* loc, const float* psi, const float* phi, const float* V,
     double gamma, float* u, float* w, void* stream);
-/* times every kernel variant (largest column TY x TZ, fitted to each box,
- * and planes per march step; 0: 24x32, 1: 16x32, 2: 32x32 with one plane,
- * 3..5 the same with two) with 1, 2, 3 and 4 resident CTAs per SM on these
+/* times every kernel variant (threads per CTA, which bound the columns that the
+ * boxes are cut into; 0..5: 256, 320, 384, 448, 640, 768) with 1, 2, 3 and 4 resident CTAs per SM on these
  * arguments and keeps the fastest; ms
  * (optional, *ncand entries) receives each candidate's time (-1: not
  * resident), *ncand the number of candidates */

@@ -21,11 +21,10 @@
 // what the V-cycle restricts next.
 //
 // One CTA takes (orbital, column) items from a work list until it is empty
-// (largest boxes first); a column is a TY x TZ window of the box marched
-// along x, each stage keeping three planes in shared memory, so the
-// orbital block is read once (plus the y / z halo) and u2, w written once.
-// The column shape and the CTAs per SM are chosen by timing
-// (mgx_local_tune); the launch can be a CUDA graph.
+// (largest orbitals first); a column is a window of the orbital's y and z
+// marched along x, so the orbital block is read once (plus the y / z halo)
+// and u2, w written once.  The threads per CTA and the CTAs per SM are chosen
+// by timing (mgx_local_tune); the launch can be a CUDA graph.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,8 +39,13 @@ namespace mgx
 {
 namespace loc
 {
-constexpr int THREADS = 256;
-constexpr int HALO    = 3;
+constexpr int HALO = 3;
+
+/* -Delta_M-like stencil: centre, faces, edges */
+struct Stencil19
+{
+    float c0, cx, cy, cz, cxy, cyz, cxz;
+};
 
 struct StepParams
 {
@@ -51,17 +55,25 @@ struct StepParams
     float* u;
     float* w;
     const int* box;       // 6 per orbital: origin, extents
+    const int* core;      // 6 per orbital: the box points with a mask that is not zero lie in
+                          // [core0, core3) x [core1, core4) x [core2, core5)
+    const int* range;     // per box column (y, z): they lie in x of [r & 0xffff, r >> 16); NULL:
+                          // the whole box
+    const size_t* roff;   // offset of an orbital's columns
     const size_t* off;    // packed offset of each orbital
     const float* mvals;   // orbital mask values, box-local
     const size_t* moff;
     const float* cvals;   // correction mask values, box-local
     const size_t* coff;
-    const int4* items;    // (orbital, 0, column origin y, z)
+    const int4* items;    // (orbital, ty | tz << 16, column origin y, z), or (orbital, 0, 0, 0):
+                          // the points outside the core
     int nitems;
     int* counter;
     int n[3];
-    float c0, cx, cy, cz, cxy, cyz, cxz; // -Delta_M
-    float gamma, jf;
+    Stencil19 lap;        // Delta_M (stage 1)
+    Stencil19 sweep;      // gamma r - jf (A gamma r - r) of r (stage 2)
+    Stencil19 A;          // -Delta_M (stage 3)
+    float jf;
 };
 
 __device__ __forceinline__ int wrapi(int i, int n)
@@ -77,86 +89,38 @@ __device__ __forceinline__ float clampm(float v, float m)
     return v;
 }
 
-/* -Delta_M at index i of plane C, with the x neighbours in planes M and P
- * (plane stride sy along y, 1 along z) */
-__device__ __forceinline__ float lap_m(const float* M, const float* C, const float* Pn, int i,
-    int sy, const StepParams& P)
-{
-    const float faces = P.cx * (M[i] + Pn[i]) + P.cy * (C[i - sy] + C[i + sy])
-        + P.cz * (C[i - 1] + C[i + 1]);
-    const float exy = M[i - sy] + M[i + sy] + Pn[i - sy] + Pn[i + sy];
-    const float eyz = C[i - sy - 1] + C[i - sy + 1] + C[i + sy - 1] + C[i + sy + 1];
-    const float exz = M[i - 1] + M[i + 1] + Pn[i - 1] + Pn[i + 1];
-    return P.c0 * C[i] + faces + P.cxy * exy + P.cyz * eyz + P.cxz * exz;
-}
+__device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
 
-/* B = 1/2 + (1/12) sum of the six faces (FDkernelRHS_4th_Mehr1) */
-__device__ __forceinline__ float rhs_b(const float* M, const float* C, const float* Pn, int i,
-    int sy)
+/* the sums of a plane at a z pair (index i, odd, of the pair's first value):
+ * the pair itself, its y neighbours, its z neighbours, its y-z diagonals.
+ * Six 8-byte loads: the pair lies across two of them, so that (z - 1, z) and
+ * (z + 1, z + 2) add up to the z neighbours of both points at once */
+struct Sums
 {
-    const float s = (M[i] + Pn[i]) + (C[i - sy] + C[i + sy]) + (C[i - 1] + C[i + 1]);
-    return 0.5f * C[i] + (1.f / 12.f) * s;
-}
-
-/* values at z - 1, z, z + 1, z + 2 of a plane column, i the (odd) index of
- * z: two 8-byte loads */
-struct Col4
-{
-    float a, b, c, d;
+    float2 a, ey, ez, q;
 };
-__device__ __forceinline__ Col4 col4(const float* A, int i)
+__device__ __forceinline__ Sums plane_sums(const float* A, int i, int pitch)
 {
     const float2 lo = *reinterpret_cast<const float2*>(A + i - 1);
     const float2 hi = *reinterpret_cast<const float2*>(A + i + 1);
-    return { lo.x, lo.y, hi.x, hi.y };
+    const float2 ls = __fadd2_rn(*reinterpret_cast<const float2*>(A + i - pitch - 1),
+        *reinterpret_cast<const float2*>(A + i + pitch - 1));
+    const float2 hs = __fadd2_rn(*reinterpret_cast<const float2*>(A + i - pitch + 1),
+        *reinterpret_cast<const float2*>(A + i + pitch + 1));
+    return { make_float2(lo.y, hi.x), make_float2(ls.y, hs.x), __fadd2_rn(lo, hi),
+        __fadd2_rn(ls, hs) };
 }
 
-/* lap_m at the z pair (i, i + 1), i odd; the same operation order as lap_m */
-__device__ __forceinline__ void lap_m2(const float* M, const float* C, const float* Pn, int i,
-    int sy, const StepParams& P, float& o0, float& o1)
+/* what a plane adds to the stencil of the planes beside it (side) and, with g the
+ * share of the plane before, to its own (mid: the centre, the largest term, last) */
+__device__ __forceinline__ float2 side(const Sums& t, const Stencil19& c)
 {
-    const Col4 c = col4(C, i), m = col4(M, i), p = col4(Pn, i);
-    const Col4 ym = col4(C, i - sy), yp = col4(C, i + sy);
-    const Col4 mym = col4(M, i - sy), myp = col4(M, i + sy);
-    const Col4 pym = col4(Pn, i - sy), pyp = col4(Pn, i + sy);
-    {
-        const float faces = P.cx * (m.b + p.b) + P.cy * (ym.b + yp.b) + P.cz * (c.a + c.c);
-        const float exy   = mym.b + myp.b + pym.b + pyp.b;
-        const float eyz   = ym.a + ym.c + yp.a + yp.c;
-        const float exz   = m.a + m.c + p.a + p.c;
-        o0 = P.c0 * c.b + faces + P.cxy * exy + P.cyz * eyz + P.cxz * exz;
-    }
-    {
-        const float faces = P.cx * (m.c + p.c) + P.cy * (ym.c + yp.c) + P.cz * (c.b + c.d);
-        const float exy   = mym.c + myp.c + pym.c + pyp.c;
-        const float eyz   = ym.b + ym.d + yp.b + yp.d;
-        const float exz   = m.b + m.d + p.b + p.d;
-        o1 = P.c0 * c.c + faces + P.cxy * exy + P.cyz * eyz + P.cxz * exz;
-    }
+    return __ffma2_rn(f2(c.cxz), t.ez, __ffma2_rn(f2(c.cxy), t.ey, __fmul2_rn(f2(c.cx), t.a)));
 }
-
-/* rhs_b at the z pair (i, i + 1), i odd; the same operation order */
-__device__ __forceinline__ void rhs_b2(const float* M, const float* C, const float* Pn, int i,
-    int sy, float& o0, float& o1)
+__device__ __forceinline__ float2 mid(const Sums& t, const Stencil19& c, float2 g)
 {
-    const Col4 c = col4(C, i);
-    const float2 m  = *reinterpret_cast<const float2*>(M + i - 1);
-    const float2 m2 = *reinterpret_cast<const float2*>(M + i + 1);
-    const float2 p  = *reinterpret_cast<const float2*>(Pn + i - 1);
-    const float2 p2 = *reinterpret_cast<const float2*>(Pn + i + 1);
-    const Col4 ym = col4(C, i - sy), yp = col4(C, i + sy);
-    const float s0 = (m.y + p.y) + (ym.b + yp.b) + (c.a + c.c);
-    const float s1 = (m2.x + p2.x) + (ym.c + yp.c) + (c.b + c.d);
-    o0 = 0.5f * c.b + (1.f / 12.f) * s0;
-    o1 = 0.5f * c.c + (1.f / 12.f) * s1;
-}
-
-/* q / d for 0 <= q < 4096 and 1 <= d <= 64 with inv = 1/d rounded to FP32:
- * (q + 1/2) / d lies at least 1/(2d) from an integer, far more than the
- * 2^-23 relative error of the product, so the truncation is exact */
-__device__ __forceinline__ int divq(int q, float inv)
-{
-    return __float2int_rz(((float)q + 0.5f) * inv);
+    return __ffma2_rn(f2(c.c0), t.a,
+        __ffma2_rn(f2(c.cy), t.ey, __ffma2_rn(f2(c.cz), t.ez, __ffma2_rn(f2(c.cyz), t.q, g))));
 }
 
 /* one periodic coordinate of a box point: b in [-3, e + 3) with e + 6 <= n */
@@ -165,45 +129,48 @@ __device__ __forceinline__ int wrap1(int g, int n)
     return g < 0 ? g + n : (g >= n ? g - n : g);
 }
 
-/* A CTA owns a ty x tz column of an orbital's box and marches along x,
- * PPS planes per step.  The column is fitted to the box: the box's y
- * extent is cut into ceil(e1 / TY) equal columns, its z extent into
- * ceil(e2 / TZ) (tz rounded up to even), so that a box a little wider than
- * TY or TZ does not pay for a second, mostly empty column; TY x TZ bounds
- * the shared-memory planes.  Plane regions shrink by one point per stage
- * in y and z: stage 0 (psi and phi - V psi) on (ty + 6) x (tz + 6), stage 1
- * (r) on (ty + 4) x (tz + 4), stage 2 (u1) on (ty + 2) x (tz + 2), stage 3
- * (u, w) on ty x tz.  Stage k makes planes PPS t + j - 3 - k (j < PPS,
- * box-local x) at step t, within [k - 3, e0 - 1 + 3 - k]; a plane needs
- * the planes p - 1 .. p + 1 of the stage before, made at this step or the
- * one before, so each stage keeps a ring of PPS + 2 planes.  Three
- * barriers per step. */
-template <int TY, int TZ, int PPS> struct Cols
+/* A CTA owns a ty x tz column of an orbital's core -- the part of its box
+ * where a mask is not zero, outside of which u = w = 0 -- and marches along x.
+ * Thread (y, z pair) of the column and its halo of 3 keeps its place in all
+ * four stages.  At step s, with p = xa - 3 + s:
+ *   stage 0 stores psi and d = phi - V psi of plane p,
+ *   stage 1 reads plane p - 1 of both and completes r of plane p - 2,
+ *   stage 2 reads plane p - 3 of r and completes u1 of plane p - 4,
+ *   stage 3 reads plane p - 5 of u1 and completes u, w of plane p - 6:
+ * every stage reads what was stored before the last barrier, so there is one
+ * barrier per step and two planes per array.  The stencil along x is
+ * accumulated: a plane's sums are formed once and give a share to three
+ * planes (Sums, side, mid).  The results next to the edge of the halo are
+ * made from values that were never set; no stage's valid region, one point
+ * narrower than that of the stage before, reads them.
+ *
+ * The inputs of the next step are loaded one step ahead.  A thread skips the
+ * planes that no mask value of its pair reaches (P.range), and does not load
+ * there.  Two steps per turn of the loop: the queues of r, u1 and the masks
+ * then need no moves.
+ *
+ * Why this form: 1536 orbitals on 160^3 (radii 4 to 8 bohr at h = 0.3; 4.4 GB,
+ * 0.65 ms at the copy rate) took 3.90 ms with a kernel that marched the whole
+ * box, mapped each stage's region to the threads anew (three barriers per
+ * plane, up to half of the threads idle in a stage's last pass, 36
+ * shared-memory wavefronts per stencil, mask values loaded where they were
+ * used: 15 % of the issue slots, long scoreboard first).  Only the core of the
+ * boxes: 3.39 ms.  This kernel: 1.96 ms with 448 threads and 2 CTAs per SM (2.36
+ * with one step per turn), 55 % of the issue slots, DRAM at 23 %: bound by
+ * instruction issue and, at 24 of 32 lanes, by the halo. */
+template <int NT> struct Plane
 {
-    static constexpr int RING = PPS + 2;
-    static constexpr int Y3 = TY + 6, Z3 = TZ + 6, N3 = Y3 * Z3;
-    static constexpr int Y2 = TY + 4, Z2 = TZ + 4, N2 = Y2 * Z2;
-    static constexpr int Y1 = TY + 2, Z1 = TZ + 2, N1 = Y1 * Z1;
-    static constexpr int N0 = TY * TZ;
-    static constexpr size_t SMEM = (size_t)(RING * (2 * N3 + N2 + N1)) * sizeof(float);
-    // ring slot of plane p >= -3
-    static __device__ __forceinline__ int slot(int p) { return (p + 3 * RING) % RING; }
-    // resident CTAs per SM the shared memory allows (the register cap of
-    // the launch bounds follows it)
-    static constexpr int MINB = (int)(227 * 1024 / (SMEM + 1024)) < 4
-                                    ? (int)(227 * 1024 / (SMEM + 1024))
-                                    : 4;
+    // the column with its halo: at most 2 NT values, and two more per row
+    // (rows of eight values or more: at most NT / 4 of them)
+    static constexpr int SIZE = 2 * NT + NT / 2;
+    static constexpr size_t SMEM = 8 * SIZE * sizeof(float);
 };
 
-template <int TY, int TZ, int PPS>
-__global__ void __launch_bounds__(THREADS, Cols<TY, TZ, PPS>::MINB) local_step_kernel(StepParams P)
+template <int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) local_step_kernel(const StepParams P)
 {
-    using C = Cols<TY, TZ, PPS>;
-    extern __shared__ __align__(16) float sm[];
-    float* s_psi = sm;                      // RING x N3
-    float* s_d   = s_psi + C::RING * C::N3; // RING x N3: phi - V psi
-    float* s_r   = s_d + C::RING * C::N3;   // RING x N2
-    float* s_u   = s_r + C::RING * C::N2;   // RING x N1
+    constexpr int PLANE = Plane<NT>::SIZE;
+    extern __shared__ __align__(16) float sm[]; // two planes each of psi, d, r, u1
     __shared__ int s_item;
     const int tid = threadIdx.x;
     for (;;)
@@ -215,189 +182,261 @@ __global__ void __launch_bounds__(THREADS, Cols<TY, TZ, PPS>::MINB) local_step_k
         if (it >= P.nitems) break;
         const int4 W = P.items[it]; // (orbital, ty | tz << 16, y0, z0)
         const int f  = W.x;
-        const int ty = W.y & 0xffff, tz = W.y >> 16;
-        // the column's plane regions of each stage (row pitch z_k, pairs
-        // per row p_k) and the reciprocals of the divisors
-        const int z3 = tz + 6, n3 = (ty + 6) * z3;
-        const int z2 = tz + 4, n2 = (ty + 4) * z2, p2 = z2 / 2;
-        const int z1 = tz + 2, n1 = (ty + 2) * z1, p1 = z1 / 2;
-        const int n0 = ty * tz, p0 = tz / 2;
-        const float i3 = 1.f / (float)z3, ip2 = 1.f / (float)p2, ip1 = 1.f / (float)p1,
-                    ip0 = 1.f / (float)p0;
+        const int ty = W.y & 0xffff, tz = W.y >> 16, y0 = W.z, z0 = W.w;
         const int* b = P.box + 6 * f;
         const int o0 = b[0], o1 = b[1], o2 = b[2], e0 = b[3], e1 = b[4], e2 = b[5];
-        const int y0 = W.z, z0 = W.w;
-        const size_t ex = (size_t)e1 * e2;
-        const float* psi = P.psi + P.off[f];
-        const float* phi = P.phi + P.off[f];
-        const float* mo  = P.mvals + P.moff[f];
-        const float* mc  = P.cvals + P.coff[f];
-        // stage 0 inputs of the next PPS planes, loaded into registers one
-        // march step ahead so that their latency overlaps stages 1 to 3
-        constexpr int NQ = (C::N3 + THREADS - 1) / THREADS;
-        float rps[PPS][NQ], rph[PPS][NQ], rv[PPS][NQ];
-        auto load_plane = [&](int p, int j) {
-            const bool in = (p >= 0 && p < e0);
-            const int gx  = wrap1(o0 + (in ? p : 0), P.n[0]);
-#pragma unroll
-            for (int k = 0; k < NQ; k++)
-            {
-                const int q  = tid + k * THREADS;
-                const int qy = divq(q, i3), qz = q - qy * z3;
-                const int by = y0 + qy - 3, bz = z0 + qz - 3;
-                float ps = 0.f, ph = 0.f, v = 0.f;
-                if (q < n3 && in && by >= 0 && by < e1 && bz >= 0 && bz < e2)
-                {
-                    const size_t li = (size_t)p * ex + (size_t)by * e2 + bz;
-                    ps              = psi[li];
-                    ph              = phi[li];
-                    const int gy = wrap1(o1 + by, P.n[1]), gz = wrap1(o2 + bz, P.n[2]);
-                    v = P.V[((size_t)gx * P.n[1] + gy) * P.n[2] + gz];
-                }
-                rps[j][k] = ps;
-                rph[j][k] = ph;
-                rv[j][k]  = v;
-            }
-        };
-#pragma unroll
-        for (int j = 0; j < PPS; j++)
-            load_plane(j - 3, j);
-        for (int t = 0; PPS * t - 6 < e0; t++)
+        const int* core = P.core + 6 * f;
+        const int xa = core[0], xb = core[3], yb = core[4], zb = core[5];
+        float* const ub = P.u + P.off[f];
+        float* const wb = P.w + P.off[f];
+        if (ty == 0)
         {
-            // stage 0: psi and phi - V psi, from the registers; then the
-            // loads of the planes of the next step
-#pragma unroll
-            for (int j = 0; j < PPS; j++)
+            // u = w = 0 outside the core, a warp per z row
+            const int ya = core[1], za = core[2];
+            for (int r = tid / 32; r < e0 * e1; r += NT / 32)
             {
-                const int p = PPS * t + j - 3;
-                if (p <= e0 + 2)
-                {
-                    float* dp = s_psi + C::slot(p) * C::N3;
-                    float* dd = s_d + C::slot(p) * C::N3;
-#pragma unroll
-                    for (int k = 0; k < NQ; k++)
+                const int x = r / e1, y = r - x * e1;
+                const bool cut = x >= xa && x < xb && y >= ya && y < yb;
+                const size_t o = (size_t)r * e2;
+                for (int z = tid & 31; z < e2; z += 32)
+                    if (!(cut && z >= za && z < zb))
                     {
-                        const int q = tid + k * THREADS;
-                        if (q < n3)
+                        ub[o + z] = 0.f;
+                        wb[o + z] = 0.f;
+                    }
+            }
+            continue;
+        }
+        const int z3 = tz + 2 * HALO, pitch = z3 + 2, rows = ty + 2 * HALO, np = z3 / 2;
+        const int qy = tid / np, qz = 2 * (tid - qy * np);
+        const int by = y0 + qy - HALO, bz = z0 + qz - HALO;
+        const int i  = qy * pitch + qz + 1;
+        const bool on  = qy < rows;
+        const bool on1 = qy >= 1 && qy < rows - 1, on2 = qy >= 2 && qy < rows - 2;
+        const bool on3 = qy >= 3 && qy < rows - 3;
+        // the pair's points in the box, and among those that this column stores
+        const bool in0 = on && by >= 0 && by < e1 && bz >= 0 && bz < e2;
+        const bool in1 = on && by >= 0 && by < e1 && bz + 1 >= 0 && bz + 1 < e2;
+        const bool st0 = on3 && by < yb && bz >= z0 && bz < min(z0 + tz, zb);
+        const bool st1 = on3 && by < yb && bz + 1 >= z0 && bz + 1 < min(z0 + tz, zb);
+        // planes [lo, hi) with a mask value at the pair, [llo, lhi) with one at a neighbour
+        int lo = 1 << 20, hi = 0, llo = 1 << 20, lhi = 0;
+        if (P.range)
+        {
+            const int* rg = P.range + P.roff[f];
+            if (on)
+                for (int dy = -1; dy <= 1; dy++)
+                    for (int dz = -1; dz <= 2; dz++)
+                    {
+                        const int y = by + dy, z = bz + dz;
+                        if (y < 0 || y >= e1 || z < 0 || z >= e2) continue;
+                        const int r = rg[y * e2 + z], l = r & 0xffff, h = r >> 16;
+                        if (l >= h) continue;
+                        llo = min(llo, max(l - 1, 0));
+                        lhi = max(lhi, min(h + 1, e0));
+                        if (dy == 0 && (dz == 0 || dz == 1))
                         {
-                            dp[q] = rps[j][k];
-                            dd[q] = rph[j][k] - rv[j][k] * rps[j][k];
+                            lo = min(lo, l);
+                            hi = max(hi, h);
                         }
                     }
-                }
-                load_plane(p + PPS, j);
-            }
-            __syncthreads();
-            // stage 1: r = Mc (B(phi - V psi) + Delta_M psi), z pairs
-#pragma unroll
-            for (int j = 0; j < PPS; j++)
+        }
+        else if (in0 || in1)
+        {
+            lo = llo = 0;
+            hi = lhi = e0;
+        }
+        const int ex = e1 * e2;
+        const int li      = by * e2 + bz;
+        const int gy      = wrap1(o1 + by, P.n[1]);
+        const int v0      = gy * P.n[2] + wrap1(o2 + bz, P.n[2]);
+        const int v1      = gy * P.n[2] + wrap1(o2 + bz + 1, P.n[2]);
+        const float* psi  = P.psi + P.off[f];
+        const float* phi  = P.phi + P.off[f];
+        const float* mo   = P.mvals + P.moff[f];
+        const float* mc   = P.cvals + P.coff[f];
+        const size_t vx   = (size_t)P.n[1] * P.n[2];
+        float2 rps, rph, rv, rmc, rmo; // of the next step
+        auto load = [&](int p) {
+            rps = rph = rv = rmc = rmo = f2(0.f);
+            if (p >= llo && p < lhi)
             {
-                const int p = PPS * t + j - 4;
-                if (p < -2 || p > e0 + 1) continue;
-                const float* M  = s_psi + C::slot(p - 1) * C::N3;
-                const float* X  = s_psi + C::slot(p) * C::N3;
-                const float* N  = s_psi + C::slot(p + 1) * C::N3;
-                const float* dM = s_d + C::slot(p - 1) * C::N3;
-                const float* dX = s_d + C::slot(p) * C::N3;
-                const float* dN = s_d + C::slot(p + 1) * C::N3;
-                float* out      = s_r + C::slot(p) * C::N2;
-                const bool in   = (p >= 0 && p < e0);
-                for (int q = tid; q < n2 / 2; q += THREADS)
+                const float* V = P.V + wrap1(o0 + p, P.n[0]) * vx;
+                const size_t q = (size_t)p * ex;
+                const float *psp = psi + q, *php = phi + q;
+                if (in0)
                 {
-                    const int qy = divq(q, ip2), qz = 2 * (q - qy * p2);
-                    const int by = y0 + qy - 2, bz = z0 + qz - 2;
-                    float m0 = 0.f, m1 = 0.f;
-                    if (in && by >= 0 && by < e1)
-                    {
-                        const float* mrow = mc + (size_t)p * ex + (size_t)by * e2;
-                        if (bz >= 0 && bz < e2) m0 = mrow[bz];
-                        if (bz + 1 >= 0 && bz + 1 < e2) m1 = mrow[bz + 1];
-                    }
-                    float r0 = 0.f, r1 = 0.f;
-                    if (m0 != 0.f || m1 != 0.f)
-                    {
-                        const int i = (qy + 1) * z3 + qz + 1;
-                        float b0, b1, l0, l1;
-                        rhs_b2(dM, dX, dN, i, z3, b0, b1);
-                        lap_m2(M, X, N, i, z3, P, l0, l1);
-                        r0 = m0 * (b0 - l0);
-                        r1 = m1 * (b1 - l1);
-                    }
-                    *reinterpret_cast<float2*>(out + qy * z2 + qz) = make_float2(r0, r1);
+                    rps.x = psp[li];
+                    rph.x = php[li];
+                    rv.x  = V[v0];
+                }
+                if (in1)
+                {
+                    rps.y = psp[li + 1];
+                    rph.y = php[li + 1];
+                    rv.y  = V[v1];
                 }
             }
-            __syncthreads();
-            // stage 2: the first sweep u1, from u0 = gamma r, z pairs
-#pragma unroll
-            for (int j = 0; j < PPS; j++)
+            if (p - 2 >= lo && p - 2 < hi)
             {
-                const int p = PPS * t + j - 5;
-                if (p < -1 || p > e0) continue;
-                const float* M = s_r + C::slot(p - 1) * C::N2;
-                const float* X = s_r + C::slot(p) * C::N2;
-                const float* N = s_r + C::slot(p + 1) * C::N2;
-                float* out     = s_u + C::slot(p) * C::N1;
-                const bool in  = (p >= 0 && p < e0);
-                for (int q = tid; q < n1 / 2; q += THREADS)
+                const float* m = mc + (size_t)(p - 2) * ex;
+                if (in0) rmc.x = m[li];
+                if (in1) rmc.y = m[li + 1];
+            }
+            if (p - 4 >= lo && p - 4 < hi)
+            {
+                const float* m = mo + (size_t)(p - 4) * ex;
+                if (in0) rmo.x = m[li];
+                if (in1) rmo.y = m[li + 1];
+            }
+        };
+        load(xa - 3);
+        float2 acc1 = f2(0.f), g1 = f2(0.f), acc2 = f2(0.f), g2 = f2(0.f), acc3 = f2(0.f),
+               g3 = f2(0.f);
+        float2 ra1 = f2(0.f), ra2 = f2(0.f), ua1 = f2(0.f), mo1 = f2(0.f), mo2 = f2(0.f);
+        const int steps = xb - xa + 9;
+#pragma unroll 2
+        for (int s = 0; s < steps; s++)
+        {
+            const int p     = xa - 3 + s;
+            float* const wr = sm + (s & 1) * PLANE;
+            const float* rd = sm + (1 - (s & 1)) * PLANE;
+            if (on)
+            {
+                const float2 mcp = rmc, mo0 = rmo;
+                const float2 d = __ffma2_rn(make_float2(-rv.x, -rv.y), rps, rph);
+                wr[i]             = rps.x;
+                wr[i + 1]         = rps.y;
+                wr[2 * PLANE + i]     = d.x;
+                wr[2 * PLANE + i + 1] = d.y;
+                load(p + 1);
+                if (on1)
                 {
-                    const int qy = divq(q, ip1), qz = 2 * (q - qy * p1);
-                    const int by = y0 + qy - 1, bz = z0 + qz - 1;
-                    float m0 = 0.f, m1 = 0.f;
-                    if (in && by >= 0 && by < e1)
+                    float2 r = f2(0.f);
+                    if (p - 1 >= lo - 1 && p - 1 < hi + 1)
                     {
-                        const float* mrow = mo + (size_t)p * ex + (size_t)by * e2;
-                        if (bz >= 0 && bz < e2) m0 = mrow[bz];
-                        if (bz + 1 >= 0 && bz + 1 < e2) m1 = mrow[bz + 1];
+                        const Sums t = plane_sums(rd, i, pitch);
+                        const Sums v = plane_sums(rd + 2 * PLANE, i, pitch);
+                        const float2 g = __ffma2_rn(f2(1.f / 12.f), v.a, side(t, P.lap));
+                        const float2 m = __ffma2_rn(f2(1.f / 12.f), __fadd2_rn(v.ey, v.ez),
+                            __ffma2_rn(f2(0.5f), v.a, g1));
+                        const float2 o = __fadd2_rn(acc1, g);
+                        acc1 = mid(t, P.lap, m);
+                        g1   = g;
+                        r    = make_float2(mcp.x != 0.f ? mcp.x * o.x : 0.f,
+                            mcp.y != 0.f ? mcp.y * o.y : 0.f);
                     }
-                    const int i = (qy + 1) * z2 + qz + 1;
-                    // outside the orbital's mask the sweep clamps to zero
-                    // whatever the stencil gives: skip the stencil there
-                    float l0 = 0.f, l1 = 0.f;
-                    if (m0 != 0.f || m1 != 0.f) lap_m2(M, X, N, i, z2, P, l0, l1);
-                    const float2 r  = make_float2(X[i], X[i + 1]);
-                    const float w0  = P.gamma * l0 - r.x;
-                    const float w1  = P.gamma * l1 - r.y;
-                    *reinterpret_cast<float2*>(out + qy * z1 + qz)
-                        = make_float2(clampm(P.gamma * r.x - P.jf * w0, m0),
-                            clampm(P.gamma * r.y - P.jf * w1, m1));
+                    wr[4 * PLANE + i]     = r.x;
+                    wr[4 * PLANE + i + 1] = r.y;
+                }
+                if (on2)
+                {
+                    float2 u = f2(0.f), ra = f2(0.f);
+                    if (p - 3 >= lo - 1 && p - 3 < hi + 1)
+                    {
+                        const Sums t   = plane_sums(rd + 4 * PLANE, i, pitch);
+                        const float2 g = side(t, P.sweep);
+                        const float2 o = __fadd2_rn(acc2, g);
+                        acc2 = mid(t, P.sweep, g2);
+                        g2   = g;
+                        ra   = t.a;
+                        u = make_float2(mo0.x != 0.f ? clampm(o.x, mo0.x) : 0.f,
+                            mo0.y != 0.f ? clampm(o.y, mo0.y) : 0.f);
+                    }
+                    wr[6 * PLANE + i]     = u.x;
+                    wr[6 * PLANE + i + 1] = u.y;
+                    if (on3)
+                    {
+                        float2 w = f2(0.f), v = f2(0.f);
+                        if (p - 5 >= lo - 1 && p - 5 < hi + 1)
+                        {
+                            const Sums t   = plane_sums(rd + 6 * PLANE, i, pitch);
+                            const float2 g = side(t, P.A);
+                            const float2 o = __fadd2_rn(acc3, g);
+                            // A u1 - r: the residual of plane p - 5 goes in here
+                            acc3 = mid(t, P.A, __fadd2_rn(make_float2(-ra2.x, -ra2.y), g3));
+                            g3   = g;
+                            const float2 x = __ffma2_rn(f2(-P.jf), o, ua1);
+                            if (mo2.x != 0.f) { w.x = clampm(o.x, mo2.x); v.x = clampm(x.x, mo2.x); }
+                            if (mo2.y != 0.f) { w.y = clampm(o.y, mo2.y); v.y = clampm(x.y, mo2.y); }
+                            ua1 = t.a;
+                        }
+                        if (p - 6 >= xa)
+                        {
+                            float* const up = ub + (size_t)(p - 6) * ex;
+                            float* const wp = wb + (size_t)(p - 6) * ex;
+                            if (st0)
+                            {
+                                up[li] = v.x;
+                                wp[li] = w.x;
+                            }
+                            if (st1)
+                            {
+                                up[li + 1] = v.y;
+                                wp[li + 1] = w.y;
+                            }
+                        }
+                    }
+                    ra2 = ra1;
+                    ra1 = ra;
+                    mo2 = mo1;
+                    mo1 = mo0;
                 }
             }
             __syncthreads();
-            // stage 3: the second sweep, stored inside the box, z pairs
-#pragma unroll
-            for (int j = 0; j < PPS; j++)
+        }
+    }
+}
+
+/* what the masks of an orbital (blockIdx.x) reach: per box column (y, z) the
+ * range [lo, hi) of x with a value of either mask that is not zero, lo | hi <<
+ * 16 (none: 0), and the bounds of all of them (none: all zero) */
+__global__ void __launch_bounds__(256) core_kernel(const float* __restrict__ mvals,
+    const size_t* __restrict__ moff, const float* __restrict__ cvals,
+    const size_t* __restrict__ coff, const int* __restrict__ box, const size_t* __restrict__ roff,
+    int* __restrict__ range, int* __restrict__ core)
+{
+    __shared__ int lo[3], hi[3];
+    const int f  = blockIdx.x;
+    const int* b = box + 6 * f;
+    if (threadIdx.x < 3)
+    {
+        lo[threadIdx.x] = 1 << 20;
+        hi[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    const float* m = mvals + moff[f];
+    const float* c = cvals + coff[f];
+    const int ex   = b[4] * b[5];
+    for (int i = threadIdx.x; i < ex; i += blockDim.x)
+    {
+        int l = 1 << 20, h = 0;
+        for (int x = 0; x < b[3]; x++)
+        {
+            const size_t k = (size_t)x * ex + i;
+            // (NaN counts as a value)
+            if (!(m[k] == 0.f && c[k] == 0.f))
             {
-                const int p = PPS * t + j - 6;
-                if (p < 0 || p >= e0) continue;
-                const float* M = s_u + C::slot(p - 1) * C::N1;
-                const float* X = s_u + C::slot(p) * C::N1;
-                const float* N = s_u + C::slot(p + 1) * C::N1;
-                const float* R = s_r + C::slot(p) * C::N2;
-                for (int q = tid; q < n0 / 2; q += THREADS)
-                {
-                    const int qy = divq(q, ip0), qz = 2 * (q - qy * p0);
-                    const int by = y0 + qy, bz = z0 + qz;
-                    if (by >= e1 || bz >= e2) continue;
-                    const size_t li = (size_t)p * ex + (size_t)by * e2 + bz;
-                    const int i     = (qy + 1) * z1 + qz + 1;
-                    const float m0  = mo[li];
-                    const float m1  = (bz + 1 < e2) ? mo[li + 1] : 0.f;
-                    // the stencil only where the mask keeps something
-                    float l0 = 0.f, l1 = 0.f;
-                    if (m0 != 0.f || m1 != 0.f) lap_m2(M, X, N, i, z1, P, l0, l1);
-                    const int ir    = (qy + 2) * z2 + qz + 2;
-                    const float w0  = l0 - R[ir];
-                    P.u[P.off[f] + li] = clampm(X[i] - P.jf * w0, m0);
-                    P.w[P.off[f] + li] = clampm(w0, m0);
-                    if (bz + 1 < e2)
-                    {
-                        const float w1 = l1 - R[ir + 1];
-                        P.u[P.off[f] + li + 1] = clampm(X[i + 1] - P.jf * w1, m1);
-                        P.w[P.off[f] + li + 1] = clampm(w1, m1);
-                    }
-                }
+                l = min(l, x);
+                h = x + 1;
             }
         }
+        range[roff[f] + i] = h ? (l | (h << 16)) : 0;
+        if (h)
+        {
+            atomicMin(lo, l);
+            atomicMax(hi, h);
+            atomicMin(lo + 1, i / b[5]);
+            atomicMax(hi + 1, i / b[5] + 1);
+            atomicMin(lo + 2, i % b[5]);
+            atomicMax(hi + 2, i % b[5] + 1);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3)
+    {
+        core[6 * f + threadIdx.x]     = hi[threadIdx.x] ? lo[threadIdx.x] : 0;
+        core[6 * f + 3 + threadIdx.x] = hi[threadIdx.x];
     }
 }
 
@@ -434,71 +473,75 @@ __global__ void __launch_bounds__(256) scatter_kernel(const float* __restrict__ 
     }
 }
 
-/* the kernel variants the tuner chooses from: largest column TY x TZ and
- * planes per march step */
-struct Shape
-{
-    int ty, tz, pps;
-};
-constexpr int NSHAPE           = 6;
-constexpr Shape SHAPES[NSHAPE] = { { 24, 32, 1 }, { 16, 32, 1 }, { 32, 32, 1 }, { 24, 32, 2 },
-    { 16, 32, 2 }, { 32, 32, 2 } };
+/* the kernel variants the tuner chooses from: threads per CTA (a column and its
+ * halo hold at most two points per thread) and the CTAs per SM that the
+ * registers are limited for */
+constexpr int NSHAPE          = 6;
+constexpr int SHAPES[NSHAPE]     = { 256, 320, 384, 448, 640, 768 };
+constexpr int SHAPE_MINB[NSHAPE] = { 3, 2, 2, 2, 1, 1 };
 
-/* kernel and dynamic shared memory of a variant */
-template <int TY, int TZ, int PPS> struct Variant
-{
-    static constexpr auto kernel() { return &local_step_kernel<TY, TZ, PPS>; }
-    static constexpr size_t smem = Cols<TY, TZ, PPS>::SMEM;
-};
+template <int S> constexpr auto variant() { return &local_step_kernel<SHAPES[S], SHAPE_MINB[S]>; }
 
-template <int TY, int TZ, int PPS> int set_attr()
-{
-    static bool done = false;
-    if (!done)
-    {
-        MGX_TRY(cuda_check(cudaFuncSetAttribute(Variant<TY, TZ, PPS>::kernel(),
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)Variant<TY, TZ, PPS>::smem),
-            "local smem"));
-        done = true;
-    }
-    return MGX_OK;
-}
-
-template <int TY, int TZ, int PPS> int occupancy()
-{
-    if (set_attr<TY, TZ, PPS>() != MGX_OK) return 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Variant<TY, TZ, PPS>::kernel(),
-            THREADS, Variant<TY, TZ, PPS>::smem)
-        != cudaSuccess)
-    {
-        cudaGetLastError();
-        return 1;
-    }
-    return std::max(n, 1);
-}
-
-/* resident CTAs per SM of variant s (also sets its shared-memory limit) */
-int max_ctas_per_sm(int s)
+/* f<S>() of variant s */
+template <template <int> class F, class... A> int with_shape(int s, A... a)
 {
     switch (s)
     {
-        case 0: return occupancy<24, 32, 1>();
-        case 1: return occupancy<16, 32, 1>();
-        case 2: return occupancy<32, 32, 1>();
-        case 3: return occupancy<24, 32, 2>();
-        case 4: return occupancy<16, 32, 2>();
-        default: return occupancy<32, 32, 2>();
+        case 0: return F<0>::run(a...);
+        case 1: return F<1>::run(a...);
+        case 2: return F<2>::run(a...);
+        case 3: return F<3>::run(a...);
+        case 4: return F<4>::run(a...);
+        default: return F<5>::run(a...);
     }
 }
 
-template <int TY, int TZ, int PPS> int launch_shape(const StepParams& P, int ctas, cudaStream_t s)
+template <int S> struct SetAttr
 {
-    Variant<TY, TZ, PPS>::kernel()<<<ctas, THREADS, Variant<TY, TZ, PPS>::smem, s>>>(P);
-    MGX_LAUNCH_CHECK("local_step_kernel");
-    return MGX_OK;
-}
+    static int run()
+    {
+        static bool done = false;
+        if (!done)
+        {
+            MGX_TRY(cuda_check(cudaFuncSetAttribute(variant<S>(),
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)Plane<SHAPES[S]>::SMEM),
+                "local smem"));
+            done = true;
+        }
+        return MGX_OK;
+    }
+};
+
+template <int S> struct Occupancy
+{
+    static int run()
+    {
+        if (SetAttr<S>::run() != MGX_OK) return 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, variant<S>(), SHAPES[S],
+                Plane<SHAPES[S]>::SMEM)
+            != cudaSuccess)
+        {
+            cudaGetLastError();
+            return 1;
+        }
+        return std::max(n, 1);
+    }
+};
+
+/* resident CTAs per SM of variant s (also sets its shared-memory limit) */
+int max_ctas_per_sm(int s) { return with_shape<Occupancy>(s); }
+
+template <int S> struct Launch
+{
+    static int run(const StepParams* P, int ctas, cudaStream_t s)
+    {
+        variant<S>()<<<ctas, SHAPES[S], Plane<SHAPES[S]>::SMEM, s>>>(*P);
+        MGX_LAUNCH_CHECK("local_step_kernel");
+        return MGX_OK;
+    }
+};
 
 } // namespace loc
 } // namespace mgx
@@ -509,20 +552,27 @@ struct mgx_local
     int nfunc          = 0;
     size_t total       = 0;
     std::vector<int> h_box;      // 6 per orbital
+    std::vector<int> h_core;     // 6 per orbital: bounds of the points that a mask reaches
     std::vector<size_t> h_off;   // nfunc + 1
-    mgx::DeviceBuffer box, off, counter;
-    mgx::DeviceBuffer items[mgx::loc::NSHAPE];
-    int nitems[mgx::loc::NSHAPE] = {};
+    std::vector<size_t> h_roff;  // nfunc + 1: box columns
+    mgx::DeviceBuffer box, off, counter, range, roff;
+    // [0]: the cores found at creation; [1]: the whole boxes, for masks that
+    // were updated in place since
+    mgx::DeviceBuffer core[2];
+    mgx::DeviceBuffer items[2][mgx::loc::NSHAPE];
+    int nitems[2][mgx::loc::NSHAPE] = {};
+    unsigned version[2] = { 0, 0 }; // of masks and corr at creation
     const mgx_masks* masks = nullptr;
     const mgx_masks* corr  = nullptr;
     // chosen configuration
-    int shape = 1, ctas_per_sm = 2, use_graph = 1;
+    int shape = 3, ctas_per_sm = 2, use_graph = 1;
     // the captured step, valid for the arguments it was captured with
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph    = nullptr;
     const void* key[5]   = { nullptr, nullptr, nullptr, nullptr, nullptr };
     double key_gamma     = 0.;
     int key_shape = -1, key_ctas = -1;
+    unsigned key_version[2] = { 0, 0 };
     ~mgx_local()
     {
         if (exec) cudaGraphExecDestroy(exec);
@@ -534,35 +584,70 @@ namespace mgx
 {
 namespace loc
 {
-int build_items(mgx_local* L, int s)
+/* the columns of a core of ey x ez for nt threads: as few as hold with the halo
+ * in two points per thread, cut into equal parts (the z part rounded up to
+ * even, as the threads work on z pairs) */
+void fit_columns(int ey, int ez, int nt, int* ty, int* tz)
 {
-    const Shape S = SHAPES[s];
+    int best = 1 << 30, area = 0;
+    for (int nz = 1; nz <= ez; nz++)
+    {
+        const int z   = (((ez + nz - 1) / nz) + 1) & ~1;
+        const int cap = 2 * nt / (z + 2 * HALO) - 2 * HALO;
+        if (cap < 1) continue;
+        const int ny = (ey + cap - 1) / cap, y = (ey + ny - 1) / ny;
+        const int n  = ((ey + y - 1) / y) * ((ez + z - 1) / z);
+        const int a  = (y + 2 * HALO) * (z + 2 * HALO);
+        if (n < best || (n == best && a < area))
+        {
+            best = n;
+            area = a;
+            *ty  = y;
+            *tz  = z;
+        }
+    }
+}
+
+int build_items(mgx_local* L, int whole, int s)
+{
     std::vector<int4> it;
-    std::vector<std::pair<size_t, int>> order; // largest box first
+    std::vector<std::pair<size_t, int>> order; // largest first
+    const int* cores = whole ? nullptr : L->h_core.data();
+    auto extent = [&](int f, int k) {
+        return cores ? cores[6 * f + 3 + k] - cores[6 * f + k] : L->h_box[6 * f + 3 + k];
+    };
     for (int f = 0; f < L->nfunc; f++)
-        order.push_back({ (size_t)L->h_box[6 * f + 3] * L->h_box[6 * f + 4] * L->h_box[6 * f + 5], f });
+        order.push_back({ (size_t)extent(f, 0) * extent(f, 1) * extent(f, 2), f });
     std::stable_sort(order.begin(), order.end(),
         [](const std::pair<size_t, int>& a, const std::pair<size_t, int>& b) { return a.first > b.first; });
     for (const auto& pr : order)
     {
-        const int f  = pr.second;
-        const int* e = &L->h_box[6 * f + 3];
-        // columns fitted to the box: equal cuts of each extent, at most
-        // S.ty x S.tz, tz even (the kernel works on z pairs)
-        const int ny = (e[1] + S.ty - 1) / S.ty, nz = (e[2] + S.tz - 1) / S.tz;
-        const int ty = (e[1] + ny - 1) / ny;
-        const int tz = (((e[2] + nz - 1) / nz) + 1) & ~1;
-        for (int y = 0; y < e[1]; y += ty)
-            for (int z = 0; z < e[2]; z += tz)
-                it.push_back(make_int4(f, ty | (tz << 16), y, z));
+        if (pr.first == 0) continue;
+        const int f = pr.second, ey = extent(f, 1), ez = extent(f, 2);
+        const int ya = cores ? cores[6 * f + 1] : 0, za = cores ? cores[6 * f + 2] : 0;
+        int ty = 1, tz = 2;
+        fit_columns(ey, ez, SHAPES[s], &ty, &tz);
+        for (int y = 0; y < ey; y += ty)
+            for (int z = 0; z < ez; z += tz)
+                it.push_back(make_int4(f, ty | (tz << 16), ya + y, za + z));
     }
-    L->nitems[s] = (int)it.size();
-    MGX_TRY(L->items[s].ensure(std::max<size_t>(it.size(), 1) * sizeof(int4)));
+    // the points outside the cores last: short items that even out the tail
+    if (cores)
+        for (const auto& pr : order)
+            it.push_back(make_int4(pr.second, 0, 0, 0));
+    L->nitems[whole][s] = (int)it.size();
+    MGX_TRY(L->items[whole][s].ensure(std::max<size_t>(it.size(), 1) * sizeof(int4)));
     if (!it.empty())
-        MGX_TRY(cuda_check(cudaMemcpy(L->items[s].ptr, it.data(), it.size() * sizeof(int4),
+        MGX_TRY(cuda_check(cudaMemcpy(L->items[whole][s].ptr, it.data(), it.size() * sizeof(int4),
                                cudaMemcpyHostToDevice),
             "items upload"));
     return MGX_OK;
+}
+
+/* whether the masks changed in place since the cores were found */
+int whole_boxes(const mgx_local* L)
+{
+    return L->masks->version != L->version[0] || L->corr->version != L->version[1];
 }
 
 StepParams params(mgx_local* L, int s, const float* psi, const float* phi, const float* V,
@@ -575,28 +660,32 @@ StepParams params(mgx_local* L, int s, const float* psi, const float* phi, const
     P.u     = u;
     P.w     = w;
     P.box   = (const int*)L->box.ptr;
+    const int whole = whole_boxes(L);
+    P.core  = (const int*)L->core[whole].ptr;
+    P.range = whole ? nullptr : (const int*)L->range.ptr;
+    P.roff  = (const size_t*)L->roff.ptr;
     P.off   = (const size_t*)L->off.ptr;
     P.mvals = (const float*)L->masks->values[0].ptr;
     P.moff  = (const size_t*)L->masks->offset[0].ptr;
     P.cvals = (const float*)L->corr->values[0].ptr;
     P.coff  = (const size_t*)L->corr->offset[0].ptr;
-    P.items   = (const int4*)L->items[s].ptr;
-    P.nitems  = L->nitems[s];
+    P.items   = (const int4*)L->items[whole][s].ptr;
+    P.nitems  = L->nitems[whole][s];
     P.counter = (int*)L->counter.ptr;
     const mgx_grid& g = L->ctx->grid;
     for (int i = 0; i < 3; i++)
         P.n[i] = g.n[i];
     const Level L0        = make_level(g, 0);
     const StencilCoeffs c = stencil_coeffs(0, L0.h);
-    P.c0    = (float)c.c0;
-    P.cx    = (float)c.cx[0];
-    P.cy    = (float)c.cy[0];
-    P.cz    = (float)c.cz[0];
-    P.cxy   = (float)c.cxy;
-    P.cyz   = (float)c.cyz;
-    P.cxz   = (float)c.cxz;
-    P.gamma = (float)gamma;
-    P.jf    = (float)jacobi_factor(0, L0.h);
+    const double jf = jacobi_factor(0, L0.h);
+    auto stencil = [&](double centre, double k) {
+        return Stencil19{ (float)(centre + k * c.c0), (float)(k * c.cx[0]), (float)(k * c.cy[0]),
+            (float)(k * c.cz[0]), (float)(k * c.cxy), (float)(k * c.cyz), (float)(k * c.cxz) };
+    };
+    P.lap   = stencil(0., -1.);
+    P.sweep = stencil(gamma + jf, -jf * gamma);
+    P.A     = stencil(0., 1.);
+    P.jf    = (float)jf;
     return P;
 }
 
@@ -609,15 +698,7 @@ int grid_ctas(mgx_local* L, int s, int ctas_per_sm)
 int enqueue(mgx_local* L, int s, int ctas, const StepParams& P, cudaStream_t st)
 {
     MGX_TRY(cuda_check(cudaMemsetAsync(L->counter.ptr, 0, sizeof(int), st), "counter reset"));
-    switch (s)
-    {
-        case 0: return launch_shape<24, 32, 1>(P, ctas, st);
-        case 1: return launch_shape<16, 32, 1>(P, ctas, st);
-        case 2: return launch_shape<32, 32, 1>(P, ctas, st);
-        case 3: return launch_shape<24, 32, 2>(P, ctas, st);
-        case 4: return launch_shape<16, 32, 2>(P, ctas, st);
-        default: return launch_shape<32, 32, 2>(P, ctas, st);
-    }
+    return with_shape<Launch>(s, &P, ctas, st);
 }
 
 int step(mgx_local* L, const float* psi, const float* phi, const float* V, double gamma, float* u,
@@ -628,7 +709,9 @@ int step(mgx_local* L, const float* psi, const float* phi, const float* V, doubl
     const int ctas      = grid_ctas(L, s, L->ctas_per_sm);
     if (!L->use_graph) return enqueue(L, s, ctas, P, st);
     const void* key[5] = { psi, phi, V, u, w };
-    bool same = L->exec && L->key_gamma == gamma && L->key_shape == s && L->key_ctas == L->ctas_per_sm;
+    bool same = L->exec && L->key_gamma == gamma && L->key_shape == s
+        && L->key_ctas == L->ctas_per_sm
+        && L->key_version[0] == L->masks->version && L->key_version[1] == L->corr->version;
     for (int i = 0; i < 5 && same; i++)
         same = (key[i] == L->key[i]);
     if (!same)
@@ -663,6 +746,8 @@ int step(mgx_local* L, const float* psi, const float* phi, const float* V, doubl
         L->key_gamma = gamma;
         L->key_shape = s;
         L->key_ctas  = L->ctas_per_sm;
+        L->key_version[0] = L->masks->version;
+        L->key_version[1] = L->corr->version;
     }
     count_launch();
     return cuda_check(cudaGraphLaunch(L->exec, st), "graph launch");
@@ -727,8 +812,43 @@ int mgx_local_create(mgx_ctx* ctx, const mgx_masks* masks, const mgx_masks* corr
                                cudaMemcpyHostToDevice),
             "offset upload"));
     }
+    const size_t nf = L->nfunc;
+    L->h_roff.assign(nf + 1, 0);
+    L->h_core.resize(6 * nf);
+    std::vector<int> whole(6 * nf, 0);
+    for (size_t f = 0; f < nf; f++)
+    {
+        const int* e      = &L->h_box[6 * f + 3];
+        L->h_roff[f + 1]  = L->h_roff[f] + (size_t)e[1] * e[2];
+        for (int k = 0; k < 3; k++)
+            whole[6 * f + 3 + k] = e[k];
+    }
+    L->version[0] = masks->version;
+    L->version[1] = corr->version;
+    MGX_TRY(L->roff.ensure((nf + 1) * sizeof(size_t)));
+    MGX_TRY(L->range.ensure(std::max<size_t>(L->h_roff[nf], 1) * sizeof(int)));
+    for (int k = 0; k < 2; k++)
+        MGX_TRY(L->core[k].ensure(std::max<size_t>(6 * nf, 1) * sizeof(int)));
+    if (nf)
+    {
+        MGX_TRY(cuda_check(cudaMemcpy(L->roff.ptr, L->h_roff.data(), (nf + 1) * sizeof(size_t),
+                               cudaMemcpyHostToDevice),
+            "column offset upload"));
+        MGX_TRY(cuda_check(cudaMemcpy(L->core[1].ptr, whole.data(), 6 * nf * sizeof(int),
+                               cudaMemcpyHostToDevice),
+            "box upload"));
+        loc::core_kernel<<<(unsigned)nf, 256>>>((const float*)masks->values[0].ptr,
+            (const size_t*)masks->offset[0].ptr, (const float*)corr->values[0].ptr,
+            (const size_t*)corr->offset[0].ptr, (const int*)L->box.ptr,
+            (const size_t*)L->roff.ptr, (int*)L->range.ptr, (int*)L->core[0].ptr);
+        MGX_LAUNCH_CHECK("core_kernel");
+        MGX_TRY(cuda_check(cudaMemcpy(L->h_core.data(), L->core[0].ptr, 6 * nf * sizeof(int),
+                               cudaMemcpyDeviceToHost),
+            "cores"));
+    }
     for (int s = 0; s < loc::NSHAPE; s++)
-        MGX_TRY(loc::build_items(L.get(), s));
+        for (int k = 0; k < 2; k++)
+            MGX_TRY(loc::build_items(L.get(), k, s));
     *out = L.release();
     return MGX_OK;
 }

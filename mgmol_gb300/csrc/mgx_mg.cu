@@ -754,6 +754,7 @@ int masks_update(mgx_ctx* ctx, mgx_masks* M, const double* centers, const double
     MGX_TRY(masks_create(ctx, M->nlevels, M->nfunc, centers, radii, M->func, M->kind,
         M->mesh_ghosts, M->dtype, &T, s));
     std::swap(*M, *T);
+    M->version = T->version + 1;
     delete T;
     return MGX_OK;
 }

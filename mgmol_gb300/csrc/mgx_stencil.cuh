@@ -164,4 +164,5 @@ struct mgx_masks
     std::vector<mgx::DeviceBuffer> state, box, offset, values;
     std::vector<std::vector<int>> h_state, h_box;
     std::vector<mgx::MaskDev> dev;
+    unsigned version = 0; // counts the updates in place
 };

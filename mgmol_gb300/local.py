@@ -22,9 +22,8 @@ from . import capi, synth
 
 # algorithmic bytes per box point: psi, phi, V, two mask values read; u, w written
 BYTES_PER_POINT = 7 * 4
-# the kernel variants of mgx_local_tune: (largest column TY x TZ, fitted to each
-# box, planes per march step)
-VARIANTS = [("24x32", 1), ("16x32", 1), ("32x32", 1), ("24x32", 2), ("16x32", 2), ("32x32", 2)]
+# the kernel variants of mgx_local_tune: threads per CTA
+VARIANTS = [256, 320, 384, 448, 640, 768]
 
 
 def build(n, h, nfunc, seed, rlo=4.0, rhi=8.0, chunk=128):
@@ -102,8 +101,7 @@ def main(argv=None):
            "box_points_total": int(loc.total), "box_points_mean": float(vols.mean()),
            "box_points_min": int(vols.min()), "box_points_max": int(vols.max()),
            "ms_per_step": t, "algorithmic_GBps": gbs, "bytes_per_point": BYTES_PER_POINT,
-           "config": {"column": VARIANTS[cfg[0]][0], "planes_per_step": VARIANTS[cfg[0]][1],
-                      "ctas_per_sm": cfg[1],
+           "config": {"threads": VARIANTS[cfg[0]], "ctas_per_sm": cfg[1],
                       "graph": bool(cfg[2])},
            "tune_ms": [round(float(x), 4) for x in ms],
            "whole_grid_points": a.nfunc * ctx.npts}

@@ -124,3 +124,33 @@ def test_box_wider_than_the_grid_is_refused():
     corr = capi.Masks(ctx, 1, c, r, func=1, kind=1, dtype=torch.float32)
     with pytest.raises(capi.MgxError):
         capi.Local(ctx, masks, corr)
+
+
+@pytest.mark.parametrize("n,h,r", [((28, 26, 26), 0.4, 2.92 * 0.4), ((50, 50, 52), 0.3, 15.3 * 0.3)])
+def test_masks_updated_in_place(n, h, r):
+    """Radii a little larger in the same boxes: the handle made before the
+    update gives what a new one gives, in every configuration; boxes of one
+    small column and of several."""
+    ll = tuple(h * x for x in n)
+    ctx = capi.Context(n, ll)
+    centers = np.array([[h * (n[0] // 2 + 0.5), h * (n[1] // 2 + 0.5), h * (n[2] // 2 + 0.5)],
+                        [0.5 * h, 1.5 * h, 0.5 * h]])
+    mk = lambda rad, func: capi.Masks(ctx, 1, centers, np.full(2, rad), func=func, kind=func,
+                                      dtype=torch.float32)
+    masks, corr = mk(r, 0), mk(r, 1)
+    loc = capi.Local(ctx, masks, corr)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda m: torch.randn(m, generator=gen, device="cuda")
+    psi, phi, V = rnd(loc.total), rnd(loc.total), rnd(int(np.prod(n)))
+    first = [t.clone() for t in loc.step(psi, phi, V, 0.03)]
+    for m in (masks, corr):
+        m.update(centers, np.full(2, r + 0.06 * h))
+    new = capi.Local(ctx, masks, corr)
+    assert np.array_equal(new.boxes, loc.boxes)
+    want = new.step(psi, phi, V, 0.03)
+    assert torch.count_nonzero(want[0]) > torch.count_nonzero(first[0]) > 0
+    for shape in range(6):
+        for handle in (loc, new):
+            handle.set_config(shape, 2, shape % 2 == 0)
+            u, w = handle.step(psi, phi, V, 0.03)
+            assert torch.equal(u, want[0]) and torch.equal(w, want[1]), shape
