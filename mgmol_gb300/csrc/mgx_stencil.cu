@@ -135,10 +135,15 @@ struct DevCoef
     T cx[4], cy[4], cz[4];
     T cxy, cyz, cxz;
     T jf;
+    // of PlaneParams, in T (in the kernels the conversion and the comparison of
+    // the doubles were redone at every use: FP64 units a quarter busy in FP32)
+    T gam, alpha;
+    int scaled;
+    int iso; // cy = cz and cxy = cxz
 };
 
 template <typename T>
-DevCoef<T> to_dev(const StencilCoeffs& c, double jf)
+DevCoef<T> to_dev(const StencilCoeffs& c, double jf, const PlaneParams& p = PlaneParams())
 {
     DevCoef<T> d;
     d.c0 = (T)c.c0;
@@ -152,6 +157,10 @@ DevCoef<T> to_dev(const StencilCoeffs& c, double jf)
     d.cyz = (T)c.cyz;
     d.cxz = (T)c.cxz;
     d.jf  = (T)jf;
+    d.gam    = (T)p.gamma_in;
+    d.alpha  = (T)p.upd_alpha;
+    d.scaled = p.gamma_in != 0.;
+    d.iso    = d.cy[0] == d.cz[0] && d.cxy == d.cxz;
     return d;
 }
 
@@ -168,6 +177,79 @@ __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+/* The same on the points of a group, two FP32 points per instruction (each
+ * half of a packed operation is rounded as the scalar one): o = a + b, a - b,
+ * c a and c a + b. */
+template <int N>
+__device__ __forceinline__ void vadd(const float (&a)[N], const float (&b)[N], float (&o)[N])
+{
+#pragma unroll
+    for (int v = 0; v < N; v += 2)
+    {
+        const float2 r = __fadd2_rn(make_float2(a[v], a[v + 1]), make_float2(b[v], b[v + 1]));
+        o[v]           = r.x;
+        o[v + 1]       = r.y;
+    }
+}
+template <int N>
+__device__ __forceinline__ void vmul(float c, const float (&a)[N], float (&o)[N])
+{
+#pragma unroll
+    for (int v = 0; v < N; v += 2)
+    {
+        const float2 r = __fmul2_rn(make_float2(c, c), make_float2(a[v], a[v + 1]));
+        o[v]           = r.x;
+        o[v + 1]       = r.y;
+    }
+}
+template <int N>
+__device__ __forceinline__ void vfma(float c, const float (&a)[N], const float (&b)[N], float (&o)[N])
+{
+#pragma unroll
+    for (int v = 0; v < N; v += 2)
+    {
+        const float2 r = __ffma2_rn(make_float2(c, c), make_float2(a[v], a[v + 1]),
+            make_float2(b[v], b[v + 1]));
+        o[v]           = r.x;
+        o[v + 1]       = r.y;
+    }
+}
+// (b exactly negated by the factor)
+template <int N>
+__device__ __forceinline__ void vsub(const float (&a)[N], const float (&b)[N], float (&o)[N])
+{
+    vfma(-1.f, b, a, o);
+}
+template <int N>
+__device__ __forceinline__ void vadd(const double (&a)[N], const double (&b)[N], double (&o)[N])
+{
+#pragma unroll
+    for (int v = 0; v < N; v++)
+        o[v] = __dadd_rn(a[v], b[v]);
+}
+template <int N>
+__device__ __forceinline__ void vsub(const double (&a)[N], const double (&b)[N], double (&o)[N])
+{
+#pragma unroll
+    for (int v = 0; v < N; v++)
+        o[v] = __dsub_rn(a[v], b[v]);
+}
+template <int N>
+__device__ __forceinline__ void vmul(double c, const double (&a)[N], double (&o)[N])
+{
+#pragma unroll
+    for (int v = 0; v < N; v++)
+        o[v] = __dmul_rn(c, a[v]);
+}
+template <int N>
+__device__ __forceinline__ void vfma(double c, const double (&a)[N], const double (&b)[N],
+    double (&o)[N])
+{
+#pragma unroll
+    for (int v = 0; v < N; v++)
+        o[v] = __fma_rn(c, a[v], b[v]);
+}
 
 __device__ __forceinline__ int wrap(int i, int n)
 {
@@ -406,7 +488,7 @@ __global__ void __launch_bounds__(256) plane_kernel(PlaneParams p, DevCoef<T> c)
     T* __restrict__ updp     = (OP == OP_JACOBI_UPD)
                                    ? reinterpret_cast<T*>(p.upd) + (size_t)f * p.ldupd
                                    : nullptr;
-    const T ualpha           = (T)p.upd_alpha;
+    const T ualpha           = c.alpha;
     const T uscale           = (OP == OP_JACOBI_UPD && p.upd_scale) ? (T)p.upd_scale[f] : (T)1;
     T* __restrict__ wp       = p.w ? reinterpret_cast<T*>(p.w) + (size_t)f * p.ldw : nullptr;
     const T* __restrict__ fp = p.f ? reinterpret_cast<const T*>(p.f) + (size_t)f * p.ldf : nullptr;
@@ -595,48 +677,118 @@ struct Vec16<double>
 
 constexpr int JJ_CS = 4; // coarse-plane slots of the folded prolongation
 
+template <typename T, typename VH>
+__device__ __forceinline__ void unpack(const typename VH::type& q, T (&o)[VH::N])
+{
+#pragma unroll
+    for (int v = 0; v < VH::N; v++)
+        o[v] = VH::get(q, v);
+}
+template <typename T, typename VH>
+__device__ __forceinline__ typename VH::type pack(const T (&a)[VH::N])
+{
+    typename VH::type q;
+#pragma unroll
+    for (int v = 0; v < VH::N; v++)
+        VH::set(q, v, a[v]);
+    return q;
+}
+
 /* In-plane part a and neighbour-plane part b of a radius-1 operator at the
  * VEC points of a group along z: centre row c0v with its z neighbours zl /
  * zr, rows y - 1 / y + 1 cmv / cpv and, for the Mehrstellen edges (EDGES),
  * their z neighbours ml, mr / pl, pr.  The y sum of each z column is formed
  * once and serves the column's own term and the edge terms of the columns
- * beside it.  Every stencil kernel that must give the same bits as another
+ * beside it.  FP64, bound by its operations (a warp instruction takes an SM's
+ * FP64 units 16 clocks): a starts from before, the part b of the plane before,
+ * which saves the addition of the two, and equal coefficients along y and z
+ * share the sum of the y and z neighbours; 14 operations per Jacobi point
+ * instead of 16.  Every stencil kernel that must give the same bits as another
  * forms a and b here. */
 template <typename T, typename VH, bool EDGES>
 __device__ __forceinline__ void vec_terms(const DevCoef<T>& c, const typename VH::type& c0v,
     const typename VH::type& cmv, const typename VH::type& cpv, T zl, T zr, T ml, T mr, T pl,
-    T pr, T* a, T* b, T* u)
+    T pr, const T (&before)[VH::N], T (&a)[VH::N], T (&b)[VH::N], T (&u)[VH::N])
 {
-    constexpr int VEC = VH::N;
-    T sy[VEC + 2];
-#pragma unroll
-    for (int v = 0; v < VEC; v++)
-        sy[v + 1] = add_rn(VH::get(cmv, v), VH::get(cpv, v));
-    if (EDGES)
+    constexpr int VEC    = VH::N;
+    constexpr bool CHAIN = sizeof(T) == 8;
+    T cm[VEC], cp[VEC], sy[VEC], sz[VEC];
+    unpack<T, VH>(c0v, u);
+    unpack<T, VH>(cmv, cm);
+    unpack<T, VH>(cpv, cp);
+    if constexpr (CHAIN)
     {
-        sy[0]       = add_rn(ml, pl);
-        sy[VEC + 1] = add_rn(mr, pr);
-    }
+        T se[VEC + 2];
 #pragma unroll
-    for (int v = 0; v < VEC; v++)
-    {
-        const T uc  = VH::get(c0v, v);
-        const T uzm = v == 0 ? zl : VH::get(c0v, v - 1);
-        const T uzp = v == VEC - 1 ? zr : VH::get(c0v, v + 1);
-        const T sz  = add_rn(uzm, uzp);
-        T aa        = fma_rn(c.cy[0], sy[v + 1], fma_rn(c.cz[0], sz, mul_rn(c.c0, uc)));
-        T bb;
+        for (int v = 0; v < VEC; v++)
+            se[v + 1] = add_rn(cm[v], cp[v]);
         if (EDGES)
         {
-            aa = fma_rn(c.cyz, add_rn(sy[v], sy[v + 2]), aa);
-            bb = fma_rn(c.cxy, sy[v + 1], fma_rn(c.cxz, sz, mul_rn(c.cx[0], uc)));
+            se[0]       = add_rn(ml, pl);
+            se[VEC + 1] = add_rn(mr, pr);
         }
-        else
-            bb = mul_rn(c.cx[0], uc);
-        a[v] = aa;
-        b[v] = bb;
-        u[v] = uc;
+#pragma unroll
+        for (int v = 0; v < VEC; v++)
+        {
+            // (with the centre last, matrices of 256 orbitals on 96^3 took 23.2 ms
+            // instead of 22.4: a longer chain after the last load)
+            T ss        = se[v + 1];
+            const T szv = add_rn(v == 0 ? zl : u[v - 1], v == VEC - 1 ? zr : u[v + 1]);
+            T aa        = fma_rn(c.c0, u[v], before[v]);
+            T bb        = mul_rn(c.cx[0], u[v]);
+            if (EDGES && c.iso)
+                ss = add_rn(ss, szv);
+            else
+            {
+                aa = fma_rn(c.cz[0], szv, aa);
+                if (EDGES) bb = fma_rn(c.cxz, szv, bb);
+            }
+            aa = fma_rn(c.cy[0], ss, aa);
+            if (EDGES)
+            {
+                aa = fma_rn(c.cyz, add_rn(se[v], se[v + 2]), aa);
+                bb = fma_rn(c.cxy, ss, bb);
+            }
+            a[v] = aa;
+            b[v] = bb;
+        }
+        return;
     }
+    vadd(cm, cp, sy);
+#pragma unroll
+    for (int v = 0; v < VEC; v++)
+        sz[v] = add_rn(v == 0 ? zl : u[v - 1], v == VEC - 1 ? zr : u[v + 1]);
+    vmul(c.c0, u, a);
+    vfma(c.cz[0], sz, a, a);
+    vfma(c.cy[0], sy, a, a);
+    vmul(c.cx[0], u, b);
+    if (EDGES)
+    {
+        const T sl = add_rn(ml, pl), sr = add_rn(mr, pr);
+        T q[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; v++)
+            q[v] = add_rn(v == 0 ? sl : sy[v - 1], v == VEC - 1 ? sr : sy[v + 1]);
+        vfma(c.cyz, q, a, a);
+        vfma(c.cxz, sz, b, b);
+        vfma(c.cxy, sy, b, b);
+    }
+}
+
+/* jacobi_point on a group: the result in u (the centre on entry), w = lap - f in w */
+template <typename T, int N>
+__device__ __forceinline__ void jacobi_group(T (&lap)[N], const T (&fv)[N], T jf, bool scaled,
+    T gam, T (&u)[N], T (&w)[N])
+{
+    if (scaled)
+    {
+        vmul(gam, lap, lap);
+        vsub(lap, u, w);
+        vmul(gam, u, u);
+    }
+    else
+        vsub(lap, fv, w);
+    vfma(-jf, w, u, u);
 }
 
 /* One Jacobi point: w = lap - f and the result ucen - jf w; scaled (the
@@ -691,8 +843,8 @@ __global__ void __launch_bounds__(256, 2) plane_vec_kernel(PlaneParams p, DevCoe
     const int x0      = tile_x * p.xc;
     const int xcount  = min(p.xc, nx - x0);
     const int nplanes = xcount + 2 + YO;
-    const bool scaled = is_jacobi(OP) && (p.gamma_in != 0.);
-    const T gam       = (T)p.gamma_in;
+    const bool scaled = is_jacobi(OP) && c.scaled;
+    const T gam       = c.gam;
 
     const size_t stage_elems = (size_t)rows * nz;
     T* stages                = reinterpret_cast<T*>(smem_raw);
@@ -787,12 +939,13 @@ __global__ void __launch_bounds__(256, 2) plane_vec_kernel(PlaneParams p, DevCoe
     T* __restrict__ updp     = (OP == OP_JACOBI_UPD)
                                    ? reinterpret_cast<T*>(p.upd) + (size_t)f * p.ldupd
                                    : nullptr;
-    const T ualpha           = (T)p.upd_alpha;
+    const T ualpha           = c.alpha;
     const T uscale           = (OP == OP_JACOBI_UPD && p.upd_scale) ? (T)p.upd_scale[f] : (T)1;
     T* __restrict__ wp       = p.w ? reinterpret_cast<T*>(p.w) + (size_t)f * p.ldw : nullptr;
     const T* __restrict__ fp = p.f ? reinterpret_cast<const T*>(p.f) + (size_t)f * p.ldf : nullptr;
     constexpr bool POINTWISE = is_jacobi(OP) || (OP == OP_HPSI_V) || (OP == OP_RHS_SUB);
     const T c12 = (T)(1. / 12.), c05 = (T)0.5;
+    constexpr bool CHAIN = sizeof(T) == 8; // A1 holds B2 as well
     // the result of 4 consecutive points (never across a 64-point block) as
     // bf16 hi = rn(r), lo = rn(r - hi) in the K-blocked operand planes, the
     // split of the tensor-core products
@@ -938,7 +1091,7 @@ __global__ void __launch_bounds__(256, 2) plane_vec_kernel(PlaneParams p, DevCoe
             V4 res;
             V4 wres;
             T ta[VEC], tb[VEC], tu[VEC];
-            if (!is_rhs_op(OP)) vec_terms<T, VH, EDGES>(c, c0v, cmv, cpv, zl, zr, ml, mr, pl, pr, ta, tb, tu);
+            if (!is_rhs_op(OP)) vec_terms<T, VH, EDGES>(c, c0v, cmv, cpv, zl, zr, ml, mr, pl, pr, B1[k], ta, tb, tu);
 #pragma unroll
             for (int v = 0; v < VEC; v++)
             {
@@ -950,7 +1103,10 @@ __global__ void __launch_bounds__(256, 2) plane_vec_kernel(PlaneParams p, DevCoe
                 T a, b;
                 if (is_rhs_op(OP))
                 {
-                    a = c05 * u + c12 * (uym + uyp + uzm + uzp);
+                    if (CHAIN)
+                        a = fma_rn(c05, u, fma_rn(c12, uym + uyp + uzm + uzp, B1[k][v]));
+                    else
+                        a = c05 * u + c12 * (uym + uyp + uzm + uzp);
                     b = c12 * u;
                 }
                 else
@@ -971,7 +1127,7 @@ __global__ void __launch_bounds__(256, 2) plane_vec_kernel(PlaneParams p, DevCoe
                 }
                 if (emit)
                 {
-                    T lap = add_rn(add_rn(A1[k][v], B2[k][v]), b);
+                    T lap = add_rn(CHAIN ? A1[k][v] : add_rn(A1[k][v], B2[k][v]), b);
                     T ucen = U1[k][v];
                     T r    = lap;
                     if (OP == OP_HPSI_V) r = lap + ucen * VH::get(pv[k], v);
@@ -1060,7 +1216,10 @@ __global__ void __launch_bounds__(256, 2) plane_vec_kernel(PlaneParams p, DevCoe
 // the results are the same bits.  The running sums keep A(x - 1) + B(x - 2)
 // as one value, the first addition of plane_vec_kernel's A1 + B2 + b, and
 // both kernels form every sum and product of a point with explicitly
-// rounded operations (vec_terms, jacobi_point, update_point, add_rn).
+// rounded operations (vec_terms, jacobi_point or jacobi_group, update_point,
+// add_rn).  192^3, 64 FP32 orbitals, both pairs of a V-cycle with the update:
+// 5.90 -> 5.47 ms with two points per instruction and the scalars of a launch
+// in the kernel's type.
 // MODE JJ_STORE stores u2 to out; JJ_UPD adds it into the update block as
 // OP_JACOBI_UPD does; JJ_RST stores it and restricts the second sweep's
 // residual into the next level's right-hand side as OP_JACOBI_RST does
@@ -1076,6 +1235,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) plane_jj_kernel(PlaneParams p, D
     constexpr bool PRO   = (MODE & JJ_PRO) != 0;
     constexpr bool RST   = ((MODE & 3) == JJ_RST);
     constexpr bool UPD   = ((MODE & 3) == JJ_UPD);
+    constexpr bool CHAIN = sizeof(T) == 8; // vec_terms adds the plane before to a
     constexpr int YO     = RST ? 1 : 0;
     extern __shared__ __align__(128) unsigned char smem_raw[];
 
@@ -1091,8 +1251,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) plane_jj_kernel(PlaneParams p, D
     const int x0      = tile_x * p.xc;
     const int xcount  = min(p.xc, nx - x0);
     const int nplanes = xcount + YO + 4; // staged planes x0 - YO - 2 .. x0 + xcount + 1
-    const bool scaled = (p.gamma_in != 0.);
-    const T gam       = (T)p.gamma_in;
+    const bool scaled = c.scaled;
+    const T gam       = c.gam;
 
     const size_t stage_elems = (size_t)rows_s * nz;
     const size_t u1_elems    = (size_t)rows1 * nz;
@@ -1228,7 +1388,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) plane_jj_kernel(PlaneParams p, D
 
     T* __restrict__ outp     = reinterpret_cast<T*>(p.out) + (size_t)f * p.ldo;
     T* __restrict__ updp     = UPD ? reinterpret_cast<T*>(p.upd) + (size_t)f * p.ldupd : nullptr;
-    const T ualpha           = (T)p.upd_alpha;
+    const T ualpha           = c.alpha;
     const T uscale           = (UPD && p.upd_scale) ? (T)p.upd_scale[f] : (T)1;
     const T* __restrict__ fp = reinterpret_cast<const T*>(p.f) + (size_t)f * p.ldf;
 
@@ -1301,7 +1461,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) plane_jj_kernel(PlaneParams p, D
 
     // in-plane part a and neighbour-plane part b of the operator at the
     // group's VEC points (vec_terms, as in plane_vec_kernel)
-    auto terms = [&](const T* q, int oc, int om, int op, T (&a)[VEC], T (&b)[VEC], T (&u)[VEC]) {
+    auto terms = [&](const T* q, int oc, int om, int op, const T (&before)[VEC], T (&a)[VEC],
+                     T (&b)[VEC], T (&u)[VEC]) {
         const V4 c0v = *reinterpret_cast<const V4*>(q + oc);
         const V4 cmv = *reinterpret_cast<const V4*>(q + oc - nz);
         const V4 cpv = *reinterpret_cast<const V4*>(q + oc + nz);
@@ -1314,7 +1475,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) plane_jj_kernel(PlaneParams p, D
             pl = q[om + nz];
             pr = q[op + nz];
         }
-        vec_terms<T, VH, EDGES>(c, c0v, cmv, cpv, zl, zr, ml, mr, pl, pr, a, b, u);
+        vec_terms<T, VH, EDGES>(c, c0v, cmv, cpv, zl, zr, ml, mr, pl, pr, before, a, b, u);
     };
 
     // OP_JACOBI_RST's restriction of the fine plane xe (odd from x0) and the
@@ -1411,22 +1572,23 @@ __global__ void __launch_bounds__(NT, 512 / NT) plane_jj_kernel(PlaneParams p, D
         {
             if (!ok1[k]) continue;
             T a[VEC], b[VEC], u[VEC];
-            terms(st, o1[k], m1[k], p1[k], a, b, u);
-            V4 res;
+            terms(st, o1[k], m1[k], p1[k], Q1[k], a, b, u);
+            if (emit1)
+            {
+                T lap[VEC], fv[VEC], w[VEC];
+                vadd(P1[k], b, lap);
+                if (!scaled) unpack<T, VH>(fa[k], fv);
+                jacobi_group<T, VEC>(lap, fv, c.jf, scaled, gam, C1[k], w);
+                *reinterpret_cast<V4*>(u1p + o1[k] - nz) = pack<T, VH>(C1[k]);
+            }
+            if (!CHAIN) vadd(a, Q1[k], P1[k]);
 #pragma unroll
             for (int v = 0; v < VEC; v++)
             {
-                if (emit1)
-                {
-                    T w;
-                    VH::set(res, v, jacobi_point<T>(add_rn(P1[k][v], b[v]), C1[k][v],
-                                        scaled ? (T)0 : VH::get(fa[k], v), c.jf, scaled, gam, w));
-                }
-                P1[k][v] = add_rn(a[v], Q1[k][v]);
+                if (CHAIN) P1[k][v] = a[v];
                 Q1[k][v] = b[v];
                 C1[k][v] = u[v];
             }
-            if (emit1) *reinterpret_cast<V4*>(u1p + o1[k] - nz) = res;
         }
         // JJ_PRO: the next staged plane, read after the barrier below
         if (PRO)
@@ -1461,36 +1623,35 @@ __global__ void __launch_bounds__(NT, 512 / NT) plane_jj_kernel(PlaneParams p, D
         {
             if (!ok2[k]) continue;
             T a[VEC], b[VEC], u[VEC];
-            terms(u1p, o2[k], m2[k], p2[k], a, b, u);
-            V4 res, wres;
+            terms(u1p, o2[k], m2[k], p2[k], Q2[k], a, b, u);
+            if (emit2)
+            {
+                T lap[VEC], fv[VEC], w[VEC];
+                vadd(P2[k], b, lap);
+                unpack<T, VH>(fb[k], fv);
+                jacobi_group<T, VEC>(lap, fv, c.jf, false, (T)0, C2[k], w);
+                if (UPD)
+                {
+                    T q[VEC];
+                    unpack<T, VH>(ub[k], q);
+                    vfma(ualpha, C2[k], q, q);
+                    vmul(uscale, q, q);
+                    *reinterpret_cast<V4*>(updp + xo2 + g2[k]) = pack<T, VH>(q);
+                }
+                else if (!RST || (r2[k] >= YO && e2 >= x0))
+                    *reinterpret_cast<V4*>(outp + xo2 + g2[k]) = pack<T, VH>(C2[k]);
+                if (RST)
+                    *reinterpret_cast<V4*>(wring + (size_t)((e2 - x0 + 1) & 3) * ring_elems
+                                           + (size_t)(o2[k] - nz)) = pack<T, VH>(w);
+            }
+            if (!CHAIN) vadd(a, Q2[k], P2[k]);
 #pragma unroll
             for (int v = 0; v < VEC; v++)
             {
-                if (emit2)
-                {
-                    T w;
-                    VH::set(res, v, jacobi_point<T>(add_rn(P2[k][v], b[v]), C2[k][v],
-                                        VH::get(fb[k], v), c.jf, false, (T)0, w));
-                    VH::set(wres, v, w);
-                }
-                P2[k][v] = add_rn(a[v], Q2[k][v]);
+                if (CHAIN) P2[k][v] = a[v];
                 Q2[k][v] = b[v];
                 C2[k][v] = u[v];
             }
-            if (!emit2) continue;
-            if (UPD)
-            {
-                V4 q = ub[k];
-#pragma unroll
-                for (int v = 0; v < VEC; v++)
-                    VH::set(q, v, update_point<T>(VH::get(q, v), VH::get(res, v), ualpha, uscale));
-                *reinterpret_cast<V4*>(updp + xo2 + g2[k]) = q;
-            }
-            else if (!RST || (r2[k] >= YO && e2 >= x0))
-                *reinterpret_cast<V4*>(outp + xo2 + g2[k]) = res;
-            if (RST)
-                *reinterpret_cast<V4*>(wring + (size_t)((e2 - x0 + 1) & 3) * ring_elems
-                                       + (size_t)(o2[k] - nz)) = wres;
         }
         if (RST && emit2 && e2 > x0 && ((e2 - x0) & 1)) pend = e2;
     }
@@ -1532,8 +1693,8 @@ __global__ void __launch_bounds__(256, 2) plane_axis_kernel(PlaneParams p, DevCo
     const int y0      = tile_y * TY;
     const int x0      = tile_x * p.xc;
     const int nplanes = min(p.xc, nx - x0) + 2 * R;
-    const bool scaled = is_jacobi(OP) && (p.gamma_in != 0.); // first sweep from gamma f
-    const float gam   = (float)p.gamma_in;
+    const bool scaled = is_jacobi(OP) && c.scaled; // first sweep from gamma f
+    const float gam   = c.gam;
 
     const size_t stage_elems = (size_t)rows * nz;
     float* stages            = reinterpret_cast<float*>(smem_raw);
@@ -1586,7 +1747,7 @@ __global__ void __launch_bounds__(256, 2) plane_axis_kernel(PlaneParams p, DevCo
     float* __restrict__ outp = reinterpret_cast<float*>(p.out) + (size_t)f * p.ldo;
     float* __restrict__ updp
         = (OP == OP_JACOBI_UPD) ? reinterpret_cast<float*>(p.upd) + (size_t)f * p.ldupd : nullptr;
-    const float ualpha = (float)p.upd_alpha;
+    const float ualpha = c.alpha;
     const float uscale = (OP == OP_JACOBI_UPD && p.upd_scale) ? (float)p.upd_scale[f] : 1.f;
     float* __restrict__ wp = p.w ? reinterpret_cast<float*>(p.w) + (size_t)f * p.ldw : nullptr;
     // pointwise operand: f of a Jacobi sweep, V of V psi
@@ -1747,8 +1908,8 @@ __global__ void __launch_bounds__(256) direct_kernel(PlaneParams p, DevCoef<T> c
     const int nx = p.n[0], ny = p.n[1], nz = p.n[2];
     const size_t npts = (size_t)nx * ny * nz;
     const int f       = blockIdx.y;
-    const bool scaled = is_jacobi(OP) && p.gamma_in != 0.; // first sweep from gamma f
-    const T gam       = scaled ? (T)p.gamma_in : (T)1;
+    const bool scaled = is_jacobi(OP) && c.scaled; // first sweep from gamma f
+    const T gam       = scaled ? c.gam : (T)1;
     const T* ub       = reinterpret_cast<const T*>(scaled ? p.f : p.u)
                   + (size_t)f * (scaled ? p.ldf : p.ldu);
     const TV* vb      = reinterpret_cast<const TV*>(p.V);
@@ -1782,7 +1943,7 @@ __global__ void __launch_bounds__(256) direct_kernel(PlaneParams p, DevCoef<T> c
         if (OP == OP_JACOBI_UPD)
         {
             T* u = reinterpret_cast<T*>(p.upd) + (size_t)f * p.ldupd + idx;
-            *u   = (p.upd_scale ? (T)p.upd_scale[f] : (T)1) * (*u + (T)p.upd_alpha * r);
+            *u   = (p.upd_scale ? (T)p.upd_scale[f] : (T)1) * (*u + c.alpha * r);
         }
         else
             reinterpret_cast<T*>(p.out)[(size_t)f * p.ldo + idx] = r;
@@ -2070,9 +2231,9 @@ int stencil_launch(int op, int lap_type, int dtype, int v_dtype,
     {
         if (dtype == MGX_F64)
             return launch_t<double, double, 0, OP_RHS, 1>(
-                p, to_dev<double>(sc, jf), nfunc, stream, force_direct);
+                p, to_dev<double>(sc, jf, p), nfunc, stream, force_direct);
         return launch_t<float, float, 0, OP_RHS, 1>(
-            p, to_dev<float>(sc, jf), nfunc, stream, force_direct);
+            p, to_dev<float>(sc, jf, p), nfunc, stream, force_direct);
     }
     if (op == OP_RHS_SPLIT)
     {
@@ -2080,20 +2241,20 @@ int stencil_launch(int op, int lap_type, int dtype, int v_dtype,
         if (dtype != MGX_F32 || !vec_ok<float, float, 0, OP_RHS_SPLIT, 1>(p, force_direct)
             || (L.npts() % 64) != 0)
             return fail(MGX_UNSUPPORTED, "split right-hand side needs the vector kernel");
-        return launch_vec<float, float, 0, OP_RHS_SPLIT, 1>(p, to_dev<float>(sc, jf), nfunc,
+        return launch_vec<float, float, 0, OP_RHS_SPLIT, 1>(p, to_dev<float>(sc, jf, p), nfunc,
             stream);
     }
     if (op == OP_RHS_SUB)
     {
         if (dtype == MGX_F64)
             return launch_t<double, double, 0, OP_RHS_SUB, 1>(
-                p, to_dev<double>(sc, jf), nfunc, stream, force_direct);
+                p, to_dev<double>(sc, jf, p), nfunc, stream, force_direct);
         return launch_t<float, float, 0, OP_RHS_SUB, 1>(
-            p, to_dev<float>(sc, jf), nfunc, stream, force_direct);
+            p, to_dev<float>(sc, jf, p), nfunc, stream, force_direct);
     }
     if (dtype == MGX_F64)
     {
-        const DevCoef<double> c = to_dev<double>(sc, jf);
+        const DevCoef<double> c = to_dev<double>(sc, jf, p);
         switch (op)
         {
             case OP_LAP:
@@ -2117,7 +2278,7 @@ int stencil_launch(int op, int lap_type, int dtype, int v_dtype,
     }
     else
     {
-        const DevCoef<float> c = to_dev<float>(sc, jf);
+        const DevCoef<float> c = to_dev<float>(sc, jf, p);
         switch (op)
         {
             case OP_LAP:
@@ -2285,12 +2446,12 @@ int jacobi2_launch(int mode, int lap_type, int dtype, const PlaneParams& p, cons
     const StencilCoeffs sc = stencil_coeffs(lap_type, L.h);
     if (dtype == MGX_F64)
     {
-        const DevCoef<double> c = to_dev<double>(sc, jf);
+        const DevCoef<double> c = to_dev<double>(sc, jf, p);
         return lap_type == 0 ? jj_mode<double, 0>(mode, p, c, nfunc, s, dry, tile_rows)
                              : jj_mode<double, 1>(mode, p, c, nfunc, s, dry, tile_rows);
     }
     if (dtype != MGX_F32) return fail(MGX_BAD_ARG, "two-sweep kernel: dtype %d", dtype);
-    const DevCoef<float> c = to_dev<float>(sc, jf);
+    const DevCoef<float> c = to_dev<float>(sc, jf, p);
     return lap_type == 0 ? jj_mode<float, 0>(mode, p, c, nfunc, s, dry, tile_rows)
                          : jj_mode<float, 1>(mode, p, c, nfunc, s, dry, tile_rows);
 }

@@ -184,3 +184,24 @@ def test_axis_kernel_tiles(n, lap):
     assert close(out, ctx.precond_mg(u.double(), lap, 0, 0.2))
     a = ctx.precond_update(u, psi.clone(), 0.4, lap, 0, 0.2)
     assert close(a, ctx.precond_update(u.double(), psi.double(), 0.4, lap, 0, 0.2))
+
+
+@pytest.mark.parametrize("h", [(0.3, 0.3, 0.3), (0.25, 0.3, 0.35), (0.3, 0.25, 0.25)])
+@pytest.mark.parametrize("n", [(32, 24, 16), (20, 18, 44)])
+def test_spacings(n, h):
+    """Equal and unequal spacings along y and z (the radius-1 FP64 kernels share
+    the sum of the y and z neighbours when the coefficients agree)."""
+    ll = tuple(a * b for a, b in zip(n, h))
+    ctx = capi.Context(n, ll)
+    rng = np.random.default_rng(3)
+    psi, V = rng.standard_normal((2, ctx.npts)), rng.standard_normal(ctx.npts)
+    for dt, tol in ((np.float64, TOL_F64), (np.float32, TOL_F32)):
+        p, v = psi.astype(dt), V.astype(dt)
+        for lap in (0, 1):
+            got = ctx.fd_apply(_dev(p, dt), lap).cpu().numpy()
+            assert rel_err(got, O.fd_apply(n, ll, lap, p.astype(np.float64))) < tol
+            got = ctx.hpsi(_dev(p, dt), _dev(v, dt), lap).cpu().numpy()
+            want = O.hpsi(n, ll, lap, p.astype(np.float64), v.astype(np.float64))
+            assert rel_err(got, want) < tol
+        got = ctx.rhs_mehr(_dev(p, dt)).cpu().numpy()
+        assert rel_err(got, O.rhs_mehr(n, ll, p.astype(np.float64))) < tol
