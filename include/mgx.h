@@ -68,7 +68,8 @@ typedef enum mgx_lap_type
 /* Arithmetic of the Gram / H contractions. */
 typedef enum mgx_gemm_mode
 {
-    MGX_GEMM_FP64   = 0, /* FP64 data, FP64 FMA (plain path) */
+    MGX_GEMM_FP64   = 0, /* FP64 data: exact BF16 slices on the tensor cores, or
+                            FP64 FMA (small products) (plain path) */
     MGX_GEMM_FP32   = 1, /* FP32 data, FP32 FMA on CUDA cores in 8-term
                           * chains, the chains summed in FP32 over 128
                           * terms and those sums in double-float (two FP32) */

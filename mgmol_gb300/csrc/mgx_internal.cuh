@@ -93,8 +93,6 @@ struct mgx_ctx
     size_t smem_optin;
     // V-cycle workspace
     mgx::DeviceBuffer vc;
-    // GEMM partials / scratch
-    mgx::DeviceBuffer gemm_ws;
     mgx::DeviceBuffer dense_ws;
     mgx::DeviceBuffer flag;
     // tensor-core GEMM: bf16 hi/lo planes, tile list, status word

@@ -16,7 +16,8 @@
 //   - digit s of A times digit t of B are integers of at most 2^14 at weight
 //     2^(-8 (s + t)).  The products of one s + t add up in an FP32 accumulator
 //     of their own, which rounds nothing while |sum| <= 2^24: after 192 values
-//     of K (256 where only s + t <= 3 are summed) it is read and added to a 64-bit integer.  (All of s + t <= 4 are
+//     of K (256 where only s + t <= 3 are summed) it is read and added to a
+//     64-bit integer.  (All of s + t <= 4 are
 //     exact for any input; of the 6 or 7 x 192 products of s + t = 5 and 6, at
 //     2^-40 and 2^-48, the last bit could round if all digits were extreme.)
 //     The sums have to be exact and not only FP32: the tensor cores truncate
@@ -28,7 +29,8 @@
 //
 // A NaN or an infinity in an operand has no digits: it raises a flag, on
 // which the kernels here do nothing and the caller's CUDA-core kernel,
-// launched behind them, does the work instead of returning at once.
+// launched behind them, does the work instead of returning at once.  A bounded
+// wait that gives up raises the same flag.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -269,8 +271,7 @@ struct Params
     const int* ka;
     const int* kb;
     Target t;
-    const int* bad;
-    int* err;
+    int* bad;
 };
 
 /* the first row tile that reaches an entry i >= c */
@@ -658,7 +659,15 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
             }
         }
     }
-    if (abort_all && threadIdx.x == 0 && p.err) atomicExch(p.err, MGX_TIMEOUT);
+    if (abort_all && threadIdx.x == 0)
+    {
+        // a wait gave up: the CUDA-core kernels form the product instead, or, where
+        // C held an operand that is overwritten in part by now, C says so
+        if (p.t.sum == nullptr && p.t.cin != nullptr && p.t.cin == p.t.C)
+            p.t.C[p.m - 1] = __longlong_as_double(0x7ff8000000000000ll);
+        else
+            atomicExch(p.bad, 1);
+    }
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
@@ -735,7 +744,7 @@ int make_planes(const View& v, size_t k0, size_t kc, const int* keys, void* plan
 }
 
 int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const void* pb,
-    const int* kb, size_t kc, const Target& t, const int* bad, int* err, cudaStream_t s)
+    const int* kb, size_t kc, const Target& t, int* bad, cudaStream_t s)
 {
     const int ns = t.sum ? NS_SUM : NS_STORE;
     if (m == 0 || n == 0 || kc == 0) return MGX_OK;
@@ -811,7 +820,6 @@ int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const vo
     p.kb  = kb;
     p.t   = t;
     p.bad = bad;
-    p.err = err;
     CUtensorMap mA, mB;
     MGX_TRY(tc::make_map_blocked(&mA, pa, m, (size_t)ns * p.kblocks, BM, 64));
     MGX_TRY(tc::make_map_blocked(&mB, pb, n, (size_t)ns * p.kblocks, p.bn, 64));
@@ -836,15 +844,14 @@ namespace
 {
 size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 
-/* keys of na + nb rows, the flag, the error word and the planes of `planes`
+/* keys of na + nb rows, the flag and the planes of `planes`
  * bytes in ctx's workspace */
 int workspace(mgx_ctx* ctx, size_t na, size_t nb, size_t planes, int** ka, int** kb, int** bad,
-    int** err, char** pl)
+    char** pl)
 {
     const size_t head = up256((na + nb + 2) * sizeof(int));
     if (ctx->slices.ensure(head + planes) != MGX_OK) return MGX_NO_MEMORY;
     *bad = (int*)ctx->slices.ptr;
-    *err = *bad + 1;
     *ka  = *bad + 2;
     *kb  = *ka + na;
     *pl  = (char*)ctx->slices.ptr + head;
@@ -871,13 +878,13 @@ int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const 
     const size_t kc  = std::min((K + 63) / 64, fit) * 64;
     const size_t pa_bytes = up256(plane_bytes(n, kc, NS_SUM)),
                  pb_bytes = up256(plane_bytes(brows, kc, NS_SUM));
-    int *ka, *kb, *err;
+    int *ka, *kb;
     char* pl;
     MGX_TRY(workspace(ctx, n, bkeys, pa_bytes + pb_bytes + sums * sizeof(unsigned long long), &ka,
-        &kb, bad, &err, &pl));
+        &kb, bad, &pl));
     char* pb  = pl + pa_bytes;
     auto* sum = (unsigned long long*)(pb + pb_bytes);
-    MGX_TRY(cuda_check(cudaMemsetAsync(*bad, 0, 2 * sizeof(int), s), "slice flags"));
+    MGX_TRY(cuda_check(cudaMemsetAsync(*bad, 0, sizeof(int), s), "slice flag"));
     MGX_TRY(cuda_check(cudaMemsetAsync(sum, 0, sums * sizeof(unsigned long long), s), "slice sums"));
     const View va = { A, ld, (size_t)n, K, true };
     MGX_TRY(row_keys(va, ka, *bad, s));
@@ -912,7 +919,7 @@ int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const 
         {
             if (!q.same) MGX_TRY(make_planes(q.v, k0, k, q.keys, pb, NS_SUM, s));
             MGX_TRY(product(ctx->sm_count, n, pl, ka, q.v.rows, q.same ? pl : pb, q.keys, k, q.t,
-                *bad, err, s));
+                *bad, s));
         }
     }
     for (int i = 0; i < nf; i++)
@@ -936,10 +943,10 @@ int store_begin(mgx_ctx* ctx, const View& A, const View& B, StorePlan* p, cudaSt
     const size_t rows = std::min(p->chunk, A.rows);
     char* pl;
     MGX_TRY(workspace(ctx, rows, B.rows, b1 + plane_bytes(rows, K, ns), &p->ka, &p->kb, &p->bad,
-        &p->err, &pl));
+        &pl));
     p->pb = pl;
     p->pa = pl + b1;
-    MGX_TRY(cuda_check(cudaMemsetAsync(p->bad, 0, 2 * sizeof(int), s), "slice flags"));
+    MGX_TRY(cuda_check(cudaMemsetAsync(p->bad, 0, sizeof(int), s), "slice flag"));
     MGX_TRY(row_keys(B, p->kb, p->bad, s));
     return make_planes(B, 0, K, p->kb, p->pb, ns, s);
 }
@@ -956,7 +963,7 @@ int store_chunk(mgx_ctx* ctx, const View& A, const View& B, const Target& t, con
     c.col0 -= (int)r0;
     MGX_TRY(row_keys(a, p.ka, p.bad, s));
     MGX_TRY(make_planes(a, 0, A.K, p.ka, p.pa, NS_STORE, s));
-    return product(ctx->sm_count, rows, p.pa, p.ka, B.rows, p.pb, p.kb, A.K, c, p.bad, p.err, s);
+    return product(ctx->sm_count, rows, p.pa, p.ka, B.rows, p.pb, p.kb, A.K, c, p.bad, s);
 }
 } // namespace sl
 } // namespace mgx

@@ -51,9 +51,10 @@ int row_keys(const View& v, int* keys, int* bad, cudaStream_t s);
 int make_planes(const View& v, size_t k0, size_t kc, const int* keys, void* planes, int ns,
     cudaStream_t s);
 /* the product of two sets of planes (NS_SUM with Target::sum, else NS_STORE) of
- * kc values of K; does nothing when *bad is set */
+ * kc values of K; does nothing when *bad is set, and sets it when a bounded wait
+ * gives up */
 int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const void* pb,
-    const int* kb, size_t kc, const Target& t, const int* bad, int* err, cudaStream_t s);
+    const int* kb, size_t kc, const Target& t, int* bad, cudaStream_t s);
 
 /* whether a product of this size is formed from slices */
 bool pays(size_t m, size_t n, size_t K);
@@ -89,7 +90,7 @@ int store(mgx_ctx* ctx, const View& A, const View& B, const Target& t, cudaStrea
 struct StorePlan
 {
     size_t chunk;
-    int *ka, *kb, *bad, *err;
+    int *ka, *kb, *bad;
     char *pa, *pb;
 };
 int store_begin(mgx_ctx* ctx, const View& A, const View& B, StorePlan* plan, cudaStream_t s);
