@@ -156,7 +156,7 @@ __device__ __forceinline__ int wrap1(int g, int n)
  * shared-memory wavefronts per stencil, mask values loaded where they were
  * used: 15 % of the issue slots, long scoreboard first).  Only the core of the
  * boxes: 3.39 ms.  This kernel: 1.96 ms with 448 threads and 2 CTAs per SM (2.36
- * with one step per turn), 55 % of the issue slots, DRAM at 23 %: bound by
+ * with one step per turn), 59 % of the issue slots, DRAM at 28 %: bound by
  * instruction issue and, at 24 of 32 lanes, by the halo. */
 template <int NT> struct Plane
 {

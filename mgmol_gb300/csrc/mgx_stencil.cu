@@ -1999,6 +1999,34 @@ static void few_tiles(int nx, int ny, int nz, int nfunc, int halo, int esz, bool
     }
 }
 
+/* Planes of an x chunk of a launch whose tiles fill the GPU: the even cut of nx
+ * whose busiest SM marches the fewest planes, halo planes of each chunk
+ * included (the kernels are bound by issue or FP64 units, so that CTAs which
+ * share an SM take turns).  Chunks of 32 planes made the pre-sweep pair march 37
+ * planes for 32; against them H psi with S, H and B of 512 FP32 orbitals on 128^3
+ * took 9.79 instead of 9.95 ms, of 256 FP64 ones on 96^3 22.2 instead of 22.4.
+ * With the CTAs resident at a time in place of SMs, 64 FP64 fields of 64^3 got
+ * one chunk and took 2 % longer. */
+static int x_chunk(int nx, size_t tiles, int halo)
+{
+    int best    = nx;
+    size_t cost = 0;
+    for (int k = 1;; k++)
+    {
+        const int x = std::min(nx, ((nx + k - 1) / k + 1) & ~1);
+        if (k > 1 && x < 16) break;
+        const size_t rounds = (tiles * ((nx + x - 1) / x) + 151) / 152;
+        const size_t c      = rounds * (size_t)(x + halo);
+        if (cost == 0 || c < cost)
+        {
+            cost = c;
+            best = x;
+        }
+        if (x <= 2) break;
+    }
+    return best;
+}
+
 /* Can the vectorised radius-1 kernel run this launch?  It needs the
  * operator to be radius 1 with a uniform element type, and every block it
  * touches 16-byte aligned with rows of whole vectors. */
@@ -2052,6 +2080,8 @@ static int launch_vec(const PlaneParams& p0, const DevCoef<T>& c, int nfunc,
     int xc = std::min(32, nx);
     if ((size_t)((ny + ty - 1) / ty) * ((nx + xc - 1) / xc) * nfunc < 4 * 152)
         few_tiles(nx, ny, nz, nfunc, 2 + YO, (int)sizeof(T), RST, &ty, &xc);
+    else
+        xc = x_chunk(nx, (size_t)((ny + ty - 1) / ty) * nfunc, 2 + YO);
     p.ty      = ty;
     p.ntile_y = (ny + ty - 1) / ty;
     p.xc      = xc;
@@ -2388,8 +2418,11 @@ static int launch_jj_nt(const PlaneParams& p0, const DevCoef<T>& c, int nfunc, c
     p.ty      = ty;
     p.ntile_y = ny / ty;
     int xc    = 32;
-    while (xc > 4 && (size_t)p.ntile_y * ((nx + xc - 1) / xc) * nfunc < 4 * 152)
-        xc /= 2;
+    if ((size_t)p.ntile_y * ((nx + xc - 1) / xc) * nfunc >= 4 * 152)
+        xc = x_chunk(nx, (size_t)p.ntile_y * nfunc, YO + 4);
+    else
+        while (xc > 4 && (size_t)p.ntile_y * ((nx + xc - 1) / xc) * nfunc < 4 * 152)
+            xc /= 2;
     if (xc > nx) xc = nx;
     p.xc      = xc;
     p.ntile_x = (nx + xc - 1) / xc;

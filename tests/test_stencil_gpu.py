@@ -205,3 +205,21 @@ def test_spacings(n, h):
             assert rel_err(got, want) < tol
         got = ctx.rhs_mehr(_dev(p, dt)).cpu().numpy()
         assert rel_err(got, O.rhs_mehr(n, ll, p.astype(np.float64))) < tol
+
+
+@pytest.mark.parametrize("n,nf", [((72, 32, 64), 150), ((37, 20, 64), 330), ((20, 16, 16), 700)])
+def test_chunks_of_a_full_launch(n, nf):
+    """Blocks that fill the GPU are cut into other x chunks than a few functions:
+    the same bits for each function."""
+    ctx = capi.Context(n, tuple(0.3 * x for x in n))
+    g = torch.Generator(device="cuda").manual_seed(8)
+    u = torch.randn((nf, ctx.npts), generator=g, device="cuda")
+    V = torch.randn(ctx.npts, generator=g, device="cuda")
+    some = torch.tensor([0, nf // 2, nf - 1], device="cuda")
+    for dt in (torch.float32, torch.float64):
+        a, v = u.to(dt), V.to(dt)
+        b = a[some].contiguous()
+        assert torch.equal(ctx.hpsi(a, v)[some], ctx.hpsi(b, v))
+        for lap in (0, 1):
+            assert torch.equal(ctx.fd_apply(a, lap)[some], ctx.fd_apply(b, lap))
+            assert torch.equal(ctx.precond_mg(a, lap, 0, 0.2)[some], ctx.precond_mg(b, lap, 0, 0.2))
