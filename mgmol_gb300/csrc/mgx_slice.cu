@@ -272,6 +272,7 @@ struct Params
     const int* kb;
     Target t;
     int* bad;
+    uint32_t polls; // after which a wait gives up
 };
 
 /* the first row tile that reaches an entry i >= c */
@@ -366,7 +367,8 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
 {
     using namespace tc;
     constexpr int B_SLICE = Form<NP, NS>::B_SLICE, STAGE = Form<NP, NS>::STAGE;
-    if (*p.bad) return;
+    // (one decision for the CTA: another one that gives up may set it just now)
+    if (__syncthreads_or(*(volatile const int*)p.bad)) return;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -375,7 +377,8 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
     uint64_t* accf  = empty + STAGES; // the MMAs up to a drain are done
     uint64_t* acce  = accf + 1;       // [NS] the epilogue warps have read accumulator a
     uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + NS);
-    __shared__ volatile int abort_all;
+    __shared__ volatile int abort_all; // a wait gave up
+    __shared__ uint64_t mma_done;
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     // diagonals s + t of walk ps: [pass_lo, pass_hi), which read slices < pass_hi
@@ -390,6 +393,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
             mbar_init(empty + s, 1);
         }
         mbar_init(accf, 1);
+        mbar_init(&mma_done, 1);
         for (int a = 0; a < NS; a++)
             mbar_init(acce + a, EPI);
         abort_all = 0;
@@ -424,7 +428,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                 for (int it = 0; it < nst; it++, g++)
                 {
                     const int b = g % STAGES;
-                    if (!mbar_wait(empty + b, (uint32_t)(((g / STAGES) & 1) ^ 1)))
+                    if (!mbar_wait(empty + b, (uint32_t)(((g / STAGES) & 1) ^ 1), p.polls))
                     {
                         abort_all = 1;
                         break;
@@ -443,6 +447,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                 }
             }
         }
+        drain_loads<STAGES>(full, g);
     }
     else if (warp == 1 && lane == 0)
     {
@@ -459,7 +464,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                 for (int it = 0; it < nst && ok; it++, g++)
                 {
                     const int b = g % STAGES;
-                    ok          = mbar_wait(full + b, (uint32_t)((g / STAGES) & 1));
+                    ok          = mbar_wait(full + b, (uint32_t)((g / STAGES) & 1), p.polls);
                     if (!ok) break;
                     fence_after_sync();
                     const uint64_t ad = desc_sw<64>(smem_u32(smem + b * STAGE));
@@ -472,7 +477,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                         if (d < lo || d >= hi || !ok) return;
                         if (fresh && drains > 0)
                         {
-                            ok = mbar_wait(acce + (d - lo), (uint32_t)((drains - 1) & 1));
+                            ok = mbar_wait(acce + (d - lo), (uint32_t)((drains - 1) & 1), p.polls);
                             if (!ok) return;
                             fence_after_sync();
                         }
@@ -509,6 +514,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                 break;
             }
         }
+        drain_mma(&mma_done);
     }
     else if (warp >= 2)
     {
@@ -543,7 +549,9 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
             bool ok      = true;
             for (int d = 0; d < na; d++, drains++)
             {
-                ok = !abort_all && mbar_wait(accf, (uint32_t)(drains & 1)) && !abort_all;
+                // (one decision for the warp, which reads TMEM together)
+                ok = __all_sync(0xffffffffu,
+                    !abort_all && mbar_wait(accf, (uint32_t)(drains & 1), p.polls) && !abort_all);
                 if (!ok) break;
                 fence_after_sync();
                 const int ps = d < nd ? 0 : 1, lo = pass_lo(ps), hi = pass_hi(ps);
@@ -659,6 +667,9 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
             }
         }
     }
+    fence_before_sync();
+    __syncthreads(); // every role is done: abort_all is final
+    fence_after_sync();
     if (abort_all && threadIdx.x == 0)
     {
         // a wait gave up: the CUDA-core kernels form the product instead, or, where
@@ -668,9 +679,6 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
         else
             atomicExch(p.bad, 1);
     }
-    fence_before_sync();
-    __syncthreads();
-    fence_after_sync();
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512)
                      : "memory");
@@ -820,6 +828,7 @@ int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const vo
     p.kb  = kb;
     p.t   = t;
     p.bad = bad;
+    p.polls = tc::wait_polls();
     CUtensorMap mA, mB;
     MGX_TRY(tc::make_map_blocked(&mA, pa, m, (size_t)ns * p.kblocks, BM, 64));
     MGX_TRY(tc::make_map_blocked(&mB, pb, n, (size_t)ns * p.kblocks, p.bn, 64));

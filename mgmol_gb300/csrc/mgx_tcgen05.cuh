@@ -7,6 +7,8 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <cstdlib>
+
 #include "mgx_internal.cuh"
 
 namespace mgx
@@ -107,6 +109,22 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar)
         : "memory");
 }
 
+/* What a role owes before its CTA ends, however it got there: the bulk loads
+ * that it has started into shared memory (the last ones of a ring of STAGES, g
+ * in all) have landed, and the MMAs that it has issued are done (bar: an
+ * mbarrier of one arrival that nothing else uses).  Bounded, like every wait. */
+template <int STAGES>
+__device__ __forceinline__ void drain_loads(uint64_t* full, int g)
+{
+    for (int k = g > STAGES ? g - STAGES : 0; k < g; k++)
+        mbar_wait(full + k % STAGES, (uint32_t)((k / STAGES) & 1));
+}
+__device__ __forceinline__ void drain_mma(uint64_t* bar)
+{
+    mma_commit(bar);
+    mbar_wait(bar, 0);
+}
+
 __device__ __forceinline__ void fence_after_sync()
 {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -139,6 +157,16 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
 {
     asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar))
                  : "memory");
+}
+
+/* Polls after which a wait of a product's pipeline gives up; MGX_WAIT_POLLS
+ * lowers it (0: every wait gives up), for the tests of what happens then. */
+constexpr uint32_t WAIT_POLLS = 1u << 26;
+inline uint32_t wait_polls()
+{
+    const char* e = getenv("MGX_WAIT_POLLS");
+    const long v  = e ? atol(e) : (long)WAIT_POLLS;
+    return v >= 0 && v < (long)WAIT_POLLS ? (uint32_t)v : WAIT_POLLS;
 }
 
 inline PFN_cuTensorMapEncodeTiled_v12000 encoder()

@@ -115,3 +115,26 @@ def test_not_finite(bad):
     want = theta.T @ hp
     assert torch.equal(torch.isnan(got), torch.isnan(want))
     assert torch.equal(torch.isinf(got), torch.isinf(want))
+
+
+@pytest.mark.parametrize("polls", ["0", "1", "3", "20"])
+def test_waits_that_give_up(polls, monkeypatch):
+    """With waits of so few polls the pipelines give up at once or on the way:
+    the CUDA-core kernels behind them form the products, and the context stays
+    usable."""
+    from mgmol_gb300 import capi
+    n = (32, 32, 20)
+    ctx = capi.Context(n, tuple(float(x) for x in n))
+    psi, hp = _block(150, ctx.npts, 21), _block(150, ctx.npts, 22)
+    theta = _block(150, 150, 23)
+    H, out = ctx.hmat(psi, hp), ctx.mult_matrix(psi, theta)
+    monkeypatch.setenv("MGX_WAIT_POLLS", polls)
+    S2, H2, out2 = ctx.gram(psi), ctx.hmat(psi, hp), ctx.mult_matrix(psi, theta)
+    torch.cuda.synchronize()
+    monkeypatch.delenv("MGX_WAIT_POLLS")
+    assert bool(((S2 - _product(psi, psi)).abs() <= _bound(psi, psi, ctx.npts)).all())
+    assert bool(((H2 - H).abs() <= _bound(psi, hp, ctx.npts)).all())
+    assert bool(((out2 - out).T.abs() <= _bound(psi.T, theta.T, 150)).all())
+    if polls == "0":  # FP64 sums in another order
+        assert not torch.equal(H2, H) and not torch.equal(out2, out)
+    assert torch.equal(ctx.hmat(psi, hp), H) and torch.equal(ctx.mult_matrix(psi, theta), out)
