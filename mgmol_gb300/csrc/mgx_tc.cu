@@ -92,6 +92,7 @@ struct Params
     double* rho       = nullptr;
     const float* rpsi = nullptr;
     size_t ldr        = 0;
+    uint32_t polls    = wait_polls(); // after which a wait gives up
 };
 
 // KIND 0: tf32 (NPROD 1); KIND 1: bf16 (NPROD 1 plain, 3 for hi/lo split).
@@ -126,6 +127,8 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel(
     uint64_t* empty = full + STAGES;
     uint64_t* accf  = empty + STAGES;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(accf + 1);
+    __shared__ uint64_t mma_done;
+    __shared__ volatile int gave_up;
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int2 tile = STORE ? make_int2((int)blockIdx.x / p.ntj, (int)blockIdx.x % p.ntj)
@@ -143,6 +146,8 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel(
             mbar_init(empty + s, 1);
         }
         mbar_init(accf, 1);
+        mbar_init(&mma_done, 1);
+        gave_up = 0;
         fence_mbar_init();
     }
     if (warp == 1)
@@ -157,7 +162,6 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel(
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = *tslot;
-    bool ok = true;
 
     if (warp == 0 && lane == 0)
     {
@@ -168,12 +172,16 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel(
             prefetch_map(&mA1);
             prefetch_map(&mB1);
         }
-        for (int it = 0; it < nkb && ok; it++)
+        int it = 0;
+        for (; it < nkb; it++)
         {
             const int s = it % STAGES;
             const uint32_t ph = (uint32_t)((it / STAGES) & 1);
-            ok = mbar_wait(empty + s, ph ^ 1u);
-            if (!ok) break;
+            if (!mbar_wait(empty + s, ph ^ 1u, p.polls))
+            {
+                gave_up = 1;
+                break;
+            }
             unsigned char* st = smem + s * STAGE;
             mbar_arrive_expect_tx(full + s, STAGE);
             const int kc = (kb0 + it) * BK;
@@ -209,18 +217,21 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel(
                 }
             }
         }
+        drain_loads<STAGES>(full, it);
     }
     else if (warp == 1 && lane == 0)
     {
         // bit 15: A is MN-major
         constexpr uint32_t idesc = instr_desc<KIND>(BM, BN) | (AMN ? (1u << 15) : 0u);
-        int it = 0;
-        for (; it < nkb && ok; it++)
+        for (int it = 0; it < nkb; it++)
         {
             const int s = it % STAGES;
             const uint32_t ph = (uint32_t)((it / STAGES) & 1);
-            ok = mbar_wait(full + s, ph);
-            if (!ok) break;
+            if (!mbar_wait(full + s, ph, p.polls))
+            {
+                gave_up = 1;
+                break;
+            }
             fence_after_sync();
             const uint32_t a0 = smem_u32(smem + s * STAGE);
             const uint32_t b0 = a0 + NOP * A_BYTES;
@@ -246,11 +257,12 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel(
         }
         // the accumulator is final once every MMA issued above completes
         mma_commit(accf);
-        if (!ok && p.err) atomicExch(p.err, MGX_TIMEOUT);
+        drain_mma(&mma_done);
     }
     else if (warp >= 2)
     {
-        const bool got = mbar_wait(accf, 0);
+        // (one decision for the warp, which reads TMEM together)
+        const bool got = __all_sync(0xffffffffu, mbar_wait(accf, 0, p.polls) && !gave_up);
         fence_after_sync();
         const int q   = warp & 3; // TMEM lane quarter this warp may access
         const int row = q * 32 + lane;
@@ -315,14 +327,15 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel(
                 }
             }
         }
-        else if (!got && p.err && lane == 0)
-            atomicExch(p.err, MGX_TIMEOUT);
+        else if (!got)
+            gave_up = 1;
         if (STORE && p.rho != nullptr && got && nkb > 0 && i < p.nrows)
             atomicAdd(p.rho + i, racc);
     }
     fence_before_sync();
-    __syncthreads();
+    __syncthreads(); // every role is done: gave_up is final
     fence_after_sync();
+    if (gave_up && threadIdx.x == 0 && p.err) atomicExch(p.err, MGX_TIMEOUT);
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
             "r"(TMEM_COLS)
@@ -348,7 +361,7 @@ inline int tile_cols(int ncols, int most)
  * on across items.  accf[b]: MMAs of accumulator b done (tcgen05.commit);
  * acce[b]: the four epilogue warps have read it.  Every wait is bounded; a
  * timeout records MGX_TIMEOUT and stops the other roles at their next
- * item. */
+ * item; the loads and MMAs in flight are waited for before the CTA ends. */
 template <int KIND, int NPROD, int BN, int STAGES, bool STORE = false, int SW = 128,
     bool AMN = false>
 __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
@@ -376,6 +389,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
     uint64_t* acce  = accf + 2;       // [2]
     uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + 2);
     __shared__ volatile int abort_all;
+    __shared__ uint64_t mma_done;
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int bn   = p.bn ? p.bn : BN;
@@ -411,6 +425,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
             mbar_init(accf + b, 1);
             mbar_init(acce + b, 4);
         }
+        mbar_init(&mma_done, 1);
         abort_all = 0;
         fence_mbar_init();
     }
@@ -445,7 +460,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
             {
                 const int s       = g % STAGES;
                 const uint32_t ph = (uint32_t)((g / STAGES) & 1);
-                if (!mbar_wait(empty + s, ph ^ 1u))
+                if (!mbar_wait(empty + s, ph ^ 1u, p.polls))
                 {
                     abort_all = 1;
                     break;
@@ -485,6 +500,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
                 }
             }
         }
+        drain_loads<STAGES>(full, g);
     }
     else if (warp == 1 && lane == 0)
     {
@@ -498,7 +514,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
             const int b       = t & 1;
             const uint32_t tb = tmem + (uint32_t)(b * BN);
             // the epilogue has drained this accumulator's previous item
-            if (!mbar_wait(acce + b, (uint32_t)(((t >> 1) & 1) ^ 1)))
+            if (!mbar_wait(acce + b, (uint32_t)(((t >> 1) & 1) ^ 1), p.polls))
             {
                 abort_all = 1;
                 break;
@@ -509,7 +525,7 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
             {
                 const int s       = g % STAGES;
                 const uint32_t ph = (uint32_t)((g / STAGES) & 1);
-                if (!mbar_wait(full + s, ph))
+                if (!mbar_wait(full + s, ph, p.polls))
                 {
                     ok = false;
                     break;
@@ -535,13 +551,11 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
                 }
                 mma_commit(empty + s);
             }
+            if (!ok) abort_all = 1; // before accf says that the accumulator is there
             mma_commit(accf + b);
-            if (!ok)
-            {
-                abort_all = 1;
-                break;
-            }
+            if (!ok) break;
         }
+        drain_mma(&mma_done);
     }
     else if (warp >= 2)
     {
@@ -553,7 +567,9 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
             int i0, j0, kb0, nkb;
             decode(w, i0, j0, kb0, nkb);
             const int b = t & 1;
-            const bool got = !abort_all && mbar_wait(accf + b, (uint32_t)((t >> 1) & 1));
+            // (one decision for the warp, which reads TMEM together)
+            const bool got = __all_sync(0xffffffffu,
+                !abort_all && mbar_wait(accf + b, (uint32_t)((t >> 1) & 1), p.polls) && !abort_all);
             if (!got)
             {
                 abort_all = 1;
@@ -625,10 +641,10 @@ __global__ void __launch_bounds__(THREADS, 1) gram_kernel_ps(
             if (lane == 0) mbar_arrive(acce + b);
         }
     }
-    if (abort_all && threadIdx.x == 0 && p.err) atomicExch(p.err, MGX_TIMEOUT);
     fence_before_sync();
-    __syncthreads();
+    __syncthreads(); // every role is done: abort_all is final
     fence_after_sync();
+    if (abort_all && threadIdx.x == 0 && p.err) atomicExch(p.err, MGX_TIMEOUT);
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
             "r"(TMEM_COLS)

@@ -89,3 +89,30 @@ def test_fused_gram_hmat_equals_separate(mode):
     assert rel_err(H.cpu().numpy(), H2.cpu().numpy()) < tol
     assert rel_err(H.cpu().numpy(), O.hmat(p, hp, ctx.vel)) < tol
     assert rel_err(S.cpu().numpy(), O.gram(p, ctx.vel)) < tol
+
+
+@pytest.mark.parametrize("polls", ["0", "1", "4", "30"])
+def test_waits_that_give_up(polls, monkeypatch):
+    """With waits of so few polls the product pipelines give up at once or on
+    the way: the call says so (or has the right result), and the context stays
+    usable."""
+    from mgmol_gb300 import capi
+    n = (32, 24, 20)
+    ctx = capi.Context(n, tuple(float(x) for x in n))
+    g = torch.Generator(device="cuda").manual_seed(7)
+    psi = torch.randn((200, ctx.npts), generator=g, device="cuda")
+    theta = torch.randn((200, 200), generator=g, dtype=torch.float64, device="cuda")
+    calls = (lambda: ctx.gram(psi, capi.GEMM_BF16X3), lambda: ctx.gram(psi, capi.GEMM_TF32),
+             lambda: ctx.mult_matrix(psi, theta, capi.GEMM_BF16X3))
+    ref = [f() for f in calls]
+    for f, want in zip(calls, ref):
+        monkeypatch.setenv("MGX_WAIT_POLLS", polls)
+        try:
+            got = f()
+        except capi.MgxError as e:
+            assert e.status == capi.MGX_TIMEOUT
+        else:
+            assert polls != "0"
+            assert float((got - want).abs().max()) <= 1e-6 * float(want.abs().max())
+        monkeypatch.delenv("MGX_WAIT_POLLS")
+        assert float((f() - want).abs().max()) <= 1e-6 * float(want.abs().max())
