@@ -301,7 +301,8 @@ int matb_cuda_cores(mgx_ctx* ctx, int dtype, const void* psi, size_t ld, size_t 
 // takes TS^2 k / 2 clocks of its SM, so the tile is the largest one that
 // still spreads over all SMs (64^3: 69 us on one SM, 5 us in 16 x 16 tiles).
 // lower_only: entries i + roff >= j; blockIdx.z: a batch of equal products at
-// strides sA, sB, sC; only_if as in gram_splitk_kernel.
+// strides sA, sB, sC; only_if as in gram_splitk_kernel, and where it says
+// sl::LOST the result is NaN.
 template <bool TA, bool TB, int TS>
 __global__ void __launch_bounds__(256) dgemm_kernel(int m, int n, int k,
     double alpha, const double* __restrict__ A, int lda,
@@ -311,7 +312,8 @@ __global__ void __launch_bounds__(256) dgemm_kernel(int m, int n, int k,
     constexpr int R = TS / 16;
     __shared__ double As[16][TS + 1];
     __shared__ double Bs[16][TS + 1];
-    if (only_if && *only_if == 0) return;
+    const int take = only_if ? *only_if : 1;
+    if (take == 0) return;
     A += blockIdx.z * sA;
     B += blockIdx.z * sB;
     C += blockIdx.z * sC;
@@ -368,7 +370,9 @@ __global__ void __launch_bounds__(256) dgemm_kernel(int m, int n, int k,
             if (i < m && j < n && (!lower_only || i + roff >= j))
             {
                 double* c = C + (size_t)j * ldc + i;
-                *c        = alpha * acc[p][q] + (beta == 0. ? 0. : beta * *c);
+                *c        = take == sl::LOST
+                                ? __longlong_as_double(0x7ff8000000000000ll)
+                                : alpha * acc[p][q] + (beta == 0. ? 0. : beta * *c);
             }
         }
 }
@@ -448,6 +452,7 @@ static int gemm(mgx_ctx* ctx, const Gemm& g, cudaStream_t s)
 /* ACC double: FP64 accumulation as the reference does for both orbital  */
 /* types; ACC float: theta rounded to FP32 and FP32 FMA.  Tiles of 128   */
 /* points x 64 functions, 8 x 4 results per thread.  cin may alias out.  */
+/* only_if as in dgemm_kernel.                                          */
 /* ------------------------------------------------------------------ */
 template <typename T, typename ACC>
 __global__ void __launch_bounds__(256) psi_theta_kernel(size_t npts, int n,
@@ -456,7 +461,8 @@ __global__ void __launch_bounds__(256) psi_theta_kernel(size_t npts, int n,
 {
     __shared__ ACC As[16][128];
     __shared__ ACC Bs[16][65];
-    if (only_if && *only_if == 0) return;
+    const int take = only_if ? *only_if : 1;
+    if (take == 0) return;
     const size_t p0 = (size_t)blockIdx.x * 128;
     const int j0 = blockIdx.y * 64;
     const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
@@ -515,6 +521,7 @@ __global__ void __launch_bounds__(256) psi_theta_kernel(size_t npts, int n,
             const size_t o = (size_t)j * ld + p;
             double r = (double)acc[u][v];
             if (beta != 0.) r += beta * (double)cin[o];
+            if (take == sl::LOST) r = __longlong_as_double(0x7ff8000000000000ll);
             out[o] = (T)r;
         }
     }

@@ -30,7 +30,8 @@
 // A NaN or an infinity in an operand has no digits: it raises a flag, on
 // which the kernels here do nothing and the caller's CUDA-core kernel,
 // launched behind them, does the work instead of returning at once.  A bounded
-// wait that gives up raises the same flag.
+// wait that gives up raises the same flag, or, when the product is added to its
+// own target and cannot be formed again, the flag that fills the target with NaN.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -673,11 +674,9 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
     if (abort_all && threadIdx.x == 0)
     {
         // a wait gave up: the CUDA-core kernels form the product instead, or, where
-        // C held an operand that is overwritten in part by now, C says so
-        if (p.t.sum == nullptr && p.t.cin != nullptr && p.t.cin == p.t.C)
-            p.t.C[p.m - 1] = __longlong_as_double(0x7ff8000000000000ll);
-        else
-            atomicExch(p.bad, 1);
+        // C held an operand that is overwritten in part by now, fill it with NaN
+        const bool lost = p.t.sum == nullptr && p.t.beta != 0. && p.t.cin == p.t.C;
+        atomicExch(p.bad, lost ? LOST : 1);
     }
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512)

@@ -52,7 +52,9 @@ int make_planes(const View& v, size_t k0, size_t kc, const int* keys, void* plan
     cudaStream_t s);
 /* the product of two sets of planes (NS_SUM with Target::sum, else NS_STORE) of
  * kc values of K; does nothing when *bad is set, and sets it when a bounded wait
- * gives up */
+ * gives up: to 1, or to LOST where Target::cin == C with beta != 0, an operand
+ * that is overwritten in part by then */
+constexpr int LOST = 2;
 int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const void* pb,
     const int* kb, size_t kc, const Target& t, int* bad, cudaStream_t s);
 
@@ -81,8 +83,8 @@ int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const 
 /* C = alpha A B^T + beta cin of FP64 operands of any layout, the rows of A
  * in chunks that bound the planes to PLANE_CAP bytes.  After each chunk
  * fallback(r0, rows, bad) enqueues the CUDA-core kernel of these rows, which
- * does nothing unless *bad is set.  MGX_NO_MEMORY: no workspace, nothing was
- * written. */
+ * does nothing unless *bad is set, and for LOST writes NaN.  MGX_NO_MEMORY: no
+ * workspace, nothing was written. */
 template <typename F>
 int store(mgx_ctx* ctx, const View& A, const View& B, const Target& t, cudaStream_t s, F fallback);
 

@@ -138,3 +138,39 @@ def test_waits_that_give_up(polls, monkeypatch):
     if polls == "0":  # FP64 sums in another order
         assert not torch.equal(H2, H) and not torch.equal(out2, out)
     assert torch.equal(ctx.hmat(psi, hp), H) and torch.equal(ctx.mult_matrix(psi, theta), out)
+
+
+@pytest.mark.parametrize("polls", ["0", "1", "3", "20"])
+def test_waits_that_give_up_in_place(polls, monkeypatch):
+    """A product that replaces its target is formed again by the CUDA cores when
+    a wait gives up; one that is added to its target cannot be, and then the
+    whole target is NaN: nothing finite is wrong."""
+    from mgmol_gb300 import capi
+    n = (32, 32, 20)
+    ctx = capi.Context(n, tuple(float(x) for x in n))
+    g = torch.Generator(device="cuda").manual_seed(31)
+    A = torch.randn((700, 700), generator=g, dtype=torch.float64, device="cuda")
+    S = A @ A.T / 700 + torch.eye(700, dtype=torch.float64, device="cuda")
+    L = torch.linalg.cholesky(S)
+    H = A + A.T
+    psi, hp = _block(150, ctx.npts, 32), _block(150, ctx.npts, 33)
+    cols = _block(150, 150, 34)
+    want = cols @ psi - hp
+    theta_ref = torch.cholesky_solve(H, L)
+    # in place: the substitutions, and columns of Psi Theta over the block they leave
+    monkeypatch.setenv("MGX_WAIT_POLLS", polls)
+    HB, Sinv = ctx.update_hb(S, H), ctx.inverse_from_cholesky(L)
+    theta, trace = ctx.theta_from_cholesky(L, H)
+    out = hp.clone()
+    ctx.residual_cols(psi, out, cols, apply_B=False, out=out)
+    torch.cuda.synchronize()
+    monkeypatch.delenv("MGX_WAIT_POLLS")
+    HB_ref = S @ H
+    assert float((HB - 0.5 * (HB_ref + HB_ref.T)).abs().max()) < 1e-11 * float(HB_ref.abs().max())
+    assert float((Sinv @ S - torch.eye(700, device="cuda")).abs().max()) < 1e-11
+    for got, ref in ((theta, theta_ref), (out, want)):
+        nan = torch.isnan(got)
+        assert bool((nan | ((got - ref).abs() < 1e-9)).all())
+        assert polls != "0" or bool(nan.all())
+    assert bool(torch.isnan(trace).any()) == bool(torch.isnan(theta.diagonal()).any())
+    assert float((ctx.update_hb(S, H) - HB).abs().max()) < 1e-11 * float(HB.abs().max())
