@@ -139,7 +139,6 @@ struct DevCoef
     // the doubles were redone at every use: FP64 units a quarter busy in FP32)
     T gam, alpha;
     int scaled;
-    int iso; // cy = cz and cxy = cxz
 };
 
 template <typename T>
@@ -160,7 +159,6 @@ DevCoef<T> to_dev(const StencilCoeffs& c, double jf, const PlaneParams& p = Plan
     d.gam    = (T)p.gamma_in;
     d.alpha  = (T)p.upd_alpha;
     d.scaled = p.gamma_in != 0.;
-    d.iso    = d.cy[0] == d.cz[0] && d.cxy == d.cxz;
     return d;
 }
 
@@ -699,12 +697,19 @@ __device__ __forceinline__ typename VH::type pack(const T (&a)[VH::N])
  * zr, rows y - 1 / y + 1 cmv / cpv and, for the Mehrstellen edges (EDGES),
  * their z neighbours ml, mr / pl, pr.  The y sum of each z column is formed
  * once and serves the column's own term and the edge terms of the columns
- * beside it.  FP64, bound by its operations (a warp instruction takes an SM's
- * FP64 units 16 clocks): a starts from before, the part b of the plane before,
- * which saves the addition of the two, and equal coefficients along y and z
- * share the sum of the y and z neighbours; 14 operations per Jacobi point
- * instead of 16.  Every stencil kernel that must give the same bits as another
- * forms a and b here. */
+ * beside it.  FP64: a comes with before, the part b of the plane before, added.
+ * The 2nd-order operator starts from it, which saves the addition (FP64 is bound
+ * by its operations: a warp instruction takes an SM's FP64 units 16 clocks).
+ * The Mehrstellen operator does not: its terms come by size, centre, faces,
+ * edges, the planes beside it last.  In the saving order, with one sum of the y
+ * and z neighbours for equal coefficients, a V-cycle of zero-mean residuals on
+ * 32^3 was off twice as far (8.5e-16 instead of 4.2e-16 in the L2 norm, the
+ * cycle restated with these sums against 80-bit arithmetic): a rounding that
+ * does not average out over neighbouring points is amplified by the cycle.  It
+ * would save 4 to 10 %: matrices of 256 orbitals on 96^3 23.1 -> 22.1 ms, the
+ * Poisson solve on 96^3 3.98 -> 3.74 ms.
+ * Every stencil kernel that must give the same bits as another forms a and b
+ * here. */
 template <typename T, typename VH, bool EDGES>
 __device__ __forceinline__ void vec_terms(const DevCoef<T>& c, const typename VH::type& c0v,
     const typename VH::type& cmv, const typename VH::type& cpv, T zl, T zr, T ml, T mr, T pl,
@@ -730,24 +735,14 @@ __device__ __forceinline__ void vec_terms(const DevCoef<T>& c, const typename VH
 #pragma unroll
         for (int v = 0; v < VEC; v++)
         {
-            // (with the centre last, matrices of 256 orbitals on 96^3 took 23.2 ms
-            // instead of 22.4: a longer chain after the last load)
-            T ss        = se[v + 1];
             const T szv = add_rn(v == 0 ? zl : u[v - 1], v == VEC - 1 ? zr : u[v + 1]);
-            T aa        = fma_rn(c.c0, u[v], before[v]);
+            T aa        = EDGES ? mul_rn(c.c0, u[v]) : fma_rn(c.c0, u[v], before[v]);
             T bb        = mul_rn(c.cx[0], u[v]);
-            if (EDGES && c.iso)
-                ss = add_rn(ss, szv);
-            else
-            {
-                aa = fma_rn(c.cz[0], szv, aa);
-                if (EDGES) bb = fma_rn(c.cxz, szv, bb);
-            }
-            aa = fma_rn(c.cy[0], ss, aa);
+            aa          = fma_rn(c.cy[0], se[v + 1], fma_rn(c.cz[0], szv, aa));
             if (EDGES)
             {
-                aa = fma_rn(c.cyz, add_rn(se[v], se[v + 2]), aa);
-                bb = fma_rn(c.cxy, ss, bb);
+                aa = add_rn(fma_rn(c.cyz, add_rn(se[v], se[v + 2]), aa), before[v]);
+                bb = fma_rn(c.cxy, se[v + 1], fma_rn(c.cxz, szv, bb));
             }
             a[v] = aa;
             b[v] = bb;

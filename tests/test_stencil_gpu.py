@@ -223,3 +223,57 @@ def test_chunks_of_a_full_launch(n, nf):
         for lap in (0, 1):
             assert torch.equal(ctx.fd_apply(a, lap)[some], ctx.fd_apply(b, lap))
             assert torch.equal(ctx.precond_mg(a, lap, 0, 0.2)[some], ctx.precond_mg(b, lap, 0, 0.2))
+
+
+def _l2(a, ref):
+    d = a.astype(np.longdouble) - ref
+    return float(np.sqrt((d * d).sum() / (ref * ref).sum()))
+
+
+def _residual_like(n, h, seed):
+    """A Gaussian with 5 % noise and no mean, as residuals of smooth orbitals have."""
+    rng = np.random.default_rng(seed)
+    x = [np.exp(-0.5 * ((np.arange(m) - m / 2.3) * h / 1.4) ** 2) for m in n]
+    u = x[0][:, None, None] * x[1][:, None] * x[2] * (1.0 + 0.05 * rng.standard_normal(n))
+    return u - u.mean()
+
+
+def _sum_axis(u, a, k=1):
+    return np.roll(u, -k, a) + np.roll(u, k, a)
+
+
+def _coefficients(ctx, n, lap, dt, offsets):
+    """The operator's coefficients as it has them: what it makes of a unit value."""
+    u = np.zeros((1, int(np.prod(n))), dt)
+    u[0, 0] = 1.0
+    r = ctx.fd_apply(_dev(u, dt), lap).cpu().numpy().reshape(n)
+    return [r[o] for o in offsets]
+
+
+def test_mehrstellen_fp64_error():
+    """The FP64 Mehrstellen operator is as close to extended precision as the
+    plain order of its sums, (centre, z, y, y-z edges), then the planes beside,
+    each product rounded with its sum (4 fields, 5 % for the field)."""
+    n, h = (32, 32, 32), 0.25
+    ctx = capi.Context(n, tuple(h * x for x in n))
+    L = np.longdouble
+    c0, fx, fy, fz, yz, xz, xy = _coefficients(ctx, n, 0, np.float64, [
+        (0, 0, 0), (1, 0, 0), (0, 1, 0), (0, 0, 1), (0, 1, 1), (1, 0, 1), (1, 1, 0)])
+
+    def neg_lap(u, fma):
+        s = [_sum_axis(u, a) for a in range(3)]
+        a = fma(yz, _sum_axis(s[1], 2), fma(fy, s[1], fma(fz, s[2], c0 * u)))
+        b = fma(xy, s[1], fma(xz, s[2], fx * u))
+        return a + np.roll(b, 1, 0) + np.roll(b, -1, 0)
+
+    def fma64(c, x, y):
+        return (L(c) * x.astype(L) + y.astype(L)).astype(np.float64)
+
+    err, plain = 0.0, 0.0
+    for seed in range(4):
+        u = _residual_like(n, h, seed)
+        ref = neg_lap(u.astype(L), lambda c, x, y: c * x + y)
+        got = ctx.fd_apply(_dev(u.reshape(1, -1), np.float64), 0).cpu().numpy().reshape(n)
+        err += _l2(got, ref)
+        plain += _l2(neg_lap(u, fma64), ref)
+    assert err < 1.05 * plain
