@@ -57,6 +57,10 @@ constexpr int DRAIN2  = 8;   // the same for the walk of s + t = 0 .. 3 alone
 constexpr int A_SLICE = BM * BK * 2;
 constexpr int EPI     = 16;  // epilogue warps: four per scheduler hide the TMEM reads
 constexpr int SUM_W   = 48;  // sums over items are kept in units of 2^-SUM_W
+// the most values of K of a sum and of a stored product: a digit product is at
+// most 2^14 and five of them share s + t = 4, so that the lower words of a sum
+// reach 5.1 K 2^30, and L of a stored product 5.1 K 2^38
+constexpr size_t MAX_K_SUM = size_t(1) << 30, MAX_K_STORE = size_t(1) << 22;
 constexpr int THREADS = 32 * (2 + EPI);
 
 /* the kernel's two forms: NP 1, all s + t in one walk over K, at most 64
@@ -267,7 +271,6 @@ struct Params
     int st_per_item; // stages of one item
     int nitems;
     int kblocks;     // 64-value blocks of K in each plane
-    int w;           // the sums are integers in units of 2^-w of a digit product
     size_t m, n;
     const int* ka;
     const int* kb;
@@ -535,8 +538,7 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
             const int ej
                 = lane < nc && j0 + lane < (long long)p.n ? key_exponent<NS>(p.kb[j0 + lane]) : 0;
             // s + t >= 4 in units of 2^-LOW of a digit product, in L (NP 1) or, until
-            // the second walk begins, in T; s + t <= 3 in units of 2^-24 (NP 1) or
-            // 2^-w, for which the sum is then rounded once
+            // the second walk begins, in T; s + t <= 3 in units of 2^-24
             constexpr int EL = Form<NP, NS>::W / 4, LOW = 8 * (NS - 1);
             long long T[EL], L[NP == 1 ? EL : 1];
 #pragma unroll
@@ -545,6 +547,11 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                 T[c] = 0;
                 if (NP == 1) L[NP == 1 ? c : 0] = 0;
             }
+            // entries of this thread: row i, columns j0 .. j0 + nc - 1 that exist
+            // (lower: from the diagonal down)
+            const int cols = i < p.m ? (int)min((long long)nc, (long long)p.n - j0) : 0;
+            const int last = p.t.lower ? (int)min((long long)cols, (long long)i + 1 - j0 - p.t.col0)
+                                       : cols;
             const int nd = (nst + DRAIN - 1) / DRAIN; // of the first walk
             const int na = NP == 1 ? nd : nd + (nst + DRAIN2 - 1) / DRAIN2;
             bool ok      = true;
@@ -558,9 +565,14 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                 const int ps = d < nd ? 0 : 1, lo = pass_lo(ps), hi = pass_hi(ps);
                 if (NP == 2 && d == nd)
                 {
+                    // s + t >= 4 goes to the lower words of the sum as it is
 #pragma unroll
                     for (int c = 0; c < EL; c++)
-                        T[c] = (T[c] + (1ll << (LOW - 1 - p.w))) >> (LOW - p.w);
+                    {
+                        if (c < last)
+                            atomicAdd(p.t.sum + (p.n + j0 + c) * p.m + i, (unsigned long long)T[c]);
+                        T[c] = 0;
+                    }
                 }
 #pragma unroll 1
                 for (int a = 0; a < NS; a++)
@@ -569,11 +581,9 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                     {
                         const int dg = lo + a;
                         // the accumulator holds integers times 2^(-8 dg): they
-                        // join the sum shifted left by sh bits
-                        const int sh   = (dg >= 4 ? LOW : NP == 1 ? 24 : p.w) - 8 * dg;
-                        const int e    = sh == 31 ? 1 : 0; // a factor of 2^31 is no int
-                        const float up = __uint_as_float((uint32_t)(127 + 8 * dg + e) << 23);
-                        const int mul  = 1 << ((sh - e) & 31);
+                        // join the sum shifted left by at most 24 bits
+                        const float up = __uint_as_float((uint32_t)(127 + 8 * dg) << 23);
+                        const int mul  = 1 << ((dg >= 4 ? LOW : 24) - 8 * dg);
 #pragma unroll
                         for (int c = 0; c < EL; c += 8)
                         {
@@ -581,26 +591,14 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                             float x[8];
                             tmem_ld8(tw + a * p.bn + c, x);
                             tmem_wait_ld(x);
-                            if (NP == 2 && sh >= 32)
-                            {
-                                // only the upper half changes
 #pragma unroll
-                                for (int i = 0; i < 8; i++)
-                                    T[c + i] += (long long)((unsigned long long)(unsigned)(
-                                                                __float2int_rn(x[i] * up) * mul)
-                                                            << 32);
-                            }
-                            else
+                            for (int i = 0; i < 8; i++)
                             {
-#pragma unroll
-                                for (int i = 0; i < 8; i++)
-                                {
-                                    const long long y = (long long)__float2int_rn(x[i] * up) * mul;
-                                    if (NP == 1 && dg >= 4)
-                                        L[NP == 1 ? c + i : 0] += y;
-                                    else
-                                        T[c + i] += y;
-                                }
+                                const long long y = (long long)__float2int_rn(x[i] * up) * mul;
+                                if (NP == 1 && dg >= 4)
+                                    L[NP == 1 ? c + i : 0] += y;
+                                else
+                                    T[c + i] += y;
                             }
                         }
                     }
@@ -614,16 +612,6 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                 abort_all = 1;
                 break;
             }
-            // the whole sum, in units of 2^-unit
-            const int unit = NP == 1 ? LOW : p.w;
-            auto whole     = [&](int c) -> __int128 {
-                return NP == 1 ? ((__int128)T[c] << (LOW - 24)) + L[NP == 1 ? c : 0] : (__int128)T[c];
-            };
-            // entries of this thread: row i, columns j0 .. j0 + nc - 1 that exist
-            // (lower: from the diagonal down)
-            const int cols = i < p.m ? (int)min((long long)nc, (long long)p.n - j0) : 0;
-            const int last = p.t.lower ? (int)min((long long)cols, (long long)i + 1 - j0 - p.t.col0)
-                                       : cols;
 #pragma unroll
             for (int c = 0; c < EL; c += 8)
             {
@@ -635,17 +623,20 @@ __global__ void __launch_bounds__(THREADS, 1) slice_product_kernel(
                     for (int x = 0; x < 8; x++)
                         if (c + x < last)
                         {
-                            const __int128 y      = whole(c + x) << (SUM_W - unit);
+                            const long long v     = T[c + x];
                             unsigned long long* o = p.t.sum + (j0 + c + x) * p.m + i;
-                            atomicAdd(o, (unsigned long long)(long long)(y >> 32));
-                            atomicAdd(o + p.n * p.m, (unsigned long long)(unsigned)y);
+                            atomicAdd(o, (unsigned long long)(v >> 8));
+                            atomicAdd(o + p.n * p.m,
+                                (unsigned long long)(((v & 255) << 24)
+                                                     + (NP == 1 ? L[NP == 1 ? c + x : 0] : 0)));
                         }
                     continue;
                 }
                 double v[8];
 #pragma unroll
                 for (int x = 0; x < 8; x++)
-                    v[x] = scaled(whole(c + x), ei - unit + __shfl_sync(0xffffffffu, ej, c + x));
+                    v[x] = scaled(((__int128)T[c + x] << (LOW - 24)) + L[NP == 1 ? c + x : 0],
+                        ei - LOW + __shfl_sync(0xffffffffu, ej, c + x));
                 if (p.t.beta != 0.)
                 {
                     double y[8];
@@ -695,8 +686,8 @@ __global__ void __launch_bounds__(256) add_sums_kernel(const unsigned long long*
     {
         const int i = (int)(t % m), j = (int)(t / m);
         if (lower && i < j + col0) continue;
-        const unsigned long long lo = sum[total + t];
-        const long long hi          = (long long)(sum[t] + (lo >> 32));
+        const long long lo = (long long)sum[total + t];
+        const long long hi = (long long)sum[t] + (lo >> 32);
         const double v = (double)hi * 4294967296. + (double)(unsigned)lo;
         C[j * ldc + i] += scalbn(v, key_exponent<7>(ka[i]) + key_exponent<7>(kb[j]) - 14 - SUM_W);
     }
@@ -797,7 +788,7 @@ int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const vo
     {
         // K split into items of whole drains: the split whose busiest SM has
         // the least to do (a drain's worth of work for the end of each item),
-        // of at most 2^17 values each, which bounds the integers below
+        // of at most 2^17 values each (T then reaches 2^55)
         const int nd = (p.nst + DRAIN - 1) / DRAIN;
         long best    = -1;
         for (int ks = 1; ks <= std::min(nd, std::max(1, 4 * sms / p.ntiles + 1)); ks++)
@@ -817,12 +808,6 @@ int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const vo
     const long items = (long)p.ntiles * ks;
     if (items > (1L << 30)) return fail(MGX_UNSUPPORTED, "too many work items");
     p.nitems = (int)items;
-    // |sum| <= 1.01 K 2^14 2^w < 2^63 (NP 2; in units of 2^-48, s + t >= 4 adds up
-    // to 5.1 K 2^30 before)
-    int lg = 0;
-    while ((1L << lg) < (long)p.st_per_item * BK) lg++;
-    if (lg > 17) return fail(MGX_UNSUPPORTED, "slices: K too large for one sum");
-    p.w = std::min(47, 48 - lg);
     p.ka  = ka;
     p.kb  = kb;
     p.t   = t;
@@ -870,6 +855,7 @@ int workspace(mgx_ctx* ctx, size_t na, size_t nb, size_t planes, int** ka, int**
 int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const Factor* f, int nf,
     int** bad, cudaStream_t s)
 {
+    if (K > MAX_K_SUM) return MGX_NO_MEMORY;
     // the planes of A and, in turn, those of each B that is not A; a sum and
     // the keys of each
     size_t brows = 0, bkeys = 0, sums = 0;
@@ -945,6 +931,7 @@ int store_begin(mgx_ctx* ctx, const View& A, const View& B, StorePlan* p, cudaSt
 {
     constexpr int ns = NS_STORE;
     const size_t K  = A.K;
+    if (K > MAX_K_STORE) return MGX_NO_MEMORY;
     const size_t b1 = up256(plane_bytes(B.rows, K, ns));
     const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(BM, K, ns));
     p->chunk = std::min((A.rows + BM - 1) / BM, fit) * BM;

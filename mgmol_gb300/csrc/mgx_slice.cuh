@@ -20,9 +20,8 @@ struct View
 
 /* What becomes of the product P = A B^T (m x n):
  *   sum given: P(i, j) is added to an integer in units of 2^-SUM_W of a digit
- *     product, its upper part in sum[j * m + i] and its lower 32 bits (with
- *     their carries) in sum[(n + j) * m + i]; K is split over CTAs that add
- *     atomically, and the order does not matter
+ *     product, sum[j * m + i] 2^32 + sum[(n + j) * m + i], both signed; K is
+ *     split over CTAs that add atomically, and the order does not matter
  *   else: C[j * ldc + i] = alpha P(i, j) + beta cin[j * ldcin + i]
  * lower: only entries i >= j + col0 (the others are left as they are). */
 struct Target
@@ -75,7 +74,7 @@ struct Factor
 /* The products of K-contiguous blocks of leading dimension ld (n rows of A),
  * in chunks of K that bound the planes to PLANE_CAP bytes; the planes of A
  * serve all of them.  *bad (device) tells whether an operand was not finite
- * and nothing was added.  MGX_NO_MEMORY: no workspace, nothing was added. */
+ * and nothing was added.  MGX_NO_MEMORY: no workspace, or K too large for the integers; nothing was added. */
 constexpr size_t PLANE_CAP = size_t(1) << 30;
 int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const Factor* f, int nf,
     int** bad, cudaStream_t s);

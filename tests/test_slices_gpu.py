@@ -174,3 +174,21 @@ def test_waits_that_give_up_in_place(polls, monkeypatch):
         assert polls != "0" or bool(nan.all())
     assert bool(torch.isnan(trace).any()) == bool(torch.isnan(theta.diagonal()).any())
     assert float((ctx.update_hb(S, H) - HB).abs().max()) < 1e-11 * float(HB.abs().max())
+
+
+def test_sums_keep_the_low_digits():
+    """Rows of one large value, in sums whose items are long: the low digits
+    reach the result whole.  Left out are at most six digit products of 2^-56,
+    2^-51.4 of x^2 for 1 <= x < 2, and 2^-56 2 of x in each operand; with the
+    rounding of the result below 2^-50."""
+    from mgmol_gb300 import capi
+    n = (64, 64, 64)
+    ctx = capi.Context(n, tuple(float(x) for x in n))
+    g = torch.Generator(device="cuda").manual_seed(41)
+    x = 1.0 + torch.rand(1024, generator=g, dtype=torch.float64, device="cuda")
+    psi = torch.zeros((1024, ctx.npts), dtype=torch.float64, device="cuda")
+    psi[torch.arange(1024, device="cuda"), 255 * torch.arange(1024, device="cuda")] = x
+    S = ctx.gram(psi)
+    d = S.diagonal()
+    assert float(((d - x * x) / (x * x)).abs().max()) < 2.0 ** -50
+    assert int(torch.count_nonzero(S)) == 1024
