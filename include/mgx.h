@@ -68,8 +68,24 @@ typedef enum mgx_lap_type
 /* Arithmetic of the Gram / H contractions. */
 typedef enum mgx_gemm_mode
 {
-    MGX_GEMM_FP64   = 0, /* FP64 data: exact BF16 slices on the tensor cores, or
-                            FP64 FMA (small products) (plain path) */
+    MGX_GEMM_FP64   = 0, /* FP64 data (plain path): BF16 slices of the operands
+                          * on the tensor cores, or FP64 FMA on the CUDA cores
+                          * (under 2^24 multiply-adds, operands with a NaN or
+                          * an infinity, mgx_set_fp64_slices off).
+                          * FP64 FMA: an entry is off by a few 2^-53 of
+                          * sum_k |a_ik b_jk|.  Slices: by 2^-54 sqrt(K)
+                          * max_k|a_ik| max_k|b_jk| (standard deviation;
+                          * never more than 2^-51 K instead of 2^-54 sqrt(K))
+                          * for the sums over grid points (S, H, B), where
+                          * every operand row is 56 bits from its largest
+                          * value down, and by 2^-60 sqrt(K) (2^-57 K) of the
+                          * same and 2^-53 of the entry for Psi Theta and the
+                          * products of N x N matrices (64 bits).  Against the
+                          * norms of the two rows that is no more than FP64
+                          * FMA for orbitals of some extent; an entry far
+                          * below them (functions that hardly overlap, rows
+                          * with single values far above the rest) loses
+                          * digits that FP64 FMA keeps. */
     MGX_GEMM_FP32   = 1, /* FP32 data, FP32 FMA on CUDA cores in 8-term
                           * chains, the chains summed in FP32 over 128
                           * terms and those sums in double-float (two FP32) */
@@ -403,6 +419,12 @@ int mgx_trace_prod(mgx_ctx* ctx, int n, const double* H, const double* Sinv,
  * not changed in between.  Off by default.  No counterpart in the
  * reference. */
 int mgx_set_reuse_conversion(mgx_ctx* ctx, int on);
+
+/* Whether the FP64 products of this context (MGX_GEMM_FP64 and the dense
+ * algebra) may be formed from BF16 slices, see MGX_GEMM_FP64 for what each
+ * form guarantees; off: all of them by FP64 FMA, 3 to 10 times slower.  On
+ * by default.  No counterpart in the reference. */
+int mgx_set_fp64_slices(mgx_ctx* ctx, int on);
 
 /* ---------------------------------------------------------------- */
 /* Residual and orbital update (rows of the ABPG step).              */

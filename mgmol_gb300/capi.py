@@ -141,6 +141,7 @@ _SIGS = {
     "mgx_cholesky": [_vp, _i, _vp, _ip, _vp],
     "mgx_cholesky_async": [_vp, _i, _vp, _vp, _vp],
     "mgx_set_reuse_conversion": [_vp, _i],
+    "mgx_set_fp64_slices": [_vp, _i],
     "mgx_timing_enable": [_i],
     "mgx_timing_read": [_i, _dp, _ip],
     "mgx_inverse_from_cholesky": [_vp, _i, _vp, _vp, _vp],
@@ -351,6 +352,14 @@ class Context:
         h = ctypes.c_void_p()
         _check(load().mgx_create(ctypes.byref(self.grid), ctypes.byref(h)))
         self.handle = h
+        self.fp64_slices = True
+
+    def set_fp64_slices(self, on):
+        """mgx_set_fp64_slices: whether FP64 products may be formed from BF16
+        slices (relative to the rows' maxima) or only by FP64 FMA (relative to
+        the sum of the absolute products)."""
+        _check(load().mgx_set_fp64_slices(self.handle, 1 if on else 0))
+        self.fp64_slices = bool(on)
 
     def set_reuse_conversion(self, on):
         """mgx_set_reuse_conversion: Psi Theta products may read the last

@@ -830,6 +830,13 @@ int mgx_set_reuse_conversion(mgx_ctx* ctx, int on)
     return MGX_OK;
 }
 
+int mgx_set_fp64_slices(mgx_ctx* ctx, int on)
+{
+    if (!ctx) return fail(MGX_BAD_ARG, "ctx is NULL");
+    ctx->fp64_slices = on ? 1 : 0;
+    return MGX_OK;
+}
+
 int mgx_cholesky_async(mgx_ctx* ctx, int n, double* A, int* info, void* stream)
 {
     if (!ctx) return fail(MGX_BAD_ARG, "ctx is NULL");

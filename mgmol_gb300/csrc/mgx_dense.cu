@@ -200,7 +200,7 @@ static int gram_add(mgx_ctx* ctx, int dtype, const void* A, size_t ld, size_t K,
     const sl::Factor* f, int nf, cudaStream_t s)
 {
     int* only_if = nullptr;
-    if (dtype == MGX_F64 && sl::pays(n, f[0].ncols, K))
+    if (dtype == MGX_F64 && sl::pays(ctx, n, f[0].ncols, K))
     {
         const int st = sl::accumulate(ctx, (const double*)A, ld, K, n, f, nf, &only_if, s);
         if (st == MGX_NO_MEMORY)
@@ -426,7 +426,7 @@ static int dgemm(const Gemm& g, int sms, cudaStream_t s, int roff = 0, const int
 static int gemm(mgx_ctx* ctx, const Gemm& g, cudaStream_t s)
 {
     if (g.m <= 0 || g.n <= 0) return MGX_OK;
-    if (g.batch == 1 && sl::pays(g.m, g.n, g.k))
+    if (g.batch == 1 && sl::pays(ctx, g.m, g.n, g.k))
     {
         const sl::View a = { g.A, (size_t)g.lda, (size_t)g.m, (size_t)g.k, g.ta };
         const sl::View b = { g.B, (size_t)g.ldb, (size_t)g.n, (size_t)g.k, !g.tb };
@@ -554,7 +554,7 @@ int psi_theta_cuda_cores(mgx_ctx* ctx, int kind, const void* psi, size_t ld, siz
         MGX_LAUNCH_CHECK("psi_theta_kernel");
         return MGX_OK;
     };
-    if (kind == 0 && sl::pays(npts, ncols, n))
+    if (kind == 0 && sl::pays(ctx, npts, ncols, n))
     {
         const sl::View a = { (const double*)psi, ld, npts, (size_t)n, false };
         const sl::View b = { theta, (size_t)ldt, (size_t)ncols, (size_t)n, true };

@@ -22,10 +22,16 @@
 //     2^-40 and 2^-48, the last bit could round if all digits were extreme.)
 //     The sums have to be exact and not only FP32: the tensor cores truncate
 //     when they add, which biases a sum of squares by 2^-24 per addition;
-//   - products of s + t > 6 (7), 2^-56 (2^-64) of |row maximum| |column maximum|
+//   - products of s + t > 6 (7), 2^-56 (2^-64) of |row scale| |column scale|
 //     and less, are left out.
-// 28 (36) bf16 products stand for one FP64 product, at 2^-56 (2^-64) of the row
-// maxima where FP64 multiply-adds round every partial sum at 2^-53.
+// 28 (36) bf16 products stand for one FP64 product.  An entry is off by about
+// 2^-54 sqrt(K) (2^-60 sqrt(K)) of row maximum x column maximum: the digits left
+// out are six (seven) products of 0.33 2^14 rms, and a row scale is up to twice (four
+// times) its maximum.  Against the norms of the rows that is what FP64
+// multiply-adds give or less, as long as a row's values of some size are not a
+// few of its K; against sum |a b|, which FP64 multiply-adds are relative to, it is not:
+// entries far below the norms lose digits, and for them the context can turn the
+// slices off.
 //
 // A NaN or an infinity in an operand has no digits: it raises a flag, on
 // which the kernels here do nothing and the caller's CUDA-core kernel,
@@ -828,9 +834,9 @@ int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const vo
     return MGX_OK;
 }
 
-bool pays(size_t m, size_t n, size_t K)
+bool pays(const mgx_ctx* ctx, size_t m, size_t n, size_t K)
 {
-    return (double)m * (double)n * (double)K >= 16. * 1024. * 1024.;
+    return ctx->fp64_slices && (double)m * (double)n * (double)K >= 16. * 1024. * 1024.;
 }
 
 namespace

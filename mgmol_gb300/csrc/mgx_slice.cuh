@@ -57,8 +57,9 @@ constexpr int LOST = 2;
 int product(int sms, size_t m, const void* pa, const int* ka, size_t n, const void* pb,
     const int* kb, size_t kc, const Target& t, int* bad, cudaStream_t s);
 
-/* whether a product of this size is formed from slices */
-bool pays(size_t m, size_t n, size_t K);
+/* whether a product of this size is formed from slices: from 2^24
+ * multiply-adds on, where the context allows it */
+bool pays(const mgx_ctx* ctx, size_t m, size_t n, size_t K);
 
 /* One product with a shared left operand: C(i, j) += sum_k A(i, k) B(j, k),
  * j < ncols, C of leading dimension n; with lower, entries i >= j + col0. */

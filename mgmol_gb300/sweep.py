@@ -146,6 +146,8 @@ class OrbitalSweep:
         self.side = torch.cuda.Stream(device=device, priority=-1) if self.use_matb else None
         self.side_after_theta = True
         self.sctx = capi.Context(ctx.n, ctx.ll) if self.use_matb else None
+        if self.sctx is not None:
+            self.sctx.set_fp64_slices(ctx.fp64_slices)
         self.info = torch.zeros(2, dtype=torch.int32, device=device)
         self.Sinv = None
         # psi does not change between the Gram products and Psi Theta: the

@@ -192,3 +192,55 @@ def test_sums_keep_the_low_digits():
     d = S.diagonal()
     assert float(((d - x * x) / (x * x)).abs().max()) < 2.0 ** -50
     assert int(torch.count_nonzero(S)) == 1024
+
+
+@pytest.mark.parametrize("peak", [1.0, 1e2, 1e4, 1e6])
+def test_error_contract(peak):
+    """Rows with one value far above the rest: from slices, an entry is off by
+    2^-54 sqrt(K) of the product of the row maxima (six standard deviations
+    here); with the slices off, by a few 2^-53 of the sum of the absolute
+    products (sums of 32 terms, those of up to 1024 parts added: 64)."""
+    from mgmol_gb300 import capi
+    n = (32, 32, 32)
+    ctx = capi.Context(n, tuple(float(x) for x in n))
+    g = torch.Generator(device="cuda").manual_seed(51)
+    a = torch.randn((70, ctx.npts), generator=g, dtype=torch.float64, device="cuda")
+    b = torch.randn((70, ctx.npts), generator=g, dtype=torch.float64, device="cuda")
+    at = torch.randint(0, ctx.npts, (2, 70), generator=g, device="cuda")
+    row = torch.arange(70, device="cuda")
+    a[row, at[0]], b[row, at[1]] = peak, peak
+    ref = _product(a, b)
+    norm = a.abs().amax(1)[:, None] * b.abs().amax(1)[None, :]
+    tail = 2.0 ** -52 * ref.abs() + 1e-14  # the result's own rounding, the filter
+    sliced = (ctx.hmat(a, b) - ref).abs()
+    assert bool((sliced <= 6 * 2.0 ** -54 * ctx.npts ** 0.5 * norm + tail).all())
+    ctx.set_fp64_slices(False)
+    units = (ctx.hmat(a, b) - ref).abs()
+    assert bool((units <= 64 * 2.0 ** -53 * (a.abs() @ b.abs().T) + tail).all())
+    if peak >= 1e4:  # what the slices cost such rows, and the FP64 units keep
+        assert float(units.max()) < 0.1 * float(sliced.max())
+
+
+def test_psi_theta_keeps_eight_digits():
+    """Psi Theta with rows of one dominant value, against extended precision:
+    2^-60 sqrt(K) of the product of the maxima (eight standard deviations) and
+    the result's rounding; seven digits would be off 2^-52 sqrt(K)."""
+    import numpy as np
+    from mgmol_gb300 import capi
+    n, nf = (17, 9, 11), 260
+    ctx = capi.Context(n, tuple(float(x) for x in n))
+    g = torch.Generator(device="cuda").manual_seed(52)
+    psi = torch.randn((nf, ctx.npts), generator=g, dtype=torch.float64, device="cuda") * 2.0 ** -20
+    theta = torch.randn((nf, nf), generator=g, dtype=torch.float64, device="cuda") * 2.0 ** -20
+    p, j = torch.arange(ctx.npts, device="cuda"), torch.arange(nf, device="cuda")
+    psi[p % nf, p] = 1.0 + psi[p % nf, p]
+    theta[(7 * j) % nf, j] = 1.0 + theta[(7 * j) % nf, j]
+    got = ctx.mult_matrix(psi, theta).cpu().numpy().astype(np.longdouble)
+    a, b = psi.cpu().numpy().astype(np.longdouble), theta.cpu().numpy().astype(np.longdouble)
+    rng = np.random.default_rng(52)
+    for jj in rng.integers(0, nf, 24):
+        pp = rng.integers(0, ctx.npts, 48)
+        ref = (b[:, jj][:, None] * a[:, pp]).sum(0)
+        size = np.abs(a[:, pp]).max(0) * np.abs(b[:, jj]).max()
+        bound = 8 * 2.0 ** -60 * nf ** 0.5 * size + 2.0 ** -52 * np.abs(ref)
+        assert np.all(np.abs(got[jj, pp] - ref) <= bound)
