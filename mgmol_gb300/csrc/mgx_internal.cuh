@@ -114,7 +114,8 @@ struct mgx_ctx
     int reuse_conversion = 0;
     // FP64 products from bf16 slices: row exponents and digit planes
     mgx::DeviceBuffer slices;
-    int fp64_slices = 1; // whether they may be formed so
+    int fp64_slices  = 1; // whether they may be formed so
+    size_t slice_cap = 0; // bytes of planes that there was memory for (0: not limited yet)
     // residual: Psi Theta when the caller passes no work block
     mgx::DeviceBuffer resid;
     // Poisson multigrid levels

@@ -43,6 +43,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <type_traits>
 #include <vector>
 
@@ -849,12 +850,37 @@ int workspace(mgx_ctx* ctx, size_t na, size_t nb, size_t planes, int** ka, int**
     char** pl)
 {
     const size_t head = up256((na + nb + 2) * sizeof(int));
+    if (const char* e = getenv("MGX_SLICE_ROOM")) // bytes, for tests: no memory for more
+        if (head + planes > (size_t)atoll(e)) return MGX_NO_MEMORY;
     if (ctx->slices.ensure(head + planes) != MGX_OK) return MGX_NO_MEMORY;
     *bad = (int*)ctx->slices.ptr;
     *ka  = *bad + 2;
     *kb  = *ka + na;
     *pl  = (char*)ctx->slices.ptr + head;
     return MGX_OK;
+}
+
+/* The bytes that planes may take at first: PLANE_CAP, MGX_SLICE_CAP for tests, or
+ * what a former call had memory for. */
+size_t plane_cap(const mgx_ctx* ctx)
+{
+    size_t cap = PLANE_CAP;
+    if (const char* e = getenv("MGX_SLICE_CAP"))
+        if (atoll(e) > 0) cap = (size_t)atoll(e);
+    return ctx->slice_cap ? std::min(cap, ctx->slice_cap) : cap;
+}
+
+/* take(cap) with half the planes each time that there is no memory for them,
+ * which the context keeps in mind: smaller chunks cost a few launches, the CUDA
+ * cores ten times the time */
+template <typename F> int with_room(mgx_ctx* ctx, F take)
+{
+    for (size_t cap = plane_cap(ctx);; cap /= 2)
+    {
+        const int st = take(cap);
+        if (st != MGX_NO_MEMORY || cap / 2 < PLANE_CAP_LEAST) return st;
+        ctx->slice_cap = cap / 2;
+    }
 }
 } // namespace
 
@@ -874,14 +900,17 @@ int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const 
         }
         sums += 2 * (size_t)n * f[i].ncols;
     }
-    const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(n + brows, 64, NS_SUM));
-    const size_t kc  = std::min((K + 63) / 64, fit) * 64;
-    const size_t pa_bytes = up256(plane_bytes(n, kc, NS_SUM)),
-                 pb_bytes = up256(plane_bytes(brows, kc, NS_SUM));
+    size_t kc, pa_bytes, pb_bytes;
     int *ka, *kb;
     char* pl;
-    MGX_TRY(workspace(ctx, n, bkeys, pa_bytes + pb_bytes + sums * sizeof(unsigned long long), &ka,
-        &kb, bad, &pl));
+    MGX_TRY(with_room(ctx, [&](size_t cap) {
+        const size_t fit = std::max<size_t>(1, cap / plane_bytes(n + brows, 64, NS_SUM));
+        kc       = std::min((K + 63) / 64, fit) * 64;
+        pa_bytes = up256(plane_bytes(n, kc, NS_SUM));
+        pb_bytes = up256(plane_bytes(brows, kc, NS_SUM));
+        return workspace(ctx, n, bkeys, pa_bytes + pb_bytes + sums * sizeof(unsigned long long),
+            &ka, &kb, bad, &pl);
+    }));
     char* pb  = pl + pa_bytes;
     auto* sum = (unsigned long long*)(pb + pb_bytes);
     MGX_TRY(cuda_check(cudaMemsetAsync(*bad, 0, sizeof(int), s), "slice flag"));
@@ -939,12 +968,14 @@ int store_begin(mgx_ctx* ctx, const View& A, const View& B, StorePlan* p, cudaSt
     const size_t K  = A.K;
     if (K > MAX_K_STORE) return MGX_NO_MEMORY;
     const size_t b1 = up256(plane_bytes(B.rows, K, ns));
-    const size_t fit = std::max<size_t>(1, PLANE_CAP / plane_bytes(BM, K, ns));
-    p->chunk = std::min((A.rows + BM - 1) / BM, fit) * BM;
-    const size_t rows = std::min(p->chunk, A.rows);
     char* pl;
-    MGX_TRY(workspace(ctx, rows, B.rows, b1 + plane_bytes(rows, K, ns), &p->ka, &p->kb, &p->bad,
-        &pl));
+    MGX_TRY(with_room(ctx, [&](size_t cap) {
+        const size_t fit = std::max<size_t>(1, cap / plane_bytes(BM, K, ns));
+        p->chunk = std::min((A.rows + BM - 1) / BM, fit) * BM;
+        const size_t rows = std::min(p->chunk, A.rows);
+        return workspace(ctx, rows, B.rows, b1 + plane_bytes(rows, K, ns), &p->ka, &p->kb, &p->bad,
+            &pl);
+    }));
     p->pb = pl;
     p->pa = pl + b1;
     MGX_TRY(cuda_check(cudaMemsetAsync(p->bad, 0, sizeof(int), s), "slice flag"));

@@ -73,15 +73,15 @@ struct Factor
 };
 
 /* The products of K-contiguous blocks of leading dimension ld (n rows of A),
- * in chunks of K that bound the planes to PLANE_CAP bytes; the planes of A
- * serve all of them.  *bad (device) tells whether an operand was not finite
+ * in chunks of K that bound the planes to PLANE_CAP bytes, or less where there
+ * is no memory for them; the planes of A serve all of them.  *bad (device) tells whether an operand was not finite
  * and nothing was added.  MGX_NO_MEMORY: no workspace, or K too large for the integers; nothing was added. */
-constexpr size_t PLANE_CAP = size_t(1) << 30;
+constexpr size_t PLANE_CAP = size_t(1) << 30, PLANE_CAP_LEAST = size_t(1) << 24;
 int accumulate(mgx_ctx* ctx, const double* A, size_t ld, size_t K, int n, const Factor* f, int nf,
     int** bad, cudaStream_t s);
 
 /* C = alpha A B^T + beta cin of FP64 operands of any layout, the rows of A
- * in chunks that bound the planes to PLANE_CAP bytes.  After each chunk
+ * in chunks that bound the planes as above.  After each chunk
  * fallback(r0, rows, bad) enqueues the CUDA-core kernel of these rows, which
  * does nothing unless *bad is set, and for LOST writes NaN.  MGX_NO_MEMORY: no
  * workspace, nothing was written. */

@@ -244,3 +244,66 @@ def test_psi_theta_keeps_eight_digits():
         size = np.abs(a[:, pp]).max(0) * np.abs(b[:, jj]).max()
         bound = 8 * 2.0 ** -60 * nf ** 0.5 * size + 2.0 ** -52 * np.abs(ref)
         assert np.all(np.abs(got[jj, pp] - ref) <= bound)
+
+
+def _products(ctx, psi, hp, theta, cols):
+    """The Gram-type products (B with a work block that cuts the functions),
+    Psi Theta and a residual over its own block, as one list."""
+    out = hp[3:3 + cols.shape[0]].clone()
+    ctx.residual_cols(psi, out, cols, apply_B=False, out=out)
+    work = torch.empty_like(psi)
+    return [*ctx.gram_hmat_matb(psi, hp, work=work),
+            ctx.matb(psi, work=work[:100]), ctx.mult_matrix(psi, theta), out]
+
+
+def _chunk_case(seed):
+    from mgmol_gb300 import capi
+    n, nf = (32, 20, 34), 150  # 170 column tiles of 128 points, the last one whole
+    ctx = capi.Context(n, tuple(float(x) for x in n))
+    psi, hp = _block(nf, ctx.npts, seed), _block(nf, ctx.npts, seed + 1)
+    theta = _block(nf, nf, seed + 2)
+    return ctx, psi, hp, theta, theta[:, 5:95].T.contiguous()
+
+
+@pytest.mark.parametrize("cap", [1, 3 << 20, 20 << 20])
+def test_chunks_of_planes(cap, monkeypatch):
+    """Planes in chunks of K (sums) and of rows (Psi Theta, the residual), down
+    to the smallest ones: the bits of one chunk; and a value that is not finite
+    in the last points makes the last chunk alone FP64 sums."""
+    ctx, psi, hp, theta, cols = _chunk_case(61)
+    want = _products(ctx, psi, hp, theta, cols)
+    monkeypatch.setenv("MGX_SLICE_CAP", str(cap))
+    for got, w in zip(_products(ctx, psi, hp, theta, cols), want):
+        assert torch.equal(got, w)
+    psi[17, -1] = float("nan")
+    hp2 = hp.clone()
+    S, H, B, B2, out, res = _products(ctx, psi, hp2, theta, cols)
+    monkeypatch.delenv("MGX_SLICE_CAP")
+    first = ctx.npts - 128  # rows of the chunks before the last at the smallest cap
+    if cap == 1:
+        assert torch.equal(out[:, :first], want[4][:, :first])
+        assert torch.equal(res[:, :first], want[5][:, :first])
+    assert float((out - want[4])[:, :-1].abs().max()) < 1e-11 * float(want[4].abs().max())
+    assert bool(torch.isnan(out[:, -1]).all()) and not bool(torch.isnan(out[:, :-1]).any())
+    assert bool(torch.isnan(res[:, -1]).all()) and not bool(torch.isnan(res[:, :-1]).any())
+    keep = [i for i in range(150) if i != 17]
+    assert float((H - want[1])[keep].abs().max()) < 1e-11 * float(want[1].abs().max())
+
+
+def test_no_memory_for_the_planes(monkeypatch):
+    """Without memory for all planes they come in smaller chunks, and without
+    memory for any the CUDA cores form the products; the context goes on."""
+    ctx, psi, hp, theta, cols = _chunk_case(71)
+    want = _products(ctx, psi, hp, theta, cols)
+    del ctx
+    ctx, *_ = _chunk_case(71)
+    monkeypatch.setenv("MGX_SLICE_ROOM", str(24 << 20))  # the first chunks want more
+    for got, w in zip(_products(ctx, psi, hp, theta, cols), want):
+        assert torch.equal(got, w)
+    monkeypatch.setenv("MGX_SLICE_ROOM", "0")
+    for got, w in zip(_products(ctx, psi, hp, theta, cols), want):
+        assert not torch.equal(got, w)
+        assert float((got - w).abs().max()) < 1e-12 * float(w.abs().max())
+    monkeypatch.delenv("MGX_SLICE_ROOM")
+    for got, w in zip(_products(ctx, psi, hp, theta, cols), want):
+        assert torch.equal(got, w)
