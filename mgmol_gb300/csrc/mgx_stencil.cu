@@ -1957,6 +1957,21 @@ constexpr int stages_for()
     return ((LAP == 0) || is_rhs_op(OP)) ? 4 : R + 4;
 }
 
+/* SMs of the current device (GB300: 152) */
+static int device_sms()
+{
+    thread_local int device = -1, sms = 152;
+    int d                   = -1;
+    if (cudaGetDevice(&d) == cudaSuccess && d != device)
+    {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d) == cudaSuccess && n > 0)
+            sms = n;
+        device = d;
+    }
+    return sms;
+}
+
 /* Tile rows and x chunk of a plane kernel that cannot fill the GPU with large
  * tiles (one field, few functions): the pair whose busiest SM has the least to
  * do.  A CTA works on (xc + halo) planes of ty rows; a point and plane costs its
@@ -1969,6 +1984,7 @@ static void few_tiles(int nx, int ny, int nz, int nfunc, int halo, int esz, bool
 {
     static const int cuts[] = { 1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 32, 48, 64 };
     const double point = esz == 8 ? 10. : 0.5;
+    const int sms      = device_sms();
     const int most     = *ty;
     double best        = -1.;
     auto up2 = [&](int v) { return even ? (v + 1) & ~1 : v; };
@@ -1980,7 +1996,7 @@ static void few_tiles(int nx, int ny, int nz, int nfunc, int halo, int esz, bool
         {
             const int x       = up2((nx + kx - 1) / kx);
             const long ctas   = (long)((ny + t - 1) / t) * ((nx + x - 1) / x) * nfunc;
-            const long per_sm = (ctas + 151) / 152;
+            const long per_sm = (ctas + sms - 1) / sms;
             const double cost = (x + halo) * (per_sm * (double)t * nz * point + 500. * ((per_sm + 1) / 2));
             if (best < 0. || cost < best)
             {
@@ -2004,13 +2020,14 @@ static void few_tiles(int nx, int ny, int nz, int nfunc, int halo, int esz, bool
  * one chunk and took 2 % longer. */
 static int x_chunk(int nx, size_t tiles, int halo)
 {
-    int best    = nx;
-    size_t cost = 0;
+    const int sms = device_sms();
+    int best      = nx;
+    size_t cost   = 0;
     for (int k = 1;; k++)
     {
         const int x = std::min(nx, ((nx + k - 1) / k + 1) & ~1);
         if (k > 1 && x < 16) break;
-        const size_t rounds = (tiles * ((nx + x - 1) / x) + 151) / 152;
+        const size_t rounds = (tiles * ((nx + x - 1) / x) + sms - 1) / sms;
         const size_t c      = rounds * (size_t)(x + halo);
         if (cost == 0 || c < cost)
         {
@@ -2073,7 +2090,7 @@ static int launch_vec(const PlaneParams& p0, const DevCoef<T>& c, int nfunc,
         if (smem_for(ty) <= smem_cap) break;
     if (ty < 1) return fail(MGX_UNSUPPORTED, "plane too large for the vector kernel");
     int xc = std::min(32, nx);
-    if ((size_t)((ny + ty - 1) / ty) * ((nx + xc - 1) / xc) * nfunc < 4 * 152)
+    if ((size_t)((ny + ty - 1) / ty) * ((nx + xc - 1) / xc) * nfunc < 4 * (size_t)device_sms())
         few_tiles(nx, ny, nz, nfunc, 2 + YO, (int)sizeof(T), RST, &ty, &xc);
     else
         xc = x_chunk(nx, (size_t)((ny + ty - 1) / ty) * nfunc, 2 + YO);
@@ -2130,7 +2147,7 @@ static int launch_axis(const PlaneParams& p0, const DevCoef<float>& c, int nfunc
     // x chunks: the march's 2R extra planes are read again by each, so no more
     // of them than give every SM several CTAs
     int cuts = 1;
-    while ((size_t)p.ntile_y * cuts * nfunc < 6 * 152 && (nx + cuts - 1) / cuts > 2 * R)
+    while ((size_t)p.ntile_y * cuts * nfunc < 6 * (size_t)device_sms() && (nx + cuts - 1) / cuts > 2 * R)
         cuts *= 2;
     p.xc      = (nx + cuts - 1) / cuts;
     p.ntile_x = (nx + p.xc - 1) / p.xc;
@@ -2198,7 +2215,7 @@ static int launch_t(const PlaneParams& p0, const DevCoef<T>& c, int nfunc,
         p.ntile_y = (ny + ty - 1) / ty;
         // x chunk: enough CTAs to fill the GPU, little halo re-read
         int xc = 32;
-        while (xc > 4 && (size_t)p.ntile_y * ((nx + xc - 1) / xc) * nfunc < 4 * 152)
+        while (xc > 4 && (size_t)p.ntile_y * ((nx + xc - 1) / xc) * nfunc < 4 * (size_t)device_sms())
             xc /= 2;
         if (xc > nx) xc = nx;
         p.xc       = xc;
@@ -2413,10 +2430,10 @@ static int launch_jj_nt(const PlaneParams& p0, const DevCoef<T>& c, int nfunc, c
     p.ty      = ty;
     p.ntile_y = ny / ty;
     int xc    = 32;
-    if ((size_t)p.ntile_y * ((nx + xc - 1) / xc) * nfunc >= 4 * 152)
+    if ((size_t)p.ntile_y * ((nx + xc - 1) / xc) * nfunc >= 4 * (size_t)device_sms())
         xc = x_chunk(nx, (size_t)p.ntile_y * nfunc, YO + 4);
     else
-        while (xc > 4 && (size_t)p.ntile_y * ((nx + xc - 1) / xc) * nfunc < 4 * 152)
+        while (xc > 4 && (size_t)p.ntile_y * ((nx + xc - 1) / xc) * nfunc < 4 * (size_t)device_sms())
             xc /= 2;
     if (xc > nx) xc = nx;
     p.xc      = xc;
