@@ -602,7 +602,10 @@ __device__ __forceinline__ double reciprocal(double d)
  * lower, column j takes G(i, j) = u_i / d_j times row j of [G^-1 | A] from
  * each row i > j, in one array whose columns before j already hold G^-1 and
  * the others what is left of A (in-place Gauss-Jordan).  L = G D^1/2 and W =
- * D^-1/2 G^-1 are scaled at the end, all columns at once.  Eight warps: two
+ * D^-1/2 G^-1 are scaled at the end, all columns at once.  1 / d_j itself stands
+ * in the array, so row and column i are taken times a power of two that brings
+ * the block's A(i, i) between 1 and 4 (the bits of L and W do not depend on it):
+ * pivots of any exponent, subnormal ones too, are factored.  Eight warps: two
  * column halves x four row groups, a lane per column, so that all four FP64
  * units work; the warp that updates the next pivot forms its reciprocal
  * before its other rows, so that the others need not wait for it.  Bound by
@@ -614,18 +617,32 @@ __global__ void __launch_bounds__(256) potrf_diag_kernel(double* A, int n, int k
     extern __shared__ double dsm[];
     double(*X)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(dsm);
     double(*U)[NB + 1] = reinterpret_cast<double(*)[NB + 1]>(dsm + NB * (NB + 1)); // u columns
-    __shared__ double inv[NB], sq[NB];
+    __shared__ double inv[NB], sq[NB], up[NB], down[NB]; // up: the powers of two of the rows
     __shared__ int bad;
     if (*info != 0) return;
     const int tid = threadIdx.x;
     for (int e = tid; e < NB * NB; e += blockDim.x)
     {
         const int i = e % NB, j = e / NB;
-        const double v = (i >= j && i < nb && j < nb) ? A[(size_t)(k0 + j) * n + k0 + i] : 0.;
+        X[i][j]     = (i >= j && i < nb && j < nb) ? A[(size_t)(k0 + j) * n + k0 + i] : 0.;
+    }
+    if (tid == 0) bad = 0;
+    __syncthreads();
+    if (tid < NB)
+    {
+        const double d = X[tid][tid];
+        const int k    = d > 0. && isfinite(d) ? ilogb(d) >> 1 : 0; // -537 .. 511
+        up[tid]        = scalbn(1., -k);
+        down[tid]      = scalbn(1., k);
+    }
+    __syncthreads();
+    for (int e = tid; e < NB * NB; e += blockDim.x)
+    {
+        const int i = e % NB, j = e / NB;
+        const double v = X[i][j] * up[i] * up[j];
         X[i][j]        = v;
         if (j == 0) U[i][0] = v;
     }
-    if (tid == 0) bad = 0;
     __syncthreads();
     // the pivot d of column j: its reciprocal, or -1 for a failure
     auto pivot = [&](int j, double d) {
@@ -705,8 +722,10 @@ __global__ void __launch_bounds__(256) potrf_diag_kernel(double* A, int n, int k
     for (int e = tid; e < nb * nb; e += blockDim.x)
     {
         const int i = e % nb, j = e / nb;
-        A[(size_t)(k0 + j) * n + k0 + i] = i > j ? U[i][j] * inv[j] : i == j ? sq[i] : 0.;
-        winv[(size_t)j * NB + i]         = i > j ? X[i][j] * inv[i] : i == j ? inv[i] : 0.;
+        A[(size_t)(k0 + j) * n + k0 + i]
+            = i > j ? U[i][j] * inv[j] * down[i] : i == j ? sq[i] * down[i] : 0.;
+        winv[(size_t)j * NB + i]
+            = i > j ? X[i][j] * inv[i] * up[j] : i == j ? inv[i] * up[j] : 0.;
     }
 }
 

@@ -138,3 +138,39 @@ def test_gram_hmat_match_reference_golden(case):
     H32 = ctx.hmat(p32, _dev(g[f"sh{case}_hpsi_f"], np.float32), mode=capi.GEMM_BF16X3).cpu().numpy()
     assert rel_err(S32, g[f"sh{case}_S_f"]) < 2e-5
     assert rel_err(H32, g[f"sh{case}_H_f"]) < 2e-5
+
+
+@pytest.mark.parametrize("n", [2, 64, 130])
+def test_cholesky_of_any_exponent(n):
+    """Pivots so small that 1 / d overflows; and rows and columns times powers
+    of two of 2^-500 to 2^500, which change no bit of the factor but its
+    exponents."""
+    ctx = capi.Context((8, 8, 8), (1, 1, 1))
+    S = np.ldexp(np.eye(n), -1039)
+    L = ctx.cholesky(_dev(S)).cpu().numpy()
+    assert np.array_equal(L, np.ldexp(np.sqrt(2.0) * np.eye(n), -520))
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n))
+    T = A @ A.T / n + np.eye(n)
+    k = rng.integers(-500, 501, n)
+    L = ctx.cholesky(_dev(T)).cpu().numpy()
+    Lk = ctx.cholesky(_dev(np.ldexp(T, k[:, None] + k[None, :]))).cpu().numpy()
+    assert np.array_equal(Lk, np.ldexp(L, np.broadcast_to(k[:, None], L.shape)))
+
+
+def test_pivot_reciprocals():
+    """The reciprocal of a pivot d against 1 / d: the second pivot of
+    [[d, d], [d, a]] is a - d (d r(d)), so that with a just above d its error
+    shows that of r: at most two roundings, of r and of d r, each 2^-53 (and
+    half a unit of the square root and of its square here)."""
+    ctx = capi.Context((8, 8, 8), (1, 1, 1))
+    rng = np.random.default_rng(9)
+    for e in (-1000, -500, -3, 0, 1, 7, 500, 1000):
+        d = np.ldexp(1.0 + rng.random(32), e)
+        d[:4] = np.ldexp([1.0, 2.0 - 2.0 ** -52, 1.0 + 2.0 ** -52, 1.5], e)
+        a = d * (1.0 + 2.0 ** -20)
+        S = np.zeros((64, 64))
+        i = 2 * np.arange(32)
+        S[i, i], S[i, i + 1], S[i + 1, i], S[i + 1, i + 1] = d, d, d, a
+        p = np.diagonal(ctx.cholesky(_dev(S)).cpu().numpy())[1::2] ** 2
+        assert np.all(np.abs(p - (a - d)) <= 2.0 ** -51 * d + 2.0 ** -51 * (a - d)), e
