@@ -174,3 +174,33 @@ def test_pivot_reciprocals():
         S[i, i], S[i, i + 1], S[i + 1, i], S[i + 1, i + 1] = d, d, d, a
         p = np.diagonal(ctx.cholesky(_dev(S)).cpu().numpy())[1::2] ** 2
         assert np.all(np.abs(p - (a - d)) <= 2.0 ** -51 * d + 2.0 ** -51 * (a - d)), e
+
+
+@pytest.mark.parametrize("n", [257, 700, 1000, 2047])
+def test_dense_algebra_of_ragged_blocks(n):
+    """Several blocks of 256, the last one ragged (down to one row), through the
+    slice products, uneven pairs of inverses among them: the factor, the
+    inverse, theta and HB against LAPACK's, and a pivot that fails in a late
+    block.  S has a condition number of about 5."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n))
+    S = A @ A.T / n + np.eye(n)
+    H = rng.standard_normal((n, n))
+    H = H + H.T
+    ctx = capi.Context((8, 8, 8), (1, 1, 1))
+    L = ctx.cholesky(_dev(S))
+    assert rel_err(L.cpu().numpy(), np.linalg.cholesky(S)) < 1e-12
+    Sinv = ctx.inverse_from_cholesky(L)
+    assert rel_err(Sinv.cpu().numpy(), np.linalg.inv(S)) < 1e-12
+    assert torch.equal(Sinv, Sinv.T)
+    want = np.linalg.solve(S, H)
+    theta, tr = ctx.theta_from_cholesky(L, _dev(H))
+    assert rel_err(theta.cpu().numpy(), want) < 1e-12
+    assert abs(float(tr) - np.trace(want)) < 1e-12 * n
+    assert rel_err(ctx.theta(Sinv, _dev(H)).cpu().numpy(), want) < 1e-12
+    HB = S @ H
+    assert rel_err(ctx.update_hb(_dev(S), _dev(H)).cpu().numpy(), 0.5 * (HB + HB.T)) < 1e-12
+    S[n - 1, n - 1] = -1.0
+    with pytest.raises(capi.MgxError) as e:
+        ctx.cholesky(_dev(S))
+    assert e.value.status == capi.MGX_NOT_SPD and f"minor {n} " in str(e.value)

@@ -159,3 +159,37 @@ def test_training_and_gain_in_the_block_iteration():
           "of", pc.functions)
     assert (its_plain <= 400).all()
     assert np.median(its_learned) <= np.median(its_plain)
+
+
+@pytest.mark.parametrize("n,nf", [((32, 16, 72), 20), ((32, 32, 64), 39)])
+def test_forms_of_large_blocks(n, nf):
+    """Enough blocks for 16 output channels and columns of 4 (last layer 8)
+    points per thread, with tiles of 32 and of 16 points along z, and the
+    halves of them on the lower levels."""
+    ll, x = _fields(n, nf, 21)
+    ctx = capi.Context(n, ll)
+    net = capi.UNet(ctx)
+    p = UO.init_params(9)
+    net.set_params(p)
+    assert rel_err(net.forward(_dev(x)).cpu().numpy(), UO.forward(n, p, x)) < TOL_FWD
+
+
+@pytest.mark.parametrize("n,nf", [((32, 16, 72), 6), ((12, 20, 40), 20)])
+def test_gradient_of_long_rows(n, nf):
+    """Weight gradients with tiles of 32 points along z (whole, cut, and on the
+    lower levels), and the data gradients' forms for many functions."""
+    ll, x = _fields(n, nf, 23)
+    _, t = _fields(n, nf, 24)
+    ctx = capi.Context(n, ll)
+    net = capi.UNet(ctx)
+    p = UO.init_params(10)
+    net.set_params(p)
+    loss, grad = net.loss_grad(_dev(x), _dev(t))
+    l_ref, g_ref = UO.loss_grad(n, p, x, t)
+    assert abs(float(loss) - l_ref) < 1e-5 * abs(l_ref)
+    g = grad.cpu().numpy()
+    o = 0
+    for ci, co, _ in UO.LAYERS:
+        k = ci * co * 27
+        assert rel_err(g[o:o + k], g_ref[o:o + k]) < TOL_GRAD, (ci, co)
+        o += k
