@@ -852,7 +852,7 @@ int workspace(mgx_ctx* ctx, size_t na, size_t nb, size_t planes, int** ka, int**
     const size_t head = up256((na + nb + 2) * sizeof(int));
     if (const char* e = getenv("MGX_SLICE_ROOM")) // bytes, for tests: no memory for more
         if (head + planes > (size_t)atoll(e)) return MGX_NO_MEMORY;
-    if (ctx->slices.ensure(head + planes) != MGX_OK) return MGX_NO_MEMORY;
+    MGX_TRY(ctx->slices.ensure(head + planes));
     *bad = (int*)ctx->slices.ptr;
     *ka  = *bad + 2;
     *kb  = *ka + na;
