@@ -11,10 +11,10 @@ conv_tol.  In Hartree sum_eig is tr(HB S^-1) (the trace in Ry, times the
 occupation 2, over 2), so the tolerances here are Hartree on that number.
 
 Two iterations start from the same seeded orbitals and potential:
-  plain  FP64 orbitals, stencils, products and V-cycle (152 s per sweep at
+  plain  FP64 orbitals, stencils, products and V-cycle (12.3 s per sweep at
          2048 orbitals on 192^3), stopped by the test on its own energies;
   mixed  FP32 orbitals and stencils with split-BF16x3 tensor-core products
-         (0.72 s per sweep there), stopped by the same test on energies
+         (0.6 s per sweep there), stopped by the same test on energies
          evaluated to FP64-class accuracy (energy_accurate): the sweep's
          own energy carries a bias and a sweep-to-sweep noise from its FP32
          stencils and FP32-accumulated products (about 1e-3 Ha and 3e-5 Ha

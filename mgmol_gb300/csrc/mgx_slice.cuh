@@ -1,4 +1,4 @@
-// FP64 products on the tensor cores by exact bf16 slices (mgx_slice.cu).
+// FP64 products on the tensor cores from bf16 slices (mgx_slice.cu).
 #pragma once
 
 #include "mgx_internal.cuh"
@@ -43,8 +43,8 @@ constexpr int NS_SUM = 7, NS_STORE = 8;
 /* bytes of the ns planes of `rows` rows of K values */
 size_t plane_bytes(size_t rows, size_t K, int ns);
 
-/* resets the keys of `rows` rows (and *bad when given) and takes the row
- * maxima of the view into them; *bad is set by a NaN or an infinity */
+/* resets the keys of the view's rows and takes the row maxima into them; *bad
+ * is set by a NaN or an infinity (and never reset here) */
 int row_keys(const View& v, int* keys, int* bad, cudaStream_t s);
 /* planes of columns [k0, k0 + kc) of the view */
 int make_planes(const View& v, size_t k0, size_t kc, const int* keys, void* planes, int ns,

@@ -2015,7 +2015,7 @@ static void few_tiles(int nx, int ny, int nz, int nfunc, int halo, int esz, bool
  * included (the kernels are bound by issue or FP64 units, so that CTAs which
  * share an SM take turns).  Chunks of 32 planes made the pre-sweep pair march 37
  * planes for 32; against them H psi with S, H and B of 512 FP32 orbitals on 128^3
- * took 9.79 instead of 9.95 ms, of 256 FP64 ones on 96^3 22.2 instead of 22.4.
+ * took 9.79 instead of 9.95 ms, and of 256 FP64 ones on 96^3 1 % less.
  * With the CTAs resident at a time in place of SMs, 64 FP64 fields of 64^3 got
  * one chunk and took 2 % longer. */
 static int x_chunk(int nx, size_t tiles, int halo)

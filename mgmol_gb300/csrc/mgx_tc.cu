@@ -1737,8 +1737,12 @@ int gram_hmat_tcgen05(mgx_ctx* ctx, int mode, const void* psi, const void* hpsi,
  * MPgemmNN product of LocGridOrbitals::multiplyByMatrix,
  * src/LocGridOrbitals.cc:793-830) on the tensor cores.  M = points,
  * N = functions, K = functions: the points are processed in chunks whose
- * transposed operand (rows = points, K = functions) fits a bounded
- * workspace; theta is converted once.  One CTA per 128 x BN output tile. */
+ * converted operand fits a bounded workspace; theta is converted once.  BF16
+ * planes are those of the Gram products (rows = functions, K = points), read
+ * MN-major: the last product's own where the caller allowed it, else made along
+ * the points chunk by chunk; FP16 and TF32 operands are transposed (rows =
+ * points, K = functions).  Persistent CTAs walk 128 x tile_cols output tiles
+ * (MGX_TC_PERSIST=0: one CTA per 128 x BN tile). */
 int psi_theta_tcgen05(mgx_ctx* ctx, int mode, const float* psi, size_t ld, size_t npts,
     int n, const double* theta, int ldt, int ncols, float beta, const float* cin, float* out,
     cudaStream_t s, double* rho)

@@ -1,7 +1,8 @@
 """FP64 products formed from exact bf16 slices on the tensor cores, against
-64-bit torch: the Gram-type products, Psi Theta and the residual's column
-chunks, at the edges of tiles (128 x at most 96), of the 256-value sums and of
-the plane chunks, and with operands that are not finite."""
+64-bit torch and extended precision: the Gram-type products, Psi Theta and the
+residual's column chunks, at the edges of tiles (128 x at most 128, or 64), of the
+sums of 192 and 256 values and of the plane chunks, with operands that are not
+finite, without memory, and after waits that give up."""
 import pytest
 import torch
 

@@ -189,8 +189,7 @@ def test_axis_kernel_tiles(n, lap):
 @pytest.mark.parametrize("h", [(0.3, 0.3, 0.3), (0.25, 0.3, 0.35), (0.3, 0.25, 0.25)])
 @pytest.mark.parametrize("n", [(32, 24, 16), (20, 18, 44)])
 def test_spacings(n, h):
-    """Equal and unequal spacings along y and z (the radius-1 FP64 kernels share
-    the sum of the y and z neighbours when the coefficients agree)."""
+    """Equal and unequal spacings along x, y and z."""
     ll = tuple(a * b for a, b in zip(n, h))
     ctx = capi.Context(n, ll)
     rng = np.random.default_rng(3)
