@@ -603,9 +603,10 @@ __device__ __forceinline__ double reciprocal(double d)
  * each row i > j, in one array whose columns before j already hold G^-1 and
  * the others what is left of A (in-place Gauss-Jordan).  L = G D^1/2 and W =
  * D^-1/2 G^-1 are scaled at the end, all columns at once.  1 / d_j itself stands
- * in the array, so row and column i are taken times a power of two that brings
- * the block's A(i, i) between 1 and 4 (the bits of L and W do not depend on it):
- * pivots of any exponent, subnormal ones too, are factored.  Eight warps: two
+ * in the array, so where the block's diagonal leaves 2^-500 .. 2^500, row and
+ * column i are taken times a power of two that brings A(i, i) between 1 and 4
+ * (the bits of L and W do not depend on it): pivots of any exponent, subnormal
+ * ones too, are factored.  (Done always, it took 2 of 73 us.)  Eight warps: two
  * column halves x four row groups, a lane per column, so that all four FP64
  * units work; the warp that updates the next pivot forms its reciprocal
  * before its other rows, so that the others need not wait for it.  Bound by
@@ -628,21 +629,22 @@ __global__ void __launch_bounds__(256) potrf_diag_kernel(double* A, int n, int k
     }
     if (tid == 0) bad = 0;
     __syncthreads();
-    if (tid < NB)
+    int k = 0; // the exponent of row tid over two, -537 .. 511
+    if (tid < nb && X[tid][tid] > 0. && isfinite(X[tid][tid])) k = ilogb(X[tid][tid]) >> 1;
+    const bool far = __syncthreads_or(k < -250 || k >= 250);
+    if (far)
     {
-        const double d = X[tid][tid];
-        const int k    = d > 0. && isfinite(d) ? ilogb(d) >> 1 : 0; // -537 .. 511
-        up[tid]        = scalbn(1., -k);
-        down[tid]      = scalbn(1., k);
+        if (tid < NB)
+        {
+            up[tid]   = scalbn(1., -k);
+            down[tid] = scalbn(1., k);
+        }
+        __syncthreads();
+        for (int e = tid; e < NB * NB; e += blockDim.x)
+            X[e % NB][e / NB] = X[e % NB][e / NB] * up[e % NB] * up[e / NB];
+        __syncthreads();
     }
-    __syncthreads();
-    for (int e = tid; e < NB * NB; e += blockDim.x)
-    {
-        const int i = e % NB, j = e / NB;
-        const double v = X[i][j] * up[i] * up[j];
-        X[i][j]        = v;
-        if (j == 0) U[i][0] = v;
-    }
+    if (tid < NB) U[tid][0] = X[tid][0];
     __syncthreads();
     // the pivot d of column j: its reciprocal, or -1 for a failure
     auto pivot = [&](int j, double d) {
@@ -722,10 +724,15 @@ __global__ void __launch_bounds__(256) potrf_diag_kernel(double* A, int n, int k
     for (int e = tid; e < nb * nb; e += blockDim.x)
     {
         const int i = e % nb, j = e / nb;
-        A[(size_t)(k0 + j) * n + k0 + i]
-            = i > j ? U[i][j] * inv[j] * down[i] : i == j ? sq[i] * down[i] : 0.;
-        winv[(size_t)j * NB + i]
-            = i > j ? X[i][j] * inv[i] * up[j] : i == j ? inv[i] * up[j] : 0.;
+        double l = i > j ? U[i][j] * inv[j] : i == j ? sq[i] : 0.;
+        double w = i > j ? X[i][j] * inv[i] : i == j ? inv[i] : 0.;
+        if (far)
+        {
+            l *= down[i];
+            w *= up[j];
+        }
+        A[(size_t)(k0 + j) * n + k0 + i] = l;
+        winv[(size_t)j * NB + i]         = w;
     }
 }
 
